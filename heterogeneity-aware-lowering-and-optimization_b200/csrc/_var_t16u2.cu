@@ -1,0 +1,365 @@
+// fp32 convolution (NHWC, one group) and batched GEMM on the CUDA cores, for graphs that run in the library's default
+// storage type.  The tensor cores have no fp32 operand type, so the bound is the FMA pipe: 128 fp32 FMA per clock and
+// SM, 74 TFLOP/s at 1965 MHz.
+//
+//   C[b][M, N] = A[b][M, K] * B[b][N, K]^T      convolution: M = N*P*Q pixels, K = R*S*C gathered on the fly
+//
+// One CTA of two warps owns a 64 x 64 tile, a thread 8 x 8 results.  Both operands sit in shared memory K-major (rows of 32
+// floats = 128 bytes), so that one 16-byte read brings four consecutive k of one row and the products go through the
+// packed fma.rn.f32x2: each accumulator is a pair (even k, odd k) that is added up at the end -- no register moves to
+// build operand pairs, 16 shared-memory reads per 128 packed FMAs.  Rows are swizzled like TMA's 128-byte mode (piece j of
+// row r at j ^ (r & 7)), which makes the eight rows a warp reads at a time land in different banks.  Operands arrive by
+// cp.async three stages deep: 16-byte pieces where four neighbouring k are contiguous and aligned, 4-byte elements otherwise
+// (a 3-channel image, an odd reduction length, a transposed operand); out-of-range pieces are zero-filled by the copy.
+//
+// Four CTAs share an SM (eight warps, 256 registers a thread).  When the tiles alone do not fill the chip the reduction is split
+// over the CTAs of a cluster: each leaves its partial tile in its own shared memory and then adds up and stores a share
+// of the rows, reading its peers' partials in rank order, so that the result does not depend on timing.
+#include <cstdio>
+#include <cstdlib>
+
+#include <algorithm>
+
+#include "epilogue.cuh"
+
+#ifndef F32_MAP
+#define F32_MAP 0
+#endif
+#ifndef F32_MINB
+#define F32_MINB 4
+#endif
+#ifndef F32_ORD
+#define F32_ORD 0
+#endif
+namespace b200 {
+namespace {
+
+#ifndef F32_TMR
+#define F32_TMR 8
+#endif
+#ifndef F32_ST
+#define F32_ST 3
+#endif
+constexpr int kTile = 64, kTileM = 8 * F32_TMR, kThreads = 64, kStages = F32_ST, kBK = 32;
+constexpr int kABytes = kTileM * kBK * 4, kStageBytes = kABytes + kTile * kBK * 4;
+constexpr int kOperandBytes = kTile * kBK * 4;                  // 8 KB per operand and stage
+constexpr int kPitch = kTile + 4;                               // floats per row of the result tile: rows land 4 banks apart
+constexpr int kSmem = kStages * kStageBytes + kTileM * 16;  // operand stages (the result tile reuses them) and the row table
+static_assert(kTileM * kPitch * 4 <= kStages * kStageBytes, "the result tile fits the operand stages");
+
+enum { LOAD_CONV_VEC, LOAD_CONV_SCALAR, LOAD_GEMM_VEC, LOAD_GEMM_SCALAR };
+
+struct F32Params {
+  int M, N, K, num_kb, m_tiles, n_tiles, splits;
+  int64_t a_row, a_col, a_batch, b_row, b_col, b_batch;
+  int H, W, C, R, S, P, Q, stride_h, stride_w, pad_t, pad_l;
+  const float *A, *B;
+  void* y;
+  Epilogue ep;
+};
+struct RowInfo { long long base; int h0, w0; };   // first input element of a pixel's window and where that window starts
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src, bool ok) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copy4(uint32_t dst, const void* src, bool ok) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(ok ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void lds_pair(uint32_t addr, unsigned long long& x, unsigned long long& y) {
+  asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "r"(addr));
+}
+__device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ uint32_t piece_at(uint32_t tile, int row, int piece) { return tile + (uint32_t)(row * 128 + ((piece ^ (row & 7)) << 4)); }
+
+// One stage of A: k-block kb of the tile's 64 rows.
+template <int LA>
+__device__ __forceinline__ void load_a(const F32Params& p, uint32_t dst, const float* A, const RowInfo* rows, int m0, int kb) {
+  const int t = threadIdx.x;
+  if (LA == LOAD_CONV_VEC) {
+    const int piece = t & 7, k = kb * kBK + piece * 4;
+    const int tap = k / p.C, c = k - tap * p.C, r = tap / p.S, s = tap - r * p.S;
+    const int64_t off = ((int64_t)r * p.W + s) * p.C + c;
+    const bool k_ok = k < p.K;
+#pragma unroll
+    for (int i = 0; i < kTileM / 8; ++i) {
+      const int row = (t >> 3) + 8 * i;
+      const RowInfo ri = rows[row];
+      const bool ok = k_ok && (unsigned)(ri.h0 + r) < (unsigned)p.H && (unsigned)(ri.w0 + s) < (unsigned)p.W;
+      copy16(piece_at(dst, row, piece), ok ? A + ri.base + off : A, ok);
+    }
+  } else if (LA == LOAD_CONV_SCALAR) {
+    const int kl = t & 31, k = kb * kBK + kl;
+    const int tap = k / p.C, c = k - tap * p.C, r = tap / p.S, s = tap - r * p.S;
+    const int64_t off = ((int64_t)r * p.W + s) * p.C + c;
+    const bool k_ok = k < p.K;
+#pragma unroll 8
+    for (int i = 0; i < kTileM / 2; ++i) {
+      const int row = (t >> 5) + 2 * i;
+      const RowInfo ri = rows[row];
+      const bool ok = k_ok && (unsigned)(ri.h0 + r) < (unsigned)p.H && (unsigned)(ri.w0 + s) < (unsigned)p.W;
+      copy4(piece_at(dst, row, kl >> 2) + (kl & 3) * 4, ok ? A + ri.base + off : A, ok);
+    }
+  } else if (LA == LOAD_GEMM_VEC) {
+    const int piece = t & 7, k = kb * kBK + piece * 4;
+#pragma unroll
+    for (int i = 0; i < kTileM / 8; ++i) {
+      const int row = (t >> 3) + 8 * i;
+      const bool ok = k < p.K && m0 + row < p.M;
+      copy16(piece_at(dst, row, piece), ok ? A + (int64_t)(m0 + row) * p.a_row + k : A, ok);
+    }
+  } else {
+    const bool along_k = p.a_col == 1;   // neighbouring lanes read neighbouring addresses whichever axis is contiguous
+#pragma unroll 8
+    for (int i = 0; i < kTileM / 2; ++i) {
+      const int row = along_k ? (t >> 5) + 2 * i : t + 64 * (i >> 5), kl = along_k ? t & 31 : i & 31, k = kb * kBK + kl;
+      const bool ok = k < p.K && m0 + row < p.M;
+      copy4(piece_at(dst, row, kl >> 2) + (kl & 3) * 4, ok ? A + (int64_t)(m0 + row) * p.a_row + (int64_t)k * p.a_col : A, ok);
+    }
+  }
+}
+template <bool VEC>
+__device__ __forceinline__ void load_b(const F32Params& p, uint32_t dst, const float* B, int n0, int kb) {
+  const int t = threadIdx.x;
+  if (VEC) {
+    const int piece = t & 7, k = kb * kBK + piece * 4;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int row = (t >> 3) + 8 * i;
+      const bool ok = k < p.K && n0 + row < p.N;
+      copy16(piece_at(dst, row, piece), ok ? B + (int64_t)(n0 + row) * p.b_col + k : B, ok);
+    }
+  } else {
+    const bool along_k = p.b_row == 1;
+#pragma unroll 8
+    for (int i = 0; i < 32; ++i) {
+      const int row = along_k ? (t >> 5) + 2 * i : t, kl = along_k ? t & 31 : i, k = kb * kBK + kl;
+      const bool ok = k < p.K && n0 + row < p.N;
+      copy4(piece_at(dst, row, kl >> 2) + (kl & 3) * 4, ok ? B + (int64_t)(n0 + row) * p.b_col + (int64_t)k * p.b_row : B, ok);
+    }
+  }
+}
+
+// Four neighbouring results of one row: the common forms on vectors, everything else through the scalar epilogue.
+__device__ __forceinline__ void finish4(const F32Params& p, float4 v, int64_t row, int col, bool plain) {
+  const Epilogue& ep = p.ep;
+  float t[4] = {v.x, v.y, v.z, v.w};
+  if (plain) {
+    if (ep.alpha != 1.f) { t[0] *= ep.alpha; t[1] *= ep.alpha; t[2] *= ep.alpha; t[3] *= ep.alpha; }
+    if (ep.add1) { const float4 a = __ldg((const float4*)(ep.add1 + col)); t[0] = __fadd_rn(t[0], a.x); t[1] = __fadd_rn(t[1], a.y); t[2] = __fadd_rn(t[2], a.z); t[3] = __fadd_rn(t[3], a.w); }
+    if (ep.add2) { const float4 a = __ldg((const float4*)(ep.add2 + col)); t[0] += a.x; t[1] += a.y; t[2] += a.z; t[3] += a.w; }
+    if (ep.act_first) apply_act_all<4>(ep.act, t, ep.act_a, ep.act_b);
+    if (ep.res) { const float4 a = *(const float4*)((const float*)ep.res + row * p.N + col); t[0] += a.x; t[1] += a.y; t[2] += a.z; t[3] += a.w; }
+    if (!ep.act_first) apply_act_all<4>(ep.act, t, ep.act_a, ep.act_b);
+    *(float4*)((float*)p.y + row * p.N + col) = make_float4(t[0], t[1], t[2], t[3]);
+  } else {
+    for (int j = 0; j < 4 && col + j < p.N; ++j) store_from_float(p.y, ep.out_dt, row * p.N + col + j, epilogue_value(ep, t[j], row, col + j, p.N));
+  }
+}
+
+template <int LA, bool BVEC>
+__global__ void __launch_bounds__(kThreads, F32_MINB) f32_tile_kernel(const F32Params p) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  RowInfo* rows = (RowInfo*)(smem + kStages * kStageBytes);
+  const int t = threadIdx.x, lane = t & 31, ty = F32_MAP ? (lane & 7) : (lane >> 2), tx = (F32_MAP ? (lane >> 3) : (lane & 3)) + 4 * (t >> 5);
+  const int per_batch = p.m_tiles * p.n_tiles, batch = (int)blockIdx.x / per_batch, tile = (int)blockIdx.x - batch * per_batch;
+  const int m0 = (tile % p.m_tiles) * kTileM, n0 = (tile / p.m_tiles) * kTile;
+  const int rank = (int)blockIdx.z;
+  const int kb_lo = (int)((int64_t)p.num_kb * rank / p.splits), kb_hi = (int)((int64_t)p.num_kb * (rank + 1) / p.splits);
+  const float *A = p.A + batch * p.a_batch, *B = p.B + batch * p.b_batch;
+  if (LA == LOAD_CONV_VEC || LA == LOAD_CONV_SCALAR) {
+    for (int rr = t; rr < kTileM; rr += kThreads) {
+    RowInfo ri;
+    const int m = m0 + rr, pq = p.P * p.Q;
+    const int img = m / pq, rem = m - img * pq, op = rem / p.Q, oq = rem - op * p.Q;
+    ri.h0 = m < p.M ? op * p.stride_h - p.pad_t : -(1 << 28);   // rows past the last pixel fail every bounds test
+    ri.w0 = oq * p.stride_w - p.pad_l;
+    ri.base = (((long long)img * p.H + ri.h0) * p.W + ri.w0) * p.C;
+    rows[rr] = ri;
+    }
+    __syncthreads();
+  }
+  const uint32_t sbase = smem_u32(smem);
+  asm volatile("griddepcontrol.wait;" ::: "memory");   // (a no-op unless launched as a programmatic dependent)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  float acc[F32_TMR][8];
+#pragma unroll
+  for (int i = 0; i < F32_TMR; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+  auto fetch = [&](int kb, int stage) {
+    if (kb < kb_hi) {
+      const uint32_t a = sbase + (uint32_t)stage * kStageBytes;
+      load_a<LA>(p, a, A, rows, m0, kb);
+      load_b<BVEC>(p, a + kABytes, B, n0, kb);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int s = 0; s < kStages - 1; ++s) fetch(kb_lo + s, s);
+  int stage = 0;
+  for (int kb = kb_lo; kb < kb_hi; ++kb) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+    __syncthreads();   // this stage has landed for every thread, and every thread is done with the stage refilled below
+    fetch(kb + kStages - 1, stage == 0 ? kStages - 1 : stage - 1);
+    const uint32_t a = sbase + (uint32_t)stage * kStageBytes + (uint32_t)(ty * 128 + (ty << 4));
+    const uint32_t b = sbase + (uint32_t)stage * kStageBytes + kABytes + (uint32_t)(tx * 128 + (tx << 4));
+#ifndef F32_UNR
+#define F32_UNR 1
+#endif
+#pragma unroll F32_UNR
+    for (int q = 0; q < 8; ++q) {
+      const uint32_t aq = a ^ (uint32_t)(q << 4), bq = b ^ (uint32_t)(q << 4);
+      float4 bv[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(bv[j].x), "=f"(bv[j].y), "=f"(bv[j].z), "=f"(bv[j].w) : "r"(bq + (uint32_t)(j * 1024)));
+#pragma unroll
+      for (int i = 0; i < F32_TMR; ++i) {
+        float4 av;
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(av.x), "=f"(av.y), "=f"(av.z), "=f"(av.w) : "r"(aq + (uint32_t)(i * 1024)));
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(av.x, bv[j].x, acc[i][j]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(av.y, bv[j].y, acc[i][j]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(av.z, bv[j].z, acc[i][j]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(av.w, bv[j].w, acc[i][j]);
+      }
+    }
+    if (++stage == kStages) stage = 0;
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  float* out = (float*)smem;
+#pragma unroll
+  for (int i = 0; i < F32_TMR; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) out[(ty + 8 * i) * kPitch + tx + 8 * j] = acc[i][j];
+  const Epilogue& ep = p.ep;
+  const bool plain = !ep.mul && !ep.add_full && (!ep.res || ep.res_dt == DT_F32) && ep.out_dt == DT_F32 && (p.N & 3) == 0;
+  const int r_lo = kTileM * rank / p.splits, r_hi = kTileM * (rank + 1) / p.splits;
+  if (p.splits > 1) {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+  } else __syncthreads();
+  for (int e = t; e < (r_hi - r_lo) * (kTile / 4); e += kThreads) {
+    const int r = r_lo + e / (kTile / 4), c = (e % (kTile / 4)) * 4;
+    if (m0 + r >= p.M || n0 + c >= p.N) continue;
+    const uint32_t at = sbase + (uint32_t)((r * kPitch + c) * 4);
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (p.splits == 1) v = *(const float4*)(out + r * kPitch + c);
+    else
+      for (int k = 0; k < p.splits; ++k) {
+        uint32_t peer;
+        float4 u;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(at), "r"(k));
+        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(u.x), "=f"(u.y), "=f"(u.z), "=f"(u.w) : "r"(peer) : "memory");
+        v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+      }
+    finish4(p, v, (int64_t)batch * p.M + m0 + r, n0 + c, plain);
+  }
+  if (p.splits > 1) {   // nobody leaves while a peer may still read its partial tile
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+  }
+}
+
+int device_sms() {
+  static int cache[16] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) return 148;
+  if (!cache[dev]) {
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+    cache[dev] = n;
+  }
+  return cache[dev];
+}
+// How many CTAs share one tile's reduction.  An SM works off its CTAs' k-blocks at full rate from two CTAs on (one CTA's
+// two warps reach two of the four schedulers), a CTA's fixed cost (filling the stages, the result tile, the cluster
+// barriers) is worth about six k-blocks, and a cluster has at most eight CTAs.
+int pick_splits(int64_t tiles, int num_kb) {
+  const int sms = device_sms();
+  int best = 1;
+  double best_cost = 0;
+  for (int n = 1; n <= 8 && n <= num_kb; ++n) {
+    const int64_t per_sm = (tiles * n + sms - 1) / sms;
+    const double cost = (double)std::max<int64_t>(per_sm, 2) * ((num_kb + n - 1) / n + (n > 1 ? 6.0 : 4.0));
+    if (n == 1 || cost < best_cost * 0.97) { best = n; best_cost = cost; }
+  }
+  return best;
+}
+template <int LA, bool BVEC>
+int launch(const F32Params& p, int64_t blocks, cudaStream_t s) {
+  static bool set[16] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 16 || !set[dev]) {
+    if (cudaFuncSetAttribute(f32_tile_kernel<LA, BVEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) { cudaGetLastError(); return -2; }
+    if (dev >= 0 && dev < 16) set[dev] = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)blocks, 1, (unsigned)p.splits);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = kSmem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  static const bool pdl = !getenv("ODLA_B200_NO_PDL");
+  int na = 0;
+  if (pdl) { attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[na].val.programmaticStreamSerializationAllowed = 1; ++na; }
+  if (p.splits > 1) {
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = 1; attr[na].val.clusterDim.y = 1; attr[na].val.clusterDim.z = (unsigned)p.splits;
+    ++na;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = na;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, f32_tile_kernel<LA, BVEC>, p);
+  if (e != cudaSuccess) { fprintf(stderr, "[odla_b200] fp32 tile kernel launch failed: %s\n", cudaGetErrorString(e)); cudaGetLastError(); return -2; }
+  return 0;
+}
+int run(F32Params p, int la, bool bvec, int64_t batch, cudaStream_t s) {
+  p.num_kb = (p.K + kBK - 1) / kBK;
+  p.m_tiles = (p.M + kTileM - 1) / kTileM;
+  p.n_tiles = (p.N + kTile - 1) / kTile;
+  const int64_t tiles = batch * p.m_tiles * p.n_tiles;
+  if (tiles <= 0) return 0;
+  if (tiles > 0x7fffffffLL) return -1;
+  p.splits = getenv("F32_SPLITS") ? std::min(atoi(getenv("F32_SPLITS")), p.num_kb) : pick_splits(tiles, p.num_kb);
+  if (la == LOAD_CONV_VEC) return launch<LOAD_CONV_VEC, true>(p, tiles, s);
+  if (la == LOAD_CONV_SCALAR) return launch<LOAD_CONV_SCALAR, true>(p, tiles, s);
+  if (la == LOAD_GEMM_VEC) return bvec ? launch<LOAD_GEMM_VEC, true>(p, tiles, s) : launch<LOAD_GEMM_VEC, false>(p, tiles, s);
+  return bvec ? launch<LOAD_GEMM_SCALAR, true>(p, tiles, s) : launch<LOAD_GEMM_SCALAR, false>(p, tiles, s);
+}
+}  // namespace
+
+bool conv_f32_supported(const ConvGeom& g) {
+  return g.groups == 1 && g.xs_c == 1 && (int64_t)g.N * g.P * g.Q < (1ll << 31) && (int64_t)g.R * g.S * g.C < (1ll << 30) && g.P > 0 && g.Q > 0;
+}
+int conv_f32(const ConvGeom& g, const void* x, const void* w, int64_t w_pitch, void* y, const Epilogue& ep, cudaStream_t s) {
+  F32Params p{};
+  p.M = g.N * g.P * g.Q; p.N = g.K; p.K = g.R * g.S * g.C;
+  p.H = g.H; p.W = g.W; p.C = g.C; p.R = g.R; p.S = g.S; p.P = g.P; p.Q = g.Q;
+  p.stride_h = g.stride_h; p.stride_w = g.stride_w; p.pad_t = g.pad_t; p.pad_l = g.pad_l;
+  p.A = (const float*)x; p.B = (const float*)w; p.y = y; p.ep = ep;
+  p.b_row = 1; p.b_col = w_pitch;
+  const bool vec = g.C % 4 == 0 && (uintptr_t)x % 16 == 0;
+  return run(p, vec ? LOAD_CONV_VEC : LOAD_CONV_SCALAR, true, 1, s);
+}
+bool gemm_f32_supported(const GemmGeom& g) { return g.M < (1ll << 31) && g.N < (1ll << 31) && g.K < (1ll << 30) && g.K > 0; }
+int gemm_f32(const GemmGeom& g, const void* A, const void* B, void* C, const Epilogue& ep, cudaStream_t s) {
+  F32Params p{};
+  p.M = (int)g.M; p.N = (int)g.N; p.K = (int)g.K;
+  p.a_row = g.a_row; p.a_col = g.a_col; p.a_batch = g.a_batch;
+  p.b_row = g.b_row; p.b_col = g.b_col; p.b_batch = g.b_batch;
+  p.A = (const float*)A; p.B = (const float*)B; p.y = C; p.ep = ep;
+  const bool avec = g.a_col == 1 && g.K % 4 == 0 && g.a_row % 4 == 0 && g.a_batch % 4 == 0 && (uintptr_t)A % 16 == 0;
+  // (pieces past K are zero on the A side, so a B row padded to a multiple of four floats may hold anything there)
+  const bool bvec = g.b_row == 1 && g.b_col % 4 == 0 && (g.K % 4 == 0 || g.b_batch == 0) && g.b_batch % 4 == 0 && (uintptr_t)B % 16 == 0;
+  return run(p, avec ? LOAD_GEMM_VEC : LOAD_GEMM_SCALAR, bvec, g.batch, s);
+}
+
+}  // namespace b200

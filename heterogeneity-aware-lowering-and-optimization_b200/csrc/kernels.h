@@ -79,6 +79,15 @@ struct GemmGeom {
 int gemm_simt(const GemmGeom& g, int in_dt, const void* A, const void* B, void* C, const Epilogue& ep,
               cudaStream_t stream);
 
+// ---- tiled fp32 path (kernels_f32.cu) ----
+// fp32 convolution over dense NHWC tensors, one group; w is [K][w_pitch] with each row the filter's R*S*C values in
+// (r, s, c) order and w_pitch a multiple of 4 (the padding holds zeros).
+bool conv_f32_supported(const ConvGeom& g);
+int conv_f32(const ConvGeom& g, const void* x, const void* w, int64_t w_pitch, void* y, const Epilogue& ep, cudaStream_t stream);
+// fp32 batched GEMM, any strides (a B with unit b_row and 16-byte rows loads widest).
+bool gemm_f32_supported(const GemmGeom& g);
+int gemm_f32(const GemmGeom& g, const void* A, const void* B, void* C, const Epilogue& ep, cudaStream_t stream);
+
 // ---- tensor-core path (kernels_umma.cu) ----
 // NHWC implicit-GEMM convolution: x [N,H,W,C], w repacked to [K][R*S*C] (K-major), y [N,P,Q,K].
 // A 1x1/stride-1 convolution with H=W=1 is a plain GEMM, which is how Gemm uses it.

@@ -123,6 +123,18 @@ std::vector<uint8_t> f32_to_storage(const std::vector<float>& f, int dt) {
   return out;
 }
 
+// fp32 [k][n] -> rows [n][pitch] with the reduction contiguous (zeros up to the pitch), in square blocks so that neither side
+// of the transposition strides through memory a line at a time.
+std::vector<uint8_t> f32_rows_kmajor(const std::vector<float>& w, int64_t k, int64_t n, int64_t pitch) {
+  std::vector<uint8_t> out((size_t)(n * pitch) * sizeof(float), 0);
+  float* o = (float*)out.data();
+  for (int64_t k0 = 0; k0 < k; k0 += 32)
+    for (int64_t n0 = 0; n0 < n; n0 += 32)
+      for (int64_t i = k0; i < std::min(k, k0 + 32); ++i)
+        for (int64_t j = n0; j < std::min(n, n0 + 32); ++j) o[j * pitch + i] = w[(size_t)(i * n + j)];
+  return out;
+}
+
 // A fused convolution / GEMM: root node plus the chain folded into its epilogue.
 struct Fused {
   V root = nullptr, out = nullptr;
@@ -929,6 +941,18 @@ odla_status Builder::emit_fused(const Item& it) {
       return ODLA_SUCCESS;
     }
     if (f.w_zp) return fail(ODLA_UNSUPPORTED_OP, "'" + root->name + "': asymmetric uint8 filters need the tensor-core path (NHWC, one group, 16-byte channel rows)");
+    if (in_dt == DT_F32 && nhwc) {
+      // fp32 storage: the tiled CUDA-core kernel, filters HWIO -> [K][R*S*C] with rows of whole 16-byte pieces
+      g.xs_c = 1; g.xs_w = g.C; g.xs_h = (int64_t)g.W * g.C; g.xs_n = (int64_t)g.H * g.W * g.C;
+      if (conv_f32_supported(g)) {
+        const int64_t kd = (int64_t)g.R * g.S * g.C, pitch = (kd + 3) / 4 * 4;
+        auto wb = prepared(f.w, "conv_f32_kmajor", [&] { return f32_rows_kmajor(const_as_f32(f.w), kd, K, pitch); });
+        const void* wk = upload(wb->data(), wb->size());
+        if (!wk) return err_status_;
+        add_launch("conv_simt", f.out, flops, bytes, [=](cudaStream_t s) { return conv_f32(g, x, wk, pitch, y, ep, s); });
+        return ODLA_SUCCESS;
+      }
+    }
     const void* wd = const_dev(f.w, in_dt);
     if (!wd) return err_status_;
     if (nhwc) {
@@ -1094,13 +1118,20 @@ odla_status Builder::emit_fused(const Item& it) {
   g.a_row = ta ? 1 : ac; g.a_col = ta ? ac : 1; g.a_batch = ar * ac;
   g.b_row = tb ? 1 : bc; g.b_col = tb ? bc : 1; g.b_batch = bbatch == 1 ? 0 : br * bc;
   const void* bp;
-  if (f.w->kind == OP_CONST) bp = const_dev(f.w, in_dt);
+  const bool f32_tiled = in_dt == DT_F32 && gemm_f32_supported(g);
+  if (f.w->kind == OP_CONST && f32_tiled && bbatch == 1 && !tb) {
+    // [K][N] weights as [N][K] rows of whole 16-byte pieces
+    const int64_t pitch = (Kd + 3) / 4 * 4;
+    auto wb = prepared(f.w, "gemm_f32_kmajor", [&] { return f32_rows_kmajor(const_as_f32(f.w), Kd, N, pitch); });
+    bp = upload(wb->data(), wb->size());
+    g.b_row = 1; g.b_col = pitch;
+  } else if (f.w->kind == OP_CONST) bp = const_dev(f.w, in_dt);
   else {
     if (dt_[resolve(f.w)] != in_dt) return fail(ODLA_UNSUPPORTED_DATATYPE, "'" + root->name + "': Gemm operand types differ");
     bp = dev_ptr(f.w);
   }
   if (!bp) return err_status_;
-  add_launch("gemm_simt", f.out, flops, bytes, with_move([=](cudaStream_t s) { return gemm_simt(g, in_dt, x, bp, y, ep, s); }));
+  add_launch("gemm_simt", f.out, flops, bytes, with_move([=](cudaStream_t s) { return f32_tiled ? gemm_f32(g, x, bp, y, ep, s) : gemm_simt(g, in_dt, x, bp, y, ep, s); }));
   if (perm_via_move) p_->launches.back().n_kernels = 2;
   return ODLA_SUCCESS;
 }

@@ -1,0 +1,54 @@
+"""The tiled fp32 kernel (kernels_f32.cu) against a float64 evaluation at the edges of its tiles, load widths and splits."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def close(got, want, k):
+    # a sum of k products in fp32: a few rounding steps of the result's magnitude
+    err = np.abs(got.astype(np.float64) - want).max() / np.sqrt(np.mean(want ** 2))
+    assert err < 4e-7 * np.sqrt(k) + 1e-6, err
+
+
+# N, H, W, C, K, R, stride, pad: 3 channels and odd channels (4-byte loads), ragged pixel and channel tiles, reductions that
+# leave a k-block nearly empty, few tiles over a long reduction (split over a cluster), one pixel
+@pytest.mark.parametrize("shape", [(2, 17, 19, 3, 64, 7, 2, 3), (1, 9, 11, 36, 65, 3, 1, 1), (1, 7, 7, 512, 72, 3, 1, 1), (3, 13, 13, 64, 255, 1, 1, 0),
+                                   (1, 8, 8, 64, 64, 1, 1, 0), (2, 8, 8, 5, 7, 2, 2, 0), (1, 1, 1, 4, 1, 1, 1, 0), (2, 28, 28, 128, 128, 3, 2, 1)])
+def test_conv_f32_matches_float64(odla, gpu_lib, shape):
+    N, H, W, C, K, R, stride, pad = shape
+    P, Q = (H + 2 * pad - R) // stride + 1, (W + 2 * pad - R) // stride + 1
+    rng = np.random.default_rng(sum(shape))
+    x = rng.standard_normal((N, H, W, C)).astype(np.float32)
+    w = (rng.standard_normal((R, R, C, K)) / np.sqrt(R * R * C)).astype(np.float32)
+    b, r = rng.standard_normal((1, 1, 1, K)).astype(np.float32), rng.standard_normal((N, P, Q, K)).astype(np.float32)
+    g = odla.Graph(gpu_lib, "c")
+    xa, ra = g.Argument("x", x.shape), g.Argument("r", r.shape)
+    y = g.Conv(xa, odla.CHANNELS_LAST, 1, g.Constant("w", w), odla.SIO, (stride, stride), (1, 1), (pad, pad), (pad, pad), None, (N, P, Q, K), "conv")
+    g.Output(g.LeakyRelu(g.Add(g.Add(y, g.Constant("b", b), "bn"), ra, "res"), 0.1, "y"))
+    got = g.run({"x": x, "r": r})["y"]
+    g.close()
+    t = torch.nn.functional.conv2d(torch.from_numpy(x).double().permute(0, 3, 1, 2), torch.from_numpy(w).double().permute(3, 2, 0, 1), stride=stride, padding=pad)
+    want = t.permute(0, 2, 3, 1).numpy() + b + r
+    close(got, np.where(want < 0, want * np.float64(np.float32(0.1)), want), R * R * C)
+
+
+# batch, M, N, K, transposed A, transposed B (None: constant weights)
+@pytest.mark.parametrize("dims", [(1, 64, 10, 784, 0, None), (1, 1, 1000, 2048, 0, None), (1, 65, 63, 33, 0, None), (1, 130, 70, 4, 1, None), (6, 77, 77, 64, 0, 1),
+                                  (6, 77, 64, 77, 0, 0), (4, 128, 64, 128, 0, 0), (1, 3, 5, 7, 0, 0)])
+def test_gemm_f32_matches_float64(odla, gpu_lib, dims):
+    batch, M, N, K, ta, tb = dims
+    rng = np.random.default_rng(sum(d or 0 for d in dims))
+    lead = (batch,) if batch > 1 else ()
+    a = rng.standard_normal(lead + ((K, M) if ta else (M, K))).astype(np.float32)
+    b = rng.standard_normal(lead + ((N, K) if tb else (K, N))).astype(np.float32)
+    c = rng.standard_normal(N).astype(np.float32)
+    g = odla.Graph(gpu_lib, "g", n_gpus=1)
+    ba = g.Constant("b", b) if tb is None else g.Argument("b", b.shape)
+    aa = g.Argument("a", a.shape)
+    g.Output(g.Gemm(aa, bool(ta), ba, bool(tb), 0.5, 2.0, g.Constant("c", c), lead + (M, N), "y"))
+    got = g.run({"a": a, "b": b} if tb is not None else {"a": a})["y"]
+    g.close()
+    af, bf = a.astype(np.float64), b.astype(np.float64)
+    close(got, 0.5 * ((af.swapaxes(-1, -2) if ta else af) @ (bf.swapaxes(-1, -2) if tb else bf)) + 2.0 * c, K)
