@@ -78,14 +78,14 @@ extern "C" int odla_b200_attention(int dtype, const void* q, const void* k, cons
     return -2;
   }
   const int dt = dtype == 0 ? DT_F16 : dtype == 1 ? DT_BF16 : -1;
-  if (dt < 0 || !attn_supported(dt, positions, channels)) return -1;
+  if (dt < 0 || positions != 128 || !attn_supported(dt, positions, channels)) return -1;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   int* status = nullptr;
   if (cudaMalloc((void**)&status, kStatusBytes) != cudaSuccess) return -2;
   cudaMemsetAsync(status, 0, kStatusBytes, (cudaStream_t)stream);
-  AttnLaunch* L = attn_prepare(dt, q, k, v, y, batch, heads, scale, merge_heads != 0, status, sms);
+  AttnLaunch* L = attn_prepare(AttnShape{dt, batch, heads, positions, 0, scale, merge_heads != 0}, q, k, v, y, status, sms);
   if (!L) { cudaFree(status); return -2; }
   int rc = attn_run(L, (cudaStream_t)stream);
   int host_status[2] = {0, 0};

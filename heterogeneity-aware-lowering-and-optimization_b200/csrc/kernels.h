@@ -128,13 +128,21 @@ UmmaLaunch* umma_conv_prepare(const UmmaConv& p, const void* x, const void* w, v
 int umma_conv_run(UmmaLaunch* l, cudaStream_t stream);
 void umma_conv_destroy(UmmaLaunch* l);
 
-// Fused attention for one shape family: softmax(scale * Q K^T) V over `batch * heads` heads of 128 positions x 64
-// channels, q / k / v laid out [batch][heads][128][64] in a two-byte type; the result is stored in the same layout or,
-// with merge_heads, as [batch][128][heads][64].  The scores stay in tensor memory.
+// Fused attention: softmax(scale * Q K^T) V over batch * heads heads of `positions` x 64 channels in a two-byte type.  q, k
+// and v lie [batch][heads][positions][64] (qkv_row_elems = 0) or as 64-column groups of rows of qkv_row_elems elements, one
+// row per (batch, position), which is how a projection leaves them; the result is stored [batch][heads][positions][64] or, with
+// merge_heads, [batch][positions][heads][64].  The scores stay in tensor memory.
+struct AttnShape {
+  int dt;
+  int64_t batch;
+  int heads;
+  int64_t positions, qkv_row_elems;
+  float scale;
+  bool merge_heads;
+};
 struct AttnLaunch;
 bool attn_supported(int dt, int64_t positions, int64_t channels);
-AttnLaunch* attn_prepare(int dt, const void* q, const void* k, const void* v, void* y, int64_t batch, int heads, float scale, bool merge_heads,
-                         int* status_word, int device_sms);
+AttnLaunch* attn_prepare(const AttnShape& a, const void* q, const void* k, const void* v, void* y, int* status_word, int device_sms);
 int attn_run(AttnLaunch* l, cudaStream_t stream);
 void attn_destroy(AttnLaunch* l);
 

@@ -1376,42 +1376,56 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 }
 
 // ------------------------------------------------------------ fused attention ----
-// softmax(scale * Q K^T) V for heads of 128 positions x 64 channels (two-byte types): one CTA works on one head at a
-// time and keeps the 128 x 128 scores in tensor memory -- they never reach global memory.  Roles: warp 0 brings Q, K, V
-// in with TMA and sends the result out, warp 1 issues the two products, warps 2-5 (one TMEM lane quarter each, a thread
-// per query row) do the soft-max between them and the final scaling.  Shared memory holds one head (no double buffer)
-// and is reused inside the head -- the probabilities overwrite Q and K, the result accumulates over the scores' tensor
-// memory columns, the result box overwrites V -- so that four CTAs share an SM and fill each other's gaps.  The probabilities go to the second product unnormalised
-// (exp(s - max), rounded to the two-byte type) and the row sums divide the result, as in any online soft-max.
+// softmax(scale * Q K^T) V for heads of 64 channels and any number of positions (two-byte types).  One CTA works on one
+// block of 128 query rows of one head at a time and keeps the scores of 128 x 128 (query, key) pairs in tensor memory -- they
+// never reach global memory.  Roles: warp 0 brings Q, K, V in with TMA and sends the result out, warp 1 issues the two
+// products, warps 2-5 (one TMEM lane quarter each, a thread per query row) do the soft-max between them and the final
+// scaling.  Shared memory holds one block (no double buffer) and is reused inside it -- the probabilities overwrite K
+// (and Q when it is not needed again), the result accumulates over the scores' tensor memory columns, the result box overwrites
+// V -- so that four (three) CTAs share an SM and fill each other's gaps.  The probabilities go to the second product
+// unnormalised (exp(s - max), rounded to the two-byte type) and the row sums divide the result, as in any online soft-max.
+//
+// MULTI = false: up to 128 positions, one key block.  MULTI = true: the key blocks of a row follow one another; each block's
+// product is read back and added to the row's 64 running results in registers, which are rescaled when the maximum moves.
+// A sequence that does not fill its last block needs no padding anywhere: TMA zero-fills loads and clips stores past the
+// last position, the products shrink to the next multiple of 16 keys and the soft-max masks the rest.
 struct AttnParams {
-  int tiles, NH, merge;          // heads in all; heads per batch element; 1: the result is stored [B][S][NH][D], 0: [B][NH][S][D]
+  int tiles, NH, S, q_tiles, k_blocks;   // query blocks in all; heads per batch element; positions; blocks per head
+  int qkv_rows;                  // 0: q, k, v lie [B][NH][S][D]; 1: heads are 64-column groups of [B * S] rows
+  int merge;                     // 1: the result is stored [B][S][NH][D], 0: [B][NH][S][D]
   float scale_log2e;             // scale * log2(e)
-  uint32_t idesc_s, idesc_o, desc_hi;
+  uint32_t idesc_s, idesc_s_last, idesc_o, desc_hi;   // (the last key block's scores product may be narrower)
+  int last_keys, last_ksteps;    // keys in the last block, and 16-key steps of its second product
   uint32_t spin_limit;
-  int bf16;
   int* status;
 };
 constexpr int kAttnS = 128, kAttnD = 64, kAttnThreads = 192;
 constexpr uint32_t kAttnBox = 16384;   // 128 rows x 128 bytes
 
-template <bool BF16>
-__global__ void __launch_bounds__(kAttnThreads, 4)
+__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z, int w) {
+  asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(smem_u32(dst)),
+               "l"((uint64_t)map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "r"(w)
+               : "memory");
+}
+
+template <bool BF16, bool MULTI>
+__global__ void __launch_bounds__(kAttnThreads, MULTI ? 3 : 4)
 attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
             const __grid_constant__ CUtensorMap tmY, const AttnParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sQ = smem;                 // [128 rows][64] K-major
   uint8_t* sK = sQ + kAttnBox;        // [128 keys][64] K-major
-  uint8_t* sV = sK + kAttnBox;        // [128 keys][64 channels]: the second product reads it MN-major
-  uint8_t* sP = sQ;                   // two k-blocks of [128 rows][64 keys], written once the first product has read Q and K
-  uint8_t* sY = sV;                   // result box, written once the second product has read V
+  uint8_t* sP = MULTI ? sK : sQ;      // two k-blocks of [128 rows][64 keys], written once the first product has read its operands
+  uint8_t* sV = sP + 2 * kAttnBox;    // [128 keys][64 channels]: the second product reads it MN-major
+  uint8_t* sY = sV;                   // result box, written once the last second product has read V
   uint64_t* bars = (uint64_t*)(sV + kAttnBox);
-  uint64_t *b_full = bars, *b_s = bars + 1, *b_p = bars + 2, *b_o = bars + 3, *b_e = bars + 4, *b_sf = bars + 5;
+  uint64_t *b_full = bars, *b_s = bars + 1, *b_p = bars + 2, *b_o = bars + 3, *b_e = bars + 4;
   uint32_t* tmem_slot = (uint32_t*)(bars + 8);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    mbar_init(b_full, 1); mbar_init(b_s, 1); mbar_init(b_p, 4); mbar_init(b_o, 1); mbar_init(b_e, 4); mbar_init(b_sf, 1);
+    mbar_init(b_full, 1); mbar_init(b_s, 1); mbar_init(b_p, 4); mbar_init(b_o, 1); mbar_init(b_e, 4);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -1427,32 +1441,41 @@ attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const uint32_t tmem_s = tmem_base, tmem_o = tmem_base;   // the result's 64 columns replace the first 64 of the scores
+  const int k_blocks = MULTI ? p.k_blocks : 1;
+  // `n` counts key blocks over all of this CTA's query blocks: its parity is the phase of every barrier
 
   if (warp == 0) {
     // ------------------------------------------------ loads and the result's store ----
     if (elect_one()) {
-      uint32_t it = 0;
-      for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x, ++it) {
-        // the previous head's products have finished reading Q, K, V and P
-        if (it > 0 && !mbar_wait(b_o, (it - 1) & 1, abort_flag, p.status, 11, p.spin_limit)) break;
-        mbar_expect_tx(b_full, 3u * kAttnBox);
-        tma_load_2d(sQ, &tmQ, b_full, 0, tile * kAttnS);
-        tma_load_2d(sK, &tmK, b_full, 0, tile * kAttnS);
-        tma_load_2d(sV, &tmV, b_full, 0, tile * kAttnS);
-        if (!mbar_wait(b_e, it & 1, abort_flag, p.status, 12, p.spin_limit)) break;
-        if (p.merge) {
-          const int b = tile / p.NH, h = tile - b * p.NH;
-          asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"((uint64_t)&tmY), "r"(smem_u32(sY)), "r"(0),
-                       "r"(h), "r"(0), "r"(b)
-                       : "memory");
-        } else {
-          asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"((uint64_t)&tmY), "r"(smem_u32(sY)), "r"(0),
-                       "r"(tile * kAttnS)
-                       : "memory");
+      uint32_t n = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x) {
+        const int head = MULTI ? tile / p.q_tiles : tile, q0 = MULTI ? (tile - head * p.q_tiles) * kAttnS : 0;
+        const int b = head / p.NH, h = head - b * p.NH;
+        auto load = [&](uint8_t* dst, const CUtensorMap* map, int s0) {
+          if (p.qkv_rows) tma_load_4d(dst, map, b_full, 0, h, s0, b); else tma_load_4d(dst, map, b_full, 0, s0, h, b);
+        };
+        for (int kb = 0; kb < k_blocks; ++kb, ++n) {
+          // the previous block's products have finished reading Q, K, V and P
+          if (n > 0 && !mbar_wait(b_o, (n - 1) & 1, abort_flag, p.status, 11, p.spin_limit)) { ok = false; break; }
+          mbar_expect_tx(b_full, (kb == 0 ? 3u : 2u) * kAttnBox);
+          if (kb == 0) load(sQ, &tmQ, q0);
+          load(sK, &tmK, kb * kAttnS);
+          load(sV, &tmV, kb * kAttnS);
         }
+        // (a wait may lag one phase behind, not two: with b_o of the last block complete, b_e of the one before it is as well)
+        if (!ok || (MULTI && !mbar_wait(b_o, (n - 1) & 1, abort_flag, p.status, 11, p.spin_limit))) break;
+        if (!mbar_wait(b_e, (n - 1) & 1, abort_flag, p.status, 12, p.spin_limit)) break;
+        if (p.merge)
+          asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"((uint64_t)&tmY), "r"(smem_u32(sY)), "r"(0),
+                       "r"(h), "r"(q0), "r"(b)
+                       : "memory");
+        else
+          asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"((uint64_t)&tmY), "r"(smem_u32(sY)), "r"(0),
+                       "r"(q0), "r"(h), "r"(b)
+                       : "memory");
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-        mbar_arrive(b_sf);
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the box is V again: the next loads are issued by this thread
       }
       asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
       // copies that were armed but never consumed (an aborted run) get a bounded chance to land
@@ -1466,20 +1489,26 @@ attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
       const uint64_t fixed = ((uint64_t)p.desc_hi << 32) | (1ull << 16);
       const uint64_t dq = fixed | (uint64_t)((smem_u32(sQ) & 0x3FFFF) >> 4), dk = fixed | (uint64_t)((smem_u32(sK) & 0x3FFFF) >> 4);
       const uint64_t dv = fixed | (uint64_t)((smem_u32(sV) & 0x3FFFF) >> 4), dp = fixed | (uint64_t)((smem_u32(sP) & 0x3FFFF) >> 4);
-      uint32_t it = 0;
-      for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x, ++it) {
-        if (!mbar_wait(b_full, it & 1, abort_flag, p.status, 13, p.spin_limit)) break;
-        tc_fence_after();
+      uint32_t n = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x)
+        for (int kb = 0; kb < k_blocks; ++kb, ++n) {
+          const bool last = kb + 1 == k_blocks;
+          if (!mbar_wait(b_full, n & 1, abort_flag, p.status, 13, p.spin_limit)) { ok = false; break; }
+          // the previous block's result has been read from the columns the scores go to
+          if (MULTI && n > 0 && !mbar_wait(b_e, (n - 1) & 1, abort_flag, p.status, 17, p.spin_limit)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t idesc_s = last ? p.idesc_s_last : p.idesc_s;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) umma_f16(tmem_s, dq + 2 * k, dk + 2 * k, p.idesc_s, k ? 1u : 0u);        // S = Q K^T, 64 deep
-        umma_commit(b_s);
-        if (!mbar_wait(b_p, it & 1, abort_flag, p.status, 14, p.spin_limit)) break;
-        tc_fence_after();
-#pragma unroll
-        for (int k = 0; k < 8; ++k)   // O = P V, 128 deep: P advances 32 bytes per step inside a k-block, V sixteen rows
-          umma_f16(tmem_o, dp + (uint64_t)((k >> 2) * (kAttnBox >> 4) + 2 * (k & 3)), dv + (uint64_t)(128 * k), p.idesc_o, k ? 1u : 0u);
-        umma_commit(b_o);
-      }
+          for (int k = 0; k < 4; ++k) umma_f16(tmem_s, dq + 2 * k, dk + 2 * k, idesc_s, k ? 1u : 0u);        // S = Q K^T, 64 deep
+          umma_commit(b_s);
+          if (!mbar_wait(b_p, n & 1, abort_flag, p.status, 14, p.spin_limit)) { ok = false; break; }
+          tc_fence_after();
+          const int ksteps = last ? p.last_ksteps : 8;
+          for (int k = 0; k < ksteps; ++k)   // O = P V: P advances 32 bytes per step inside a k-block, V sixteen rows
+            umma_f16(tmem_o, dp + (uint64_t)((k >> 2) * (kAttnBox >> 4) + 2 * (k & 3)), dv + (uint64_t)(128 * k), p.idesc_o, k ? 1u : 0u);
+          umma_commit(b_o);
+        }
     }
   } else {
     // ------------------------------------------------ soft-max and the final scaling ----
@@ -1487,76 +1516,115 @@ attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
     const uint32_t p_row = smem_u32(sP) + (uint32_t)row * 128u, y_row = smem_u32(sY) + (uint32_t)row * 128u;
     const int rx = row & 7;
-    uint32_t it = 0;
-    for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x, ++it) {
-      if (!mbar_wait(b_s, it & 1, abort_flag, p.status, 15, p.spin_limit)) break;
-      tc_fence_after();
-      float mx = -3.402823466e+38f;
-#pragma unroll 1
-      for (int c = 0; c < 8; ++c) {
-        uint32_t r[16];
-        tmem_ld16(tmem_s + lane_addr + (uint32_t)(c * 16), r);
-        tmem_ld_wait_regs<16>(r);
+    uint32_t n = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x) {
+      // a warp whose 32 rows all lie past the last position has nothing to compute: what it leaves in shared memory only
+      // reaches rows that the store clips
+      const bool live = (MULTI ? (tile % p.q_tiles) * kAttnS : 0) + quarter * 32 < p.S;
+      float run_max = -3.402823466e+38f, sum = 0.f;
+      float o[MULTI ? kAttnD : 1];
+      if (MULTI) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) mx = fmaxf(mx, __uint_as_float(r[j]) * p.scale_log2e);
+        for (int j = 0; j < (MULTI ? kAttnD : 1); ++j) o[j] = 0.f;
       }
-      float sum = 0.f;
+      for (int kb = 0; kb < k_blocks; ++kb, ++n) {
+        const bool last = kb + 1 == k_blocks;
+        const int keys = last ? p.last_keys : kAttnS, chunks = (keys + 15) >> 4;
+        if (!mbar_wait(b_s, n & 1, abort_flag, p.status, 15, p.spin_limit)) { ok = false; break; }
+        tc_fence_after();
+        float corr = 0.f;
+        if (live) {
+          float mx = run_max;
 #pragma unroll 1
-      for (int c = 0; c < 8; ++c) {
-        uint32_t r[16];
-        tmem_ld16(tmem_s + lane_addr + (uint32_t)(c * 16), r);
-        tmem_ld_wait_regs<16>(r);
-        float e[16];
+          for (int c = 0; c < chunks; ++c) {
+            uint32_t r[16];
+            tmem_ld16(tmem_s + lane_addr + (uint32_t)(c * 16), r);
+            tmem_ld_wait_regs<16>(r);
+            if (c * 16 + 16 <= keys) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          e[j] = fmaf(__uint_as_float(r[j]), p.scale_log2e, -mx);
-          asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(e[j]));
-          sum += e[j];
-        }
-        // keys c*16 .. c*16+15 are pieces (c & 3) * 2, +1 of this row in k-block c >> 2
+              for (int j = 0; j < 16; ++j) mx = fmaxf(mx, __uint_as_float(r[j]) * p.scale_log2e);
+            } else {
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          uint4 u;
-          uint32_t* w = (uint32_t*)&u;
-#pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            if (BF16) { __nv_bfloat162 h = __floats2bfloat162_rn(e[q * 8 + 2 * t], e[q * 8 + 2 * t + 1]); w[t] = *(uint32_t*)&h; }
-            else { __half2 h = __floats2half2_rn(e[q * 8 + 2 * t], e[q * 8 + 2 * t + 1]); w[t] = *(uint32_t*)&h; }
+              for (int j = 0; j < 16; ++j) if (c * 16 + j < keys) mx = fmaxf(mx, __uint_as_float(r[j]) * p.scale_log2e);
+            }
           }
-          sts128(p_row + (uint32_t)(c >> 2) * kAttnBox + (uint32_t)(((((c & 3) << 1) + q) ^ rx) << 4), u);
-        }
-      }
-      tc_fence_before();
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the tensor cores read P through the async proxy
-      __syncwarp();
-      if (lane == 0) mbar_arrive(b_p);
-      const float inv = __fdividef(1.0f, sum);
-      if (!mbar_wait(b_o, it & 1, abort_flag, p.status, 16, p.spin_limit)) break;
-      tc_fence_after();
-      // the store of the previous head has finished reading the result box
-      if (it > 0 && !mbar_wait(b_sf, (it - 1) & 1, abort_flag, p.status, 17, p.spin_limit)) break;
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        uint32_t r[16];
-        tmem_ld16(tmem_o + lane_addr + (uint32_t)(c * 16), r);
-        tmem_ld_wait_regs<16>(r);
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          uint4 u;
-          uint32_t* w = (uint32_t*)&u;
-#pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            const float a = __uint_as_float(r[q * 8 + 2 * t]) * inv, b = __uint_as_float(r[q * 8 + 2 * t + 1]) * inv;
-            if (BF16) { __nv_bfloat162 h = __floats2bfloat162_rn(a, b); w[t] = *(uint32_t*)&h; }
-            else { __half2 h = __floats2half2_rn(a, b); w[t] = *(uint32_t*)&h; }
+          if (MULTI) {
+            corr = run_max - mx;   // 1 when the maximum has not moved, 0 for the first block
+            asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(corr));
+            sum *= corr;
+            run_max = mx;
           }
-          sts128(y_row + (uint32_t)((((c << 1) + q) ^ rx) << 4), u);
+#pragma unroll 1
+          for (int c = 0; c < chunks; ++c) {
+            uint32_t r[16];
+            tmem_ld16(tmem_s + lane_addr + (uint32_t)(c * 16), r);
+            tmem_ld_wait_regs<16>(r);
+            float e[16];
+            const bool whole = c * 16 + 16 <= keys;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              e[j] = fmaf(__uint_as_float(r[j]), p.scale_log2e, -mx);
+              asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(e[j]));
+              if (!whole && c * 16 + j >= keys) e[j] = 0.f;
+              sum += e[j];
+            }
+            // keys c*16 .. c*16+15 are pieces (c & 3) * 2, +1 of this row in k-block c >> 2
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              uint4 u;
+              uint32_t* w = (uint32_t*)&u;
+#pragma unroll
+              for (int t = 0; t < 4; ++t) {
+                if (BF16) { __nv_bfloat162 h = __floats2bfloat162_rn(e[q * 8 + 2 * t], e[q * 8 + 2 * t + 1]); w[t] = *(uint32_t*)&h; }
+                else { __half2 h = __floats2half2_rn(e[q * 8 + 2 * t], e[q * 8 + 2 * t + 1]); w[t] = *(uint32_t*)&h; }
+              }
+              sts128(p_row + (uint32_t)(c >> 2) * kAttnBox + (uint32_t)(((((c & 3) << 1) + q) ^ rx) << 4), u);
+            }
+          }
         }
+        tc_fence_before();
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the tensor cores read P through the async proxy
+        __syncwarp();
+        if (lane == 0) mbar_arrive(b_p);
+        const float inv = last ? __fdividef(1.0f, sum) : 1.f;
+        if (!mbar_wait(b_o, n & 1, abort_flag, p.status, 16, p.spin_limit)) { ok = false; break; }
+        tc_fence_after();
+        if (live) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            uint32_t r[16];
+            tmem_ld16(tmem_o + lane_addr + (uint32_t)(c * 16), r);
+            tmem_ld_wait_regs<16>(r);
+            if (MULTI) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                float& acc = o[MULTI ? c * 16 + j : 0];
+                acc = fmaf(acc, corr, __uint_as_float(r[j]));
+                r[j] = __float_as_uint(acc);
+              }
+            }
+            if (!MULTI || last) {
+#pragma unroll
+              for (int q = 0; q < 2; ++q) {
+                uint4 u;
+                uint32_t* w = (uint32_t*)&u;
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                  const float a = __uint_as_float(r[q * 8 + 2 * t]) * inv, b = __uint_as_float(r[q * 8 + 2 * t + 1]) * inv;
+                  if (BF16) { __nv_bfloat162 h = __floats2bfloat162_rn(a, b); w[t] = *(uint32_t*)&h; }
+                  else { __half2 h = __floats2half2_rn(a, b); w[t] = *(uint32_t*)&h; }
+                }
+                sts128(y_row + (uint32_t)((((c << 1) + q) ^ rx) << 4), u);
+              }
+            }
+          }
+        }
+        tc_fence_before();
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(b_e);
       }
-      tc_fence_before();
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(b_e);
     }
   }
   tc_fence_before();
@@ -1923,56 +1991,49 @@ struct AttnLaunch {
   AttnParams p;
   int grid;
   size_t smem;
-  bool bf16;
+  bool bf16, multi;
 };
-bool attn_supported(int dt, int64_t S, int64_t D) { return (dt == DT_F16 || dt == DT_BF16) && S == kAttnS && D == kAttnD; }
-AttnLaunch* attn_prepare(int dt, const void* q, const void* k, const void* v, void* y, int64_t batch, int heads, float scale, bool merge_heads, int* status,
-                         int sms) {
-  if (!attn_supported(dt, kAttnS, kAttnD) || batch * heads <= 0 || batch * heads * kAttnS >= (1ll << 31) || !load_driver_entry_points()) return nullptr;
-  if ((uintptr_t)q % 16 || (uintptr_t)k % 16 || (uintptr_t)v % 16 || (uintptr_t)y % 16) return nullptr;
+bool attn_supported(int dt, int64_t S, int64_t D) { return (dt == DT_F16 || dt == DT_BF16) && S >= 1 && S <= 65536 && D == kAttnD; }
+AttnLaunch* attn_prepare(const AttnShape& a, const void* q, const void* k, const void* v, void* y, int* status, int sms) {
+  const int64_t S = a.positions, q_tiles = (S + kAttnS - 1) / kAttnS, batch = a.batch, heads = a.heads, ld = a.qkv_row_elems;
+  if (!attn_supported(a.dt, S, kAttnD) || batch * heads <= 0 || batch * heads * q_tiles >= (1ll << 31) || batch * S >= (1ll << 31) || !load_driver_entry_points()) return nullptr;
+  if ((uintptr_t)q % 16 || (uintptr_t)k % 16 || (uintptr_t)v % 16 || (uintptr_t)y % 16 || ld % 8) return nullptr;
   auto* L = new AttnLaunch();
   AttnParams& p = L->p;
-  p.tiles = (int)(batch * heads); p.NH = heads; p.merge = merge_heads ? 1 : 0;
-  p.scale_log2e = scale * 1.4426950408889634f;
-  p.bf16 = dt == DT_BF16; L->bf16 = dt == DT_BF16;
-  const uint32_t fmt = dt == DT_BF16 ? 1u : 0u;
-  p.idesc_s = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(kAttnS >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-  p.idesc_o = (1u << 4) | (fmt << 7) | (fmt << 10) | (1u << 16) | ((uint32_t)(kAttnD >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);   // B (= V) is MN-major
+  p.NH = (int)heads; p.S = (int)S; p.q_tiles = (int)q_tiles; p.k_blocks = (int)q_tiles;
+  p.tiles = (int)(batch * heads * q_tiles);
+  p.qkv_rows = ld > 0 ? 1 : 0; p.merge = a.merge_heads ? 1 : 0;
+  p.scale_log2e = a.scale * 1.4426950408889634f;
+  L->bf16 = a.dt == DT_BF16; L->multi = q_tiles > 1;
+  p.last_keys = (int)(S - (q_tiles - 1) * kAttnS);
+  p.last_ksteps = (p.last_keys + 15) / 16;
+  const uint32_t fmt = a.dt == DT_BF16 ? 1u : 0u, common = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(128 >> 4) << 24);
+  p.idesc_s = common | ((uint32_t)(kAttnS >> 3) << 17);
+  p.idesc_s_last = common | ((uint32_t)(2 * p.last_ksteps) << 17);                 // as many keys as are left, in sixteens
+  p.idesc_o = common | (1u << 16) | ((uint32_t)(kAttnD >> 3) << 17);               // B (= V) is MN-major
   p.desc_hi = ((uint32_t)(8 * 128) >> 4) | (1u << 14) | (2u << 29);
   p.spin_limit = kSpinLimit;
   p.status = status;
-  L->grid = p.tiles < 4 * sms ? p.tiles : 4 * sms;
-  L->smem = 3 * (size_t)kAttnBox + 1024 /*alignment slack*/ + 256 /*barriers*/;
-  const CUtensorMapDataType tdt = dt == DT_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-  const cuuint64_t rows = (cuuint64_t)p.tiles * kAttnS;
-  cuuint64_t dims[2] = {(cuuint64_t)kAttnD, rows};
-  cuuint64_t strides[1] = {(cuuint64_t)kAttnD * 2};
-  cuuint32_t box[2] = {(cuuint32_t)kAttnD, (cuuint32_t)kAttnS};
-  cuuint32_t estr[2] = {1, 1};
+  const int per_sm = L->multi ? 3 : 4;
+  L->grid = p.tiles < per_sm * sms ? p.tiles : per_sm * sms;
+  L->smem = (L->multi ? 4 : 3) * (size_t)kAttnBox + 1024 /*alignment slack*/ + 256 /*barriers*/;
+  const CUtensorMapDataType tdt = a.dt == DT_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+  // heads inside rows: (channel, head, position, batch); heads outside: (channel, position, head, batch)
+  auto encode = [&](CUtensorMap* m, const void* base, bool rows, int64_t row_elems, CUtensorMapL2promotion l2) {
+    const cuuint64_t D = (cuuint64_t)kAttnD, hs = (cuuint64_t)heads, ps = (cuuint64_t)S, bs = (cuuint64_t)batch, re = (cuuint64_t)row_elems * 2;
+    cuuint64_t dr[4] = {D, hs, ps, bs}, sr[3] = {D * 2, re, ps * re}, dh[4] = {D, ps, hs, bs}, sh[3] = {D * 2, ps * D * 2, hs * ps * D * 2};
+    cuuint32_t br[4] = {(cuuint32_t)kAttnD, 1, (cuuint32_t)kAttnS, 1}, bh[4] = {(cuuint32_t)kAttnD, (cuuint32_t)kAttnS, 1, 1}, e[4] = {1, 1, 1, 1};
+    return g_encode_tiled(m, tdt, 4, (void*)base, rows ? dr : dh, rows ? sr : sh, rows ? br : bh, e, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, l2,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
   CUresult r = CUDA_SUCCESS;
   const void* src[3] = {q, k, v};
   CUtensorMap* maps[3] = {&L->tmQ, &L->tmK, &L->tmV};
-  for (int i = 0; i < 3 && r == CUDA_SUCCESS; ++i)
-    r = g_encode_tiled(maps[i], tdt, 2, (void*)src[i], dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                       CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r == CUDA_SUCCESS) {
-    if (merge_heads) {   // [B][S][NH][D]: a head's 128 rows lie NH * D elements apart
-      cuuint64_t d4[4] = {(cuuint64_t)kAttnD, (cuuint64_t)heads, (cuuint64_t)kAttnS, (cuuint64_t)batch};
-      cuuint64_t s4[3] = {(cuuint64_t)kAttnD * 2, (cuuint64_t)heads * kAttnD * 2, (cuuint64_t)kAttnS * heads * kAttnD * 2};
-      cuuint32_t b4[4] = {(cuuint32_t)kAttnD, 1, (cuuint32_t)kAttnS, 1};
-      cuuint32_t e4[4] = {1, 1, 1, 1};
-      r = g_encode_tiled(&L->tmY, tdt, 4, y, d4, s4, b4, e4, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    } else {
-      r = g_encode_tiled(&L->tmY, tdt, 2, y, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    }
-  }
+  for (int i = 0; i < 3 && r == CUDA_SUCCESS; ++i) r = encode(maps[i], src[i], ld > 0, ld, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
+  if (r == CUDA_SUCCESS) r = encode(&L->tmY, y, a.merge_heads, heads * kAttnD, CU_TENSOR_MAP_L2_PROMOTION_NONE);
   if (r != CUDA_SUCCESS) { fprintf(stderr, "[odla_b200] tensor map (attention) encode failed: %d\n", (int)r); delete L; return nullptr; }
-  if (cudaFuncSetAttribute(attn_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L->smem) != cudaSuccess ||
-      cudaFuncSetAttribute(attn_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L->smem) != cudaSuccess) {
-    cudaGetLastError(); delete L; return nullptr;
-  }
+  auto* fn = L->multi ? (L->bf16 ? attn_kernel<true, true> : attn_kernel<false, true>) : (L->bf16 ? attn_kernel<true, false> : attn_kernel<false, false>);
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L->smem) != cudaSuccess) { cudaGetLastError(); delete L; return nullptr; }
   return L;
 }
 int attn_run(AttnLaunch* L, cudaStream_t stream) {
@@ -1989,8 +2050,8 @@ int attn_run(AttnLaunch* L, cudaStream_t stream) {
   if (pdl) { attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[na].val.programmaticStreamSerializationAllowed = 1; ++na; }
   cfg.attrs = attr;
   cfg.numAttrs = na;
-  cudaError_t le = L->bf16 ? cudaLaunchKernelEx(&cfg, attn_kernel<true>, L->tmQ, L->tmK, L->tmV, L->tmY, L->p)
-                           : cudaLaunchKernelEx(&cfg, attn_kernel<false>, L->tmQ, L->tmK, L->tmV, L->tmY, L->p);
+  auto* fn = L->multi ? (L->bf16 ? attn_kernel<true, true> : attn_kernel<false, true>) : (L->bf16 ? attn_kernel<true, false> : attn_kernel<false, false>);
+  const cudaError_t le = cudaLaunchKernelEx(&cfg, fn, L->tmQ, L->tmK, L->tmV, L->tmY, L->p);
   if (le != cudaSuccess) { fprintf(stderr, "[odla_b200] attention launch failed: %s\n", cudaGetErrorString(le)); cudaGetLastError(); return -2; }
   return 0;
 }

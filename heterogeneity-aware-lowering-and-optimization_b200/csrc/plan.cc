@@ -125,14 +125,18 @@ std::vector<uint8_t> f32_to_storage(const std::vector<float>& f, int dt) {
 
 // fp32 [k][n] -> rows [n][pitch] with the reduction contiguous (zeros up to the pitch), in square blocks so that neither side
 // of the transposition strides through memory a line at a time.
-std::vector<uint8_t> f32_rows_kmajor(const std::vector<float>& w, int64_t k, int64_t n, int64_t pitch) {
-  std::vector<uint8_t> out((size_t)(n * pitch) * sizeof(float), 0);
-  float* o = (float*)out.data();
+std::vector<float> transpose_rows(const std::vector<float>& w, int64_t k, int64_t n, int64_t pitch) {
+  std::vector<float> o((size_t)(n * pitch), 0.f);
   for (int64_t k0 = 0; k0 < k; k0 += 32)
     for (int64_t n0 = 0; n0 < n; n0 += 32)
       for (int64_t i = k0; i < std::min(k, k0 + 32); ++i)
-        for (int64_t j = n0; j < std::min(n, n0 + 32); ++j) o[j * pitch + i] = w[(size_t)(i * n + j)];
-  return out;
+        for (int64_t j = n0; j < std::min(n, n0 + 32); ++j) o[(size_t)(j * pitch + i)] = w[(size_t)(i * n + j)];
+  return o;
+}
+std::vector<uint8_t> f32_rows_kmajor(const std::vector<float>& w, int64_t k, int64_t n, int64_t pitch) { return f32_to_storage(transpose_rows(w, k, n, pitch), DT_F32); }
+// A Gemm's weights as K-major rows [n][k] of storage type dt; `w` is [k][n], or already [n][k] when `transposed`.
+std::vector<uint8_t> rows_kmajor(const std::vector<float>& w, int64_t k, int64_t n, bool transposed, int dt) {
+  return f32_to_storage(transposed ? w : transpose_rows(w, k, n, k), dt);
 }
 
 // A fused convolution / GEMM: root node plus the chain folded into its epilogue.
@@ -166,6 +170,9 @@ struct Item {               // one launch-list entry before emission
   // items of their own, their operands are read here
   V attn_q = nullptr, attn_k = nullptr;
   float attn_scale = 1.f;
+  int64_t attn_row_elems = 0;   // 0: q, k, v are head-split; else they are column groups of projection rows this wide
+  // projections of one tensor that run as a single Gemm (columns side by side): their roots, this item's own first
+  std::vector<V> group;
 };
 
 class Builder {
@@ -255,6 +262,8 @@ class Builder {
   odla_status place();
   odla_status emit();
   void try_attention(Item& it, const Fused& f);
+  bool can_group(const std::vector<V>& roots);
+  odla_status emit_group(const Item& it);
   odla_status emit_fused(const Item& it);
   odla_status emit_plain(const Item& it);
   void add_launch(const char* op, V out, double flops, double bytes, std::function<int(cudaStream_t)> fn) {
@@ -544,10 +553,12 @@ odla_status Builder::place() {
     for (auto& kv : alias_) if (resolve(kv.first) == v) aliased = true;
     if ((K * 2) % 16 != 0 && !aliased) pitch_[v] = (K + 7) / 8 * 8;
   }
+  std::map<V, int64_t> grouped;   // a group's first value holds the columns of all of them
+  for (auto& it : items_) if (!it.group.empty()) grouped[it.out] = (int64_t)it.group.size();
   auto bytes_of = [&](V v) {
     auto pi = pitch_.find(v);
     if (pi != pitch_.end()) { const auto& sh = v->type.shape; return count(v) / sh.dims[sh.size - 1] * pi->second * storage_size(dt_[v]); }
-    return count(v) * storage_size(dt_[v]);
+    return count(v) * storage_size(dt_[v]) * (grouped.count(v) ? grouped.at(v) : 1);
   };
   for (V a : c_->args) {
     Slot s; s.dt = dt_[a]; s.bytes = bytes_of(a); s.offset = arena.alloc(s.bytes);
@@ -633,22 +644,134 @@ void Builder::try_attention(Item& it, const Fused& f) {
   const auto &qs = q->type.shape, &ks = k->type.shape, &vs = v->type.shape;
   if (qs.size != 4 || ks.size != 4 || vs.size != 4) return;
   const int64_t B = qs.dims[0], NH = qs.dims[1], S = qs.dims[2], D = qs.dims[3];
-  if (!attn_supported(fs, S, D)) return;
+  if (!attn_supported(fs, S, D) || B * NH * S >= (1ll << 31)) return;
   for (int d = 0; d < 4; ++d) if (ks.dims[d] != qs.dims[d] || vs.dims[d] != qs.dims[d]) return;
   if (ps.dims[0] != B || ps.dims[1] != NH || ps.dims[2] != S || ps.dims[3] != S) return;
   if (f.perm_mode == 2 && (f.perm_NH != NH || f.perm_S != S || f.perm_D != D)) return;
   if (dt_[q] != fs || dt_[k] != fs || dt_[v] != fs || alias_.count(q) || alias_.count(k) || alias_.count(v)) return;
   if (pitch_.count(q) || pitch_.count(k) || pitch_.count(v)) return;
   // the two earlier launches go; nothing else reads what they would have written
-  size_t removed = 0;
-  for (size_t i = items_.size(); i-- > 0;)
-    if (items_[i].out == sm || items_[i].out == sc_out) { items_.erase(items_.begin() + (long)i); ++removed; }
-  if (removed != 2) { B2_WARN("attention pattern at '%s' matched but its producers were not separate launches", root->name.c_str()); }
+  auto drop = [&](V out) {
+    for (size_t i = items_.size(); i-- > 0;)
+      if (items_[i].out == out) { items_.erase(items_.begin() + (long)i); return 1; }
+    return 0;
+  };
+  if (drop(sm) + drop(sc_out) != 2) { B2_WARN("attention pattern at '%s' matched but its producers were not separate launches", root->name.c_str()); }
   it.attn_q = q;
   it.attn_k = k;
   it.attn_scale = sc_root->fa[0] * g.scalar_mul;
   it.reads.clear();
   it.reads.push_back(q); it.reads.push_back(k); it.reads.push_back(v);
+  // q, k and v that are head splits of projections nobody else reads stay as the projections leave them: the kernel
+  // addresses a head as a group of 64 columns, so that neither a permuting store nor a sequence of whole boxes is needed.
+  std::vector<V> roots;
+  for (V t : {q, k, v}) {
+    auto ti = fused_into_.find(t);
+    V r = ti != fused_into_.end() ? ti->second : nullptr;
+    if (!r || r->kind != OP_GEMM || !fused_.count(r) || fused_[r]->out != t || fused_[r]->perm_mode != 1 || users_[t] != 1 || t->is_output) return;
+    if (fused_[r]->w->kind != OP_CONST || r->type.shape.size != 2) return;
+    roots.push_back(r);
+  }
+  if (roots[0] == roots[1] || roots[1] == roots[2] || roots[0] == roots[2]) return;
+  for (V r : roots) fused_[r]->perm_mode = 0;
+  it.attn_row_elems = NH * D;
+  if (!can_group(roots)) return;
+  // ... and when they project the same tensor the three Gemms are one with three times the columns, which fills the chip
+  // better and reads the tensor once
+  for (auto& other : items_)
+    if (other.out == q) { other.group = roots; it.attn_row_elems = 3 * NH * D; }
+  if (it.attn_row_elems != 3 * NH * D) return;
+  drop(k);
+  drop(v);
+  it.reads.clear();
+  it.reads.push_back(q);
+}
+
+// Whether plain Gemms with constant weights can run as one Gemm over their columns side by side.
+bool Builder::can_group(const std::vector<V>& roots) {
+  V a = roots[0];
+  const Fused& fa = *fused_[a];
+  const auto &as = a->in[0]->type.shape, &ws = fa.w->type.shape;
+  if (as.size != 2 || ws.size != 2 || a->ia[0] != 0) return false;
+  for (V r : roots) {
+    const Fused& f = *fused_[r];
+    if (f.x != fa.x || r->in[0] != a->in[0] || f.int8 != fa.int8 || f.x_scale != fa.x_scale || f.w_zp || f.res || f.act != ACT_NONE || f.quant_scale || f.has_scalar_mul || f.perm_mode) return false;
+    if (r->ia[0] != a->ia[0] || r->ia[1] != a->ia[1] || r->fa[0] != a->fa[0] || r->fa[1] != a->fa[1]) return false;
+    if (f.w->kind != OP_CONST || f.w->type.shape.size != 2 || f.w->type.shape.dims[0] != ws.dims[0] || f.w->type.shape.dims[1] != ws.dims[1]) return false;
+    if (!f.add_const != !fa.add_const || !r->in[2] != !a->in[2] || (r->in[2] && r->in[2]->kind != OP_CONST)) return false;
+    if (r->in[2] && numel(r->in[2]->type.shape) != 1 && numel(r->in[2]->type.shape) != r->type.shape.dims[1]) return false;
+  }
+  const int64_t M = shape(a).dims[0], N = a->type.shape.dims[1] * (int64_t)roots.size();
+  if (M >= (1ll << 31)) return false;
+  return umma_conv_supported(UmmaConv{1, 1, (int)M, (int)as.dims[1], (int)N, 1, 1, 1, (int)M, 1, 1, 0, 0, fa.int8 ? DT_S8 : FS()});
+}
+
+// |accumulator| <= 128 * sum |w[k,:]| (activations lie in [-128, 127]); below 2^22 for every output channel the epilogue can
+// convert the accumulators without the conversion pipe.  The output channel is the last axis of w, or its first (k_last false).
+int accumulators_small(const std::vector<int>& w, int64_t K, bool k_last) {
+  const int64_t n = (int64_t)w.size();
+  if (getenv("ODLA_B200_NO_ACC_SMALL") || K <= 0 || n % K != 0) return 0;
+  const int64_t inner = n / K;
+  std::vector<int64_t> sum((size_t)K, 0);
+  for (int64_t i = 0; i < n; ++i) sum[(size_t)(k_last ? i % K : i / inner)] += std::abs(w[(size_t)i]);
+  return *std::max_element(sum.begin(), sum.end()) * 128 < (1ll << 22) ? 1 : 0;
+}
+
+// Several projections of one tensor as one Gemm: weights, multipliers and addends side by side, [rows][sum of columns] out.
+odla_status Builder::emit_group(const Item& it) {
+  V root = it.fused->root;
+  const bool int8 = it.fused->int8, tb = root->ia[1] != 0;
+  const int in_dt = int8 ? DT_S8 : FS();
+  if (dt_[resolve(it.fused->x)] != in_dt) return fail(ODLA_UNSUPPORTED_DATATYPE, "'" + root->name + "': operand storage type does not match the compute type");
+  const int64_t N = root->type.shape.dims[1], Kd = root->in[0]->type.shape.dims[1], M = shape(root).dims[0], G = (int64_t)it.group.size();
+  std::vector<float> mul, add1, add2;
+  Epilogue ep;
+  ep.alpha = root->fa[0];
+  ep.out_dt = dt_[it.out];
+  ep.acc_small = int8 ? 1 : 0;
+  std::string form = "gemm_kmajor_group dt" + std::to_string(in_dt) + (tb ? " t" : " n");
+  for (V r : it.group) {
+    const Fused& f = *fused_[r];
+    form += " " + std::to_string(f.w->index);
+    if (int8) {
+      auto sx = const_as_f32(f.x_scale), sw = const_as_f32(f.w_scale);
+      for (int64_t n = 0; n < N; ++n) mul.push_back(sx[0] * sw[sw.size() == 1 ? 0 : n]);
+      const int8_t* w = (const int8_t*)f.w->host;
+      if (!accumulators_small(std::vector<int>(w, w + N * Kd), N, !tb)) ep.acc_small = 0;
+    }
+    if (r->in[2] && root->fa[1] != 0.f) {
+      auto c = const_as_f32(r->in[2]);
+      for (int64_t n = 0; n < N; ++n) add1.push_back(root->fa[1] * c[c.size() == 1 ? 0 : n]);
+    }
+    if (f.add_const) { auto c = const_as_f32(f.add_const); add2.insert(add2.end(), c.begin(), c.end()); }
+  }
+  if (!mul.empty()) ep.mul = upload_f32(mul);
+  if (!add1.empty()) ep.add1 = upload_f32(add1);
+  if (!add2.empty()) ep.add2 = upload_f32(add2);
+  auto wb = prepared(it.fused->w, form, [&] {
+    std::vector<uint8_t> all;
+    for (V r : it.group) {
+      auto part = rows_kmajor(const_as_f32(fused_[r]->w), Kd, N, tb, in_dt);
+      all.insert(all.end(), part.begin(), part.end());
+    }
+    return all;
+  });
+  void* wd = upload(wb->data(), wb->size());
+  if (!wd) return err_status_;
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p_->device);
+  UmmaLaunch* ul = umma_conv_prepare(UmmaConv{1, 1, (int)M, (int)Kd, (int)(G * N), 1, 1, 1, (int)M, 1, 1, 0, 0, in_dt}, dev_ptr(it.fused->x), wd, dev_ptr(it.out), ep, p_->status, sms);
+  if (!ul) return fail(ODLA_FAILURE, "'" + root->name + "': tensor-map encoding failed");
+  p_->umma.push_back(ul);
+  // one entry of the launch list per value; the kernel belongs to the first
+  add_launch("gemm_umma", it.out, 2.0 * M * N * Kd * G, tensor_bytes(it.fused->x) + G * tensor_bytes(it.out) + (double)(G * N * Kd) * storage_size(in_dt),
+             [ul](cudaStream_t s) { return umma_conv_run(ul, s); });
+  p_->launches.back().out_ptr = nullptr;   // (not a dense tensor of the value's own size: no range record)
+  for (size_t i = 1; i < it.group.size(); ++i) {
+    add_launch("gemm_umma", fused_[it.group[i]]->out, 0, 0, [](cudaStream_t) { return 0; });
+    p_->launches.back().n_kernels = 0;
+  }
+  return ODLA_SUCCESS;
 }
 
 odla_status Builder::emit_fused(const Item& it) {
@@ -658,8 +781,11 @@ odla_status Builder::emit_fused(const Item& it) {
     const int64_t B = shape(it.attn_q).dims[0], NH = qs.dims[1], S = qs.dims[2], D = qs.dims[3];
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p_->device);
-    AttnLaunch* al = attn_prepare(FS(), dev_ptr(it.attn_q), dev_ptr(it.attn_k), dev_ptr(f.w), dev_ptr(f.out), B, (int)NH, it.attn_scale, f.perm_mode == 2,
-                                  p_->status, sms);
+    const char* qp = (const char*)dev_ptr(it.attn_q);
+    const bool grouped = it.attn_row_elems > NH * D;   // k and v are the columns after q's
+    const void* kp = grouped ? qp + NH * D * storage_size(FS()) : dev_ptr(it.attn_k);
+    const void* vp = grouped ? qp + 2 * NH * D * storage_size(FS()) : dev_ptr(f.w);
+    AttnLaunch* al = attn_prepare(AttnShape{FS(), B, (int)NH, S, it.attn_row_elems, it.attn_scale, f.perm_mode == 2}, qp, kp, vp, dev_ptr(f.out), p_->status, sms);
     if (!al) return fail(ODLA_FAILURE, "'" + f.root->name + "': fused attention could not be prepared");
     p_->attn.push_back(al);
     const double flops = 2.0 * 2.0 * (double)B * NH * S * S * D;
@@ -667,6 +793,7 @@ odla_status Builder::emit_fused(const Item& it) {
     add_launch("attention", f.out, flops, bytes, [al](cudaStream_t s) { return attn_run(al, s); });
     return ODLA_SUCCESS;
   }
+  if (!it.group.empty()) return emit_group(it);
   const Fused& f = *it.fused;
   V root = f.root;
   int in_dt = f.int8 ? DT_S8 : FS();
@@ -696,23 +823,9 @@ odla_status Builder::emit_fused(const Item& it) {
     } else {
       for (int64_t i = 0; i < wn; ++i) wint[(size_t)i] = ((const int8_t*)f.w->host)[i];
     }
-    // |accumulator| <= 128 * sum |w[k,:]| (activations lie in [-128, 127]); below 2^22 for every output channel the
-    // epilogue can convert the accumulators without the conversion pipe.
-    if (f.w->kind == OP_CONST && !getenv("ODLA_B200_NO_ACC_SMALL")) {
-      const int* wq = wint.data();
-      const int64_t n = wn;
-      // filters are [.., K] (HWIO) and Gemm weights [Kd, N] or, transposed, [N, Kd]: the output channel is the last
-      // axis unless the Gemm's B is transposed
-      const bool k_last = !(root->kind == OP_GEMM && root->ia[1] != 0);
-      std::vector<int64_t> sum((size_t)K, 0);
-      if (n % K == 0) {
-        const int64_t inner = n / K;
-        for (int64_t i = 0; i < n; ++i) sum[(size_t)(k_last ? i % K : i / inner)] += std::abs((int)wq[i]);
-        int64_t worst = 0;
-        for (int64_t k = 0; k < K; ++k) worst = std::max(worst, sum[(size_t)k]);
-        ep.acc_small = worst * 128 < (1ll << 22) ? 1 : 0;
-      }
-    }
+    // filters are [.., K] (HWIO) and Gemm weights [Kd, N] or, transposed, [N, Kd]: the output channel is the last axis
+    // unless the Gemm's B is transposed
+    if (f.w->kind == OP_CONST) ep.acc_small = accumulators_small(wint, K, !(root->kind == OP_GEMM && root->ia[1] != 0));
   }
   if (f.add_const) ep.add2 = (const float*)const_dev(f.add_const, DT_F32);
   if (f.res) {
@@ -1061,11 +1174,7 @@ odla_status Builder::emit_fused(const Item& it) {
             }
           return out;
         }
-        auto wf = f.int8 ? std::vector<float>(wint.begin(), wint.end()) : const_as_f32(f.w);
-        std::vector<float> w2;
-        if (tb) w2 = wf;  // already [N][K]
-        else { w2.resize(wf.size()); for (int64_t k = 0; k < Kd; ++k) for (int64_t n = 0; n < N; ++n) w2[(size_t)(n * Kd + k)] = wf[(size_t)(k * N + n)]; }
-        return f32_to_storage(w2, in_dt);
+        return rows_kmajor(f.int8 ? std::vector<float>(wint.begin(), wint.end()) : const_as_f32(f.w), Kd, N, tb, in_dt);
       });
       void* wd = upload(wb->data(), wb->size());
       if (!wd) return err_status_;
