@@ -6,9 +6,36 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <cstdlib>
+
 #include "kernels.h"
 
 namespace b200 {
+
+// ---- launches ----
+// Every kernel of this library is launched as a programmatic dependent of the one in front of it (its blocks may be placed
+// while that one drains) and therefore begins with dependency_wait(): wait until the kernels it depends on have completed and
+// their writes are visible, then let the next kernel's blocks come.
+__device__ __forceinline__ void dependency_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... P, typename... A>
+inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+  static const bool pdl = !getenv("ODLA_B200_NO_PDL");
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);   // (the caller asks cudaGetLastError)
+}
+
 
 __device__ __forceinline__ float load_as_float(const void* p, int dt, int64_t i) {
   switch (dt) {

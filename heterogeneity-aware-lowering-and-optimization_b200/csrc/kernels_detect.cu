@@ -2,10 +2,13 @@
 // (odla_ops_nn.h:757-759).
 //
 // Greedy non-maximum suppression is a walk over the candidates in descending score order; sorting them first is what
-// a CPU does.  Here one CTA owns one (batch, class) problem and repeats: block-wide arg-max over the candidates that
-// are still eligible (score, then the lower index on a tie -- the order a stable descending sort gives), record it,
-// strike what it suppresses.  That is the same walk without the sort, costs one pass over the scores per SELECTED box
-// (a few dozen for real detectors) and needs no scratch beyond a bit mask in shared memory.
+// a CPU does.  Here one CTA owns one (batch, class) problem: one coalesced pass over the scores gathers the candidates above
+// the threshold -- a few dozen of ten thousand for real detectors -- with their boxes in shared memory, and then one warp
+// repeats: arg-max over the candidates that are still eligible (score, then the lower index on a tie -- the order a stable
+// descending sort gives, whatever order they were gathered in), record it, strike what it suppresses.  Bound by latency: the
+// pass over the scores is a dozen loads per thread, a selection a few hundred cycles.  When more candidates pass the
+// threshold than fit, the whole block walks the scores once per SELECTED box instead, with a bit mask of the eligible ones in
+// shared memory.
 //
 //   mode 0  odla_NMS: the ONNX NonMaxSuppression rule the reference's emitter maps to it
 //           (lib/target/generic_cpp/nms.cc:22-69): boxes [B, N, 4] as (y1, x1, y2, x2) in any corner order, scores
@@ -15,6 +18,7 @@
 //           box only, scores below the threshold are skipped, boxes are (y_min, x_min, y_max, x_max).
 //
 // Every floating-point step uses the *_rn intrinsics in the order of the CPU oracle, so both pick the same boxes.
+#include <algorithm>
 #include <cstdio>
 
 #include "epilogue.cuh"
@@ -69,16 +73,91 @@ __device__ __forceinline__ bool overlaps_yolo(const float (&s)[4], const float (
   return __fdiv_rn(comm, __fsub_rn(__fadd_rn(sa, ca), comm)) > thr;
 }
 
+constexpr int kGathered = 1024;   // candidates of one problem kept in shared memory: boxes 16 KB, scores and indices 8 KB
+constexpr int kNmsThreads = 512;
+constexpr int kNmsSmem = kGathered * 24;
+
 // grid = problems (batch x class); sel[p][k] = k-th selected box of problem p, cnt[p] = how many.
 template <int MODE>
-__global__ void greedy_nms_kernel(const void* __restrict__ boxes, int box_dt, const void* __restrict__ scores, int score_dt, int C, int N, int max_sel,
-                                  float iou_thr, float score_thr, int* __restrict__ sel, int* __restrict__ cnt) {
-  extern __shared__ uint32_t alive[];          // MODE 0: one bit per candidate
+__global__ void __launch_bounds__(kNmsThreads)
+greedy_nms_kernel(const void* __restrict__ boxes, int box_dt, const void* __restrict__ scores, int score_dt, int C, int N, int max_sel,
+                  float iou_thr, float score_thr, int* __restrict__ sel, int* __restrict__ cnt) {
+  dependency_wait();
+  extern __shared__ uint32_t alive[];          // the gathered candidates; MODE 0 without them: one bit per candidate
   __shared__ Cand warp_c[32];
   __shared__ Cand chosen;
+  __shared__ int n_gathered;
   const int p = blockIdx.x, b = p / C;
   const int64_t sbase = (int64_t)p * N, bbase = (int64_t)b * N;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  {
+    float4* g_box = (float4*)alive;
+    float* g_score = (float*)(g_box + kGathered);
+    int* g_idx = (int*)(g_score + kGathered);
+    if (threadIdx.x == 0) n_gathered = 0;
+    __syncthreads();
+    for (int i0 = threadIdx.x; i0 < N; i0 += 8 * blockDim.x) {
+      float sc[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) { const int i = i0 + u * blockDim.x; if (i < N) sc[u] = load_as_float(scores, score_dt, sbase + i); }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int i = i0 + u * blockDim.x;
+        if (i < N && (MODE == 0 ? sc[u] > score_thr : !(sc[u] < score_thr))) {
+          const int at = atomicAdd(&n_gathered, 1);
+          if (at < kGathered) { g_score[at] = sc[u]; g_idx[at] = i; }
+        }
+      }
+    }
+    __syncthreads();
+    const int n = n_gathered;
+    if (n <= kGathered) {
+      for (int k = threadIdx.x; k < n; k += blockDim.x) {
+        float v[4];
+        load_box(boxes, box_dt, bbase + g_idx[k], v);
+        g_box[k] = make_float4(v[0], v[1], v[2], v[3]);
+      }
+      __syncthreads();
+      if (warp != 0) return;
+      uint32_t gone = 0;            // MODE 0: lane's candidate k = lane + 32 * j has been selected or suppressed (bit j)
+      Cand last; last.score = 0.f; last.idx = -1;
+      float lb[4] = {0.f, 0.f, 0.f, 0.f};
+      int n_sel = 0;
+      while (n_sel < max_sel) {
+        Cand best; best.score = 0.f; best.idx = -1;
+        int best_k = -1;
+        for (int k = lane, j = 0; k < n; k += 32, ++j) {
+          if (MODE == 0 && ((gone >> j) & 1u)) continue;
+          Cand c; c.score = g_score[k]; c.idx = g_idx[k];
+          if (MODE != 0 && last.idx >= 0) {
+            // after the last selected one in (score descending, index ascending) order, and not overlapping it
+            if (!better(last, c)) continue;
+            const float4 f = g_box[k];
+            const float cb[4] = {f.x, f.y, f.z, f.w};
+            if (overlaps_yolo(lb, cb, iou_thr)) continue;
+          }
+          if (best.idx < 0 || better(c, best)) { best = c; best_k = k; }
+        }
+        last = warp_best(best);
+        if (last.idx < 0) break;
+        if (lane == 0) sel[(int64_t)p * max_sel + n_sel] = last.idx;
+        ++n_sel;
+        const int owner = __ffs(__ballot_sync(0xffffffffu, best.idx == last.idx)) - 1;
+        const float4 f = g_box[__shfl_sync(0xffffffffu, best_k, owner)];
+        lb[0] = f.x; lb[1] = f.y; lb[2] = f.z; lb[3] = f.w;
+        if (MODE == 0)
+          for (int k = lane, j = 0; k < n; k += 32, ++j) {
+            if ((gone >> j) & 1u) continue;
+            const float4 q = g_box[k];
+            const float cb[4] = {q.x, q.y, q.z, q.w};
+            if (g_idx[k] == last.idx || overlaps_onnx(lb, cb, iou_thr)) gone |= 1u << j;
+          }
+      }
+      if (lane == 0) cnt[p] = n_sel;
+      return;
+    }
+    __syncthreads();   // the gathered ones are given up: the mask below reuses their memory
+  }
   if (MODE == 0) {
     for (int w = threadIdx.x; w < (N + 31) / 32; w += blockDim.x) {
       uint32_t m = 0;
@@ -147,18 +226,38 @@ __global__ void greedy_nms_kernel(const void* __restrict__ boxes, int box_dt, co
 
 // Selections of all problems in (batch, class, selection order) order -> rows (batch, class, box) of the output,
 // at most `rows`; the rest is filled with -1.
-__global__ void nms_emit_kernel(const int* __restrict__ sel, const int* __restrict__ cnt, int problems, int C, int max_sel, int rows, int out64, void* out) {
+__global__ void __launch_bounds__(1024)
+nms_emit_kernel(const int* __restrict__ sel, const int* __restrict__ cnt, int problems, int C, int max_sel, int rows, int out64, void* out) {
+  dependency_wait();
   __shared__ int start[1025];
-  if (threadIdx.x == 0) { int s = 0; for (int p = 0; p < problems; ++p) { start[p] = s; s += cnt[p]; } start[problems] = s; }
+  __shared__ int warp_sum[32];
+  // exclusive prefix sums of the (at most 1024) counts; every block makes its own copy
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  int v = t < problems ? cnt[t] : 0;
+  const int own = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += u; }
+  if (lane == 31) warp_sum[warp] = v;
   __syncthreads();
-  for (int r = threadIdx.x; r < rows; r += blockDim.x) {
-    int v[3] = {-1, -1, -1};
+  if (warp == 0) {
+    int w = warp_sum[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, w, o); if (lane >= o) w += u; }
+    warp_sum[lane] = w;
+  }
+  __syncthreads();
+  v += warp > 0 ? warp_sum[warp - 1] : 0;
+  if (t < problems) start[t] = v - own;
+  if (t == problems - 1) start[problems] = v;
+  __syncthreads();
+  for (int r = blockIdx.x * blockDim.x + t; r < rows; r += gridDim.x * blockDim.x) {
+    int o[3] = {-1, -1, -1};
     if (r < start[problems]) {
       int lo = 0, hi = problems;   // the problem whose range holds row r
       while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if (start[mid] <= r) lo = mid; else hi = mid; }
-      v[0] = lo / C; v[1] = lo % C; v[2] = sel[(int64_t)lo * max_sel + (r - start[lo])];
+      o[0] = lo / C; o[1] = lo % C; o[2] = sel[(int64_t)lo * max_sel + (r - start[lo])];
     }
-    for (int k = 0; k < 3; ++k) { if (out64) ((long long*)out)[r * 3 + k] = v[k]; else ((int*)out)[r * 3 + k] = v[k]; }
+    for (int k = 0; k < 3; ++k) { if (out64) ((long long*)out)[r * 3 + k] = o[k]; else ((int*)out)[r * 3 + k] = o[k]; }
   }
 }
 
@@ -167,6 +266,7 @@ __global__ void nms_emit_kernel(const int* __restrict__ sel, const int* __restri
 // objectness e/(e+1), class scores e/(e+1) * objectness.  One thread per (cell, anchor).
 __global__ void yolo_decode_kernel(const void* __restrict__ head, int dt, int nchw, int S, int cls, int first, int N, const unsigned* __restrict__ anchors6,
                                    const unsigned* __restrict__ img_w, const unsigned* __restrict__ img_h, float* __restrict__ boxes, float* __restrict__ scores) {
+  dependency_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= S * S * 3) return;
   const int a = t % 3, x = (t / 3) % S, y = t / (3 * S);
@@ -198,6 +298,7 @@ __global__ void yolo_decode_kernel(const void* __restrict__ head, int dt, int nc
 // selected_info[c][k] = (y_min, x_min, y_max, x_max, score) of class c's k-th selection, zeros beyond the count.
 __global__ void yolo_emit_kernel(const int* __restrict__ sel, const int* __restrict__ cnt, const float* __restrict__ boxes, const float* __restrict__ scores,
                                  int cls, int N, int per_class, float* __restrict__ info, unsigned* __restrict__ num) {
+  dependency_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < cls) num[t] = (unsigned)cnt[t];
   if (t >= cls * per_class) return;
@@ -218,10 +319,10 @@ int nms(int B, int C, int N, int max_sel, float iou_thr, float score_thr, int bo
   if (B * C <= 0 || out_rows <= 0) return 0;
   if (B * C > 1024 || N > 1500000) return -1;
   if (N > 0 && max_sel > 0) {
-    greedy_nms_kernel<0><<<B * C, 256, ((N + 31) / 32) * 4, s>>>(boxes, box_dt, scores, score_dt, C, N, max_sel, iou_thr, score_thr, sel, cnt);
+    launch(greedy_nms_kernel<0>, B * C, kNmsThreads, std::max(kNmsSmem, ((N + 31) / 32) * 4), s, boxes, box_dt, scores, score_dt, C, N, max_sel, iou_thr, score_thr, sel, cnt);
     if (int rc = check_launch()) return rc;
   } else if (cudaMemsetAsync(cnt, 0, sizeof(int) * B * C, s) != cudaSuccess) return -2;
-  nms_emit_kernel<<<1, 256, 0, s>>>(sel, cnt, B * C, C, max_sel > 0 ? max_sel : 1, out_rows, out64, out);
+  launch(nms_emit_kernel, std::min((out_rows + 1023) / 1024, 64), 1024, 0, s, sel, cnt, B * C, C, max_sel > 0 ? max_sel : 1, out_rows, out64, out);
   return check_launch();
 }
 
@@ -233,12 +334,12 @@ int yolo_postprocess(int cls, const int* S3, const void* const* heads, int dt, c
   for (int i = 0; i < 3; ++i) {
     const int threads = S3[i] * S3[i] * 3;
     // the coarsest head (stride 32) uses the largest anchors: rows 2, 1, 0 of the anchor table for 13, 26, 52
-    yolo_decode_kernel<<<(threads + 127) / 128, 128, 0, s>>>(heads[i], dt, nchw3[i], S3[i], cls, first[i], N, anchors18 + 6 * (2 - i), img_w, img_h, boxes, scores);
+    launch(yolo_decode_kernel, (threads + 127) / 128, 128, 0, s, heads[i], dt, nchw3[i], S3[i], cls, first[i], N, anchors18 + 6 * (2 - i), img_w, img_h, boxes, scores);
     if (int rc = check_launch()) return rc;
   }
-  greedy_nms_kernel<1><<<cls, 256, 0, s>>>(boxes, DT_F32, scores, DT_F32, cls, N, per_class, 0.45f, 0.3f, sel, cnt);
+  launch(greedy_nms_kernel<1>, cls, kNmsThreads, kNmsSmem, s, boxes, DT_F32, scores, DT_F32, cls, N, per_class, 0.45f, 0.3f, sel, cnt);
   if (int rc = check_launch()) return rc;
-  yolo_emit_kernel<<<(cls * per_class + 127) / 128, 128, 0, s>>>(sel, cnt, boxes, scores, cls, N, per_class, info, num);
+  launch(yolo_emit_kernel, (cls * per_class + 127) / 128, 128, 0, s, sel, cnt, boxes, scores, cls, N, per_class, info, num);
   return check_launch();
 }
 

@@ -67,6 +67,7 @@ __device__ __forceinline__ void store_result(const Epilogue& ep, void* y, int64_
 // One thread per output element, output channel fastest so filter reads coalesce for HWIO.
 template <typename T, typename ACC>
 __global__ void conv_direct_kernel(ConvGeom g, const T* __restrict__ x, const T* __restrict__ w, void* y, Epilogue ep) {
+  dependency_wait();
   int64_t total = (int64_t)g.N * g.P * g.Q * g.K;
   int cg = g.C / g.groups, kg = g.K / g.groups;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
@@ -96,6 +97,7 @@ __global__ void conv_direct_kernel(ConvGeom g, const T* __restrict__ x, const T*
 
 template <typename T, typename ACC>
 __global__ void gemm_direct_kernel(GemmGeom g, const T* __restrict__ A, const T* __restrict__ B, void* C, Epilogue ep) {
+  dependency_wait();
   int64_t total = g.batch * g.M * g.N;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     int n = (int)(e % g.N);
@@ -112,6 +114,7 @@ __global__ void gemm_direct_kernel(GemmGeom g, const T* __restrict__ A, const T*
 // ------------------------------------------------------------------ pooling ----
 template <bool IS_MAX>
 __global__ void pool_generic_kernel(PoolGeom g, int dt, const void* x, void* y) {
+  dependency_wait();
   int64_t total = (int64_t)g.N * g.P * g.Q * g.C;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     int c = (int)(e % g.C);
@@ -172,6 +175,7 @@ template <> struct VecMax<float, 4> {
 // the rows shared by neighbouring output rows are found in L2.
 template <typename T, int VEC>
 __global__ void maxpool_nhwc_vec_kernel(PoolGeom g, const T* __restrict__ x, T* __restrict__ y) {
+  dependency_wait();
   const int cv = g.C / VEC, row_items = g.Q * cv;
   const int rows = g.N * g.P;
   for (int row = blockIdx.y; row < rows; row += gridDim.y) {
@@ -206,6 +210,7 @@ __global__ void maxpool_nhwc_vec_kernel(PoolGeom g, const T* __restrict__ x, T* 
 // thread's life R*S trips to memory long.
 template <typename T, int VEC, int R, int S>
 __global__ void maxpool_nhwc_win_kernel(PoolGeom g, const T* __restrict__ x, T* __restrict__ y) {
+  dependency_wait();
   const int cv = g.C / VEC, row_items = g.Q * cv;
   const int rows = g.N * g.P;
   for (int row = blockIdx.y; row < rows; row += gridDim.y) {
@@ -263,11 +268,13 @@ __device__ __forceinline__ float unary_one(int op, float x, float a, float b) {
   return x;
 }
 __global__ void unary_kernel(int op, int dt_in, int dt_out, const void* x, void* y, int64_t n, float a, float b) {
+  dependency_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     store_from_float(y, dt_out, i, unary_one(op, load_as_float(x, dt_in, i), a, b));
 }
 // 16-byte path for fp16 -> fp16.
 __global__ void unary_h8_kernel(int op, const uint4* __restrict__ x, uint4* __restrict__ y, int64_t n8, float a, float b) {
+  dependency_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n8; i += (int64_t)gridDim.x * blockDim.x) {
     uint4 v = x[i];
     __half* h = (__half*)&v;
@@ -289,6 +296,7 @@ __device__ __forceinline__ float binary_one(int op, float x, float y) {
 }
 __global__ void binary_kernel(int op, BinaryGeom g, int dt_l, int dt_r, int dt_out, const void* l, const void* r, void* y,
                               int64_t total, int act, float act_a) {
+  dependency_wait();
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     int64_t rem = e, li = 0, ri = 0;
     for (int d = g.rank - 1; d >= 0; --d) {
@@ -304,6 +312,7 @@ __global__ void binary_kernel(int op, BinaryGeom g, int dt_l, int dt_r, int dt_o
 // Same-shape fp16 fast path, 16 bytes per thread.
 __global__ void binary_same_h8_kernel(int op, const uint4* __restrict__ l, const uint4* __restrict__ r, uint4* __restrict__ y,
                                       int64_t n8, int act, float act_a) {
+  dependency_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n8; i += (int64_t)gridDim.x * blockDim.x) {
     uint4 a = l[i], b = r[i];
     __half* ha = (__half*)&a;
@@ -320,6 +329,7 @@ __global__ void binary_same_h8_kernel(int op, const uint4* __restrict__ l, const
 template <typename T, typename RT>
 __global__ void binary_period_vec_kernel(int op, const uint4* __restrict__ l, const RT* __restrict__ r, uint4* __restrict__ y, int64_t n8, int64_t period8,
                                          int act, float act_a) {
+  dependency_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n8; i += (int64_t)gridDim.x * blockDim.x) {
     uint4 a = l[i];
     const int64_t j = (i % period8) * 8;
@@ -341,6 +351,7 @@ __global__ void binary_period_vec_kernel(int op, const uint4* __restrict__ l, co
 }
 __global__ void channel_affine_kernel(int dt, const void* x, void* y, const float* a, const float* b, int64_t total, int64_t C,
                                       int64_t inner) {
+  dependency_wait();
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     int c = (int)((e / inner) % C);
     store_from_float(y, dt, e, __fadd_rn(__fmul_rn(load_as_float(x, dt, e), a[c]), b[c]));
@@ -380,6 +391,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 }
 // One warp per row along a contiguous last axis.
 __global__ void softmax_rows_kernel(int dt, const void* x, void* y, int64_t rows, int64_t dim, int log_form) {
+  dependency_wait();
   int lane = threadIdx.x & 31;
   int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5, nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t row = warp; row < rows; row += nwarps) {
@@ -432,6 +444,7 @@ __device__ __forceinline__ void load_row_pieces(const uint4* row, int pieces, in
 }
 template <typename T, int NP, int LPR>
 __global__ void softmax_rows_vec_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, int64_t rows, int pieces, int log_form) {
+  dependency_wait();
   constexpr int RPW = 32 / LPR;  // rows per warp
   const int lane = threadIdx.x & 31, l = lane % LPR;
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5, nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -479,6 +492,7 @@ __global__ void softmax_rows_vec_kernel(const uint4* __restrict__ x, uint4* __re
 template <typename T, int NP, int LPR, bool QUANT>
 __global__ void layernorm_rows_vec_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, const float* __restrict__ gamma, const float* __restrict__ beta,
                                           int64_t rows, int pieces, float eps, uint2* __restrict__ qout, const float* __restrict__ qscale) {
+  dependency_wait();
   const QuantDiv qd(QUANT ? qscale[0] : 1.f);
   constexpr int RPW = 32 / LPR;
   const int lane = threadIdx.x & 31, l = lane % LPR;
@@ -545,9 +559,9 @@ bool launch_rows_vec(bool is_softmax, const void* x, void* y, const float* gamma
   const int grid = grid_for(rows * lpr, 256);
 #define B2_ROWS(NP, LPR)                                                                                                                      \
   do {                                                                                                                                        \
-    if (is_softmax) softmax_rows_vec_kernel<T, NP, LPR><<<grid, 256, 0, s>>>((const uint4*)x, (uint4*)y, rows, pieces, log_form);             \
-    else if (q) layernorm_rows_vec_kernel<T, NP, LPR, true><<<grid, 256, 0, s>>>((const uint4*)x, (uint4*)y, gamma, beta, rows, pieces, eps, (uint2*)q, qscale); \
-    else layernorm_rows_vec_kernel<T, NP, LPR, false><<<grid, 256, 0, s>>>((const uint4*)x, (uint4*)y, gamma, beta, rows, pieces, eps, nullptr, nullptr); \
+    if (is_softmax) launch(softmax_rows_vec_kernel<T, NP, LPR>, grid, 256, 0, s, (const uint4*)x, (uint4*)y, rows, pieces, log_form);             \
+    else if (q) launch(layernorm_rows_vec_kernel<T, NP, LPR, true>, grid, 256, 0, s, (const uint4*)x, (uint4*)y, gamma, beta, rows, pieces, eps, (uint2*)q, qscale); \
+    else launch(layernorm_rows_vec_kernel<T, NP, LPR, false>, grid, 256, 0, s, (const uint4*)x, (uint4*)y, gamma, beta, rows, pieces, eps, nullptr, nullptr); \
   } while (0)
   if (lpr == 8) B2_ROWS(1, 8);
   else if (lpr == 16) B2_ROWS(1, 16);
@@ -561,6 +575,7 @@ bool launch_rows_vec(bool is_softmax, const void* x, void* y, const float* gamma
 }
 // Strided axis: one thread per (outer, inner) pair.
 __global__ void softmax_strided_kernel(int dt, const void* x, void* y, int64_t outer, int64_t dim, int64_t inner, int log_form) {
+  dependency_wait();
   int64_t total = outer * inner;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     int64_t base = (e / inner) * dim * inner + e % inner;
@@ -575,6 +590,7 @@ __global__ void softmax_strided_kernel(int dt, const void* x, void* y, int64_t o
   }
 }
 __global__ void reduce_mean_axis_kernel(int dt_in, int dt_out, const void* x, void* y, int64_t before, int64_t dim, int64_t after) {
+  dependency_wait();
   int64_t total = before * after;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     int64_t i = e / after, k = e % after;
@@ -585,6 +601,7 @@ __global__ void reduce_mean_axis_kernel(int dt_in, int dt_out, const void* x, vo
 }
 __global__ void layernorm_kernel(int dt, const void* x, void* y, const float* gamma, const float* beta, int64_t rows, int64_t dim,
                                  float eps) {
+  dependency_wait();
   int lane = threadIdx.x & 31;
   int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5, nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t row = warp; row < rows; row += nwarps) {
@@ -605,6 +622,7 @@ __global__ void layernorm_kernel(int dt, const void* x, void* y, const float* ga
 // ------------------------------------------------------------- quantisation ----
 __global__ void quantize_kernel(int dt_in, const void* x, void* q, const float* scale, const int* zp, int64_t total, int64_t adim,
                                 int64_t inner, int per_axis, int is_unsigned) {
+  dependency_wait();
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     int a = per_axis ? (int)((e / inner) % adim) : 0;
     float r = rintf(__fdiv_rn(load_as_float(x, dt_in, e), scale[a]));
@@ -614,6 +632,7 @@ __global__ void quantize_kernel(int dt_in, const void* x, void* q, const float* 
 }
 // Per-tensor fp32 -> int8, 16 elements per thread (four 16-byte loads, one 16-byte store).
 __global__ void quantize_f32_s8_vec_kernel(const float4* __restrict__ x, uint4* __restrict__ q, const float* scale, int64_t n16) {
+  dependency_wait();
   const QuantDiv qd(scale[0]);
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n16; i += (int64_t)gridDim.x * blockDim.x) {
     uint4 out;
@@ -629,11 +648,13 @@ __global__ void quantize_f32_s8_vec_kernel(const float4* __restrict__ x, uint4* 
   }
 }
 __global__ void requantize_kernel(int dt_in, const void* x, int8_t* q, float inv, int64_t n) {
+  dependency_wait();
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x)
     q[e] = (int8_t)rne_sat_s8(__fmul_rn(load_as_float(x, dt_in, e), inv));
 }
 __global__ void dequantize_kernel(int dt_out, const void* q, void* x, const float* scale, const int* zp, int64_t total, int64_t adim,
                                   int64_t inner, int per_axis, int is_unsigned) {
+  dependency_wait();
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     int a = per_axis ? (int)((e / inner) % adim) : 0;
     float v = is_unsigned ? (float)((const uint8_t*)q)[e] : (float)((const int8_t*)q)[e];
@@ -642,6 +663,7 @@ __global__ void dequantize_kernel(int dt_out, const void* q, void* x, const floa
   }
 }
 __global__ void convert_kernel(int dt_in, int dt_out, const void* x, void* y, int64_t n) {
+  dependency_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     if (dt_in == DT_S64 && dt_out == DT_S32) { ((int32_t*)y)[i] = (int32_t)((const long long*)x)[i]; continue; }
     if (dt_in == DT_S32 && dt_out == DT_S64) { ((long long*)y)[i] = ((const int32_t*)x)[i]; continue; }
@@ -650,6 +672,7 @@ __global__ void convert_kernel(int dt_in, int dt_out, const void* x, void* y, in
 }
 // fp32 -> fp16, 8 elements per thread.
 __global__ void convert_f32_f16_vec_kernel(const float4* __restrict__ x, uint4* __restrict__ y, int64_t n8) {
+  dependency_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n8; i += (int64_t)gridDim.x * blockDim.x) {
     float4 a = x[2 * i], b = x[2 * i + 1];
     uint4 o;
@@ -663,6 +686,7 @@ __global__ void convert_f32_f16_vec_kernel(const float4* __restrict__ x, uint4* 
 // ------------------------------------------------------------- data movement ----
 template <typename T>
 __global__ void move_kernel(MoveGeom g, const T* __restrict__ x, T* __restrict__ y, int64_t total) {
+  dependency_wait();
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     int64_t rem = e, si = g.in_offset, di = g.out_offset;
     for (int d = g.rank - 1; d >= 0; --d) {
@@ -676,6 +700,7 @@ __global__ void move_kernel(MoveGeom g, const T* __restrict__ x, T* __restrict__
 }
 template <typename T>
 __global__ void pad_channels_kernel(const T* __restrict__ x, uint4* __restrict__ y, int64_t pixels, int C) {
+  dependency_wait();
   constexpr int CP = 32 / (int)sizeof(T);
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < pixels; p += (int64_t)gridDim.x * blockDim.x) {
     uint4 out[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
@@ -690,6 +715,7 @@ __global__ void pad_channels_kernel(const T* __restrict__ x, uint4* __restrict__
 }
 template <typename T>
 __global__ void stem_widen_kernel(const T* __restrict__ x, uint4* __restrict__ y, int N, int H, int W, int C, int Q) {
+  dependency_wait();
   constexpr int PER = 16 / (int)sizeof(T);       // elements per 16-byte piece
   constexpr int PIECES = 32 / PER;                // pieces per widened pixel (32 elements)
   const int64_t total = (int64_t)N * H * Q * PIECES;
@@ -712,6 +738,7 @@ __global__ void stem_widen_kernel(const T* __restrict__ x, uint4* __restrict__ y
 // to Wp pixels on the right.
 template <typename T, int CP>
 __global__ void stem_pad_kernel(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int W, int C, int lp, int Wp) {
+  dependency_wait();
   static_assert(sizeof(T) * CP == 4 || sizeof(T) * CP == 8 || sizeof(T) * CP == 16, "a padded pixel is 4, 8 or 16 bytes");
   const int64_t total = rows * Wp;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
@@ -732,6 +759,7 @@ __global__ void stem_pad_kernel(const T* __restrict__ x, T* __restrict__ y, int6
 }
 template <typename T>
 __global__ void resize_nearest_kernel(const T* __restrict__ x, T* __restrict__ y, int N, int H, int W, int C, int P, int Q, int nhwc) {
+  dependency_wait();
   int64_t total = (int64_t)N * P * Q * C;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     int c, q, p, n;
@@ -748,6 +776,7 @@ __global__ void resize_nearest_kernel(const T* __restrict__ x, T* __restrict__ y
 template <typename T>
 __global__ void gather_kernel(const T* __restrict__ x, const void* idx, int idx_dt, T* __restrict__ y, int64_t outer, int64_t axis_dim,
                               int64_t n_idx, int64_t inner) {
+  dependency_wait();
   int64_t total = outer * n_idx * inner;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     int64_t i = e % inner, k = (e / inner) % n_idx, o = e / (inner * n_idx);
@@ -766,10 +795,10 @@ int conv_simt(const ConvGeom& g, int in_dt, const void* x, const void* w, void* 
   if (total <= 0) return 0;
   int grid = grid_for(total, 256);
   switch (in_dt) {
-    case DT_F32: conv_direct_kernel<float, float><<<grid, 256, 0, s>>>(g, (const float*)x, (const float*)w, y, ep); break;
-    case DT_F16: conv_direct_kernel<__half, float><<<grid, 256, 0, s>>>(g, (const __half*)x, (const __half*)w, y, ep); break;
-    case DT_BF16: conv_direct_kernel<__nv_bfloat16, float><<<grid, 256, 0, s>>>(g, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, y, ep); break;
-    case DT_S8: conv_direct_kernel<int8_t, int><<<grid, 256, 0, s>>>(g, (const int8_t*)x, (const int8_t*)w, y, ep); break;
+    case DT_F32: launch(conv_direct_kernel<float, float>, grid, 256, 0, s, g, (const float*)x, (const float*)w, y, ep); break;
+    case DT_F16: launch(conv_direct_kernel<__half, float>, grid, 256, 0, s, g, (const __half*)x, (const __half*)w, y, ep); break;
+    case DT_BF16: launch(conv_direct_kernel<__nv_bfloat16, float>, grid, 256, 0, s, g, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, y, ep); break;
+    case DT_S8: launch(conv_direct_kernel<int8_t, int>, grid, 256, 0, s, g, (const int8_t*)x, (const int8_t*)w, y, ep); break;
     default: return -1;
   }
   return check_launch();
@@ -779,10 +808,10 @@ int gemm_simt(const GemmGeom& g, int in_dt, const void* A, const void* B, void* 
   if (total <= 0) return 0;
   int grid = grid_for(total, 256);
   switch (in_dt) {
-    case DT_F32: gemm_direct_kernel<float, float><<<grid, 256, 0, s>>>(g, (const float*)A, (const float*)B, C, ep); break;
-    case DT_F16: gemm_direct_kernel<__half, float><<<grid, 256, 0, s>>>(g, (const __half*)A, (const __half*)B, C, ep); break;
-    case DT_BF16: gemm_direct_kernel<__nv_bfloat16, float><<<grid, 256, 0, s>>>(g, (const __nv_bfloat16*)A, (const __nv_bfloat16*)B, C, ep); break;
-    case DT_S8: gemm_direct_kernel<int8_t, int><<<grid, 256, 0, s>>>(g, (const int8_t*)A, (const int8_t*)B, C, ep); break;
+    case DT_F32: launch(gemm_direct_kernel<float, float>, grid, 256, 0, s, g, (const float*)A, (const float*)B, C, ep); break;
+    case DT_F16: launch(gemm_direct_kernel<__half, float>, grid, 256, 0, s, g, (const __half*)A, (const __half*)B, C, ep); break;
+    case DT_BF16: launch(gemm_direct_kernel<__nv_bfloat16, float>, grid, 256, 0, s, g, (const __nv_bfloat16*)A, (const __nv_bfloat16*)B, C, ep); break;
+    case DT_S8: launch(gemm_direct_kernel<int8_t, int>, grid, 256, 0, s, g, (const int8_t*)A, (const int8_t*)B, C, ep); break;
     default: return -1;
   }
   return check_launch();
@@ -803,8 +832,8 @@ int pool2d(const PoolGeom& g, int dt, bool is_max, const void* x, void* y, cudaS
   if (is_max && nhwc_dense && aligned && g.H >= 1 && g.W >= 1 && ((g.R == 3 && g.S == 3) || (g.R == 2 && g.S == 2)) && !getenv("ODLA_B200_POOL_RUNTIME_WINDOW")) {
 #define B2_POOL_WIN(T, V)                                                                                                          \
     do {                                                                                                                           \
-      if (g.R == 3) maxpool_nhwc_win_kernel<T, V, 3, 3><<<pool_grid(g, V), 256, 0, s>>>(g, (const T*)x, (T*)y);                    \
-      else maxpool_nhwc_win_kernel<T, V, 2, 2><<<pool_grid(g, V), 256, 0, s>>>(g, (const T*)x, (T*)y);                             \
+      if (g.R == 3) launch(maxpool_nhwc_win_kernel<T, V, 3, 3>, pool_grid(g, V), 256, 0, s, g, (const T*)x, (T*)y);                    \
+      else launch(maxpool_nhwc_win_kernel<T, V, 2, 2>, pool_grid(g, V), 256, 0, s, g, (const T*)x, (T*)y);                             \
       return check_launch();                                                                                                       \
     } while (0)
     if (dt == DT_F16 && g.C % 8 == 0) B2_POOL_WIN(__half, 8);
@@ -814,22 +843,22 @@ int pool2d(const PoolGeom& g, int dt, bool is_max, const void* x, void* y, cudaS
 #undef B2_POOL_WIN
   }
   if (is_max && nhwc_dense && aligned) {
-    if (dt == DT_F16 && g.C % 8 == 0) { maxpool_nhwc_vec_kernel<__half, 8><<<pool_grid(g, 8), 256, 0, s>>>(g, (const __half*)x, (__half*)y); return check_launch(); }
-    if (dt == DT_BF16 && g.C % 8 == 0) { maxpool_nhwc_vec_kernel<__nv_bfloat16, 8><<<pool_grid(g, 8), 256, 0, s>>>(g, (const __nv_bfloat16*)x, (__nv_bfloat16*)y); return check_launch(); }
-    if (dt == DT_S8 && g.C % 16 == 0) { maxpool_nhwc_vec_kernel<int8_t, 16><<<pool_grid(g, 16), 256, 0, s>>>(g, (const int8_t*)x, (int8_t*)y); return check_launch(); }
-    if (dt == DT_F32 && g.C % 4 == 0) { maxpool_nhwc_vec_kernel<float, 4><<<pool_grid(g, 4), 256, 0, s>>>(g, (const float*)x, (float*)y); return check_launch(); }
+    if (dt == DT_F16 && g.C % 8 == 0) { launch(maxpool_nhwc_vec_kernel<__half, 8>, pool_grid(g, 8), 256, 0, s, g, (const __half*)x, (__half*)y); return check_launch(); }
+    if (dt == DT_BF16 && g.C % 8 == 0) { launch(maxpool_nhwc_vec_kernel<__nv_bfloat16, 8>, pool_grid(g, 8), 256, 0, s, g, (const __nv_bfloat16*)x, (__nv_bfloat16*)y); return check_launch(); }
+    if (dt == DT_S8 && g.C % 16 == 0) { launch(maxpool_nhwc_vec_kernel<int8_t, 16>, pool_grid(g, 16), 256, 0, s, g, (const int8_t*)x, (int8_t*)y); return check_launch(); }
+    if (dt == DT_F32 && g.C % 4 == 0) { launch(maxpool_nhwc_vec_kernel<float, 4>, pool_grid(g, 4), 256, 0, s, g, (const float*)x, (float*)y); return check_launch(); }
   }
-  if (is_max) pool_generic_kernel<true><<<grid_for(total, 256), 256, 0, s>>>(g, dt, x, y);
-  else pool_generic_kernel<false><<<grid_for(total, 256), 256, 0, s>>>(g, dt, x, y);
+  if (is_max) launch(pool_generic_kernel<true>, grid_for(total, 256), 256, 0, s, g, dt, x, y);
+  else launch(pool_generic_kernel<false>, grid_for(total, 256), 256, 0, s, g, dt, x, y);
   return check_launch();
 }
 int unary(int op, int dt_in, int dt_out, const void* x, void* y, int64_t n, float a, float b, cudaStream_t s) {
   if (n <= 0) return 0;
   if (dt_in == DT_F16 && dt_out == DT_F16 && n % 8 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)y % 16 == 0) {
-    unary_h8_kernel<<<grid_for(n / 8, 256), 256, 0, s>>>(op, (const uint4*)x, (uint4*)y, n / 8, a, b);
+    launch(unary_h8_kernel, grid_for(n / 8, 256), 256, 0, s, op, (const uint4*)x, (uint4*)y, n / 8, a, b);
     return check_launch();
   }
-  unary_kernel<<<grid_for(n, 256), 256, 0, s>>>(op, dt_in, dt_out, x, y, n, a, b);
+  launch(unary_kernel, grid_for(n, 256), 256, 0, s, op, dt_in, dt_out, x, y, n, a, b);
   return check_launch();
 }
 int binary(int op, const BinaryGeom& g, int dt_l, int dt_r, int dt_out, const void* l, const void* r, void* y, int act, float act_a,
@@ -845,7 +874,7 @@ int binary(int op, const BinaryGeom& g, int dt_l, int dt_r, int dt_out, const vo
   if (total <= 0) return 0;
   if (same && dt_l == DT_F16 && dt_r == DT_F16 && dt_out == DT_F16 && total % 8 == 0 && (uintptr_t)l % 16 == 0 &&
       (uintptr_t)r % 16 == 0 && (uintptr_t)y % 16 == 0) {
-    binary_same_h8_kernel<<<grid_for(total / 8, 256), 256, 0, s>>>(op, (const uint4*)l, (const uint4*)r, (uint4*)y, total / 8, act, act_a);
+    launch(binary_same_h8_kernel, grid_for(total / 8, 256), 256, 0, s, op, (const uint4*)l, (const uint4*)r, (uint4*)y, total / 8, act, act_a);
     return check_launch();
   }
   // left operand dense, right operand a broadcast over the leading dims (zero strides there, dense strides after)
@@ -862,20 +891,20 @@ int binary(int op, const BinaryGeom& g, int dt_l, int dt_r, int dt_out, const vo
     }
     if (l_dense && r_suffix && period % 8 == 0 && period >= 8) {
       const int grid = grid_for(total / 8, 256);
-      if (dt_out == DT_F16 && dt_r == DT_F16) binary_period_vec_kernel<__half, __half><<<grid, 256, 0, s>>>(op, (const uint4*)l, (const __half*)r, (uint4*)y, total / 8, period / 8, act, act_a);
-      else if (dt_out == DT_F16) binary_period_vec_kernel<__half, float><<<grid, 256, 0, s>>>(op, (const uint4*)l, (const float*)r, (uint4*)y, total / 8, period / 8, act, act_a);
-      else if (dt_r == DT_BF16) binary_period_vec_kernel<__nv_bfloat16, __nv_bfloat16><<<grid, 256, 0, s>>>(op, (const uint4*)l, (const __nv_bfloat16*)r, (uint4*)y, total / 8, period / 8, act, act_a);
-      else binary_period_vec_kernel<__nv_bfloat16, float><<<grid, 256, 0, s>>>(op, (const uint4*)l, (const float*)r, (uint4*)y, total / 8, period / 8, act, act_a);
+      if (dt_out == DT_F16 && dt_r == DT_F16) launch(binary_period_vec_kernel<__half, __half>, grid, 256, 0, s, op, (const uint4*)l, (const __half*)r, (uint4*)y, total / 8, period / 8, act, act_a);
+      else if (dt_out == DT_F16) launch(binary_period_vec_kernel<__half, float>, grid, 256, 0, s, op, (const uint4*)l, (const float*)r, (uint4*)y, total / 8, period / 8, act, act_a);
+      else if (dt_r == DT_BF16) launch(binary_period_vec_kernel<__nv_bfloat16, __nv_bfloat16>, grid, 256, 0, s, op, (const uint4*)l, (const __nv_bfloat16*)r, (uint4*)y, total / 8, period / 8, act, act_a);
+      else launch(binary_period_vec_kernel<__nv_bfloat16, float>, grid, 256, 0, s, op, (const uint4*)l, (const float*)r, (uint4*)y, total / 8, period / 8, act, act_a);
       return check_launch();
     }
   }
-  binary_kernel<<<grid_for(total, 256), 256, 0, s>>>(op, g, dt_l, dt_r, dt_out, l, r, y, total, act, act_a);
+  launch(binary_kernel, grid_for(total, 256), 256, 0, s, op, g, dt_l, dt_r, dt_out, l, r, y, total, act, act_a);
   return check_launch();
 }
 int channel_affine(int dt, const void* x, void* y, const float* a, const float* b, int64_t outer, int64_t C, int64_t inner, cudaStream_t s) {
   int64_t total = outer * C * inner;
   if (total <= 0) return 0;
-  channel_affine_kernel<<<grid_for(total, 256), 256, 0, s>>>(dt, x, y, a, b, total, C, inner);
+  launch(channel_affine_kernel, grid_for(total, 256), 256, 0, s, dt, x, y, a, b, total, C, inner);
   return check_launch();
 }
 // fp32 rows of up to 32 * NP elements, one warp per row: the row is read once into registers (lane l holds elements
@@ -883,6 +912,7 @@ int channel_affine(int dt, const void* x, void* y, const float* a, const float* 
 template <int NP, bool SOFTMAX>
 __global__ void rows_f32_reg_kernel(const float* __restrict__ x, float* __restrict__ y, const float* __restrict__ gamma, const float* __restrict__ beta,
                                     int64_t rows, int dim, float eps, int log_form) {
+  dependency_wait();
   const int lane = threadIdx.x & 31;
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5, nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t row = warp; row < rows; row += nwarps) {
@@ -929,8 +959,8 @@ static bool launch_rows_f32(bool is_softmax, const void* x, void* y, const float
   const int grid = grid_for(rows * 32, 128);
 #define B2_ROWS32(NP)                                                                                                                              \
   do {                                                                                                                                             \
-    if (is_softmax) rows_f32_reg_kernel<NP, true><<<grid, 128, 0, s>>>((const float*)x, (float*)y, gamma, beta, rows, (int)dim, eps, log_form);     \
-    else rows_f32_reg_kernel<NP, false><<<grid, 128, 0, s>>>((const float*)x, (float*)y, gamma, beta, rows, (int)dim, eps, log_form);               \
+    if (is_softmax) launch(rows_f32_reg_kernel<NP, true>, grid, 128, 0, s, (const float*)x, (float*)y, gamma, beta, rows, (int)dim, eps, log_form);     \
+    else launch(rows_f32_reg_kernel<NP, false>, grid, 128, 0, s, (const float*)x, (float*)y, gamma, beta, rows, (int)dim, eps, log_form);               \
   } while (0)
   if (dim <= 128) B2_ROWS32(4);
   else if (dim <= 512) B2_ROWS32(16);
@@ -944,8 +974,8 @@ int softmax(int dt, const void* x, void* y, int64_t outer, int64_t dim, int64_t 
   if (inner == 1 && dt == DT_F32 && launch_rows_f32(true, x, y, nullptr, nullptr, outer, dim, 0.f, log_form, s)) return check_launch();
   if (inner == 1 && dt == DT_F16 && launch_rows_vec<__half>(true, x, y, nullptr, nullptr, outer, dim, 0.f, log_form, s)) return check_launch();
   if (inner == 1 && dt == DT_BF16 && launch_rows_vec<__nv_bfloat16>(true, x, y, nullptr, nullptr, outer, dim, 0.f, log_form, s)) return check_launch();
-  if (inner == 1) softmax_rows_kernel<<<grid_for(outer * 32, 256), 256, 0, s>>>(dt, x, y, outer, dim, log_form);
-  else softmax_strided_kernel<<<grid_for(outer * inner, 128), 128, 0, s>>>(dt, x, y, outer, dim, inner, log_form);
+  if (inner == 1) launch(softmax_rows_kernel, grid_for(outer * 32, 256), 256, 0, s, dt, x, y, outer, dim, log_form);
+  else launch(softmax_strided_kernel, grid_for(outer * inner, 128), 128, 0, s, dt, x, y, outer, dim, inner, log_form);
   return check_launch();
 }
 // Mean along one axis with 16-byte loads across the kept inner axis: a thread owns VEC neighbouring outputs and adds
@@ -961,6 +991,7 @@ template <typename IN> __device__ __forceinline__ void red_load(const IN* p, flo
 }
 template <typename IN>
 __global__ void reduce_mean_axis_vec_kernel(int dt_out, const IN* __restrict__ x, void* __restrict__ y, int64_t before, int64_t dim, int64_t after, float in_scale) {
+  dependency_wait();
   constexpr int VEC = RedVec<IN>::N;
   const int64_t av = after / VEC, total = before * av;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
@@ -983,6 +1014,7 @@ __global__ void reduce_mean_axis_vec_kernel(int dt_out, const IN* __restrict__ x
 // right and divided.  All D1 * D2 loads of a thread are independent, so they overlap instead of waiting in a loop.
 template <typename IN, int D1, int D2>
 __global__ void reduce_mean_two_axes_kernel(int dt_out, const IN* __restrict__ x, void* __restrict__ y, int64_t before, int64_t after, float in_scale) {
+  dependency_wait();
   constexpr int VEC = RedVec<IN>::N;
   const int64_t av = after / VEC, total = before * av;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
@@ -1014,13 +1046,14 @@ int reduce_mean_two_axes(int dt_in, int dt_out, const void* x, void* y, int64_t 
   if (d1 != 7 || d2 != 7 || after % vec != 0 || (uintptr_t)x % 16 != 0 || before * after <= 0) return 1;   // not taken: the caller runs the two passes
   if (!(dt_in == DT_F32 || dt_in == DT_F16 || dt_in == DT_BF16 || dt_in == DT_S8)) return 1;
   const int grid = grid_for(before * (after / vec), 128);
-  if (dt_in == DT_F32) reduce_mean_two_axes_kernel<float, 7, 7><<<grid, 128, 0, s>>>(dt_out, (const float*)x, y, before, after, in_scale);
-  else if (dt_in == DT_F16) reduce_mean_two_axes_kernel<__half, 7, 7><<<grid, 128, 0, s>>>(dt_out, (const __half*)x, y, before, after, in_scale);
-  else if (dt_in == DT_BF16) reduce_mean_two_axes_kernel<__nv_bfloat16, 7, 7><<<grid, 128, 0, s>>>(dt_out, (const __nv_bfloat16*)x, y, before, after, in_scale);
-  else reduce_mean_two_axes_kernel<int8_t, 7, 7><<<grid, 128, 0, s>>>(dt_out, (const int8_t*)x, y, before, after, in_scale);
+  if (dt_in == DT_F32) launch(reduce_mean_two_axes_kernel<float, 7, 7>, grid, 128, 0, s, dt_out, (const float*)x, y, before, after, in_scale);
+  else if (dt_in == DT_F16) launch(reduce_mean_two_axes_kernel<__half, 7, 7>, grid, 128, 0, s, dt_out, (const __half*)x, y, before, after, in_scale);
+  else if (dt_in == DT_BF16) launch(reduce_mean_two_axes_kernel<__nv_bfloat16, 7, 7>, grid, 128, 0, s, dt_out, (const __nv_bfloat16*)x, y, before, after, in_scale);
+  else launch(reduce_mean_two_axes_kernel<int8_t, 7, 7>, grid, 128, 0, s, dt_out, (const int8_t*)x, y, before, after, in_scale);
   return check_launch();
 }
 __global__ void reduce_mean_axis_s8_kernel(int dt_out, const int8_t* x, void* y, int64_t before, int64_t dim, int64_t after, float in_scale) {
+  dependency_wait();
   int64_t total = before * after;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     int64_t i = e / after, k = e % after;
@@ -1035,14 +1068,14 @@ int reduce_mean_axis(int dt_in, int dt_out, const void* x, void* y, int64_t befo
   if ((dt_in == DT_F32 || dt_in == DT_F16 || dt_in == DT_BF16 || dt_in == DT_S8) && after % vec == 0 && (uintptr_t)x % 16 == 0) {
     const int64_t work = before * (after / vec);
     const int grid = grid_for(work, 128);
-    if (dt_in == DT_F32) reduce_mean_axis_vec_kernel<float><<<grid, 128, 0, s>>>(dt_out, (const float*)x, y, before, dim, after, in_scale);
-    else if (dt_in == DT_F16) reduce_mean_axis_vec_kernel<__half><<<grid, 128, 0, s>>>(dt_out, (const __half*)x, y, before, dim, after, in_scale);
-    else if (dt_in == DT_BF16) reduce_mean_axis_vec_kernel<__nv_bfloat16><<<grid, 128, 0, s>>>(dt_out, (const __nv_bfloat16*)x, y, before, dim, after, in_scale);
-    else reduce_mean_axis_vec_kernel<int8_t><<<grid, 128, 0, s>>>(dt_out, (const int8_t*)x, y, before, dim, after, in_scale);
+    if (dt_in == DT_F32) launch(reduce_mean_axis_vec_kernel<float>, grid, 128, 0, s, dt_out, (const float*)x, y, before, dim, after, in_scale);
+    else if (dt_in == DT_F16) launch(reduce_mean_axis_vec_kernel<__half>, grid, 128, 0, s, dt_out, (const __half*)x, y, before, dim, after, in_scale);
+    else if (dt_in == DT_BF16) launch(reduce_mean_axis_vec_kernel<__nv_bfloat16>, grid, 128, 0, s, dt_out, (const __nv_bfloat16*)x, y, before, dim, after, in_scale);
+    else launch(reduce_mean_axis_vec_kernel<int8_t>, grid, 128, 0, s, dt_out, (const int8_t*)x, y, before, dim, after, in_scale);
     return check_launch();
   }
-  if (dt_in == DT_S8) reduce_mean_axis_s8_kernel<<<grid_for(before * after, 128), 128, 0, s>>>(dt_out, (const int8_t*)x, y, before, dim, after, in_scale);
-  else reduce_mean_axis_kernel<<<grid_for(before * after, 128), 128, 0, s>>>(dt_in, dt_out, x, y, before, dim, after);
+  if (dt_in == DT_S8) launch(reduce_mean_axis_s8_kernel, grid_for(before * after, 128), 128, 0, s, dt_out, (const int8_t*)x, y, before, dim, after, in_scale);
+  else launch(reduce_mean_axis_kernel, grid_for(before * after, 128), 128, 0, s, dt_in, dt_out, x, y, before, dim, after);
   return check_launch();
 }
 int layernorm(int dt, const void* x, void* y, const float* gamma, const float* beta, int64_t rows, int64_t dim, float eps, cudaStream_t s) {
@@ -1050,7 +1083,7 @@ int layernorm(int dt, const void* x, void* y, const float* gamma, const float* b
   if (dt == DT_F16 && launch_rows_vec<__half>(false, x, y, gamma, beta, rows, dim, eps, 0, s)) return check_launch();
   if (dt == DT_BF16 && launch_rows_vec<__nv_bfloat16>(false, x, y, gamma, beta, rows, dim, eps, 0, s)) return check_launch();
   if (dt == DT_F32 && launch_rows_f32(false, x, y, gamma, beta, rows, dim, eps, 0, s)) return check_launch();
-  layernorm_kernel<<<grid_for(rows * 32, 256), 256, 0, s>>>(dt, x, y, gamma, beta, rows, dim, eps);
+  launch(layernorm_kernel, grid_for(rows * 32, 256), 256, 0, s, dt, x, y, gamma, beta, rows, dim, eps);
   return check_launch();
 }
 int quantize(int dt_in, const void* x, void* q, const float* scale, const int* zp, int64_t outer, int64_t adim, int64_t inner,
@@ -1067,6 +1100,7 @@ int layernorm_quantize(int dt, const void* x, void* y, const float* gamma, const
 // Per-tensor two-byte float -> int8, 16 elements per thread (two 16-byte loads, one 16-byte store).
 template <typename T>
 __global__ void quantize_h_s8_vec_kernel(const uint4* __restrict__ x, uint4* __restrict__ q, const float* scale, int64_t n16) {
+  dependency_wait();
   const QuantDiv qd(scale[0]);
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n16; i += (int64_t)gridDim.x * blockDim.x) {
     uint4 out;
@@ -1091,20 +1125,21 @@ int quantize(int dt_in, const void* x, void* q, const float* scale, const int* z
   int64_t total = outer * adim * inner;
   if (total <= 0) return 0;
   if (dt_in == DT_F32 && !per_axis && !zp && !is_unsigned && total % 16 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)q % 16 == 0) {
-    quantize_f32_s8_vec_kernel<<<grid_for(total / 16, 256), 256, 0, s>>>((const float4*)x, (uint4*)q, scale, total / 16);
+    launch(quantize_f32_s8_vec_kernel, grid_for(total / 16, 256), 256, 0, s, (const float4*)x, (uint4*)q, scale, total / 16);
     return check_launch();
   }
   if ((dt_in == DT_F16 || dt_in == DT_BF16) && !per_axis && !zp && !is_unsigned && total % 16 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)q % 16 == 0) {
-    if (dt_in == DT_F16) quantize_h_s8_vec_kernel<__half><<<grid_for(total / 16, 256), 256, 0, s>>>((const uint4*)x, (uint4*)q, scale, total / 16);
-    else quantize_h_s8_vec_kernel<__nv_bfloat16><<<grid_for(total / 16, 256), 256, 0, s>>>((const uint4*)x, (uint4*)q, scale, total / 16);
+    if (dt_in == DT_F16) launch(quantize_h_s8_vec_kernel<__half>, grid_for(total / 16, 256), 256, 0, s, (const uint4*)x, (uint4*)q, scale, total / 16);
+    else launch(quantize_h_s8_vec_kernel<__nv_bfloat16>, grid_for(total / 16, 256), 256, 0, s, (const uint4*)x, (uint4*)q, scale, total / 16);
     return check_launch();
   }
-  quantize_kernel<<<grid_for(total, 256), 256, 0, s>>>(dt_in, x, q, scale, zp, total, adim, inner, per_axis, is_unsigned);
+  launch(quantize_kernel, grid_for(total, 256), 256, 0, s, dt_in, x, q, scale, zp, total, adim, inner, per_axis, is_unsigned);
   return check_launch();
 }
 // Per-tensor int8 -> float storage type, 16 elements per thread: x = fl(float(q) * scale), one rounding to the storage type.
 template <typename OUT>
 __global__ void dequantize_s8_vec_kernel(const uint4* __restrict__ q, OUT* __restrict__ x, const float* __restrict__ scale, int64_t n16) {
+  dependency_wait();
   const float s = scale[0];
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n16; i += (int64_t)gridDim.x * blockDim.x) {
     const uint4 u = q[i];
@@ -1126,6 +1161,7 @@ __global__ void dequantize_s8_vec_kernel(const uint4* __restrict__ q, OUT* __res
 // Requantisation of a value computed from int32 accumulators: q = sat(rne(x * inv)), 16 elements per thread.
 template <typename IN>
 __global__ void requantize_vec_kernel(const IN* __restrict__ x, uint4* __restrict__ q, float inv, int64_t n16) {
+  dependency_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n16; i += (int64_t)gridDim.x * blockDim.x) {
     float f[16];
     if constexpr (sizeof(IN) == 4) {
@@ -1155,12 +1191,12 @@ int requantize(int dt_in, const void* x, void* q, float inv_scale, int64_t n, cu
   if (n <= 0) return 0;
   if (n % 16 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)q % 16 == 0 && (dt_in == DT_F32 || dt_in == DT_F16 || dt_in == DT_BF16)) {
     const int grid = grid_for(n / 16, 256);
-    if (dt_in == DT_F32) requantize_vec_kernel<float><<<grid, 256, 0, s>>>((const float*)x, (uint4*)q, inv_scale, n / 16);
-    else if (dt_in == DT_F16) requantize_vec_kernel<__half><<<grid, 256, 0, s>>>((const __half*)x, (uint4*)q, inv_scale, n / 16);
-    else requantize_vec_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>((const __nv_bfloat16*)x, (uint4*)q, inv_scale, n / 16);
+    if (dt_in == DT_F32) launch(requantize_vec_kernel<float>, grid, 256, 0, s, (const float*)x, (uint4*)q, inv_scale, n / 16);
+    else if (dt_in == DT_F16) launch(requantize_vec_kernel<__half>, grid, 256, 0, s, (const __half*)x, (uint4*)q, inv_scale, n / 16);
+    else launch(requantize_vec_kernel<__nv_bfloat16>, grid, 256, 0, s, (const __nv_bfloat16*)x, (uint4*)q, inv_scale, n / 16);
     return check_launch();
   }
-  requantize_kernel<<<grid_for(n, 256), 256, 0, s>>>(dt_in, x, (int8_t*)q, inv_scale, n);
+  launch(requantize_kernel, grid_for(n, 256), 256, 0, s, dt_in, x, (int8_t*)q, inv_scale, n);
   return check_launch();
 }
 int dequantize(int dt_out, const void* q, void* x, const float* scale, const int* zp, int64_t outer, int64_t adim, int64_t inner,
@@ -1170,27 +1206,28 @@ int dequantize(int dt_out, const void* q, void* x, const float* scale, const int
   if (!per_axis && !zp && !is_unsigned && total % 16 == 0 && (uintptr_t)q % 16 == 0 && (uintptr_t)x % 16 == 0 &&
       (dt_out == DT_F32 || dt_out == DT_F16 || dt_out == DT_BF16)) {
     const int grid = grid_for(total / 16, 256);
-    if (dt_out == DT_F32) dequantize_s8_vec_kernel<float><<<grid, 256, 0, s>>>((const uint4*)q, (float*)x, scale, total / 16);
-    else if (dt_out == DT_F16) dequantize_s8_vec_kernel<__half><<<grid, 256, 0, s>>>((const uint4*)q, (__half*)x, scale, total / 16);
-    else dequantize_s8_vec_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>((const uint4*)q, (__nv_bfloat16*)x, scale, total / 16);
+    if (dt_out == DT_F32) launch(dequantize_s8_vec_kernel<float>, grid, 256, 0, s, (const uint4*)q, (float*)x, scale, total / 16);
+    else if (dt_out == DT_F16) launch(dequantize_s8_vec_kernel<__half>, grid, 256, 0, s, (const uint4*)q, (__half*)x, scale, total / 16);
+    else launch(dequantize_s8_vec_kernel<__nv_bfloat16>, grid, 256, 0, s, (const uint4*)q, (__nv_bfloat16*)x, scale, total / 16);
     return check_launch();
   }
-  dequantize_kernel<<<grid_for(total, 256), 256, 0, s>>>(dt_out, q, x, scale, zp, total, adim, inner, per_axis, is_unsigned);
+  launch(dequantize_kernel, grid_for(total, 256), 256, 0, s, dt_out, q, x, scale, zp, total, adim, inner, per_axis, is_unsigned);
   return check_launch();
 }
 int convert(int dt_in, int dt_out, const void* x, void* y, int64_t n, cudaStream_t s) {
   if (n <= 0) return 0;
   if (dt_in == DT_F32 && dt_out == DT_F16 && n % 8 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)y % 16 == 0) {
-    convert_f32_f16_vec_kernel<<<grid_for(n / 8, 256), 256, 0, s>>>((const float4*)x, (uint4*)y, n / 8);
+    launch(convert_f32_f16_vec_kernel, grid_for(n / 8, 256), 256, 0, s, (const float4*)x, (uint4*)y, n / 8);
     return check_launch();
   }
   // two-byte -> fp32 (an fp16 / bf16 graph whose API outputs are fp32): four values per thread, as one long row
   if ((dt_in == DT_F16 || dt_in == DT_BF16) && dt_out == DT_F32 && n % 4 == 0 && n < (1 << 30) && (uintptr_t)x % 8 == 0 && (uintptr_t)y % 16 == 0)
     return convert_rows(dt_in, dt_out, x, y, 1, n, n, s);
-  convert_kernel<<<grid_for(n, 256), 256, 0, s>>>(dt_in, dt_out, x, y, n);
+  launch(convert_kernel, grid_for(n, 256), 256, 0, s, dt_in, dt_out, x, y, n);
   return check_launch();
 }
 __global__ void convert_rows_kernel(int dt_in, int dt_out, const void* x, void* y, int64_t rows, int64_t K, int64_t Kp) {
+  dependency_wait();
   const int64_t total = rows * K;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = e / K, k = e - r * K;
@@ -1201,6 +1238,7 @@ __global__ void convert_rows_kernel(int dt_in, int dt_out, const void* x, void* 
 // one contiguous run): four values per thread as one 16-byte store when the rows allow it, one value per thread otherwise.
 template <typename IN>
 __global__ void convert_rows_h_f32_v4_kernel(const IN* __restrict__ x, float4* __restrict__ y, int64_t total4, int K4, int64_t Kp) {
+  dependency_wait();
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total4; e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = e / K4;
     const int k = (int)(e - r * K4) * 4;
@@ -1211,6 +1249,7 @@ __global__ void convert_rows_h_f32_v4_kernel(const IN* __restrict__ x, float4* _
 }
 template <typename IN>
 __global__ void convert_rows_h_f32_flat_kernel(const IN* __restrict__ x, float* __restrict__ y, int64_t total, int K, int64_t Kp) {
+  dependency_wait();
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = e / K;
     y[e] = (float)x[r * Kp + (e - r * K)];
@@ -1223,28 +1262,30 @@ int convert_rows(int dt_in, int dt_out, const void* x, void* y, int64_t rows, in
     if (v4) {
       const int64_t total4 = rows * (K / 4);
       const int grid = grid_for(total4, 256);
-      if (dt_in == DT_F16) convert_rows_h_f32_v4_kernel<__half><<<grid, 256, 0, s>>>((const __half*)x, (float4*)y, total4, (int)(K / 4), Kp);
-      else convert_rows_h_f32_v4_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>((const __nv_bfloat16*)x, (float4*)y, total4, (int)(K / 4), Kp);
+      if (dt_in == DT_F16) launch(convert_rows_h_f32_v4_kernel<__half>, grid, 256, 0, s, (const __half*)x, (float4*)y, total4, (int)(K / 4), Kp);
+      else launch(convert_rows_h_f32_v4_kernel<__nv_bfloat16>, grid, 256, 0, s, (const __nv_bfloat16*)x, (float4*)y, total4, (int)(K / 4), Kp);
     } else {
       const int grid = grid_for(rows * K, 256);
-      if (dt_in == DT_F16) convert_rows_h_f32_flat_kernel<__half><<<grid, 256, 0, s>>>((const __half*)x, (float*)y, rows * K, (int)K, Kp);
-      else convert_rows_h_f32_flat_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>((const __nv_bfloat16*)x, (float*)y, rows * K, (int)K, Kp);
+      if (dt_in == DT_F16) launch(convert_rows_h_f32_flat_kernel<__half>, grid, 256, 0, s, (const __half*)x, (float*)y, rows * K, (int)K, Kp);
+      else launch(convert_rows_h_f32_flat_kernel<__nv_bfloat16>, grid, 256, 0, s, (const __nv_bfloat16*)x, (float*)y, rows * K, (int)K, Kp);
     }
     return check_launch();
   }
-  convert_rows_kernel<<<grid_for(rows * K, 256), 256, 0, s>>>(dt_in, dt_out, x, y, rows, K, Kp);
+  launch(convert_rows_kernel, grid_for(rows * K, 256), 256, 0, s, dt_in, dt_out, x, y, rows, K, Kp);
   return check_launch();
 }
 // ---- range profiling: min / max per tensor and per channel (last axis) ----
 // A float maps to an unsigned key that orders the same way (sign bit flipped for positives, all bits for negatives).
 __device__ __forceinline__ unsigned range_key(float f) { const unsigned b = __float_as_uint(f); return (b & 0x80000000u) ? ~b : (b | 0x80000000u); }
 __global__ void range_reset_kernel(unsigned* stats, int64_t channels) {
+  dependency_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < 2 + 2 * channels; i += (int64_t)gridDim.x * blockDim.x)
     stats[i] = (i == 0 || (i >= 2 && i < 2 + channels)) ? 0xffffffffu : 0u;   // minima start at the largest key, maxima at the smallest
 }
 // A block takes a contiguous run of rows; thread t keeps channels t, t + 256, ... (up to 16 of them) in registers and
 // publishes them with one atomic pair per channel at the end.
 __global__ void range_minmax_kernel(int dt, const void* __restrict__ x, int64_t rows, int channels, unsigned* __restrict__ stats) {
+  dependency_wait();
   const int64_t per_block = (rows + gridDim.x - 1) / gridDim.x, r0 = blockIdx.x * per_block, r1 = min(rows, r0 + per_block);
   for (int c0 = 0; c0 < channels; c0 += 16 * blockDim.x) {
     float mn[16], mx[16];
@@ -1270,7 +1311,7 @@ __global__ void range_minmax_kernel(int dt, const void* __restrict__ x, int64_t 
   }
 }
 int range_stats_reset(unsigned* stats, int64_t channels, cudaStream_t s) {
-  range_reset_kernel<<<grid_for(2 + 2 * channels, 256), 256, 0, s>>>(stats, channels);
+  launch(range_reset_kernel, grid_for(2 + 2 * channels, 256), 256, 0, s, stats, channels);
   return check_launch();
 }
 int range_minmax(int dt, const void* x, int64_t count, int64_t channels, unsigned* stats, cudaStream_t s) {
@@ -1278,13 +1319,14 @@ int range_minmax(int dt, const void* x, int64_t count, int64_t channels, unsigne
   if (dt != DT_F32 && dt != DT_F16 && dt != DT_BF16) return 0;
   const int64_t rows = count / channels;
   int grid = (int)std::min<int64_t>(rows, (int64_t)sm_count() * 8);
-  range_minmax_kernel<<<grid > 0 ? grid : 1, 256, 0, s>>>(dt, x, rows, (int)channels, stats);
+  launch(range_minmax_kernel, grid > 0 ? grid : 1, 256, 0, s, dt, x, rows, (int)channels, stats);
   return check_launch();
 }
 // out[b][n][k] = in[b][k][n]: the last two axes swapped, through 32 x 32 shared-memory tiles so that both the reads
 // (along n) and the writes (along k) are contiguous.
 template <typename T>
 __global__ void transpose_last2_kernel(const T* __restrict__ x, T* __restrict__ y, int64_t in_off, int64_t out_off, int N, int K, int tiles_n, int tiles_k) {
+  dependency_wait();
   __shared__ T tile[32][33];
   const int64_t b = blockIdx.x / (tiles_n * tiles_k);
   const int t = (int)(blockIdx.x % (tiles_n * tiles_k));
@@ -1313,7 +1355,7 @@ static bool launch_transpose_last2(const MoveGeom& g, const void* x, void* y, cu
   const int tn = (int)((N + 31) / 32), tk = (int)((K + 31) / 32);
   const int64_t blocks = B * tn * tk;
   if (blocks <= 0 || blocks > 0x7fffffffLL) return false;
-  transpose_last2_kernel<T><<<(unsigned)blocks, dim3(32, 8), 0, s>>>((const T*)x, (T*)y, g.in_offset, g.out_offset, (int)N, (int)K, tn, tk);
+  launch(transpose_last2_kernel<T>, (unsigned)blocks, dim3(32, 8), 0, s, (const T*)x, (T*)y, g.in_offset, g.out_offset, (int)N, (int)K, tn, tk);
   return true;
 }
 int move(const MoveGeom& g0, int esz, const void* x, void* y, cudaStream_t s) {
@@ -1361,11 +1403,11 @@ int move(const MoveGeom& g0, int esz, const void* x, void* y, cudaStream_t s) {
   if (total <= 0) return 0;
   int grid = grid_for(total, 256);
   switch (esz) {
-    case 16: move_kernel<uint4><<<grid, 256, 0, s>>>(g, (const uint4*)x, (uint4*)y, total); break;
-    case 1: move_kernel<uint8_t><<<grid, 256, 0, s>>>(g, (const uint8_t*)x, (uint8_t*)y, total); break;
-    case 2: move_kernel<uint16_t><<<grid, 256, 0, s>>>(g, (const uint16_t*)x, (uint16_t*)y, total); break;
-    case 4: move_kernel<uint32_t><<<grid, 256, 0, s>>>(g, (const uint32_t*)x, (uint32_t*)y, total); break;
-    case 8: move_kernel<uint64_t><<<grid, 256, 0, s>>>(g, (const uint64_t*)x, (uint64_t*)y, total); break;
+    case 16: launch(move_kernel<uint4>, grid, 256, 0, s, g, (const uint4*)x, (uint4*)y, total); break;
+    case 1: launch(move_kernel<uint8_t>, grid, 256, 0, s, g, (const uint8_t*)x, (uint8_t*)y, total); break;
+    case 2: launch(move_kernel<uint16_t>, grid, 256, 0, s, g, (const uint16_t*)x, (uint16_t*)y, total); break;
+    case 4: launch(move_kernel<uint32_t>, grid, 256, 0, s, g, (const uint32_t*)x, (uint32_t*)y, total); break;
+    case 8: launch(move_kernel<uint64_t>, grid, 256, 0, s, g, (const uint64_t*)x, (uint64_t*)y, total); break;
     default: return -1;
   }
   return check_launch();
@@ -1374,8 +1416,8 @@ int pad_channels(int esz, const void* x, void* y, int64_t pixels, int C, int Cp,
   if (pixels <= 0) return 0;
   if (Cp * esz != 32 || C > Cp || (uintptr_t)y % 16 != 0) return -1;
   int grid = grid_for(pixels, 256);
-  if (esz == 1) pad_channels_kernel<uint8_t><<<grid, 256, 0, s>>>((const uint8_t*)x, (uint4*)y, pixels, C);
-  else if (esz == 2) pad_channels_kernel<uint16_t><<<grid, 256, 0, s>>>((const uint16_t*)x, (uint4*)y, pixels, C);
+  if (esz == 1) launch(pad_channels_kernel<uint8_t>, grid, 256, 0, s, (const uint8_t*)x, (uint4*)y, pixels, C);
+  else if (esz == 2) launch(pad_channels_kernel<uint16_t>, grid, 256, 0, s, (const uint16_t*)x, (uint4*)y, pixels, C);
   else return -1;
   return check_launch();
 }
@@ -1384,8 +1426,8 @@ int stem_widen(int esz, const void* x, void* y, int N, int H, int W, int C, int 
   if (total <= 0) return 0;
   if (C > 4 || (uintptr_t)y % 16 != 0) return -1;
   int grid = grid_for(total, 256);
-  if (esz == 1) stem_widen_kernel<uint8_t><<<grid, 256, 0, s>>>((const uint8_t*)x, (uint4*)y, N, H, W, C, Q);
-  else if (esz == 2) stem_widen_kernel<uint16_t><<<grid, 256, 0, s>>>((const uint16_t*)x, (uint4*)y, N, H, W, C, Q);
+  if (esz == 1) launch(stem_widen_kernel<uint8_t>, grid, 256, 0, s, (const uint8_t*)x, (uint4*)y, N, H, W, C, Q);
+  else if (esz == 2) launch(stem_widen_kernel<uint16_t>, grid, 256, 0, s, (const uint16_t*)x, (uint4*)y, N, H, W, C, Q);
   else return -1;
   return check_launch();
 }
@@ -1395,11 +1437,11 @@ int stem_pad(int esz, const void* x, void* y, int N, int H, int W, int C, int pi
   const int cp = pixel_bytes / esz;
   if (C > cp || (uintptr_t)y % 16 != 0) return -1;
   int grid = grid_for(total, 256);
-  if (esz == 1 && cp == 4) stem_pad_kernel<uint8_t, 4><<<grid, 256, 0, s>>>((const uint8_t*)x, (uint8_t*)y, rows, W, C, lp, Wp);
-  else if (esz == 1 && cp == 8) stem_pad_kernel<uint8_t, 8><<<grid, 256, 0, s>>>((const uint8_t*)x, (uint8_t*)y, rows, W, C, lp, Wp);
-  else if (esz == 1 && cp == 16) stem_pad_kernel<uint8_t, 16><<<grid, 256, 0, s>>>((const uint8_t*)x, (uint8_t*)y, rows, W, C, lp, Wp);
-  else if (esz == 2 && cp == 4) stem_pad_kernel<uint16_t, 4><<<grid, 256, 0, s>>>((const uint16_t*)x, (uint16_t*)y, rows, W, C, lp, Wp);
-  else if (esz == 2 && cp == 8) stem_pad_kernel<uint16_t, 8><<<grid, 256, 0, s>>>((const uint16_t*)x, (uint16_t*)y, rows, W, C, lp, Wp);
+  if (esz == 1 && cp == 4) launch(stem_pad_kernel<uint8_t, 4>, grid, 256, 0, s, (const uint8_t*)x, (uint8_t*)y, rows, W, C, lp, Wp);
+  else if (esz == 1 && cp == 8) launch(stem_pad_kernel<uint8_t, 8>, grid, 256, 0, s, (const uint8_t*)x, (uint8_t*)y, rows, W, C, lp, Wp);
+  else if (esz == 1 && cp == 16) launch(stem_pad_kernel<uint8_t, 16>, grid, 256, 0, s, (const uint8_t*)x, (uint8_t*)y, rows, W, C, lp, Wp);
+  else if (esz == 2 && cp == 4) launch(stem_pad_kernel<uint16_t, 4>, grid, 256, 0, s, (const uint16_t*)x, (uint16_t*)y, rows, W, C, lp, Wp);
+  else if (esz == 2 && cp == 8) launch(stem_pad_kernel<uint16_t, 8>, grid, 256, 0, s, (const uint16_t*)x, (uint16_t*)y, rows, W, C, lp, Wp);
   else return -1;
   return check_launch();
 }
@@ -1408,14 +1450,14 @@ int resize_nearest(int esz, const void* x, void* y, int N, int H, int W, int C, 
   if (total <= 0) return 0;
   if (nhwc && ((int64_t)C * esz) % 16 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)y % 16 == 0) {  // whole 16-byte pieces of a pixel per thread
     const int C16 = (int)((int64_t)C * esz / 16);
-    resize_nearest_kernel<uint4><<<grid_for((int64_t)N * P * Q * C16, 256), 256, 0, s>>>((const uint4*)x, (uint4*)y, N, H, W, C16, P, Q, 1);
+    launch(resize_nearest_kernel<uint4>, grid_for((int64_t)N * P * Q * C16, 256), 256, 0, s, (const uint4*)x, (uint4*)y, N, H, W, C16, P, Q, 1);
     return check_launch();
   }
   int grid = grid_for(total, 256);
   switch (esz) {
-    case 1: resize_nearest_kernel<uint8_t><<<grid, 256, 0, s>>>((const uint8_t*)x, (uint8_t*)y, N, H, W, C, P, Q, nhwc); break;
-    case 2: resize_nearest_kernel<uint16_t><<<grid, 256, 0, s>>>((const uint16_t*)x, (uint16_t*)y, N, H, W, C, P, Q, nhwc); break;
-    case 4: resize_nearest_kernel<uint32_t><<<grid, 256, 0, s>>>((const uint32_t*)x, (uint32_t*)y, N, H, W, C, P, Q, nhwc); break;
+    case 1: launch(resize_nearest_kernel<uint8_t>, grid, 256, 0, s, (const uint8_t*)x, (uint8_t*)y, N, H, W, C, P, Q, nhwc); break;
+    case 2: launch(resize_nearest_kernel<uint16_t>, grid, 256, 0, s, (const uint16_t*)x, (uint16_t*)y, N, H, W, C, P, Q, nhwc); break;
+    case 4: launch(resize_nearest_kernel<uint32_t>, grid, 256, 0, s, (const uint32_t*)x, (uint32_t*)y, N, H, W, C, P, Q, nhwc); break;
     default: return -1;
   }
   return check_launch();
@@ -1426,14 +1468,14 @@ int gather(int esz, const void* x, const void* idx, int idx_dt, void* y, int64_t
   if (total <= 0) return 0;
   if ((inner * esz) % 16 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)y % 16 == 0) {  // rows are copied in 16-byte pieces
     const int64_t inner16 = inner * esz / 16;
-    gather_kernel<uint4><<<grid_for(outer * n_idx * inner16, 256), 256, 0, s>>>((const uint4*)x, idx, idx_dt, (uint4*)y, outer, axis_dim, n_idx, inner16);
+    launch(gather_kernel<uint4>, grid_for(outer * n_idx * inner16, 256), 256, 0, s, (const uint4*)x, idx, idx_dt, (uint4*)y, outer, axis_dim, n_idx, inner16);
     return check_launch();
   }
   int grid = grid_for(total, 256);
   switch (esz) {
-    case 1: gather_kernel<uint8_t><<<grid, 256, 0, s>>>((const uint8_t*)x, idx, idx_dt, (uint8_t*)y, outer, axis_dim, n_idx, inner); break;
-    case 2: gather_kernel<uint16_t><<<grid, 256, 0, s>>>((const uint16_t*)x, idx, idx_dt, (uint16_t*)y, outer, axis_dim, n_idx, inner); break;
-    case 4: gather_kernel<uint32_t><<<grid, 256, 0, s>>>((const uint32_t*)x, idx, idx_dt, (uint32_t*)y, outer, axis_dim, n_idx, inner); break;
+    case 1: launch(gather_kernel<uint8_t>, grid, 256, 0, s, (const uint8_t*)x, idx, idx_dt, (uint8_t*)y, outer, axis_dim, n_idx, inner); break;
+    case 2: launch(gather_kernel<uint16_t>, grid, 256, 0, s, (const uint16_t*)x, idx, idx_dt, (uint16_t*)y, outer, axis_dim, n_idx, inner); break;
+    case 4: launch(gather_kernel<uint32_t>, grid, 256, 0, s, (const uint32_t*)x, idx, idx_dt, (uint32_t*)y, outer, axis_dim, n_idx, inner); break;
     default: return -1;
   }
   return check_launch();
