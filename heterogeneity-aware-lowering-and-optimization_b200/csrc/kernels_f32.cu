@@ -249,6 +249,51 @@ __global__ void __launch_bounds__(kThreads, 4) f32_tile_kernel(const F32Params p
   }
 }
 
+// Few results over a long reduction (a classifier behind a small batch): a 64 x 64 tile would leave most of its threads and
+// nearly all SMs without work and walk the reduction serially, 2 us per k-block.  Here a warp owns 4 x 2 results, its lanes
+// share the reduction (16-byte loads, everything from L2) and the sums meet in shuffles.  64 x 10 results over 784: 20 -> 4 us.
+constexpr int kFewRows = 4, kFewCols = 2;
+__global__ void __launch_bounds__(128) f32_few_results_kernel(const F32Params p) {
+  const int lane = threadIdx.x & 31, col_groups = (p.N + kFewCols - 1) / kFewCols, row_groups = (p.M + kFewRows - 1) / kFewRows;
+  const int64_t w = blockIdx.x * 4 + (threadIdx.x >> 5), per_batch = (int64_t)col_groups * row_groups;
+  dependency_wait();
+  const int64_t batch = w / per_batch, g = w - batch * per_batch;
+  const int m0 = (int)(g / col_groups) * kFewRows, n0 = (int)(g % col_groups) * kFewCols;
+  if (batch >= p.splits) return;   // (splits holds the batch count here)
+  const float *A = p.A + batch * p.a_batch, *B = p.B + batch * p.b_batch;
+  float acc[kFewRows][kFewCols] = {};
+#pragma unroll 4
+  for (int k = lane * 4; k < p.K; k += 128) {
+    float4 a[kFewRows], b[kFewCols];
+#pragma unroll
+    for (int i = 0; i < kFewRows; ++i) a[i] = *(const float4*)(A + (int64_t)min(m0 + i, p.M - 1) * p.a_row + k);
+#pragma unroll
+    for (int j = 0; j < kFewCols; ++j) b[j] = __ldg((const float4*)(B + (int64_t)min(n0 + j, p.N - 1) * p.b_col + k));
+#pragma unroll
+    for (int i = 0; i < kFewRows; ++i)
+#pragma unroll
+      for (int j = 0; j < kFewCols; ++j) {
+        acc[i][j] = fmaf(a[i].x, b[j].x, acc[i][j]); acc[i][j] = fmaf(a[i].y, b[j].y, acc[i][j]);
+        acc[i][j] = fmaf(a[i].z, b[j].z, acc[i][j]); acc[i][j] = fmaf(a[i].w, b[j].w, acc[i][j]);
+      }
+  }
+  float mine = 0.f;   // lane i * kFewCols + j finishes result (i, j)
+#pragma unroll
+  for (int i = 0; i < kFewRows; ++i)
+#pragma unroll
+    for (int j = 0; j < kFewCols; ++j) {
+      float v = acc[i][j];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane == i * kFewCols + j) mine = v;
+    }
+  const int m = m0 + lane / kFewCols, n = n0 + lane % kFewCols;
+  if (lane < kFewRows * kFewCols && m < p.M && n < p.N) {
+    const int64_t row = batch * p.M + m;
+    store_from_float(p.y, p.ep.out_dt, row * p.N + n, epilogue_value(p.ep, mine, row, n, p.N));
+  }
+}
+
 int device_sms() {
   static int cache[16] = {0};
   int dev = 0;
@@ -276,7 +321,7 @@ int pick_splits(int64_t tiles, int num_kb) {
   return best;
 }
 template <int LA, bool BVEC>
-int launch(const F32Params& p, int64_t blocks, cudaStream_t s) {
+int launch_tiles(const F32Params& p, int64_t blocks, cudaStream_t s) {
   static bool set[16] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -312,10 +357,10 @@ int run(F32Params p, int la, bool bvec, int64_t batch, cudaStream_t s) {
   if (tiles <= 0) return 0;
   if (tiles > 0x7fffffffLL) return -1;
   p.splits = pick_splits(tiles, p.num_kb);
-  if (la == LOAD_CONV_VEC) return launch<LOAD_CONV_VEC, true>(p, tiles, s);
-  if (la == LOAD_CONV_SCALAR) return launch<LOAD_CONV_SCALAR, true>(p, tiles, s);
-  if (la == LOAD_GEMM_VEC) return bvec ? launch<LOAD_GEMM_VEC, true>(p, tiles, s) : launch<LOAD_GEMM_VEC, false>(p, tiles, s);
-  return bvec ? launch<LOAD_GEMM_SCALAR, true>(p, tiles, s) : launch<LOAD_GEMM_SCALAR, false>(p, tiles, s);
+  if (la == LOAD_CONV_VEC) return launch_tiles<LOAD_CONV_VEC, true>(p, tiles, s);
+  if (la == LOAD_CONV_SCALAR) return launch_tiles<LOAD_CONV_SCALAR, true>(p, tiles, s);
+  if (la == LOAD_GEMM_VEC) return bvec ? launch_tiles<LOAD_GEMM_VEC, true>(p, tiles, s) : launch_tiles<LOAD_GEMM_VEC, false>(p, tiles, s);
+  return bvec ? launch_tiles<LOAD_GEMM_SCALAR, true>(p, tiles, s) : launch_tiles<LOAD_GEMM_SCALAR, false>(p, tiles, s);
 }
 }  // namespace
 
@@ -342,6 +387,13 @@ int gemm_f32(const GemmGeom& g, const void* A, const void* B, void* C, const Epi
   const bool avec = g.a_col == 1 && g.K % 4 == 0 && g.a_row % 4 == 0 && g.a_batch % 4 == 0 && (uintptr_t)A % 16 == 0;
   // (pieces past K are zero on the A side, so a B row padded to a multiple of four floats may hold anything there)
   const bool bvec = g.b_row == 1 && g.b_col % 4 == 0 && (g.K % 4 == 0 || g.b_batch == 0) && g.b_batch % 4 == 0 && (uintptr_t)B % 16 == 0;
+  // up to 16384 results the warps of one launch fit the chip at once and the operands are re-read from L2 only
+  if (avec && bvec && g.K % 4 == 0 && g.batch > 0 && g.batch * g.M * g.N <= 16384) {
+    p.splits = (int)g.batch;
+    const int64_t warps = g.batch * ((g.M + kFewRows - 1) / kFewRows) * ((g.N + kFewCols - 1) / kFewCols);
+    b200::launch(f32_few_results_kernel, (unsigned)((warps + 3) / 4), 128, 0, s, p);
+    return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  }
   return run(p, avec ? LOAD_GEMM_VEC : LOAD_GEMM_SCALAR, bvec, g.batch, s);
 }
 
