@@ -111,7 +111,7 @@ struct Plan {
   int64_t arena_bytes = 0;
   char* consts = nullptr;          // converted / repacked constants
   int64_t const_bytes = 0;
-  int* status = nullptr;           // device status block (kStatusBytes): word 0 non-zero when a bounded wait expired
+  int* status = nullptr;           // device address of the replica's status block: word 0 non-zero when a bounded wait expired
   std::vector<void*> extra_allocs; // uploaded constants and scratch
   std::vector<UmmaLaunch*> umma;   // prepared tensor-core launches (own their tensor maps)
   std::vector<AttnLaunch*> attn;   // prepared fused-attention launches
@@ -136,7 +136,7 @@ struct Plan {
 struct Replica {
   int device = 0;
   int64_t shard_start = 0, shard_batch = 0;  // rows [start, start+batch) of dim 0
-  int* host_status = nullptr;      // pinned copy of the plan's device status word
+  int* host_status = nullptr;      // pinned, mapped status block (kStatusBytes) the plan's kernels write to
   std::unique_ptr<Plan> plan;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev_begin = nullptr, ev_end = nullptr;

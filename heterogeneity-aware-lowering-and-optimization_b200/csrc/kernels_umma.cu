@@ -149,7 +149,8 @@ __device__ __forceinline__ bool mbar_wait_impl(uint64_t* bar, uint32_t parity, v
     if ((i & 63) == 63 && *abort_flag) return false;
   }
   *abort_flag = 1;
-  if (status) { atomicCAS(status, 0, code); status[1] = (int)blockIdx.x; }
+  // (the block may be host memory: plain stores, the last of several expiring waits wins)
+  if (status) { *(volatile int*)status = code; ((volatile int*)status)[1] = (int)blockIdx.x; __threadfence_system(); }
   return false;
 }
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {

@@ -41,7 +41,6 @@ Plan::~Plan() {
   for (auto* a : attn) attn_destroy(a);
   for (void* p : extra_allocs) cudaFree(p);
   if (arena) cudaFree(arena);
-  if (status) cudaFree(status);
 }
 
 namespace {
@@ -612,8 +611,6 @@ odla_status Builder::place() {
   p_->arena_bytes = arena.top;
   if (inject_fault("alloc") || cudaMalloc((void**)&p_->arena, (size_t)std::max<int64_t>(p_->arena_bytes, 1024)) != cudaSuccess)
     return fail(ODLA_MEM_ERROR, "arena allocation failed");
-  if (cudaMalloc((void**)&p_->status, kStatusBytes) != cudaSuccess) return fail(ODLA_MEM_ERROR, "status word allocation failed");
-  cudaMemset(p_->status, 0, kStatusBytes);
   return ODLA_SUCCESS;
 }
 
@@ -1778,10 +1775,13 @@ static odla_status build_replicas(_odla_computation* c, int visible, int64_t B, 
     B2_CUDA("stream", cudaStreamCreateWithFlags(&r.stream, cudaStreamNonBlocking), ODLA_FAILURE);
     B2_CUDA("event", cudaEventCreate(&r.ev_begin), ODLA_FAILURE);
     B2_CUDA("event", cudaEventCreate(&r.ev_end), ODLA_FAILURE);
-    B2_CUDA("alloc", cudaMallocHost((void**)&r.host_status, 256), ODLA_MEM_ERROR);
-    memset(r.host_status, 0, 256);
+    // The status block is pinned host memory that the kernels address directly: nothing is written there unless a bounded
+    // wait expires, so reading it costs an execute no copy.
+    B2_CUDA("alloc", cudaHostAlloc((void**)&r.host_status, kStatusBytes, cudaHostAllocMapped), ODLA_MEM_ERROR);
+    memset(r.host_status, 0, kStatusBytes);
     r.plan = std::make_unique<Plan>();
     r.plan->device = r.device;
+    B2_CUDA("alloc", cudaHostGetDevicePointer((void**)&r.plan->status, r.host_status, 0), ODLA_MEM_ERROR);
     r.plan->batch = r.shard_batch;
     Builder b(c, r.plan.get(), c->shardable ? B : r.shard_batch, r.shard_batch, r.shard_start);
     odla_status s = b.run();
@@ -1939,20 +1939,22 @@ int run_launches(Replica& r, _odla_context* ctx, bool use_graph, long long* n_la
 }
 }  // namespace
 
-// Enqueues one replica's share of an execute on its own stream: input copies, the launch list, output copies, the
-// status read-back and the two events that time it.  Nothing here waits for the GPU.
+// Enqueues one replica's share of an execute on its own stream: input copies, the launch list, output copies and the two
+// events that time it.  Nothing here waits for the GPU.
 static odla_status enqueue_replica(Replica& r, size_t index, _odla_context* ctx, bool use_graph, long long* launched) {
   Plan& p = *r.plan;
   auto fail_here = [&](odla_status s, const char* what) { B2_ERR("GPU %d: %s failed", r.device, what); return s; };
   if (cudaSetDevice(r.device) != cudaSuccess) return fail_here(ODLA_FAILURE, "cudaSetDevice");
   cudaEventRecord(r.ev_begin, r.stream);
+  // where a bound pointer lives only has to be looked up when it may be another GPU's memory; cudaMemcpyDefault tells host from device
+  const bool one_gpu = visible_devices() == 1;
   for (auto& io : p.inputs) {
     const char* src = (const char*)ctx->in.find(io.v)->second + io.user_offset;  // every argument is bound (checked by the caller)
-    int pd = pointer_device(src);
+    const int pd = one_gpu ? -1 : pointer_device(src);
     cudaError_t e;
     if (inject_fault("h2d")) e = cudaErrorUnknown;
     else if (pd >= 0 && pd != r.device) e = cudaMemcpyPeerAsync(p.arena + io.stage, r.device, src, pd, (size_t)io.api_bytes, r.stream);
-    else e = cudaMemcpyAsync(p.arena + io.stage, src, (size_t)io.api_bytes, pd >= 0 ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, r.stream);
+    else e = cudaMemcpyAsync(p.arena + io.stage, src, (size_t)io.api_bytes, cudaMemcpyDefault, r.stream);
     if (e != cudaSuccess) return fail_here(ODLA_FAILURE, "input copy");
   }
   // With contexts on several lanes in flight, this execute's kernels start behind the kernels of the execute that was
@@ -1982,17 +1984,16 @@ static odla_status enqueue_replica(Replica& r, size_t index, _odla_context* ctx,
     if (bound == ctx->out.end()) continue;
     if (!io.per_shard && index != 0) continue;  // a value that does not depend on the batch: the first replica writes it
     char* dst = (char*)bound->second + io.user_offset;
-    int pd = pointer_device(dst);
+    const int pd = one_gpu ? -1 : pointer_device(dst);
     cudaError_t e;
     if (inject_fault("d2h")) e = cudaErrorUnknown;
     else if (io.const_host) {
-      e = cudaMemcpyAsync(dst, io.const_host, (size_t)io.api_bytes, pd >= 0 ? cudaMemcpyHostToDevice : cudaMemcpyHostToHost, r.stream);
+      e = cudaMemcpyAsync(dst, io.const_host, (size_t)io.api_bytes, cudaMemcpyDefault, r.stream);
     } else if (pd >= 0 && pd != r.device) {
       e = inject_fault("peer") ? cudaErrorUnknown : cudaMemcpyPeerAsync(dst, pd, p.arena + io.stage, r.device, (size_t)io.api_bytes, r.stream);
-    } else e = cudaMemcpyAsync(dst, p.arena + io.stage, (size_t)io.api_bytes, pd >= 0 ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, r.stream);
+    } else e = cudaMemcpyAsync(dst, p.arena + io.stage, (size_t)io.api_bytes, cudaMemcpyDefault, r.stream);
     if (e != cudaSuccess) return fail_here(ODLA_FAILURE, "output copy");
   }
-  cudaMemcpyAsync(r.host_status, p.status, sizeof(int) * 4, cudaMemcpyDeviceToHost, r.stream);
   cudaEventRecord(r.ev_end, r.stream);
   return ODLA_SUCCESS;
 }
@@ -2052,8 +2053,7 @@ odla_status execute(_odla_computation* c, _odla_context* ctx) {
       if (cudaEventElapsedTime(&ms, r.ev_begin, r.ev_end) == cudaSuccess) worst = std::max(worst, ms); else cudaGetLastError();
       if (r.host_status[0] != 0) {
         B2_ERR("GPU %d: a bounded wait inside a kernel expired (code %d, detail %d)", r.device, r.host_status[0], r.host_status[1]);
-        cudaMemsetAsync(r.plan->status, 0, kStatusBytes, r.stream);
-        cudaStreamSynchronize(r.stream);
+        memset(r.host_status, 0, kStatusBytes);   // (the stream is idle)
         result = ODLA_TIMEOUT;
       }
     }
