@@ -116,6 +116,8 @@ struct UmmaConv {
   // R x S window of x.  A filter whose values do not fit the operand type is split into terms that do (uint8 weights
   // minus their zero point span [-255, 255]: two or three int8 terms).  0 and 1 both mean a single term.
   int w_terms = 0;
+  // w is written by no kernel (a constant uploaded before the first launch): its loads need not wait for the kernel in front.
+  int w_constant = 0;
 };
 // True when the tensor-core kernel can run this problem.
 bool umma_conv_supported(const UmmaConv& p);

@@ -84,6 +84,7 @@ struct UmmaParams {
   int fast_variant;    // mode 1: accumulator conversion (0 fp32, 1 int32 by conversion, 2 int32 by integer add) * 2 + residual
   int tmem_cols;
   uint32_t spin_limit;  // attempts before a bounded wait gives up
+  int early_b;         // stages whose B boxes are requested before the previous kernel has finished (0: B is a run-time tensor)
   int test_skip_stage;  // test hook: the producer of CTA 0 leaves the last stage of its first tile unarmed, so the MMA lane's wait runs out
   void* y;
   int* status;
@@ -282,6 +283,9 @@ template <> __device__ __forceinline__ void tmem_ld_wait_regs<16>(uint32_t (&r)[
 template <> __device__ __forceinline__ void tmem_ld_wait_regs<32>(uint32_t (&r)[32]) { tmem_ld_wait(); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// Waits until the kernels this launch depends on have completed and their writes are visible (programmatic dependent launch).
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* m) { asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)m) : "memory"); }
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(
@@ -935,6 +939,37 @@ __device__ __forceinline__ void box_gelu_s8(const UmmaParams& p, uint32_t taddr,
   }
 }
 
+// The products of one k-block: 32 bytes of K per instruction.  Everything that does not change from instruction to
+// instruction is decided outside -- the issuing lane's instruction stream is what the tensor pipe waits for.
+template <bool PAIR, bool INT>
+__device__ __forceinline__ void issue_four(uint32_t d, uint64_t da, uint64_t db, uint64_t bstep, uint32_t idesc, uint32_t accum) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if constexpr (PAIR && INT) umma_i8_pair(d, da + 2 * k, db + bstep * k, idesc, k ? 1u : accum);
+    else if constexpr (PAIR) umma_f16_pair(d, da + 2 * k, db + bstep * k, idesc, k ? 1u : accum);
+    else if constexpr (INT) umma_i8(d, da + 2 * k, db + bstep * k, idesc, k ? 1u : accum);
+    else umma_f16(d, da + 2 * k, db + bstep * k, idesc, k ? 1u : accum);
+  }
+}
+template <bool PAIR>
+__device__ __forceinline__ void issue_kblock(const UmmaParams& p, uint32_t d, uint64_t da, uint64_t db, int ksteps, uint32_t accum) {
+  if (ksteps == 4) {
+    if (p.acc_int) issue_four<PAIR, true>(d, da, db, 2, p.idesc, accum);
+    else issue_four<PAIR, false>(d, da, db, (uint64_t)p.b_kstep, p.idesc, accum);
+    return;
+  }
+  for (int k = 0; k < ksteps; ++k) {
+    if constexpr (PAIR) {
+      if (p.acc_int) umma_i8_pair(d, da + 2 * k, db + 2 * k, p.idesc, accum);
+      else umma_f16_pair(d, da + 2 * k, db + 2 * k, p.idesc, accum);
+    } else {
+      if (p.acc_int) umma_i8(d, da + 2 * k, db + 2 * k, p.idesc, accum);
+      else umma_f16(d, da + 2 * k, db + (uint64_t)(p.b_kstep * k), p.idesc, accum);
+    }
+    accum = 1;
+  }
+}
+
 // --------------------------------------------------------------------- kernel ----
 // MODE 3: staged epilogue, further straight-line forms: LeakyReLU before the optional residual (Darknet) or GELU, two-byte
 //         outputs (box_leaky); int8 operands, GELU, requantised int8 output (box_gelu_s8).
@@ -993,10 +1028,9 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  // Programmatic dependent launch: everything above overlapped the previous kernel's tail; from here on
-  // this kernel reads what that kernel wrote.  The next kernel may start its own prologue now.
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // Programmatic dependent launch: everything above overlapped the previous kernel's tail.  Only the threads that touch
+  // tensors other kernels write or read wait for that kernel (grid_dependency_wait): the producer -- which first issues
+  // the filter loads of its first stages, constants nobody writes --, the residual loader, the storer and direct epilogues.
   if (threadIdx.x == 0) TS(0);
 
   const uint32_t a_box = (uint32_t)(BM * p.kb_bytes), b_box = (uint32_t)(p.bn_load * p.kb_bytes);
@@ -1009,12 +1043,62 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // One lane runs this loop; it is kept free of divisions (filter tap, channel chunk, stage and
     // phase are running counters) because its instruction rate bounds the rate of k-blocks.
     if (elect_one()) {
-      int s = 0;
-      uint32_t ph = 0;
+      prefetch_map(&tmB);
+      prefetch_map(&tmA);
+      // where the walk over a tile's k-blocks and over the stage ring stands
+      struct Walk { int tap, fr, fs, c0, left, s; uint32_t ph; };
+      Walk k{0, 0, 0, 0, 0, 0, 0};
+      int w0 = 0, h0 = 0, img = 0, m0 = 0, n0 = 0, bidx = 0;
+      // One stage: its k-blocks of A (do_a) and B (do_b), each load signalling the stage's barrier, which do_b arms with the
+      // byte count of both.
+      auto fill = [&](bool do_a, bool do_b, bool skip) {
+        const int nb = k.left < p.bps ? k.left : p.bps;
+        k.left -= nb;
+        uint8_t* sa = smem + (size_t)k.s * stage_bytes;
+        uint8_t* sb = sa + (size_t)p.bps * a_box;
+        uint64_t* fb = full_bar + k.s;
+        uint32_t fbc = 0;
+        if constexpr (PAIR) {
+          // the first CTA's barrier counts the bytes of both CTAs; only it is armed
+          if (do_b && rank == 0) mbar_expect_tx(fb, 2u * (uint32_t)nb * (a_box + b_box));
+          fbc = map_to_cta(smem_u32(fb), 0);
+        } else if (do_b && !skip) mbar_expect_tx(fb, (uint32_t)nb * (a_box + b_box));
+        for (int j = 0; j < nb; ++j) {
+          if constexpr (PAIR) {
+            if (do_b) {
+              const int nb0 = n0 + rank * p.bn_load;
+              if (p.rows_per_batch) tma_load_3d_pair(sb, &tmB, fbc, k.c0, nb0, bidx);
+              else tma_load_3d_pair(sb, &tmB, fbc, k.c0, k.tap, nb0);
+            }
+            if (do_a) {
+              if (p.im2col) tma_load_im2col_4d_pair(sa, &tmA, fbc, k.c0, w0, h0, img, (uint16_t)k.fs, (uint16_t)k.fr);
+              else tma_load_2d_pair(sa, &tmA, fbc, k.c0, m0);
+            }
+          } else if (!skip) {
+            if (do_b) {
+              if (p.rows_per_batch) tma_load_3d(sb, &tmB, fb, p.b_n_major ? n0 : k.c0, p.b_n_major ? k.c0 : n0, bidx);
+              else tma_load_3d(sb, &tmB, fb, k.c0, k.tap, n0);
+            }
+            if (do_a) {
+              if (p.im2col) tma_load_im2col_4d(sa, &tmA, fb, k.c0, w0, h0, img, (uint16_t)k.fs, (uint16_t)k.fr);
+              else tma_load_2d(sa, &tmA, fb, k.c0, m0);
+            }
+          }
+          sa += a_box;
+          sb += b_box;
+          k.c0 += p.kbe;
+          if (k.c0 >= p.C) {
+            k.c0 = 0;
+            ++k.tap;
+            if (++k.fs == p.S) { k.fs = 0; if (++k.fr == p.R) k.fr = 0; }   // the next filter term walks the window again
+          }
+        }
+        if (++k.s == p.stages) { k.s = 0; k.ph ^= 1; }
+      };
       bool ok = true;
       for (int tile = tile_first; tile < p.total_tiles && ok; tile += tile_step) {
-        const int m0 = (((tile % p.m_tiles) << kPair) + rank) * BM, n0 = (tile / p.m_tiles) * p.BN;
-        int w0 = 0, h0 = 0, img = 0;
+        m0 = (((tile % p.m_tiles) << kPair) + rank) * BM;
+        n0 = (tile / p.m_tiles) * p.BN;
         if (p.im2col) {
           const int pq = p.P * p.Q;
           img = m0 / pq;
@@ -1023,64 +1107,31 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           w0 = oq * p.stride_w - p.pad_l;
           h0 = op * p.stride_h - p.pad_t;
         }
-        int tap = 0, fr = 0, fs = 0, c0 = 0, left = p.num_kb;
-        const int bidx = p.rows_per_batch ? m0 / p.rows_per_batch : 0;
-        for (int it = 0; it < p.num_it; ++it) {
-          if (!mbar_wait(empty_bar + s, ph ^ 1, abort_flag, p.status, 1, p.spin_limit)) { ok = false; break; }
-          const int nb = left < p.bps ? left : p.bps;
-          left -= nb;
-          uint8_t* sa = smem + (size_t)s * stage_bytes;
-          uint8_t* sb = sa + (size_t)p.bps * a_box;
-          uint64_t* fb = full_bar + s;
-          if constexpr (PAIR) {
-            // the first CTA's barrier counts the bytes of both CTAs; only it is armed
-            if (rank == 0) mbar_expect_tx(fb, 2u * (uint32_t)nb * (a_box + b_box));
-            const uint32_t fbc = map_to_cta(smem_u32(fb), 0);
-            const int nb0 = n0 + rank * p.bn_load;
-            for (int j = 0; j < nb; ++j) {
-              if (p.im2col) tma_load_im2col_4d_pair(sa, &tmA, fbc, c0, w0, h0, img, (uint16_t)fs, (uint16_t)fr);
-              else tma_load_2d_pair(sa, &tmA, fbc, c0, m0);
-              if (p.rows_per_batch) tma_load_3d_pair(sb, &tmB, fbc, c0, nb0, bidx);
-              else tma_load_3d_pair(sb, &tmB, fbc, c0, tap, nb0);
-              sa += a_box;
-              sb += b_box;
-              c0 += p.kbe;
-              if (c0 >= p.C) {
-                c0 = 0;
-                ++tap;
-                if (++fs == p.S) { fs = 0; if (++fr == p.R) fr = 0; }   // the next filter term walks the window again
-              }
-            }
-            if (++s == p.stages) { s = 0; ph ^= 1; }
-            continue;
-          }
+        k.tap = k.fr = k.fs = k.c0 = 0;
+        k.left = p.num_kb;
+        bidx = p.rows_per_batch ? m0 / p.rows_per_batch : 0;
+        int it = 0;
+        if (tile == tile_first) {
+          // The first stages are free: their filter boxes are on the way before the previous kernel has finished.
+          const int early = p.early_b < p.num_it ? p.early_b : p.num_it;
+          const Walk start = k;
+          for (int e = 0; e < early; ++e) fill(false, true, false);
+          grid_dependency_wait();
+          asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the next kernel may start its own prologue now
+          k = start;
+          for (; it < early; ++it) fill(true, false, false);
+        }
+        for (; it < p.num_it; ++it) {
+          if (!mbar_wait(empty_bar + k.s, k.ph ^ 1, abort_flag, p.status, 1, p.spin_limit)) { ok = false; break; }
           // Test hook (never set by the planner): this stage is neither armed nor loaded, so its barrier can never
           // complete and the MMA lane's bounded wait reports a timeout; nothing faults and nothing spins for ever.
-          const bool skip = p.test_skip_stage && blockIdx.x == 0 && tile == tile_first && it == p.num_it - 1;
-          if (!skip) mbar_expect_tx(fb, (uint32_t)nb * (a_box + b_box));
-          for (int j = 0; j < nb; ++j) {
-            if (skip) {}
-            else if (p.im2col) tma_load_im2col_4d(sa, &tmA, fb, c0, w0, h0, img, (uint16_t)fs, (uint16_t)fr);
-            else tma_load_2d(sa, &tmA, fb, c0, m0);
-            if (skip) {}
-            else if (p.rows_per_batch) tma_load_3d(sb, &tmB, fb, p.b_n_major ? n0 : c0, p.b_n_major ? c0 : n0, bidx);
-            else tma_load_3d(sb, &tmB, fb, c0, tap, n0);
-            sa += a_box;
-            sb += b_box;
-            c0 += p.kbe;
-            if (c0 >= p.C) {
-              c0 = 0;
-              ++tap;
-              if (++fs == p.S) { fs = 0; if (++fr == p.R) fr = 0; }   // the next filter term walks the window again
-            }
-          }
-          if (++s == p.stages) { s = 0; ph ^= 1; }
+          fill(true, true, p.test_skip_stage && blockIdx.x == 0 && tile == tile_first && it == p.num_it - 1);
         }
       }
       if (!ok) {
         // give copies already in flight a bounded chance to land before shared memory goes away
         for (int i = 0; i < p.stages; ++i)
-          for (uint32_t k = 0; k < 4096; ++k)
+          for (uint32_t n = 0; n < 4096; ++n)
             if (mbar_try_wait(&full_bar[i], 0) || mbar_try_wait(&full_bar[i], 1)) break;
       }
     }
@@ -1109,16 +1160,8 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           for (int j = 0; j < nb; ++j) {
             const uint64_t da = desc_fixed | (uint64_t)((sa & 0x3FFFF) >> 4);
             const uint64_t db = desc_fixed | (uint64_t)((sb & 0x3FFFF) >> 4);
-            for (int k = 0; k < ksteps; ++k) {
-              if constexpr (PAIR) {
-                if (p.acc_int) umma_i8_pair(tmem_d, da + 2 * k, db + 2 * k, p.idesc, accum);
-                else umma_f16_pair(tmem_d, da + 2 * k, db + 2 * k, p.idesc, accum);
-              } else {
-                if (p.acc_int) umma_i8(tmem_d, da + 2 * k, db + 2 * k, p.idesc, accum);
-                else umma_f16(tmem_d, da + 2 * k, db + (uint64_t)(p.b_kstep * k), p.idesc, accum);
-              }
-              accum = 1;
-            }
+            issue_kblock<PAIR>(p, tmem_d, da, db, ksteps, accum);
+            accum = 1;
             sa += a_box;
             sb += b_box;
           }
@@ -1132,6 +1175,10 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   } else if (warp == kLoaderWarp) {
     // -------------------------------------------- staging ring: arm boxes (residual loads) ----
     if (STAGED && elect_one()) {
+      if (p.res_tma) {
+        prefetch_map(&tmR);
+        grid_dependency_wait();
+      }
       const int cols_per_box = 128 / p.out_esz;
       int slot = 0;
       uint32_t ph = 0;
@@ -1161,6 +1208,8 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   } else if (warp == kStorerWarp) {
     // ------------------------------------------------ staging ring: store finished boxes ----
     if (STAGED && elect_one()) {
+      prefetch_map(&tmY);
+      grid_dependency_wait();   // earlier kernels may still read what the stores overwrite
       const int cols_per_box = 128 / p.out_esz;
       const uint32_t staging_u32 = smem_u32(staging);
       int slot = 0, prev = -1;
@@ -1309,6 +1358,7 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     } else {
       // Direct epilogue: rows go straight to global memory.  Residual rows can be fetched before the
       // accumulator is ready: they only depend on the tile.
+      grid_dependency_wait();
       const bool res_vec = p.ep.res && (p.K_out & 15) == 0 && (p.ep.res_dt == DT_F16 || p.ep.res_dt == DT_BF16 || p.ep.res_dt == DT_S8);
       const int res_q = p.ep.res_dt == DT_S8 ? 2 : 4;       // 16-byte pieces per 32 channels
       const int res_esz = p.ep.res_dt == DT_S8 ? 1 : 2;
@@ -1844,6 +1894,7 @@ UmmaLaunch* umma_conv_prepare(const UmmaConv& c, const void* x, const void* w, v
   // Test hooks for the time-out path (tests/test_conv_umma_gpu.py): a short limit and one deliberately unarmed stage.
   if (const char* e = getenv("ODLA_B200_TEST_SPIN_LIMIT")) { const long v = atol(e); if (v >= 64 && v <= (1l << 18)) p.spin_limit = (uint32_t)v; }
   if (getenv("ODLA_B200_TEST_SKIP_STAGE") && !p.pair) p.test_skip_stage = 1;
+  p.early_b = c.w_constant && !p.test_skip_stage ? p.stages : 0;
   L->grid = p.pair ? (2 * p.total_tiles < (sms & ~1) ? 2 * p.total_tiles : (sms & ~1)) : (p.total_tiles < sms ? p.total_tiles : sms);
   L->smem = (size_t)p.stages * stage_bytes + (size_t)p.ring_boxes * 16384 + 1024 /*alignment slack*/ + 1024 /*barriers*/;
   if (L->smem > 227 * 1024) { delete L; return nullptr; }

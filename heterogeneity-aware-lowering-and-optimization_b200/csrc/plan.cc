@@ -757,7 +757,9 @@ odla_status Builder::emit_group(const Item& it) {
   if (!wd) return err_status_;
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p_->device);
-  UmmaLaunch* ul = umma_conv_prepare(UmmaConv{1, 1, (int)M, (int)Kd, (int)(G * N), 1, 1, 1, (int)M, 1, 1, 0, 0, in_dt}, dev_ptr(it.fused->x), wd, dev_ptr(it.out), ep, p_->status, sms);
+  UmmaConv uc{1, 1, (int)M, (int)Kd, (int)(G * N), 1, 1, 1, (int)M, 1, 1, 0, 0, in_dt};
+  uc.w_constant = 1;
+  UmmaLaunch* ul = umma_conv_prepare(uc, dev_ptr(it.fused->x), wd, dev_ptr(it.out), ep, p_->status, sms);
   if (!ul) return fail(ODLA_FAILURE, "'" + root->name + "': tensor-map encoding failed");
   p_->umma.push_back(ul);
   // one entry of the launch list per value; the kernel belongs to the first
@@ -1029,6 +1031,7 @@ odla_status Builder::emit_fused(const Item& it) {
       void* wd = upload(wb->data(), wb->size());
       if (!wd) return err_status_;
       if (pitch_.count(f.out)) uc.y_pitch = (int)pitch_[f.out];
+      uc.w_constant = 1;
       UmmaLaunch* ul = umma_conv_prepare(uc, x_umma, wd, y, ep, p_->status, sms);
       if (!ul) return fail(ODLA_FAILURE, "'" + root->name + "': tensor-map encoding failed");
       p_->umma.push_back(ul);
@@ -1155,6 +1158,7 @@ odla_status Builder::emit_fused(const Item& it) {
     if (store_direct) set_store(uc);
     if (Mt < (1ll << 31) && umma_conv_supported(uc)) {
       if (w_terms > 1) uc.w_terms = w_terms;
+      uc.w_constant = 1;
       auto wb = prepared(f.w, std::string("gemm_kmajor dt") + std::to_string(in_dt) + (tb ? " t" : " n") + " terms" + std::to_string(w_terms) +
                                   (f.w_zp ? " zp" + std::to_string((int)const_as_f32(f.w_zp)[0]) : std::string()), [&] {
         if (w_terms > 1) {
