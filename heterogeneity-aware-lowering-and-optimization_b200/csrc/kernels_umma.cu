@@ -11,12 +11,13 @@
 // 128/64/32-byte swizzled K-major layout that tcgen05.mma reads through shared-memory descriptors.
 //
 // One persistent CTA per SM walks its tiles (128 pixels x BN channels):
-//   warp 0      producer: waits for a free stage, arms its mbarrier with the byte count, issues TMA
+//   warp 0      producer of A: waits for a free stage, arms its mbarrier with the byte count, issues TMA
 //   warp 1      allocates tensor memory, issues tcgen05.mma (one lane), commits to mbarriers
 //   16 warps    staged epilogue: tcgen05.ld the fp32 / int32 accumulators (one TMEM lane = one output pixel per
 //               thread), apply the fused epilogue, write 16-byte pieces into a ring of 128-row x 128-byte boxes
-//   2 warps     feed the ring (TMA loads of residual boxes) and drain it (TMA stores, plain or through a 4-d map
-//               of a head-permuted tensor)
+//   1 warp      producer of B, on the same stages and barriers
+//   1 warp      drains the ring (TMA stores, plain or through a 4-d map of a head-permuted tensor) and arms freed
+//               boxes again (TMA loads of residual boxes)
 //   (the direct variant, for fp32 / int32 outputs, runs 8 epilogue warps that store rows straight to global memory)
 // Two accumulator buffers in tensor memory let the epilogue of tile i overlap the MMAs of tile i+1.
 //
@@ -46,8 +47,8 @@ constexpr int BM = 128;
 template <bool STAGED> struct EpiCfg {
   static constexpr int kWarps = STAGED ? 16 : 8;     // epilogue warps (a multiple of 4: one per TMEM lane quarter)
   static constexpr int kChunk = STAGED ? 16 : 32;    // accumulator columns per tcgen05.ld
-  static constexpr int kLoaderWarp = 2 + kWarps;      // brings residual boxes into the staging ring
-  static constexpr int kStorerWarp = 3 + kWarps;      // drains finished boxes with TMA stores
+  static constexpr int kFilterWarp = 2 + kWarps;      // producer of B
+  static constexpr int kStorerWarp = 3 + kWarps;      // drains finished boxes with TMA stores, arms them again (residual loads)
   static constexpr int kThreads = 32 * (4 + kWarps);
 };
 constexpr int kMaxRing = 8;
@@ -84,7 +85,7 @@ struct UmmaParams {
   int fast_variant;    // mode 1: accumulator conversion (0 fp32, 1 int32 by conversion, 2 int32 by integer add) * 2 + residual
   int tmem_cols;
   uint32_t spin_limit;  // attempts before a bounded wait gives up
-  int early_b;         // stages whose B boxes are requested before the previous kernel has finished (0: B is a run-time tensor)
+  int b_constant;      // B is written by no kernel: its loads need not wait for the kernel in front
   int test_skip_stage;  // test hook: the producer of CTA 0 leaves the last stage of its first tile unarmed, so the MMA lane's wait runs out
   void* y;
   int* status;
@@ -159,19 +160,6 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
                "l"((uint64_t)map), "r"(smem_u32(bar)), "r"(x), "r"(y)
                : "memory");
 }
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z) {
-  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
-               "l"((uint64_t)map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
-               : "memory");
-}
-__device__ __forceinline__ void tma_load_im2col_4d(void* dst, const CUtensorMap* map, uint64_t* bar, int c, int w, int h, int n,
-                                                   uint16_t off_w, uint16_t off_h) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2], {%7, %8};" ::"r"(
-          smem_u32(dst)),
-      "l"((uint64_t)map), "r"(smem_u32(bar)), "r"(c), "r"(w), "r"(h), "r"(n), "h"(off_w), "h"(off_h)
-      : "memory");
-}
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -188,6 +176,49 @@ __device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t da, uint64_t d
 }
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// The same on 32-bit shared-memory addresses, for the loops of the producing and issuing lanes: one lane's dependent
+// instructions bound the rate of stages there, so that neither pointer arithmetic nor divisions belong in them.
+__device__ __forceinline__ bool mbar_try_wait_at(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ void mbar_expect_tx_at(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+template <bool PAIR> __device__ __forceinline__ void load_2d_at(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
+  if constexpr (PAIR)
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
+                 "l"((uint64_t)map), "r"(bar), "r"(x), "r"(y) : "memory");
+  else
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
+                 "l"((uint64_t)map), "r"(bar), "r"(x), "r"(y) : "memory");
+}
+template <bool PAIR> __device__ __forceinline__ void load_3d_at(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z) {
+  if constexpr (PAIR)
+    asm volatile("cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst),
+                 "l"((uint64_t)map), "r"(bar), "r"(x), "r"(y), "r"(z) : "memory");
+  else
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst),
+                 "l"((uint64_t)map), "r"(bar), "r"(x), "r"(y), "r"(z) : "memory");
+}
+template <bool PAIR>
+__device__ __forceinline__ void load_im2col_at(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c, int w, int h, int n, uint16_t off_w, uint16_t off_h) {
+  if constexpr (PAIR)
+    asm volatile(
+        "cp.async.bulk.tensor.4d.im2col.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2], {%7, %8};" ::"r"(dst),
+        "l"((uint64_t)map), "r"(bar), "r"(c), "r"(w), "r"(h), "r"(n), "h"(off_w), "h"(off_h) : "memory");
+  else
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2], {%7, %8};" ::"r"(dst),
+        "l"((uint64_t)map), "r"(bar), "r"(c), "r"(w), "r"(h), "r"(n), "h"(off_w), "h"(off_h) : "memory");
 }
 // ---- CTA-pair (cta_group::2) forms.  Both CTAs of the pair issue their own loads; the byte counts land on
 // the barrier of the pair's first CTA (`bar_cluster` is that barrier's shared::cluster address), whose MMA lane
@@ -208,24 +239,6 @@ __device__ __forceinline__ void cluster_sync_all() {
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory");
-}
-__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, uint32_t bar_cluster, int x, int y) {
-  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(dst)),
-               "l"((uint64_t)map), "r"(bar_cluster), "r"(x), "r"(y)
-               : "memory");
-}
-__device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* map, uint32_t bar_cluster, int x, int y, int z) {
-  asm volatile("cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
-               "l"((uint64_t)map), "r"(bar_cluster), "r"(x), "r"(y), "r"(z)
-               : "memory");
-}
-__device__ __forceinline__ void tma_load_im2col_4d_pair(void* dst, const CUtensorMap* map, uint32_t bar_cluster, int c, int w, int h, int n,
-                                                        uint16_t off_w, uint16_t off_h) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.im2col.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2], {%7, %8};" ::"r"(
-          smem_u32(dst)),
-      "l"((uint64_t)map), "r"(bar_cluster), "r"(c), "r"(w), "r"(h), "r"(n), "h"(off_w), "h"(off_h)
-      : "memory");
 }
 __device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -939,36 +952,52 @@ __device__ __forceinline__ void box_gelu_s8(const UmmaParams& p, uint32_t taddr,
   }
 }
 
-// The products of one k-block: 32 bytes of K per instruction.  Everything that does not change from instruction to
-// instruction is decided outside -- the issuing lane's instruction stream is what the tensor pipe waits for.
+// The products of one k-block: 32 bytes of K per instruction; `la`, `lb` are the low words of the operands' descriptors.
+// Everything that does not change from instruction to instruction is decided outside -- the issuing lane's instruction
+// stream is what the tensor pipe waits for.
+__device__ __forceinline__ uint64_t desc64(uint32_t lo, uint32_t hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
+  return d;
+}
 template <bool PAIR, bool INT>
-__device__ __forceinline__ void issue_four(uint32_t d, uint64_t da, uint64_t db, uint64_t bstep, uint32_t idesc, uint32_t accum) {
+__device__ __forceinline__ void issue_one(uint32_t d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accum) {
+  if constexpr (PAIR && INT) umma_i8_pair(d, da, db, idesc, accum);
+  else if constexpr (PAIR) umma_f16_pair(d, da, db, idesc, accum);
+  else if constexpr (INT) umma_i8(d, da, db, idesc, accum);
+  else umma_f16(d, da, db, idesc, accum);
+}
+template <bool PAIR, bool INT>
+__device__ __forceinline__ void issue_four(uint32_t d, uint32_t la, uint32_t lb, uint32_t bstep, uint32_t hi, uint32_t idesc, uint32_t accum) {
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    if constexpr (PAIR && INT) umma_i8_pair(d, da + 2 * k, db + bstep * k, idesc, k ? 1u : accum);
-    else if constexpr (PAIR) umma_f16_pair(d, da + 2 * k, db + bstep * k, idesc, k ? 1u : accum);
-    else if constexpr (INT) umma_i8(d, da + 2 * k, db + bstep * k, idesc, k ? 1u : accum);
-    else umma_f16(d, da + 2 * k, db + bstep * k, idesc, k ? 1u : accum);
-  }
+  for (int k = 0; k < 4; ++k) issue_one<PAIR, INT>(d, desc64(la + 2 * k, hi), desc64(lb + bstep * k, hi), idesc, k ? 1u : accum);
 }
 template <bool PAIR>
-__device__ __forceinline__ void issue_kblock(const UmmaParams& p, uint32_t d, uint64_t da, uint64_t db, int ksteps, uint32_t accum) {
+__device__ __forceinline__ void issue_kblock(const UmmaParams& p, uint32_t d, uint32_t la, uint32_t lb, int ksteps, uint32_t accum) {
   if (ksteps == 4) {
-    if (p.acc_int) issue_four<PAIR, true>(d, da, db, 2, p.idesc, accum);
-    else issue_four<PAIR, false>(d, da, db, (uint64_t)p.b_kstep, p.idesc, accum);
+    if (p.acc_int) issue_four<PAIR, true>(d, la, lb, 2, p.desc_hi, p.idesc, accum);
+    else if (p.b_kstep == 2) issue_four<PAIR, false>(d, la, lb, 2, p.desc_hi, p.idesc, accum);
+    else issue_four<PAIR, false>(d, la, lb, (uint32_t)p.b_kstep, p.desc_hi, p.idesc, accum);
     return;
   }
   for (int k = 0; k < ksteps; ++k) {
-    if constexpr (PAIR) {
-      if (p.acc_int) umma_i8_pair(d, da + 2 * k, db + 2 * k, p.idesc, accum);
-      else umma_f16_pair(d, da + 2 * k, db + 2 * k, p.idesc, accum);
-    } else {
-      if (p.acc_int) umma_i8(d, da + 2 * k, db + 2 * k, p.idesc, accum);
-      else umma_f16(d, da + 2 * k, db + (uint64_t)(p.b_kstep * k), p.idesc, accum);
-    }
+    if (p.acc_int) issue_one<PAIR, true>(d, desc64(la + 2 * k, p.desc_hi), desc64(lb + 2 * k, p.desc_hi), p.idesc, accum);
+    else issue_one<PAIR, false>(d, desc64(la + 2 * k, p.desc_hi), desc64(lb + (uint32_t)(p.b_kstep * k), p.desc_hi), p.idesc, accum);
     accum = 1;
   }
 }
+// Row and column of a tile; consecutive tiles of a unit lie tile_step apart.
+template <bool V> struct BoolConst { static constexpr bool value = V; };
+struct TileWalk {
+  int mi, ni;
+  __device__ __forceinline__ TileWalk(const UmmaParams& p, int tile) { ni = tile / p.m_tiles; mi = tile - ni * p.m_tiles; }
+  __device__ __forceinline__ bool next(const UmmaParams& p, int step) {   // true when the column changed
+    mi += step;
+    const bool wrapped = mi >= p.m_tiles;
+    while (mi >= p.m_tiles) { mi -= p.m_tiles; ++ni; }
+    return wrapped;
+  }
+};
 
 // --------------------------------------------------------------------- kernel ----
 // MODE 3: staged epilogue, further straight-line forms: LeakyReLU before the optional residual (Darknet) or GELU, two-byte
@@ -985,7 +1014,7 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                  const __grid_constant__ CUtensorMap tmR, const UmmaParams p) {
   constexpr bool STAGED = MODE != 0;
   constexpr int kPair = PAIR ? 1 : 0;
-  constexpr int kEpilogueWarps = EpiCfg<STAGED>::kWarps, kLoaderWarp = EpiCfg<STAGED>::kLoaderWarp, kStorerWarp = EpiCfg<STAGED>::kStorerWarp;
+  constexpr int kEpilogueWarps = EpiCfg<STAGED>::kWarps, kFilterWarp = EpiCfg<STAGED>::kFilterWarp, kStorerWarp = EpiCfg<STAGED>::kStorerWarp;
   constexpr int CW = EpiCfg<STAGED>::kChunk;
   extern __shared__ uint8_t smem_raw[];
   if (threadIdx.x == 0) TS(7);
@@ -1000,16 +1029,15 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint64_t* tempty_bar = tfull_bar + 2;            // [2]
   uint64_t* box_full = tempty_bar + 2;             // [ring] box is armed: free, and its residual (if any) has landed
   uint64_t* box_done = box_full + kMaxRing;        // [ring] every epilogue warp that owns part of the box has written it
-  uint64_t* box_free = box_done + kMaxRing;        // [ring] the TMA store has finished reading the box
-  uint32_t* tmem_slot = (uint32_t*)(box_free + kMaxRing);
+  uint32_t* tmem_slot = (uint32_t*)(box_done + kMaxRing);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < p.stages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (int s = 0; s < p.stages; ++s) { mbar_init(&full_bar[s], 2); mbar_init(&empty_bar[s], 1); }   // (a full stage: both producers have armed it and every byte has landed)
     // in pair mode the epilogue warps of both CTAs release an accumulator on the first CTA's barrier
     for (int a = 0; a < 2; ++a) { mbar_init(&tfull_bar[a], 1); mbar_init(&tempty_bar[a], (uint32_t)(kEpilogueWarps << kPair)); }
-    for (int b = 0; b < kMaxRing; ++b) { mbar_init(&box_full[b], 1); mbar_init(&box_done[b], (uint32_t)p.box_arrivals); mbar_init(&box_free[b], 1); }
+    for (int b = 0; b < kMaxRing; ++b) { mbar_init(&box_full[b], 1); mbar_init(&box_done[b], (uint32_t)p.box_arrivals); }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -1029,8 +1057,8 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   // Programmatic dependent launch: everything above overlapped the previous kernel's tail.  Only the threads that touch
-  // tensors other kernels write or read wait for that kernel (grid_dependency_wait): the producer -- which first issues
-  // the filter loads of its first stages, constants nobody writes --, the residual loader, the storer and direct epilogues.
+  // tensors other kernels write or read wait for that kernel (grid_dependency_wait): the producer of A, the storer and direct
+  // epilogues.  The producer of B does not when its boxes come from constants: they are on the way early.
   if (threadIdx.x == 0) TS(0);
 
   const uint32_t a_box = (uint32_t)(BM * p.kb_bytes), b_box = (uint32_t)(p.bn_load * p.kb_bytes);
@@ -1039,97 +1067,108 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int rank = PAIR ? (int)cluster_ctarank() : 0;
   const int tile_first = (int)(blockIdx.x >> kPair), tile_step = (int)(gridDim.x >> kPair);
   if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer ----
-    // One lane runs this loop; it is kept free of divisions (filter tap, channel chunk, stage and
-    // phase are running counters) because its instruction rate bounds the rate of k-blocks.
+    // ------------------------------------------------------------ producer of A ----
+    // One lane; its instruction rate bounds the rate of stages.  The pixel a tile starts at is carried from tile to tile.
+    if (elect_one()) {
+      prefetch_map(&tmA);
+      grid_dependency_wait();
+      asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the next kernel may start its own prologue now
+      const uint32_t bytes_kb = PAIR ? 2u * a_box : a_box;              // the first CTA's barrier counts the bytes of both
+      const uint32_t sa0 = smem_u32(smem), full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
+      const uint32_t land0 = PAIR ? map_to_cta(full0, 0) : full0;       // the barriers the copies signal
+      auto produce = [&](auto im2col_mode) {
+        constexpr bool IM2COL = decltype(im2col_mode)::value;
+        bool ok = true;
+        int s = 0;
+        uint32_t ph = 1, sa_stage = sa0;   // a stage is free when its phase differs: the first round passes at once
+        TileWalk at(p, tile_first);
+        int img = 0, op = 0, oq = 0, d_img = 0, d_op = 0, d_oq = 0;
+        auto locate = [&](int pix, int& i, int& r, int& c) { const int pq = p.P * p.Q; i = pix / pq; pix -= i * pq; r = pix / p.Q; c = pix - r * p.Q; };
+        if (IM2COL) {
+          locate(((at.mi << kPair) + rank) * BM, img, op, oq);
+          locate((tile_step << kPair) * BM, d_img, d_op, d_oq);
+        }
+        for (int tile = tile_first; tile < p.total_tiles && ok; tile += tile_step) {
+          const int m0 = ((at.mi << kPair) + rank) * BM;
+          const int w0 = oq * p.stride_w - p.pad_l, h0 = op * p.stride_h - p.pad_t;
+          int fr = 0, fs = 0, c0 = 0, left = p.num_kb;
+          while (left > 0) {
+            if (!mbar_try_wait_at(empty0 + 8u * s, ph) && !mbar_wait(empty_bar + s, ph, abort_flag, p.status, 1, p.spin_limit)) { ok = false; break; }
+            const int nb = left < p.bps ? left : p.bps;
+            left -= nb;
+            // Test hook (never set by the planner): this stage is neither armed nor loaded, so its barrier can never
+            // complete and the MMA lane's bounded wait reports a timeout; nothing faults and nothing spins for ever.
+            const bool skip = !PAIR && p.test_skip_stage && blockIdx.x == 0 && tile == tile_first && left == 0;
+            if (!skip && (!PAIR || rank == 0)) mbar_expect_tx_at(full0 + 8u * s, (uint32_t)nb * bytes_kb);
+            const uint32_t land = land0 + 8u * s;
+            uint32_t sa = sa_stage;
+            for (int j = skip ? nb : 0; j < nb; ++j) {
+              if (IM2COL) load_im2col_at<PAIR>(sa, &tmA, land, c0, w0, h0, img, (uint16_t)fs, (uint16_t)fr);
+              else load_2d_at<PAIR>(sa, &tmA, land, c0, m0);
+              sa += a_box;
+              c0 += p.kbe;
+              if (c0 >= p.C) {
+                c0 = 0;
+                if (IM2COL && ++fs == p.S) { fs = 0; if (++fr == p.R) fr = 0; }   // the next filter term walks the window again
+              }
+            }
+            sa_stage += (uint32_t)stage_bytes;
+            if (++s == p.stages) { s = 0; ph ^= 1; sa_stage = sa0; }
+          }
+          const bool wrapped = at.next(p, tile_step);
+          if (IM2COL) {
+            if (wrapped) locate(((at.mi << kPair) + rank) * BM, img, op, oq);
+            else {
+              oq += d_oq; if (oq >= p.Q) { oq -= p.Q; ++op; }
+              op += d_op; if (op >= p.P) { op -= p.P; ++img; }
+              img += d_img;
+            }
+          }
+        }
+        if (!ok) {
+          // give copies already in flight a bounded chance to land before shared memory goes away
+          for (int i = 0; i < p.stages; ++i)
+            for (uint32_t n = 0; n < 4096; ++n)
+              if (mbar_try_wait(&full_bar[i], 0) || mbar_try_wait(&full_bar[i], 1)) break;
+        }
+      };
+      if (p.im2col) produce(BoolConst<true>{}); else produce(BoolConst<false>{});
+    }
+  } else if (warp == kFilterWarp) {
+    // ------------------------------------------------------------ producer of B ----
     if (elect_one()) {
       prefetch_map(&tmB);
-      prefetch_map(&tmA);
-      // where the walk over a tile's k-blocks and over the stage ring stands
-      struct Walk { int tap, fr, fs, c0, left, s; uint32_t ph; };
-      Walk k{0, 0, 0, 0, 0, 0, 0};
-      int w0 = 0, h0 = 0, img = 0, m0 = 0, n0 = 0, bidx = 0;
-      // One stage: its k-blocks of A (do_a) and B (do_b), each load signalling the stage's barrier, which do_b arms with the
-      // byte count of both.
-      auto fill = [&](bool do_a, bool do_b, bool skip) {
-        const int nb = k.left < p.bps ? k.left : p.bps;
-        k.left -= nb;
-        uint8_t* sa = smem + (size_t)k.s * stage_bytes;
-        uint8_t* sb = sa + (size_t)p.bps * a_box;
-        uint64_t* fb = full_bar + k.s;
-        uint32_t fbc = 0;
-        if constexpr (PAIR) {
-          // the first CTA's barrier counts the bytes of both CTAs; only it is armed
-          if (do_b && rank == 0) mbar_expect_tx(fb, 2u * (uint32_t)nb * (a_box + b_box));
-          fbc = map_to_cta(smem_u32(fb), 0);
-        } else if (do_b && !skip) mbar_expect_tx(fb, (uint32_t)nb * (a_box + b_box));
-        for (int j = 0; j < nb; ++j) {
-          if constexpr (PAIR) {
-            if (do_b) {
-              const int nb0 = n0 + rank * p.bn_load;
-              if (p.rows_per_batch) tma_load_3d_pair(sb, &tmB, fbc, k.c0, nb0, bidx);
-              else tma_load_3d_pair(sb, &tmB, fbc, k.c0, k.tap, nb0);
-            }
-            if (do_a) {
-              if (p.im2col) tma_load_im2col_4d_pair(sa, &tmA, fbc, k.c0, w0, h0, img, (uint16_t)k.fs, (uint16_t)k.fr);
-              else tma_load_2d_pair(sa, &tmA, fbc, k.c0, m0);
-            }
-          } else if (!skip) {
-            if (do_b) {
-              if (p.rows_per_batch) tma_load_3d(sb, &tmB, fb, p.b_n_major ? n0 : k.c0, p.b_n_major ? k.c0 : n0, bidx);
-              else tma_load_3d(sb, &tmB, fb, k.c0, k.tap, n0);
-            }
-            if (do_a) {
-              if (p.im2col) tma_load_im2col_4d(sa, &tmA, fb, k.c0, w0, h0, img, (uint16_t)k.fs, (uint16_t)k.fr);
-              else tma_load_2d(sa, &tmA, fb, k.c0, m0);
-            }
-          }
-          sa += a_box;
-          sb += b_box;
-          k.c0 += p.kbe;
-          if (k.c0 >= p.C) {
-            k.c0 = 0;
-            ++k.tap;
-            if (++k.fs == p.S) { k.fs = 0; if (++k.fr == p.R) k.fr = 0; }   // the next filter term walks the window again
-          }
-        }
-        if (++k.s == p.stages) { k.s = 0; k.ph ^= 1; }
-      };
+      if (!p.b_constant) grid_dependency_wait();
+      const uint32_t bytes_kb = PAIR ? 2u * b_box : b_box;
+      const uint32_t sb0 = smem_u32(smem) + (uint32_t)p.bps * a_box, full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
+      const uint32_t land0 = PAIR ? map_to_cta(full0, 0) : full0;
       bool ok = true;
-      for (int tile = tile_first; tile < p.total_tiles && ok; tile += tile_step) {
-        m0 = (((tile % p.m_tiles) << kPair) + rank) * BM;
-        n0 = (tile / p.m_tiles) * p.BN;
-        if (p.im2col) {
-          const int pq = p.P * p.Q;
-          img = m0 / pq;
-          const int rem = m0 - img * pq;
-          const int op = rem / p.Q, oq = rem - op * p.Q;
-          w0 = oq * p.stride_w - p.pad_l;
-          h0 = op * p.stride_h - p.pad_t;
-        }
-        k.tap = k.fr = k.fs = k.c0 = 0;
-        k.left = p.num_kb;
-        bidx = p.rows_per_batch ? m0 / p.rows_per_batch : 0;
-        int it = 0;
-        if (tile == tile_first) {
-          // The first stages are free: their filter boxes are on the way before the previous kernel has finished.
-          const int early = p.early_b < p.num_it ? p.early_b : p.num_it;
-          const Walk start = k;
-          for (int e = 0; e < early; ++e) fill(false, true, false);
-          grid_dependency_wait();
-          asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the next kernel may start its own prologue now
-          k = start;
-          for (; it < early; ++it) fill(true, false, false);
-        }
-        for (; it < p.num_it; ++it) {
-          if (!mbar_wait(empty_bar + k.s, k.ph ^ 1, abort_flag, p.status, 1, p.spin_limit)) { ok = false; break; }
-          // Test hook (never set by the planner): this stage is neither armed nor loaded, so its barrier can never
-          // complete and the MMA lane's bounded wait reports a timeout; nothing faults and nothing spins for ever.
-          fill(true, true, p.test_skip_stage && blockIdx.x == 0 && tile == tile_first && it == p.num_it - 1);
+      int s = 0;
+      uint32_t ph = 1, sb_stage = sb0;
+      TileWalk at(p, tile_first);
+      for (int tile = tile_first; tile < p.total_tiles && ok; tile += tile_step, at.next(p, tile_step)) {
+        const int n0 = at.ni * p.BN + (PAIR ? rank * p.bn_load : 0);
+        const int bidx = p.rows_per_batch ? ((at.mi << kPair) + rank) * BM / p.rows_per_batch : 0;
+        int c0 = 0, tap = 0, left = p.num_kb;
+        while (left > 0) {
+          if (!mbar_try_wait_at(empty0 + 8u * s, ph) && !mbar_wait(empty_bar + s, ph, abort_flag, p.status, 8, p.spin_limit)) { ok = false; break; }
+          const int nb = left < p.bps ? left : p.bps;
+          left -= nb;
+          if (!PAIR || rank == 0) mbar_expect_tx_at(full0 + 8u * s, (uint32_t)nb * bytes_kb);
+          const uint32_t land = land0 + 8u * s;
+          uint32_t sb = sb_stage;
+          for (int j = 0; j < nb; ++j) {
+            if (p.rows_per_batch) load_3d_at<PAIR>(sb, &tmB, land, p.b_n_major ? n0 : c0, p.b_n_major ? c0 : n0, bidx);
+            else load_3d_at<PAIR>(sb, &tmB, land, c0, tap, n0);
+            sb += b_box;
+            c0 += p.kbe;
+            if (c0 >= p.C) { c0 = 0; ++tap; }
+          }
+          sb_stage += (uint32_t)stage_bytes;
+          if (++s == p.stages) { s = 0; ph ^= 1; sb_stage = sb0; }
         }
       }
       if (!ok) {
-        // give copies already in flight a bounded chance to land before shared memory goes away
         for (int i = 0; i < p.stages; ++i)
           for (uint32_t n = 0; n < 4096; ++n)
             if (mbar_try_wait(&full_bar[i], 0) || mbar_try_wait(&full_bar[i], 1)) break;
@@ -1141,9 +1180,11 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       int s = 0;
       uint32_t ph = 0, tcount = 0;
       bool ok = true;
-      const uint32_t smem_base = smem_u32(smem);
-      const uint64_t desc_fixed = ((uint64_t)p.desc_hi << 32) | (1ull << 16);
       const int ksteps = p.kb_bytes >> 5;  // 32 bytes of K per instruction
+      // low descriptor words of the current stage's first boxes (addresses in 16-byte units; shared memory ends below 2^18)
+      const uint32_t lo0 = (1u << 16) | (smem_u32(smem) >> 4), lo_stage = (uint32_t)stage_bytes >> 4, lo_b = ((uint32_t)p.bps * a_box) >> 4;
+      const uint32_t full0 = smem_u32(full_bar);
+      uint32_t lo = lo0;
       for (int tile = tile_first; tile < p.total_tiles && ok; tile += tile_step, ++tcount) {
         const uint32_t acc = tcount & 1, acc_ph = (tcount >> 1) & 1;
         if (!mbar_wait(&tempty_bar[acc], acc_ph ^ 1, abort_flag, p.status, 2, p.spin_limit)) { ok = false; break; }
@@ -1151,83 +1192,69 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const uint32_t tmem_d = tmem_base + acc * (uint32_t)p.BN;
         int left = p.num_kb;
         uint32_t accum = 0;
-        for (int it = 0; it < p.num_it; ++it) {
-          if (!mbar_wait(full_bar + s, ph, abort_flag, p.status, 3, p.spin_limit)) { ok = false; break; }
+        while (left > 0) {
+          if (!mbar_try_wait_at(full0 + 8u * s, ph) && !mbar_wait(full_bar + s, ph, abort_flag, p.status, 3, p.spin_limit)) { ok = false; break; }
           tc_fence_after();
           const int nb = left < p.bps ? left : p.bps;
           left -= nb;
-          uint32_t sa = smem_base + (uint32_t)s * (uint32_t)stage_bytes, sb = sa + (uint32_t)p.bps * a_box;
+          uint32_t la = lo, lb = lo + lo_b;
           for (int j = 0; j < nb; ++j) {
-            const uint64_t da = desc_fixed | (uint64_t)((sa & 0x3FFFF) >> 4);
-            const uint64_t db = desc_fixed | (uint64_t)((sb & 0x3FFFF) >> 4);
-            issue_kblock<PAIR>(p, tmem_d, da, db, ksteps, accum);
+            issue_kblock<PAIR>(p, tmem_d, la, lb, ksteps, accum);
             accum = 1;
-            sa += a_box;
-            sb += b_box;
+            la += a_box >> 4;
+            lb += b_box >> 4;
           }
           if constexpr (PAIR) umma_commit_pair(empty_bar + s); else umma_commit(empty_bar + s);  // frees the stage once these MMAs have read it
-          if (++s == p.stages) { s = 0; ph ^= 1; }
+          lo += lo_stage;
+          if (++s == p.stages) { s = 0; ph ^= 1; lo = lo0; }
         }
         if (ok) { if constexpr (PAIR) umma_commit_pair(&tfull_bar[acc]); else umma_commit(&tfull_bar[acc]); }  // accumulator complete
         if (tcount == 0) TS(3);
       }
     }
-  } else if (warp == kLoaderWarp) {
-    // -------------------------------------------- staging ring: arm boxes (residual loads) ----
-    if (STAGED && elect_one()) {
-      if (p.res_tma) {
-        prefetch_map(&tmR);
-        grid_dependency_wait();
-      }
-      const int cols_per_box = 128 / p.out_esz;
-      int slot = 0;
-      uint32_t ph = 0;
-      bool ok = true;
-      for (int tile = tile_first; tile < p.total_tiles && ok; tile += tile_step) {
-        const int m0 = (((tile % p.m_tiles) << kPair) + rank) * BM, n0 = (tile / p.m_tiles) * p.BN;
-        for (int bx = 0; bx < p.stage_boxes; ++bx) {
-          const int x0 = n0 + bx * cols_per_box;
-          if (x0 >= p.K_out) break;
-          if (!mbar_wait(box_free + slot, ph ^ 1, abort_flag, p.status, 5, p.spin_limit)) { ok = false; break; }
-          if (p.res_tma) {
-            mbar_expect_tx(box_full + slot, 16384u);
-            tma_load_2d(staging + slot * 16384, &tmR, box_full + slot, x0, m0);
-          } else {
-            mbar_arrive(box_full + slot);
-          }
-          if (++slot == p.ring_boxes) { slot = 0; ph ^= 1; }
-        }
-      }
-      if (!ok && p.res_tma) {
-        // residual loads already in flight get a bounded chance to land before shared memory goes away
-        for (int i = 0; i < p.ring_boxes; ++i)
-          for (uint32_t k = 0; k < 4096; ++k)
-            if (mbar_try_wait(&box_full[i], 0) || mbar_try_wait(&box_full[i], 1)) break;
-      }
-    }
   } else if (warp == kStorerWarp) {
-    // ------------------------------------------------ staging ring: store finished boxes ----
+    // -------------------------- staging ring: store finished boxes, arm them again (residual loads) ----
     if (STAGED && elect_one()) {
       prefetch_map(&tmY);
-      grid_dependency_wait();   // earlier kernels may still read what the stores overwrite
+      if (p.res_tma) prefetch_map(&tmR);
+      grid_dependency_wait();   // earlier kernels may still read what the stores overwrite, and write the residual
       const int cols_per_box = 128 / p.out_esz;
       const uint32_t staging_u32 = smem_u32(staging);
-      int slot = 0, prev = -1;
+      // Arming runs ring_boxes ahead of storing: a box is armed for its next use as soon as its store has read it.
+      int a_tile = tile_first, a_bx = 0, a_slot = 0;
+      TileWalk a_at(p, tile_first);
+      auto arm = [&]() {
+        if (a_tile >= p.total_tiles) return;
+        if (p.res_tma) {
+          mbar_expect_tx(box_full + a_slot, 16384u);
+          tma_load_2d(staging + a_slot * 16384, &tmR, box_full + a_slot, a_at.ni * p.BN + a_bx * cols_per_box, ((a_at.mi << kPair) + rank) * BM);
+        } else {
+          mbar_arrive(box_full + a_slot);
+        }
+        if (++a_slot == p.ring_boxes) a_slot = 0;
+        if (++a_bx == p.stage_boxes || a_at.ni * p.BN + a_bx * cols_per_box >= p.K_out) { a_bx = 0; a_tile += tile_step; a_at.next(p, tile_step); }
+      };
+      for (int b = 0; b < p.ring_boxes; ++b) arm();
+      int slot = 0;
+      bool unread = false;   // the newest store may still be reading its box
       uint32_t ph = 0;
       bool ok = true;
-      for (int tile = tile_first; tile < p.total_tiles && ok; tile += tile_step) {
-        const int m0 = (((tile % p.m_tiles) << kPair) + rank) * BM, n0 = (tile / p.m_tiles) * p.BN;
+      TileWalk at(p, tile_first);
+      for (int tile = tile_first; tile < p.total_tiles && ok; tile += tile_step, at.next(p, tile_step)) {
+        const int m0 = ((at.mi << kPair) + rank) * BM, n0 = at.ni * p.BN;
         for (int bx = 0; bx < p.stage_boxes; ++bx) {
           const int x0 = n0 + bx * cols_per_box;
           if (x0 >= p.K_out) break;
           // Nothing to send yet: use the wait to let the last store finish reading its box and hand that box back,
           // so that the next tile's epilogue never waits for this tile's boxes to be stored.
-          if (prev >= 0 && !mbar_try_wait(box_done + slot, ph)) {
-            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-            mbar_arrive(box_free + prev);
-            prev = -1;
+          if (!mbar_try_wait(box_done + slot, ph)) {
+            if (unread) {
+              asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+              arm();
+              unread = false;
+            }
+            if (!mbar_wait(box_done + slot, ph, abort_flag, p.status, 7, p.spin_limit)) { ok = false; break; }
           }
-          if (!mbar_wait(box_done + slot, ph, abort_flag, p.status, 7, p.spin_limit)) { ok = false; break; }
           if (p.store_mode == 0) {
             asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"((uint64_t)&tmY),
                          "r"(staging_u32 + (uint32_t)slot * 16384u), "r"(x0), "r"(m0)
@@ -1243,13 +1270,19 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                          : "memory");
           }
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-          if (prev >= 0) {
+          if (unread) {
             asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");  // every store but the newest has read its box
-            mbar_arrive(box_free + prev);
+            arm();
           }
-          prev = slot;
+          unread = true;
           if (++slot == p.ring_boxes) { slot = 0; ph ^= 1; }
         }
+      }
+      if (!ok && p.res_tma) {
+        // residual loads already in flight get a bounded chance to land before shared memory goes away
+        for (int i = 0; i < p.ring_boxes; ++i)
+          for (uint32_t k = 0; k < 4096; ++k)
+            if (mbar_try_wait(&box_full[i], 0) || mbar_try_wait(&box_full[i], 1)) break;
       }
       asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // stores complete before shared memory is released
     }
@@ -1279,9 +1312,10 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const bool fast_relu = p.ep.act == ACT_RELU;
       const float fast_lo = fast_relu ? 0.f : -128.f;
       const uint32_t fast_floor = fast_relu ? 0u : (OUT == DT_F16 ? 0xFC00FC00u : 0xFF80FF80u);
-      for (int tile = tile_first; tile < p.total_tiles && ok; tile += tile_step, ++tcount) {
+      TileWalk at(p, tile_first);
+      for (int tile = tile_first; tile < p.total_tiles && ok; tile += tile_step, ++tcount, at.next(p, tile_step)) {
         const uint32_t acc = tcount & 1, acc_ph = (tcount >> 1) & 1;
-        const int n0 = (tile / p.m_tiles) * p.BN;
+        const int n0 = at.ni * p.BN;
         if (!mbar_wait(&tfull_bar[acc], acc_ph, abort_flag, p.status, 4, p.spin_limit)) { ok = false; break; }
         tc_fence_after();
         if (tcount == 0 && threadIdx.x == 64) TS(4);
@@ -1894,7 +1928,7 @@ UmmaLaunch* umma_conv_prepare(const UmmaConv& c, const void* x, const void* w, v
   // Test hooks for the time-out path (tests/test_conv_umma_gpu.py): a short limit and one deliberately unarmed stage.
   if (const char* e = getenv("ODLA_B200_TEST_SPIN_LIMIT")) { const long v = atol(e); if (v >= 64 && v <= (1l << 18)) p.spin_limit = (uint32_t)v; }
   if (getenv("ODLA_B200_TEST_SKIP_STAGE") && !p.pair) p.test_skip_stage = 1;
-  p.early_b = c.w_constant && !p.test_skip_stage ? p.stages : 0;
+  p.b_constant = c.w_constant;
   L->grid = p.pair ? (2 * p.total_tiles < (sms & ~1) ? 2 * p.total_tiles : (sms & ~1)) : (p.total_tiles < sms ? p.total_tiles : sms);
   L->smem = (size_t)p.stages * stage_bytes + (size_t)p.ring_boxes * 16384 + 1024 /*alignment slack*/ + 1024 /*barriers*/;
   if (L->smem > 227 * 1024) { delete L; return nullptr; }
