@@ -118,6 +118,8 @@ struct UmmaConv {
   int w_terms = 0;
   // w is written by no kernel (a constant uploaded before the first launch): its loads need not wait for the kernel in front.
   int w_constant = 0;
+  // Output rows of the whole recorded batch when this launch computes a share of them (0: all of them are here).
+  long long rows_full = 0;
 };
 // True when the tensor-core kernel can run this problem.
 bool umma_conv_supported(const UmmaConv& p);

@@ -29,6 +29,7 @@
 // exit where tensor memory is released.  The host reports ODLA_TIMEOUT.
 #include <cuda.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -85,6 +86,10 @@ struct UmmaParams {
   int fast_variant;    // mode 1: accumulator conversion (0 fp32, 1 int32 by conversion, 2 int32 by integer add) * 2 + residual
   int tmem_cols;
   uint32_t spin_limit;  // attempts before a bounded wait gives up
+  int splits;          // > 1: the split kernel, this many CTAs share a tile's reduction
+  int bm;              // rows of its tiles: 128 or 64
+  int split_data_bytes;  // ... shared memory before its barriers: the operand stages, reused by the partial tile
+  int y_ld;            // row pitch of y in elements (split kernel)
   int b_constant;      // B is written by no kernel: its loads need not wait for the kernel in front
   int test_skip_stage;  // test hook: the producer of CTA 0 leaves the last stage of its first tile unarmed, so the MMA lane's wait runs out
   void* y;
@@ -1460,6 +1465,275 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
 }
 
+// ------------------------------------------------------- few tiles: split reductions ----
+// A launch whose tiles leave most of the chip idle (a batch of one, the deep layers of a few images, a classifier) is bound by
+// the serial walk of each tile over its k-blocks, not by any throughput.  Here the 2 to 8 CTAs of a cluster share a tile of 64
+// or 128 rows by 16 to 64 columns: each walks a contiguous share of the k-blocks, leaves its 32-bit partial tile in its own
+// shared memory, and after a cluster barrier adds up, finishes and stores a share of the rows, reading its peers' partials in
+// rank order, so that the result does not depend on timing (int32 partial sums are exact).  Residuals are fetched while the
+// products run.
+constexpr int kSplitThreads = 352, kSplitEpiWarps = 8;   // producer of A, MMA issuer, eight warps that empty tensor memory, producer of B
+constexpr int kSplitRows = 4;                             // rows one thread finishes, at most (128 rows x 16 pieces / 2 CTAs / 256 threads)
+struct SplitShared { uint64_t full[8], empty[8], done; uint32_t tmem; int abort; };
+
+// What four neighbouring columns need from the epilogue's per-channel vectors; one thread keeps the same columns for all its rows.
+struct FourColumns { float mul[4], add1[4], add2[4]; };
+__device__ __forceinline__ void load_four_columns(const Epilogue& ep, int col, FourColumns& f) {
+  auto vec = [&](const float* src, float (&o)[4]) { const float4 v = __ldg((const float4*)(src + col)); o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w; };
+  if (ep.mul) vec(ep.mul, f.mul);
+  if (ep.add1) vec(ep.add1, f.add1);
+  if (ep.add2) vec(ep.add2, f.add2);
+}
+// The residual of four neighbouring results as it lies in memory (up to 16 bytes).
+__device__ __forceinline__ uint4 load_four_residuals(const Epilogue& ep, int64_t at) {
+  uint4 u = make_uint4(0, 0, 0, 0);
+  if (ep.res_dt == DT_F16 || ep.res_dt == DT_BF16) { const uint2 t = *(const uint2*)((const uint16_t*)ep.res + at); u.x = t.x; u.y = t.y; }
+  else if (ep.res_dt == DT_S8) u.x = *(const uint32_t*)((const int8_t*)ep.res + at);
+  else u = *(const uint4*)((const float*)ep.res + at);
+  return u;
+}
+// Finishes and stores four neighbouring results of one row, with the arithmetic of epilogue_value (every step rounded by itself).
+__device__ __forceinline__ void finish_four(const UmmaParams& p, float (&v)[4], int64_t row, int col, const FourColumns& f, const uint4& res) {
+  const Epilogue& ep = p.ep;
+  if (ep.mul) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = __fmul_rn(v[j], f.mul[j]);
+  }
+  if (ep.alpha != 1.f) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = __fmul_rn(v[j], ep.alpha);
+  }
+  if (ep.add1) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = __fadd_rn(v[j], f.add1[j]);
+  }
+  if (ep.add2) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = __fadd_rn(v[j], f.add2[j]);
+  }
+  if (ep.act_first) apply_act_all<4>(ep.act, v, ep.act_a, ep.act_b);
+  if (ep.res) {
+    const uint32_t w[4] = {res.x, res.y, res.z, res.w};
+    float r[4];
+    if (ep.res_dt == DT_F16 || ep.res_dt == DT_BF16) {
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        const float2 h = ep.res_dt == DT_F16 ? __half22float2(*(const __half2*)&w[t]) : __bfloat1622float2(*(const __nv_bfloat162*)&w[t]);
+        r[2 * t] = h.x; r[2 * t + 1] = h.y;
+      }
+    } else if (ep.res_dt == DT_S8) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) r[j] = __fmul_rn((float)(signed char)(w[0] >> (8 * j)), ep.res_scale);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) r[j] = __uint_as_float(w[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = __fadd_rn(v[j], r[j]);
+  }
+  if (!ep.act_first) apply_act_all<4>(ep.act, v, ep.act_a, ep.act_b);
+  const int64_t at = row * p.y_ld + col;
+  if (ep.out_dt == DT_F16 || ep.out_dt == DT_BF16) {
+    uint2 u;
+    uint32_t* w = (uint32_t*)&u;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      if (ep.out_dt == DT_F16) { const __half2 h = __floats2half2_rn(v[2 * t], v[2 * t + 1]); w[t] = *(const uint32_t*)&h; }
+      else { const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * t], v[2 * t + 1]); w[t] = *(const uint32_t*)&h; }
+    }
+    *(uint2*)((uint16_t*)p.y + at) = u;
+  } else if (ep.out_dt == DT_S8) {
+    uint32_t q[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) q[j] = (uint32_t)rne_sat_s8(ep.out_multiply ? __fmul_rn(v[j], ep.out_inv) : __fdiv_rn(v[j], ep.out_scale));
+    *(uint32_t*)((int8_t*)p.y + at) = __byte_perm(__byte_perm(q[0], q[1], 0x0040), __byte_perm(q[2], q[3], 0x0040), 0x5410);
+  } else {
+    *(float4*)((float*)p.y + at) = make_float4(v[0], v[1], v[2], v[3]);
+  }
+}
+
+__global__ void __launch_bounds__(kSplitThreads, 2)
+umma_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const UmmaParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  const int stage_bytes = p.bps * (p.bm + p.bn_load) * p.kb_bytes;
+  SplitShared& sh = *(SplitShared*)(smem + p.split_data_bytes);
+  volatile int* abort_flag = &sh.abort;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int swz = p.BN >= 32 ? 7 : 3;   // a row of the partial tile has BN / 4 pieces, at least 4
+  const int rank = (int)blockIdx.x % p.splits, tile = (int)blockIdx.x / p.splits;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < p.stages; ++s) { mbar_init(&sh.full[s], 2); mbar_init(&sh.empty[s], 1); }
+    mbar_init(&sh.done, 1);
+    sh.abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh.tmem)), "r"((uint32_t)p.tmem_cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = sh.tmem;
+  const uint32_t a_box = (uint32_t)(p.bm * p.kb_bytes), b_box = (uint32_t)(p.bn_load * p.kb_bytes);
+  const int ni = tile / p.m_tiles, m0 = (tile - ni * p.m_tiles) * p.bm, n0 = ni * p.BN;
+  const int kb_lo = (int)((int64_t)p.num_kb * rank / p.splits), kb_hi = (int)((int64_t)p.num_kb * (rank + 1) / p.splits);
+  // A thread's place in the final pass: four columns, the same for all its rows (the pass's 256 threads span whole rows).
+  const int per_row = p.BN >> 2, t = (int)threadIdx.x - 64, c4 = t & (per_row - 1), col = n0 + 4 * c4, row_step = (kSplitEpiWarps * 32) / per_row;
+  const int rows = min(p.bm, p.M_total - m0), r_lo = rows * rank / p.splits, r_hi = rows * (rank + 1) / p.splits;
+  const bool vec = (p.K_out & 3) == 0, finisher = warp >= 2 && warp < 2 + kSplitEpiWarps && col < p.K_out;
+  FourColumns fc;
+  uint4 res[kSplitRows];
+  if (warp == 0 || warp == 2 + kSplitEpiWarps) {
+    // ------------------------------------------------------------ producers of A and B ----
+    if (elect_one()) {
+      const bool do_a = warp == 0;
+      prefetch_map(do_a ? &tmA : &tmB);
+      if (do_a || !p.b_constant) grid_dependency_wait();
+      if (do_a) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+      int w0 = 0, h0 = 0, img = 0;
+      if (do_a && p.im2col) {
+        const int pq = p.P * p.Q;
+        img = m0 / pq;
+        const int rem = m0 - img * pq, op = rem / p.Q, oq = rem - op * p.Q;
+        w0 = oq * p.stride_w - p.pad_l;
+        h0 = op * p.stride_h - p.pad_t;
+      }
+      const int bidx = p.rows_per_batch ? m0 / p.rows_per_batch : 0;
+      int tap = kb_lo / p.chunks_per_tap, c0 = (kb_lo - tap * p.chunks_per_tap) * p.kbe;
+      int fr = (tap % (p.R * p.S)) / p.S, fs = tap % p.S, left = kb_hi - kb_lo, s = 0;
+      uint32_t ph = 1;
+      const uint32_t first = smem_u32(smem) + (do_a ? 0u : (uint32_t)p.bps * a_box), box = do_a ? a_box : b_box;
+      uint32_t at_stage = first;
+      bool ok = true;
+      while (left > 0) {
+        if (!mbar_wait(&sh.empty[s], ph, abort_flag, p.status, do_a ? 21 : 23, p.spin_limit)) { ok = false; break; }
+        const int nb = left < p.bps ? left : p.bps;
+        left -= nb;
+        const bool skip = do_a && p.test_skip_stage && blockIdx.x == 0 && left == 0;   // (the test hook of the persistent kernel)
+        const uint32_t land = smem_u32(&sh.full[s]);
+        if (!skip) mbar_expect_tx_at(land, (uint32_t)nb * box);
+        uint32_t dst = at_stage;
+        for (int j = skip ? nb : 0; j < nb; ++j) {
+          if (!do_a) {
+            if (p.rows_per_batch) load_3d_at<false>(dst, &tmB, land, p.b_n_major ? n0 : c0, p.b_n_major ? c0 : n0, bidx);
+            else load_3d_at<false>(dst, &tmB, land, c0, tap, n0);
+          } else if (p.im2col) load_im2col_at<false>(dst, &tmA, land, c0, w0, h0, img, (uint16_t)fs, (uint16_t)fr);
+          else load_2d_at<false>(dst, &tmA, land, c0, m0);
+          dst += box;
+          c0 += p.kbe;
+          if (c0 >= p.C) { c0 = 0; ++tap; if (++fs == p.S) { fs = 0; if (++fr == p.R) fr = 0; } }
+        }
+        at_stage += (uint32_t)stage_bytes;
+        if (++s == p.stages) { s = 0; ph ^= 1; at_stage = first; }
+      }
+      if (!ok)   // copies in flight get a bounded chance to land before shared memory goes away
+        for (int i = 0; i < p.stages; ++i)
+          for (uint32_t n = 0; n < 4096; ++n)
+            if (mbar_try_wait(&sh.full[i], 0) || mbar_try_wait(&sh.full[i], 1)) break;
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      int s = 0, left = kb_hi - kb_lo;
+      uint32_t ph = 0, accum = 0;
+      const int ksteps = p.kb_bytes >> 5;
+      const uint32_t lo0 = (1u << 16) | (smem_u32(smem) >> 4), lo_stage = (uint32_t)stage_bytes >> 4, lo_b = ((uint32_t)p.bps * a_box) >> 4;
+      uint32_t lo = lo0;
+      bool ok = true;
+      while (left > 0) {
+        if (!mbar_wait(&sh.full[s], ph, abort_flag, p.status, 22, p.spin_limit)) { ok = false; break; }
+        tc_fence_after();
+        const int nb = left < p.bps ? left : p.bps;
+        left -= nb;
+        uint32_t la = lo, lb = lo + lo_b;
+        for (int j = 0; j < nb; ++j) {
+          issue_kblock<false>(p, tmem, la, lb, ksteps, accum);
+          accum = 1;
+          la += a_box >> 4;
+          lb += b_box >> 4;
+        }
+        umma_commit(&sh.empty[s]);
+        lo += lo_stage;
+        if (++s == p.stages) { s = 0; ph ^= 1; lo = lo0; }
+      }
+      if (ok) umma_commit(&sh.done);
+    }
+  } else {
+    if (finisher && vec) load_four_columns(p.ep, col, fc);
+    grid_dependency_wait();   // residuals are read, and tensors earlier kernels may still read overwritten, from here on
+    if (finisher && vec && p.ep.res) {
+#pragma unroll
+      for (int i = 0; i < kSplitRows; ++i) {
+        const int r = r_lo + t / per_row + i * row_step;
+        if (r < r_hi) res[i] = load_four_residuals(p.ep, ((int64_t)m0 + r) * p.K_out + col);
+      }
+    }
+    // the accumulators go to shared memory as 16-byte pieces, row r's piece c at c ^ (r & 7): rows apart by whole bank cycles
+    // are then written, and neighbouring pieces of a row read, without conflicts
+    // (64-row products occupy the first 16 lanes of every quarter of tensor memory)
+    const int quarter = warp & 3, r = p.bm == 64 ? quarter * 16 + (lane & 15) : quarter * 32 + lane;
+    const bool lane_ok = p.bm == 128 || lane < 16;
+    if (mbar_wait(&sh.done, 0, abort_flag, p.status, 24, p.spin_limit)) {
+      tc_fence_after();
+      const uint32_t row_at = smem_u32(smem) + (uint32_t)(r * p.BN * 4);
+      for (int c = (warp - 2) >> 2; c < p.BN / 16; c += kSplitEpiWarps / 4) {
+        uint32_t v[16];
+        tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(c * 16), v);
+        tmem_ld_wait_regs<16>(v);
+        if (lane_ok) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) sts128(row_at + (uint32_t)(((4 * c + q) ^ (r & swz)) << 4), make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
+        }
+      }
+    }
+  }
+  __syncwarp();
+  tc_fence_before();
+  cluster_sync_all();
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)p.tmem_cols) : "memory");
+  }
+  if (finisher) {
+    const uint32_t base = smem_u32(smem);
+#pragma unroll
+    for (int i = 0; i < kSplitRows; ++i) {
+      const int r = r_lo + t / per_row + i * row_step;
+      if (r >= r_hi) break;
+      const uint32_t at = base + (uint32_t)(r * p.BN * 4) + (uint32_t)((c4 ^ (r & swz)) << 4);
+      const int64_t row = (int64_t)m0 + r;
+      uint4 u[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (k < p.splits)
+          asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(u[k].x), "=r"(u[k].y), "=r"(u[k].z), "=r"(u[k].w) : "r"(map_to_cta(at, (uint32_t)k)) : "memory");
+      float v[4];
+      if (p.acc_int) {
+        int4 a = make_int4((int)u[0].x, (int)u[0].y, (int)u[0].z, (int)u[0].w);
+#pragma unroll
+        for (int k = 1; k < 8; ++k) if (k < p.splits) { a.x += (int)u[k].x; a.y += (int)u[k].y; a.z += (int)u[k].z; a.w += (int)u[k].w; }
+        if (p.ep.out_dt == DT_S32) {
+          const int raw[4] = {a.x, a.y, a.z, a.w};
+          for (int j = 0; j < 4 && col + j < p.K_out; ++j) ((int32_t*)p.y)[row * p.K_out + col + j] = raw[j];
+          continue;
+        }
+        v[0] = (float)a.x; v[1] = (float)a.y; v[2] = (float)a.z; v[3] = (float)a.w;
+      } else {
+        v[0] = __uint_as_float(u[0].x); v[1] = __uint_as_float(u[0].y); v[2] = __uint_as_float(u[0].z); v[3] = __uint_as_float(u[0].w);
+#pragma unroll
+        for (int k = 1; k < 8; ++k)
+          if (k < p.splits) { v[0] += __uint_as_float(u[k].x); v[1] += __uint_as_float(u[k].y); v[2] += __uint_as_float(u[k].z); v[3] += __uint_as_float(u[k].w); }
+      }
+      if (vec && !p.ep.add_full) finish_four(p, v, row, col, fc, res[i]);
+      else
+        for (int j = 0; j < 4 && col + j < p.K_out; ++j) store_from_float(p.y, p.ep.out_dt, row * p.y_ld + col + j, epilogue_value(p.ep, v[j], row, col + j, p.K_out));
+    }
+  }
+  cluster_sync_all();   // nobody leaves while a peer may still read its partial tile
+}
+
 // ------------------------------------------------------------ fused attention ----
 // softmax(scale * Q K^T) V for heads of 64 channels and any number of positions (two-byte types).  One CTA works on one
 // block of 128 query rows of one head at a time and keeps the scores of 128 x 128 (query, key) pairs in tensor memory -- they
@@ -1780,6 +2054,41 @@ bool umma_store_perm_ok(const UmmaConv& c, const Epilogue& ep, const void* y) {
   return M % ((long long)c.store_S * c.store_NH) == 0 && c.K == c.store_D;
 }
 
+// Whether the CTAs of a cluster share each tile's reduction (umma_split_kernel), and over which tiles.  How many share it
+// changes the order in which floating-point sums are taken, so that number is decided from the rows of the whole recorded
+// batch and not from this launch's share of them: a row's result does not depend on how a batch is cut over GPUs or
+// sub-batches.  The tile's shape then follows the launch's own rows.  In clocks, measured on 3x3 layers of one image with 9 to
+// 144 k-blocks: one takes 176 of a persistent CTA's walk, 200 of a cluster's, whose barriers and slower way out cost 4500.
+// 7 x 7 x 512 -> 512: 22.4 -> 13.7 us.
+void choose_split(const UmmaConv& c, int sms, UmmaParams& p) {
+  p.splits = 1;
+  p.bm = BM;
+  if (p.pair || c.store_mode != 0 || getenv("ODLA_B200_NO_SPLIT")) return;
+  auto tiles = [](int64_t n, int64_t t) { return (n + t - 1) / t; };
+  const int64_t rows_full = std::max<int64_t>(c.rows_full, p.M_total);
+  double best = 176.0 * p.num_kb;
+  for (int n = 2; n <= 8 && n <= p.num_kb; n *= 2) {
+    // enough SMs for clusters over 64-column tiles of the whole batch
+    if (tiles(rows_full, BM) * tiles(c.K, 64) * n > sms) break;
+    const double cost = 200.0 * tiles(p.num_kb, n) + 4500.0;
+    if (cost < best) { best = cost; p.splits = n; }
+  }
+  if (p.splits == 1) return;
+  // the smallest tiles that still find an SM each: fewer bytes per k-block and CTA
+  best = -1;
+  for (int bm = BM; bm >= 64; bm /= 2)
+    for (int bn = 64; bn >= 16; bn /= 2) {
+      if (c.w_batches > 0 && (bm != BM || (c.w_n_major && bn != 64))) continue;   // B boxes of a batched GEMM follow 128-row tiles
+      const int64_t ctas = tiles(p.M_total, bm) * tiles(c.K, bn) * p.splits;
+      const double cost = (double)tiles(ctas, sms) * std::max((bm + bn) * p.kb_bytes / 80.0, 200.0);
+      if (best < 0 || cost < best) { best = cost; p.bm = bm; p.BN = bn; }
+    }
+  p.bn_load = p.BN;
+  p.m_tiles = (int)tiles(p.M_total, p.bm);
+  p.n_tiles = (int)tiles(c.K, p.BN);
+  p.total_tiles = p.m_tiles * p.n_tiles;
+}
+
 UmmaLaunch* umma_conv_prepare(const UmmaConv& c, const void* x, const void* w, void* y, const Epilogue& ep, int* status, int sms) {
   if (!umma_conv_supported(c) || !load_driver_entry_points()) return nullptr;
   auto* L = new UmmaLaunch();
@@ -1822,14 +2131,16 @@ UmmaLaunch* umma_conv_prepare(const UmmaConv& c, const void* x, const void* w, v
       p.total_tiles = p.m_tiles * p.n_tiles;
     }
   }
+  choose_split(c, sms, p);
   // Several k-blocks share one pipeline stage (one mbarrier round trip) when they are small: up to
   // 48 KB per stage, balanced over the tile's k-blocks.
-  const int box_bytes = (BM + p.bn_load) * p.kb_bytes;
+  const int box_bytes = (p.bm + p.bn_load) * p.kb_bytes;
   int bps_max = (48 * 1024) / box_bytes;
   if (bps_max < 1) bps_max = 1;
   if (bps_max > 8) bps_max = 8;
-  const int iters = (p.num_kb + bps_max - 1) / bps_max;
-  p.bps = (p.num_kb + iters - 1) / iters;
+  const int share_kb = (p.num_kb + p.splits - 1) / p.splits;   // k-blocks one CTA walks
+  const int iters = (share_kb + bps_max - 1) / bps_max;
+  p.bps = (share_kb + iters - 1) / iters;
   p.num_it = (p.num_kb + p.bps - 1) / p.bps;
   const int stage_bytes = p.bps * box_bytes;
   // Staged epilogue: the output tile goes through shared memory (128-byte-swizzled boxes of 128 rows)
@@ -1839,7 +2150,8 @@ UmmaLaunch* umma_conv_prepare(const UmmaConv& c, const void* x, const void* w, v
   // The residual of a staged launch always comes through the staging box, so it must have the output's type.
   const bool res_ok = !ep.res || (ep.res_dt == ep.out_dt && (uintptr_t)ep.res % 16 == 0);
   const int64_t y_cols = c.y_pitch > 0 ? c.y_pitch : c.K;  // row pitch of y in elements
-  p.staged = (ep.out_dt == DT_F16 || ep.out_dt == DT_BF16 || ep.out_dt == DT_S8) && (y_cols * p.out_esz) % 16 == 0 && !ep.add_full && res_ok &&
+  p.y_ld = (int)y_cols;
+  p.staged = p.splits == 1 && (ep.out_dt == DT_F16 || ep.out_dt == DT_BF16 || ep.out_dt == DT_S8) && (y_cols * p.out_esz) % 16 == 0 && !ep.add_full && res_ok &&
              (c.y_pitch == 0 || (c.y_pitch >= c.K && !ep.res && c.store_mode == 0)) &&
              ((uintptr_t)y % 16 == 0) && !getenv("ODLA_B200_DIRECT_EPILOGUE");
   p.stage_boxes = p.staged ? (p.BN * p.out_esz + 127) / 128 : 0;
@@ -1884,7 +2196,7 @@ UmmaLaunch* umma_conv_prepare(const UmmaConv& c, const void* x, const void* w, v
   }
   {
     // 16 epilogue warps = 4 groups; a group owns BN/64 consecutive 16-column chunks, a box holds 128/out_esz/16
-    const int per_group = p.BN / 64, per_box = 128 / p.out_esz / 16;
+    const int per_group = std::max(p.BN / 64, 1), per_box = 128 / p.out_esz / 16;
     const int groups_per_box = per_box / per_group < 4 ? per_box / per_group : 4;
     p.box_arrivals = 4 * (groups_per_box < 1 ? 1 : groups_per_box);
     // Contiguous runs let the groups work on different boxes at once, which pays when boxes need no residual and
@@ -1905,12 +2217,12 @@ UmmaLaunch* umma_conv_prepare(const UmmaConv& c, const void* x, const void* w, v
   p.acc_int = c.in_dt == DT_S8;
   p.store_mode = c.store_mode; p.store_S = c.store_S; p.store_NH = c.store_NH;
   if (p.store_mode && (!p.staged || !umma_store_perm_ok(c, ep, y))) { delete L; return nullptr; }
-  if (c.y_pitch > 0 && !p.staged) { delete L; return nullptr; }  // the direct epilogue writes rows of K elements
+  if (c.y_pitch > 0 && !p.staged && (p.splits == 1 || ep.res)) { delete L; return nullptr; }  // the direct epilogue writes rows of K elements
   p.rows_per_batch = c.w_batches > 0 ? c.rows_per_batch : 0;
-  p.tmem_cols = 2 * p.BN;  // 128, 256 or 512: powers of two >= 32
+  p.tmem_cols = p.splits > 1 ? std::max(p.BN, 32) : 2 * p.BN;  // 32 to 512: powers of two
   const uint32_t fmt = c.in_dt == DT_BF16 ? 1u : (c.in_dt == DT_S8 ? 1u : 0u);      // bf16 / signed 8-bit / f16
   const uint32_t cfmt = p.acc_int ? 2u : 1u;                                        // s32 / f32 accumulators
-  p.idesc = (cfmt << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.BN >> 3) << 17) | ((uint32_t)((BM << p.pair) >> 4) << 24);
+  p.idesc = (cfmt << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.BN >> 3) << 17) | ((uint32_t)((p.bm << p.pair) >> 4) << 24);
   // B stored [k][n]: the instruction reads it MN-major (descriptor bit 16).  A box is then 64 k-rows of 128 bytes: the
   // 8-row group pitch (SBO) is the same 1024 bytes, and 32 bytes of K are 16 rows = 2048 bytes further on.
   p.b_n_major = c.w_n_major ? 1 : 0;
@@ -1931,6 +2243,12 @@ UmmaLaunch* umma_conv_prepare(const UmmaConv& c, const void* x, const void* w, v
   p.b_constant = c.w_constant;
   L->grid = p.pair ? (2 * p.total_tiles < (sms & ~1) ? 2 * p.total_tiles : (sms & ~1)) : (p.total_tiles < sms ? p.total_tiles : sms);
   L->smem = (size_t)p.stages * stage_bytes + (size_t)p.ring_boxes * 16384 + 1024 /*alignment slack*/ + 1024 /*barriers*/;
+  if (p.splits > 1) {
+    p.stages = std::max(1, std::min({200 * 1024 / stage_bytes, 8, (share_kb + p.bps - 1) / p.bps}));
+    p.split_data_bytes = (std::max(p.stages * stage_bytes, p.bm * p.BN * 4) + 1023) / 1024 * 1024;
+    L->grid = p.total_tiles * p.splits;
+    L->smem = (size_t)p.split_data_bytes + 1024 /*alignment slack*/ + 256 /*barriers*/;
+  }
   if (L->smem > 227 * 1024) { delete L; return nullptr; }
 
   const CUtensorMapDataType dt = c.in_dt == DT_S8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : (c.in_dt == DT_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16);
@@ -1946,7 +2264,7 @@ UmmaLaunch* umma_conv_prepare(const UmmaConv& c, const void* x, const void* w, v
     int upper[2] = {(c.Q - 1) * c.stride_w - c.pad_l - (c.W - 1), (c.P - 1) * c.stride_h - c.pad_t - (c.H - 1)};
     if (upper[0] < -128 || upper[0] > 127 || upper[1] < -128 || upper[1] > 127) { delete L; return nullptr; }
     cuuint32_t estr[4] = {1, (cuuint32_t)c.stride_w, (cuuint32_t)c.stride_h, 1};
-    r = g_encode_im2col(&L->tmA, dt, 4, (void*)x, dims, strides, lower, upper, (cuuint32_t)p.kbe, (cuuint32_t)BM, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
+    r = g_encode_im2col(&L->tmA, dt, 4, (void*)x, dims, strides, lower, upper, (cuuint32_t)p.kbe, (cuuint32_t)p.bm, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r == CUDA_SUCCESS) {
       // Drivers up to 13.1 encode small im2col tensors (< 128 KiB) with a flag that makes the load
@@ -1960,7 +2278,7 @@ UmmaLaunch* umma_conv_prepare(const UmmaConv& c, const void* x, const void* w, v
   } else {
     cuuint64_t dims[2] = {(cuuint64_t)c.C, (cuuint64_t)p.M_total};
     cuuint64_t strides[1] = {(cuuint64_t)c.C * es};
-    cuuint32_t box[2] = {(cuuint32_t)p.kbe, (cuuint32_t)BM};
+    cuuint32_t box[2] = {(cuuint32_t)p.kbe, (cuuint32_t)p.bm};
     cuuint32_t estr[2] = {1, 1};
     r = g_encode_tiled(&L->tmA, dt, 2, (void*)x, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -2023,6 +2341,7 @@ UmmaLaunch* umma_conv_prepare(const UmmaConv& c, const void* x, const void* w, v
    cudaFuncSetAttribute(umma_conv_kernel<O, M, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) == cudaSuccess)
     bool ok = B2_SMEM(DT_F16, 1) && B2_SMEM(DT_BF16, 1) && B2_SMEM(DT_S8, 1) && B2_SMEM(DT_F16, 2) && B2_SMEM(DT_BF16, 2) && B2_SMEM(DT_S8, 2) && B2_SMEM(DT_F16, 3) && B2_SMEM(DT_BF16, 3) && B2_SMEM(DT_S8, 3) && B2_SMEM(-1, 0);
 #undef B2_SMEM
+    ok = ok && cudaFuncSetAttribute(umma_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) == cudaSuccess;
     if (!ok) { cudaGetLastError(); delete L; return nullptr; }
     attr_set[dev] = true;
   }
@@ -2035,7 +2354,7 @@ int umma_conv_run(UmmaLaunch* L, cudaStream_t stream) {
   const UmmaParams& p = L->p;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)L->grid);
-  cfg.blockDim = dim3(p.staged ? EpiCfg<true>::kThreads : EpiCfg<false>::kThreads);
+  cfg.blockDim = dim3(p.splits > 1 ? kSplitThreads : p.staged ? EpiCfg<true>::kThreads : EpiCfg<false>::kThreads);
   cfg.dynamicSmemBytes = L->smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
@@ -2046,9 +2365,9 @@ int umma_conv_run(UmmaLaunch* L, cudaStream_t stream) {
     attr[na].val.programmaticStreamSerializationAllowed = 1;
     ++na;
   }
-  if (p.pair) {
+  if (p.pair || p.splits > 1) {
     attr[na].id = cudaLaunchAttributeClusterDimension;
-    attr[na].val.clusterDim.x = 2;
+    attr[na].val.clusterDim.x = p.pair ? 2 : (unsigned)p.splits;
     attr[na].val.clusterDim.y = 1;
     attr[na].val.clusterDim.z = 1;
     ++na;
@@ -2059,7 +2378,8 @@ int umma_conv_run(UmmaLaunch* L, cudaStream_t stream) {
 #define B2_LAUNCH(O, M)                                                                                   \
   le = p.pair ? cudaLaunchKernelEx(&cfg, umma_conv_kernel<O, M, true>, L->tmA, L->tmB, L->tmY, L->tmR, p) \
               : cudaLaunchKernelEx(&cfg, umma_conv_kernel<O, M, false>, L->tmA, L->tmB, L->tmY, L->tmR, p)
-  if (p.epi_mode == 0) B2_LAUNCH(-1, 0);
+  if (p.splits > 1) le = cudaLaunchKernelEx(&cfg, umma_split_kernel, L->tmA, L->tmB, p);
+  else if (p.epi_mode == 0) B2_LAUNCH(-1, 0);
   else if (p.epi_mode == 1) { if (p.ep.out_dt == DT_F16) B2_LAUNCH(DT_F16, 1); else if (p.ep.out_dt == DT_BF16) B2_LAUNCH(DT_BF16, 1); else B2_LAUNCH(DT_S8, 1); }
   else if (p.epi_mode == 3) { if (p.ep.out_dt == DT_F16) B2_LAUNCH(DT_F16, 3); else if (p.ep.out_dt == DT_BF16) B2_LAUNCH(DT_BF16, 3); else B2_LAUNCH(DT_S8, 3); }
   else { if (p.ep.out_dt == DT_F16) B2_LAUNCH(DT_F16, 2); else if (p.ep.out_dt == DT_BF16) B2_LAUNCH(DT_BF16, 2); else B2_LAUNCH(DT_S8, 2); }

@@ -211,6 +211,11 @@ class Builder {
     return s;
   }
   int64_t count(V v) const { return numel(shape(v)); }
+  // Rows of the whole recorded batch behind `rows` rows of this shard of `v`.
+  int64_t rows_of_batch(V v, int64_t rows) const {
+    auto it = carries_batch_.find(v);
+    return it != carries_batch_.end() && it->second && b_ > 0 && rows % b_ == 0 ? rows / b_ * B_ : rows;
+  }
   int storage_of(V v) const {
     if (is_float_type(v->type.element_type)) return FS();
     return api_dt(v->type.element_type);
@@ -759,6 +764,7 @@ odla_status Builder::emit_group(const Item& it) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p_->device);
   UmmaConv uc{1, 1, (int)M, (int)Kd, (int)(G * N), 1, 1, 1, (int)M, 1, 1, 0, 0, in_dt};
   uc.w_constant = 1;
+  uc.rows_full = rows_of_batch(root, (int64_t)uc.N * uc.P * uc.Q);
   UmmaLaunch* ul = umma_conv_prepare(uc, dev_ptr(it.fused->x), wd, dev_ptr(it.out), ep, p_->status, sms);
   if (!ul) return fail(ODLA_FAILURE, "'" + root->name + "': tensor-map encoding failed");
   p_->umma.push_back(ul);
@@ -1032,6 +1038,7 @@ odla_status Builder::emit_fused(const Item& it) {
       if (!wd) return err_status_;
       if (pitch_.count(f.out)) uc.y_pitch = (int)pitch_[f.out];
       uc.w_constant = 1;
+      uc.rows_full = rows_of_batch(root, (int64_t)uc.N * uc.P * uc.Q);
       UmmaLaunch* ul = umma_conv_prepare(uc, x_umma, wd, y, ep, p_->status, sms);
       if (!ul) return fail(ODLA_FAILURE, "'" + root->name + "': tensor-map encoding failed");
       p_->umma.push_back(ul);
@@ -1159,6 +1166,7 @@ odla_status Builder::emit_fused(const Item& it) {
     if (Mt < (1ll << 31) && umma_conv_supported(uc)) {
       if (w_terms > 1) uc.w_terms = w_terms;
       uc.w_constant = 1;
+      uc.rows_full = rows_of_batch(root, (int64_t)uc.N * uc.P * uc.Q);
       auto wb = prepared(f.w, std::string("gemm_kmajor dt") + std::to_string(in_dt) + (tb ? " t" : " n") + " terms" + std::to_string(w_terms) +
                                   (f.w_zp ? " zp" + std::to_string((int)const_as_f32(f.w_zp)[0]) : std::string()), [&] {
         if (w_terms > 1) {
@@ -1195,6 +1203,7 @@ odla_status Builder::emit_fused(const Item& it) {
     UmmaConv uc{1, 1, (int)(batch * M), (int)Kd, (int)N, 1, 1, 1, (int)(batch * M), 1, 1, 0, 0, in_dt};
     uc.w_batches = (int)batch;
     uc.rows_per_batch = (int)M;
+    uc.rows_full = rows_of_batch(root, batch * M);
     if (store_direct) set_store(uc);
     // a [batch, K, 64] operand (attention probabilities x V) is read as it lies; other widths are transposed first
     if (!tb && N == 64 && Kd % 64 == 0 && !getenv("ODLA_B200_NO_N_MAJOR")) uc.w_n_major = 1;
