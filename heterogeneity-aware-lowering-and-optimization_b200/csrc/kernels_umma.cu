@@ -2054,6 +2054,8 @@ bool umma_store_perm_ok(const UmmaConv& c, const Epilogue& ep, const void* y) {
   return M % ((long long)c.store_S * c.store_NH) == 0 && c.K == c.store_D;
 }
 
+constexpr int kLongReduction = 12;   // k-blocks from which a tile's time is its operands' and MMAs', not its epilogue's
+
 // Whether the CTAs of a cluster share each tile's reduction (umma_split_kernel), and over which tiles.  How many share it
 // changes the order in which floating-point sums are taken, so that number is decided from the rows of the whole recorded
 // batch and not from this launch's share of them: a row's result does not depend on how a batch is cut over GPUs or
@@ -2121,7 +2123,7 @@ UmmaLaunch* umma_conv_prepare(const UmmaConv& c, const void* x, const void* w, v
   {
     // (the thresholds can be moved through the environment, which the tests use to run every shape on pairs)
     const int pair_min_bn = getenv("ODLA_B200_PAIR_MIN_BN") ? atoi(getenv("ODLA_B200_PAIR_MIN_BN")) : 128;
-    const int pair_min_kb = getenv("ODLA_B200_PAIR_MIN_KB") ? atoi(getenv("ODLA_B200_PAIR_MIN_KB")) : 12;
+    const int pair_min_kb = getenv("ODLA_B200_PAIR_MIN_KB") ? atoi(getenv("ODLA_B200_PAIR_MIN_KB")) : kLongReduction;
     const bool pair_s8 = getenv("ODLA_B200_PAIR_S8") != nullptr;
     p.pair = ((c.in_dt != DT_S8 || pair_s8) && p.BN >= pair_min_bn && p.num_kb >= pair_min_kb && p.M_total % (2 * BM) == 0 && sms >= 2 &&
               c.w_batches == 0) ? 1 : 0;
@@ -2191,7 +2193,17 @@ UmmaLaunch* umma_conv_prepare(const UmmaConv& c, const void* x, const void* w, v
     p.ring_boxes = (budget - want_stages * stage_bytes) / 16384;
     if (p.ring_boxes > kMaxRing) p.ring_boxes = kMaxRing;
     if (p.ring_boxes > ring_want) p.ring_boxes = ring_want;
-    if (p.ring_boxes < p.stage_boxes) p.ring_boxes = p.stage_boxes;
+    int ring_min = p.stage_boxes;
+    // Long reductions are bound by how many operand bytes are on their way: a stage is 1400 clocks from its request to its
+    // MMAs and 700 more to its next request, in which the tensor cores take in 130 KB of a 256 x 256 pair tile's operands.
+    // Their epilogues have time, so two boxes go round (one being written, one being stored), a tile's worth where a residual
+    // is fetched ahead and four stages remain.  3x3 256 -> 512 at 26 x 26 x 16: 40.7 -> 36.7 us, 1024 -> 256 at 14 x 14 x 256: 40.8 -> 36.9 us, a
+    // 3072-deep projection of 8192 rows: 48.7 -> 45.0 us.
+    if (p.num_kb >= kLongReduction) {
+      ring_min = ep.res && budget - p.stage_boxes * 16384 >= 4 * stage_bytes ? p.stage_boxes : 2;
+      if (p.ring_boxes > ring_min) p.ring_boxes = ring_min;
+    }
+    if (p.ring_boxes < ring_min) p.ring_boxes = ring_min;
     if (p.ring_boxes < 2) p.ring_boxes = 2;  // the store of box i frees box i-1
   }
   {
@@ -2201,7 +2213,7 @@ UmmaLaunch* umma_conv_prepare(const UmmaConv& c, const void* x, const void* w, v
     p.box_arrivals = 4 * (groups_per_box < 1 ? 1 : groups_per_box);
     // Contiguous runs let the groups work on different boxes at once, which pays when boxes need no residual and
     // the CTA has many tiles to stream through; otherwise finishing box after box gets the first store out sooner.
-    p.epi_interleave = ep.res != nullptr || (p.total_tiles << p.pair) < 16 * sms;
+    p.epi_interleave = ep.res != nullptr || (p.total_tiles << p.pair) < 16 * sms || p.ring_boxes < p.stage_boxes;
     if (getenv("ODLA_B200_EPI_INTERLEAVE")) p.epi_interleave = atoi(getenv("ODLA_B200_EPI_INTERLEAVE"));
     if (p.epi_interleave) p.box_arrivals = 16;
   }
