@@ -2065,7 +2065,7 @@ constexpr int kLongReduction = 12;   // k-blocks from which a tile's time is its
 void choose_split(const UmmaConv& c, int sms, UmmaParams& p) {
   p.splits = 1;
   p.bm = BM;
-  if (p.pair || c.store_mode != 0 || getenv("ODLA_B200_NO_SPLIT")) return;
+  if (c.store_mode != 0 || getenv("ODLA_B200_NO_SPLIT") || getenv("ODLA_B200_PAIR_MIN_KB")) return;
   auto tiles = [](int64_t n, int64_t t) { return (n + t - 1) / t; };
   const int64_t rows_full = std::max<int64_t>(c.rows_full, p.M_total);
   double best = 176.0 * p.num_kb;
@@ -2087,6 +2087,48 @@ void choose_split(const UmmaConv& c, int sms, UmmaParams& p) {
     }
   p.bn_load = p.BN;
   p.m_tiles = (int)tiles(p.M_total, p.bm);
+  p.n_tiles = (int)tiles(c.K, p.BN);
+  p.total_tiles = p.m_tiles * p.n_tiles;
+}
+
+// The tile of a persistent launch whose p.BN is at least 128: how many columns, and whether CTA pairs (tcgen05 cta_group::2)
+// share it.  A pair computes 256 rows x BN columns and each CTA loads only half of the filter tile.  That pays where
+// operand traffic into shared memory is the limit -- two-byte operands and a long reduction (measured: 12 or more k-blocks,
+// e.g. a 768-deep transformer projection; at 8 a ResNet layer loses) -- and costs where the epilogue is, because the pair's
+// CTAs then wait for each other's accumulators.  Needs an even grid.
+// Long reductions also choose their columns: a launch takes whole rounds of tiles, and 96 tiles of 256 columns on 74 pairs
+// are two rounds as long as 148 would be.  192 columns make them 128 shorter ones.  In clocks, from the walk's own
+// timing: a k-block of 256, 192, 128 columns takes 560, 430, 390 on pairs and 600, 470, 415 on single CTAs, a tile 1200 to
+// start, the last tile's epilogue 20 a column and a pair's setting up 400.  3x3 512 -> 1024 at 13 x 13 x 16: 43 -> 35 us, a
+// 3072 -> 768 projection of 8192 rows with a residual: 49 -> 45 us.  (192 columns are one and a half boxes of one-byte results: not there.)
+void choose_tile(const UmmaConv& c, const Epilogue& ep, int sms, UmmaParams& p) {
+  p.pair = 0;
+  p.bn_load = p.BN;
+  if (p.BN < 128 && !getenv("ODLA_B200_PAIR_MIN_BN")) return;
+  // (the thresholds can be moved through the environment, which the tests use to run every shape on pairs)
+  const int pair_min_bn = getenv("ODLA_B200_PAIR_MIN_BN") ? atoi(getenv("ODLA_B200_PAIR_MIN_BN")) : 128;
+  const int pair_min_kb = getenv("ODLA_B200_PAIR_MIN_KB") ? atoi(getenv("ODLA_B200_PAIR_MIN_KB")) : kLongReduction;
+  const bool pairs = (c.in_dt != DT_S8 || getenv("ODLA_B200_PAIR_S8")) && p.num_kb >= pair_min_kb && sms >= 2 && c.w_batches == 0 &&
+                     (c.store_mode == 0 || p.M_total % (2 * BM) == 0);
+  auto tiles = [](int64_t n, int64_t t) { return (n + t - 1) / t; };
+  const bool choose = p.num_kb >= kLongReduction && p.BN >= 128 && c.w_batches == 0;
+  const int out_esz = storage_size_of(ep.out_dt);
+  double best = -1;
+  int best_bn = p.BN, best_pair = 0;
+  for (int bn = choose ? pick_bn(c.K) : p.BN; bn >= (choose ? 128 : p.BN); bn -= 64) {
+    if (bn == 192 && (out_esz != 2 || p.kb_bytes != 128)) continue;
+    for (int pair = pairs && bn >= pair_min_bn ? 1 : 0; pair >= 0; --pair) {
+      const double kb = bn > 192 ? (pair ? 560 : 600) : (bn > 128 ? (pair ? 430 : 470) : (pair ? 390 : 415));
+      const int64_t rounds = tiles(tiles(p.M_total, BM << pair) * tiles(c.K, bn), pair ? sms / 2 : sms);
+      const double cost = (double)rounds * (p.num_kb * kb + 1200.0) + 20.0 * bn + 400.0 * pair;
+      if (best < 0 || cost < best) { best = cost; best_bn = bn; best_pair = pair; }
+      if (pair && !choose) break;   // (only tests come here: short reductions on pairs)
+    }
+  }
+  p.BN = best_bn;
+  p.pair = best_pair;
+  p.bn_load = p.BN >> p.pair;
+  p.m_tiles = (int)tiles(p.M_total, BM << p.pair);
   p.n_tiles = (int)tiles(c.K, p.BN);
   p.total_tiles = p.m_tiles * p.n_tiles;
 }
@@ -2115,25 +2157,8 @@ UmmaLaunch* umma_conv_prepare(const UmmaConv& c, const void* x, const void* w, v
   }
   p.n_tiles = (c.K + p.BN - 1) / p.BN;
   p.total_tiles = p.m_tiles * p.n_tiles;
-  // CTA pairs (tcgen05 cta_group::2): a pair computes 256 rows x BN columns and each CTA loads only half of the
-  // filter tile.  That pays where operand traffic into shared memory is the limit -- two-byte operands and a long
-  // reduction (measured: 12 or more k-blocks, e.g. a 768-deep transformer projection; at 8 a ResNet layer loses) -- and
-  // costs where the epilogue is, because the pair's CTAs then wait for each other's accumulators.  Needs whole 256-row
-  // tiles and an even grid.
-  {
-    // (the thresholds can be moved through the environment, which the tests use to run every shape on pairs)
-    const int pair_min_bn = getenv("ODLA_B200_PAIR_MIN_BN") ? atoi(getenv("ODLA_B200_PAIR_MIN_BN")) : 128;
-    const int pair_min_kb = getenv("ODLA_B200_PAIR_MIN_KB") ? atoi(getenv("ODLA_B200_PAIR_MIN_KB")) : kLongReduction;
-    const bool pair_s8 = getenv("ODLA_B200_PAIR_S8") != nullptr;
-    p.pair = ((c.in_dt != DT_S8 || pair_s8) && p.BN >= pair_min_bn && p.num_kb >= pair_min_kb && p.M_total % (2 * BM) == 0 && sms >= 2 &&
-              c.w_batches == 0) ? 1 : 0;
-    p.bn_load = p.pair ? p.BN / 2 : p.BN;
-    if (p.pair) {
-      p.m_tiles = p.M_total / (2 * BM);
-      p.total_tiles = p.m_tiles * p.n_tiles;
-    }
-  }
   choose_split(c, sms, p);
+  if (p.splits == 1) choose_tile(c, ep, sms, p);
   // Several k-blocks share one pipeline stage (one mbarrier round trip) when they are small: up to
   // 48 KB per stage, balanced over the tile's k-blocks.
   const int box_bytes = (p.bm + p.bn_load) * p.kb_bytes;
@@ -2213,7 +2238,7 @@ UmmaLaunch* umma_conv_prepare(const UmmaConv& c, const void* x, const void* w, v
     p.box_arrivals = 4 * (groups_per_box < 1 ? 1 : groups_per_box);
     // Contiguous runs let the groups work on different boxes at once, which pays when boxes need no residual and
     // the CTA has many tiles to stream through; otherwise finishing box after box gets the first store out sooner.
-    p.epi_interleave = ep.res != nullptr || (p.total_tiles << p.pair) < 16 * sms || p.ring_boxes < p.stage_boxes;
+    p.epi_interleave = ep.res != nullptr || (p.total_tiles << p.pair) < 16 * sms || p.ring_boxes < p.stage_boxes || p.BN == 192;
     if (getenv("ODLA_B200_EPI_INTERLEAVE")) p.epi_interleave = atoi(getenv("ODLA_B200_EPI_INTERLEAVE"));
     if (p.epi_interleave) p.box_arrivals = 16;
   }
@@ -2231,7 +2256,7 @@ UmmaLaunch* umma_conv_prepare(const UmmaConv& c, const void* x, const void* w, v
   if (p.store_mode && (!p.staged || !umma_store_perm_ok(c, ep, y))) { delete L; return nullptr; }
   if (c.y_pitch > 0 && !p.staged && (p.splits == 1 || ep.res)) { delete L; return nullptr; }  // the direct epilogue writes rows of K elements
   p.rows_per_batch = c.w_batches > 0 ? c.rows_per_batch : 0;
-  p.tmem_cols = p.splits > 1 ? std::max(p.BN, 32) : 2 * p.BN;  // 32 to 512: powers of two
+  p.tmem_cols = p.splits > 1 ? std::max(p.BN, 32) : (p.BN > 128 ? 512 : 2 * p.BN);  // 32 to 512: powers of two
   const uint32_t fmt = c.in_dt == DT_BF16 ? 1u : (c.in_dt == DT_S8 ? 1u : 0u);      // bf16 / signed 8-bit / f16
   const uint32_t cfmt = p.acc_int ? 2u : 1u;                                        // s32 / f32 accumulators
   p.idesc = (cfmt << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.BN >> 3) << 17) | ((uint32_t)((p.bm << p.pair) >> 4) << 24);

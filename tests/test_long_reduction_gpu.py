@@ -1,0 +1,55 @@
+"""Long reductions on the tensor cores: tiles whose reduction the CTAs of a cluster share, 192-column tiles and CTA pairs whose
+second half has no rows, against float64."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def run_conv(odla, lib, N, H, W, C, K, R, residual, dtype):
+    rng = np.random.default_rng(N * H * W + C + K)
+    pad = R // 2
+    x = rng.standard_normal((N, H, W, C)).astype(np.float32)
+    w = (rng.standard_normal((R, R, C, K)) / np.sqrt(R * R * C)).astype(np.float32)
+    b = rng.standard_normal(K).astype(np.float32)
+    r = rng.standard_normal((N, H, W, K)).astype(np.float32)
+    g = odla.Graph(lib, "c", fp16=dtype == "f16", bf16=dtype == "bf16", n_gpus=1)
+    io, td = (odla.FLOAT16, torch.float16) if dtype == "f16" else (odla.FLOAT32, torch.float32)
+    half = torch.float16 if dtype == "f16" else torch.bfloat16
+    y = g.Conv(g.Argument("x", (N, H, W, C), io), odla.CHANNELS_LAST, 1, g.Constant("w", w), odla.SIO, (1, 1), (1, 1), (pad, pad), (pad, pad), None, (N, H, W, K), "conv")
+    y = g.Add(y, g.Constant("b", b.reshape(1, 1, 1, K)), "bias")
+    if residual:
+        y = g.Add(y, g.Argument("r", (N, H, W, K), io), "sum")
+    g.Output(g.Relu(y, "y"))
+    tx, tr = torch.from_numpy(x).to(half).to(td).cuda(), torch.from_numpy(r).to(half).to(td).cuda()
+    o = torch.empty((N, H, W, K), dtype=td, device="cuda")
+    g.bind_input("x", tx.data_ptr())
+    if residual:
+        g.bind_input("r", tr.data_ptr())
+    g.bind_output(g.out_names[0], o.data_ptr())
+    torch.cuda.synchronize()
+    assert g.execute() == 0
+    assert any(p["op"] == "conv_umma" for p in g.profile(runs=1))
+    g.close()
+    xd, wd = torch.from_numpy(x).to(half).double(), torch.from_numpy(w).to(half).double()
+    ref = torch.nn.functional.conv2d(xd.permute(0, 3, 1, 2).cuda(), wd.permute(3, 2, 0, 1).cuda(), padding=pad).permute(0, 2, 3, 1).cpu().numpy() + b
+    if residual:
+        ref = ref + torch.from_numpy(r).to(half).double().numpy()
+    return o.float().cpu().numpy(), np.maximum(ref, 0)
+
+
+SIZES = [  # N, H, W, C, K, R
+    (1, 7, 7, 512, 512, 3), (1, 5, 13, 256, 72, 3), (1, 1, 130, 2048, 1000, 1), (2, 7, 9, 520, 24, 3), (1, 14, 14, 1024, 256, 1), (1, 1, 1, 4096, 8, 1),   # clusters of 2 to 8
+    (1, 65, 100, 768, 320, 1), (1, 64, 100, 768, 320, 1),   # 192 columns: 51 row tiles (a half-empty pair) and 50
+]
+
+
+@pytest.mark.parametrize("size", SIZES)
+@pytest.mark.parametrize("residual", [False, True])
+@pytest.mark.parametrize("dtype", ["f16", "bf16"])
+def test_long_reductions(odla, gpu_lib, size, residual, dtype):
+    got, ref = run_conv(odla, gpu_lib, *size, residual, dtype)
+    # one rounding of the sum before the residual and one after it, of values below eight
+    step = 2.0 ** (-10 if dtype == "f16" else -7)
+    np.testing.assert_allclose(got, ref, rtol=step, atol=2 * step)
