@@ -489,9 +489,16 @@ __global__ void softmax_rows_vec_kernel(const uint4* __restrict__ x, uint4* __re
       }
   }
 }
-template <typename T, int NP, int LPR, bool QUANT>
-__global__ void layernorm_rows_vec_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, const float* __restrict__ gamma, const float* __restrict__ beta,
-                                          int64_t rows, int pieces, float eps, uint2* __restrict__ qout, const float* __restrict__ qscale) {
+// A row's time is a chain of latencies (its loads, two rounds of shuffles, gamma and beta, the stores), so the bound is how many
+// rows are under way: blocks of four warps, seven to an SM (72 registers a thread), leave no gap that blocks of eight do.
+// 8192 rows of 768 two-byte values: 15.8 -> 13.9 us, with their int8 copy 18.2 -> 16.8 (a bracketed launch alone is 2.6).
+// Ten blocks spill.
+// EARLY: gamma and beta are requested with the row instead of after its sums.  That takes 48 more registers, i.e. rows under
+// way, and so pays where all rows are under way anyway (693 rows: 9.2 -> 7.6 us) and loses where they queue (8192: 15.8).
+constexpr int kLayernormThreads = 128;
+template <typename T, int NP, int LPR, bool QUANT, bool EARLY>
+__global__ void __launch_bounds__(kLayernormThreads, EARLY ? 4 : 7) layernorm_rows_vec_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, const float* __restrict__ gamma,
+                                          const float* __restrict__ beta, int64_t rows, int pieces, float eps, uint2* __restrict__ qout, const float* __restrict__ qscale) {
   dependency_wait();
   const QuantDiv qd(QUANT ? qscale[0] : 1.f);
   constexpr int RPW = 32 / LPR;
@@ -504,6 +511,16 @@ __global__ void layernorm_rows_vec_kernel(const uint4* __restrict__ x, uint4* __
     float v[NP][8];
     bool have[NP];
     load_row_pieces<T, NP, LPR>(x + row * pieces, pieces, l, row_ok, v, have);
+    float4 gm4[NP][2], bt4[NP][2];
+    if (EARLY) {
+#pragma unroll
+      for (int i = 0; i < NP; ++i)
+        if (l + LPR * i < pieces) {
+          const int d0 = (l + LPR * i) * 8;
+          if (gamma) { gm4[i][0] = __ldg((const float4*)(gamma + d0)); gm4[i][1] = __ldg((const float4*)(gamma + d0 + 4)); }
+          if (beta) { bt4[i][0] = __ldg((const float4*)(beta + d0)); bt4[i][1] = __ldg((const float4*)(beta + d0 + 4)); }
+        }
+    }
     float s = 0.f;
 #pragma unroll
     for (int i = 0; i < NP; ++i)
@@ -525,8 +542,12 @@ __global__ void layernorm_rows_vec_kernel(const uint4* __restrict__ x, uint4* __
       if (have[i]) {
         const int d0 = (l + LPR * i) * 8;
         float gm[8], bt[8];
-        if (gamma) { const float4 g0 = *(const float4*)(gamma + d0), g1 = *(const float4*)(gamma + d0 + 4); gm[0] = g0.x; gm[1] = g0.y; gm[2] = g0.z; gm[3] = g0.w; gm[4] = g1.x; gm[5] = g1.y; gm[6] = g1.z; gm[7] = g1.w; }
-        if (beta) { const float4 b0 = *(const float4*)(beta + d0), b1 = *(const float4*)(beta + d0 + 4); bt[0] = b0.x; bt[1] = b0.y; bt[2] = b0.z; bt[3] = b0.w; bt[4] = b1.x; bt[5] = b1.y; bt[6] = b1.z; bt[7] = b1.w; }
+        if (!EARLY) {
+          if (gamma) { gm4[i][0] = __ldg((const float4*)(gamma + d0)); gm4[i][1] = __ldg((const float4*)(gamma + d0 + 4)); }
+          if (beta) { bt4[i][0] = __ldg((const float4*)(beta + d0)); bt4[i][1] = __ldg((const float4*)(beta + d0 + 4)); }
+        }
+        if (gamma) { const float4 g0 = gm4[i][0], g1 = gm4[i][1]; gm[0] = g0.x; gm[1] = g0.y; gm[2] = g0.z; gm[3] = g0.w; gm[4] = g1.x; gm[5] = g1.y; gm[6] = g1.z; gm[7] = g1.w; }
+        if (beta) { const float4 b0 = bt4[i][0], b1 = bt4[i][1]; bt[0] = b0.x; bt[1] = b0.y; bt[2] = b0.z; bt[3] = b0.w; bt[4] = b1.x; bt[5] = b1.y; bt[6] = b1.z; bt[7] = b1.w; }
         uint32_t w[4];
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
@@ -557,11 +578,18 @@ bool launch_rows_vec(bool is_softmax, const void* x, void* y, const float* gamma
   const int pieces = (int)(dim / 8);
   const int lpr = pieces <= 8 ? 8 : (pieces <= 16 ? 16 : 32), np = (pieces + lpr - 1) / lpr;
   const int grid = grid_for(rows * lpr, 256);
+  const int norm_grid = grid_for(rows * lpr, kLayernormThreads);
+  const bool early = rows * lpr <= (int64_t)sm_count() * 16 * 32;   // 16 warps of the EARLY form fit an SM
+#define B2_NORM(NP, LPR, Q, EARLY)                                                                                                            \
+  do {                                                                                                                                        \
+    if (EARLY) launch(layernorm_rows_vec_kernel<T, NP, LPR, Q, true>, norm_grid, kLayernormThreads, 0, s, (const uint4*)x, (uint4*)y, gamma, beta, rows, pieces, eps, (uint2*)q, qscale); \
+    else launch(layernorm_rows_vec_kernel<T, NP, LPR, Q, false>, norm_grid, kLayernormThreads, 0, s, (const uint4*)x, (uint4*)y, gamma, beta, rows, pieces, eps, (uint2*)q, qscale); \
+  } while (0)
 #define B2_ROWS(NP, LPR)                                                                                                                      \
   do {                                                                                                                                        \
     if (is_softmax) launch(softmax_rows_vec_kernel<T, NP, LPR>, grid, 256, 0, s, (const uint4*)x, (uint4*)y, rows, pieces, log_form);             \
-    else if (q) launch(layernorm_rows_vec_kernel<T, NP, LPR, true>, grid, 256, 0, s, (const uint4*)x, (uint4*)y, gamma, beta, rows, pieces, eps, (uint2*)q, qscale); \
-    else launch(layernorm_rows_vec_kernel<T, NP, LPR, false>, grid, 256, 0, s, (const uint4*)x, (uint4*)y, gamma, beta, rows, pieces, eps, nullptr, nullptr); \
+    else if (q) B2_NORM(NP, LPR, true, early);                                                                                                \
+    else B2_NORM(NP, LPR, false, early);                                                                                                      \
   } while (0)
   if (lpr == 8) B2_ROWS(1, 8);
   else if (lpr == 16) B2_ROWS(1, 16);
@@ -571,6 +599,7 @@ bool launch_rows_vec(bool is_softmax, const void* x, void* y, const float* gamma
   else if (np <= 4) B2_ROWS(4, 32);
   else B2_ROWS(8, 32);
 #undef B2_ROWS
+#undef B2_NORM
   return true;
 }
 // Strided axis: one thread per (outer, inner) pair.
