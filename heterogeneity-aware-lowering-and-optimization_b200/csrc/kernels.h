@@ -81,12 +81,14 @@ int gemm_simt(const GemmGeom& g, int in_dt, const void* A, const void* B, void* 
 
 // ---- tiled fp32 path (kernels_f32.cu) ----
 // fp32 convolution over dense NHWC tensors, one group; w is [K][w_pitch] with each row the filter's R*S*C values in
-// (r, s, c) order and w_pitch a multiple of 4 (the padding holds zeros).
+// (r, s, c) order and w_pitch a multiple of 4 (the padding holds zeros).  images_full: images of the whole recorded batch, of
+// which g.N are here.  It alone decides the order of the sums, so that an image's result does not depend on how a batch is cut.
 bool conv_f32_supported(const ConvGeom& g);
-int conv_f32(const ConvGeom& g, const void* x, const void* w, int64_t w_pitch, void* y, const Epilogue& ep, cudaStream_t stream);
-// fp32 batched GEMM, any strides (a B with unit b_row and 16-byte rows loads widest).
+int conv_f32(const ConvGeom& g, int64_t images_full, const void* x, const void* w, int64_t w_pitch, void* y, const Epilogue& ep, cudaStream_t stream);
+// fp32 batched GEMM, any strides (a B with unit b_row and 16-byte rows loads widest).  batch_full and rows_full: g.batch and g.M
+// of the whole recorded batch, as above.
 bool gemm_f32_supported(const GemmGeom& g);
-int gemm_f32(const GemmGeom& g, const void* A, const void* B, void* C, const Epilogue& ep, cudaStream_t stream);
+int gemm_f32(const GemmGeom& g, int64_t batch_full, int64_t rows_full, const void* A, const void* B, void* C, const Epilogue& ep, cudaStream_t stream);
 
 // ---- tensor-core path (kernels_umma.cu) ----
 // NHWC implicit-GEMM convolution: x [N,H,W,C], w repacked to [K][R*S*C] (K-major), y [N,P,Q,K].

@@ -38,7 +38,7 @@ static_assert(kTile * kPitch * 4 <= kStages * 2 * kOperandBytes, "the result til
 enum { LOAD_CONV_VEC, LOAD_CONV_SCALAR, LOAD_GEMM_VEC, LOAD_GEMM_SCALAR };
 
 struct F32Params {
-  int M, N, K, num_kb, m_tiles, n_tiles, splits;
+  int M, N, K, num_kb, m_tiles, n_tiles, splits, batches;
   int64_t a_row, a_col, a_batch, b_row, b_col, b_batch;
   int H, W, C, R, S, P, Q, stride_h, stride_w, pad_t, pad_l;
   const float *A, *B;
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(128) f32_few_results_kernel(const F32Params p)
   dependency_wait();
   const int64_t batch = w / per_batch, g = w - batch * per_batch;
   const int m0 = (int)(g / col_groups) * kFewRows, n0 = (int)(g % col_groups) * kFewCols;
-  if (batch >= p.splits) return;   // (splits holds the batch count here)
+  if (batch >= p.batches) return;
   const float *A = p.A + batch * p.a_batch, *B = p.B + batch * p.b_batch;
   float acc[kFewRows][kFewCols] = {};
 #pragma unroll 4
@@ -309,6 +309,8 @@ int device_sms() {
 // busiest SM works off its CTAs in pairs -- one CTA's two warps reach two of the four schedulers, so an odd CTA costs as
 // much as two -- at 1.04 us per k-block and CTA; every round of four resident CTAs pays about 4 us for filling the stages and
 // writing the tile, a cluster 2 us more for its barriers and remote reads (measured on ResNet-50's layers at batch 8).
+// `tiles` are those of the whole recorded batch: the number of shares is the order of the sums, and a launch that computes a
+// part of the batch (another GPU's or sub-batch's rows) has to take the same one.
 int pick_splits(int64_t tiles, int num_kb) {
   const int sms = device_sms();
   int best = 1;
@@ -349,14 +351,14 @@ int launch_tiles(const F32Params& p, int64_t blocks, cudaStream_t s) {
   if (e != cudaSuccess) { fprintf(stderr, "[odla_b200] fp32 tile kernel launch failed: %s\n", cudaGetErrorString(e)); cudaGetLastError(); return -2; }
   return 0;
 }
-int run(F32Params p, int la, bool bvec, int64_t batch, cudaStream_t s) {
+int run(F32Params p, int la, bool bvec, int64_t batch, int64_t batch_full, int64_t rows_full, cudaStream_t s) {
   p.num_kb = (p.K + kBK - 1) / kBK;
   p.m_tiles = (p.M + kTile - 1) / kTile;
   p.n_tiles = (p.N + kTile - 1) / kTile;
   const int64_t tiles = batch * p.m_tiles * p.n_tiles;
   if (tiles <= 0) return 0;
   if (tiles > 0x7fffffffLL) return -1;
-  p.splits = pick_splits(tiles, p.num_kb);
+  p.splits = pick_splits(batch_full * ((rows_full + kTile - 1) / kTile) * p.n_tiles, p.num_kb);
   if (la == LOAD_CONV_VEC) return launch_tiles<LOAD_CONV_VEC, true>(p, tiles, s);
   if (la == LOAD_CONV_SCALAR) return launch_tiles<LOAD_CONV_SCALAR, true>(p, tiles, s);
   if (la == LOAD_GEMM_VEC) return bvec ? launch_tiles<LOAD_GEMM_VEC, true>(p, tiles, s) : launch_tiles<LOAD_GEMM_VEC, false>(p, tiles, s);
@@ -367,7 +369,7 @@ int run(F32Params p, int la, bool bvec, int64_t batch, cudaStream_t s) {
 bool conv_f32_supported(const ConvGeom& g) {
   return g.groups == 1 && g.xs_c == 1 && (int64_t)g.N * g.P * g.Q < (1ll << 31) && (int64_t)g.R * g.S * g.C < (1ll << 30) && g.P > 0 && g.Q > 0;
 }
-int conv_f32(const ConvGeom& g, const void* x, const void* w, int64_t w_pitch, void* y, const Epilogue& ep, cudaStream_t s) {
+int conv_f32(const ConvGeom& g, int64_t images_full, const void* x, const void* w, int64_t w_pitch, void* y, const Epilogue& ep, cudaStream_t s) {
   F32Params p{};
   p.M = g.N * g.P * g.Q; p.N = g.K; p.K = g.R * g.S * g.C;
   p.H = g.H; p.W = g.W; p.C = g.C; p.R = g.R; p.S = g.S; p.P = g.P; p.Q = g.Q;
@@ -375,10 +377,10 @@ int conv_f32(const ConvGeom& g, const void* x, const void* w, int64_t w_pitch, v
   p.A = (const float*)x; p.B = (const float*)w; p.y = y; p.ep = ep;
   p.b_row = 1; p.b_col = w_pitch;
   const bool vec = g.C % 4 == 0 && (uintptr_t)x % 16 == 0;
-  return run(p, vec ? LOAD_CONV_VEC : LOAD_CONV_SCALAR, true, 1, s);
+  return run(p, vec ? LOAD_CONV_VEC : LOAD_CONV_SCALAR, true, 1, 1, images_full * g.P * g.Q, s);
 }
 bool gemm_f32_supported(const GemmGeom& g) { return g.M < (1ll << 31) && g.N < (1ll << 31) && g.K < (1ll << 30) && g.K > 0; }
-int gemm_f32(const GemmGeom& g, const void* A, const void* B, void* C, const Epilogue& ep, cudaStream_t s) {
+int gemm_f32(const GemmGeom& g, int64_t batch_full, int64_t rows_full, const void* A, const void* B, void* C, const Epilogue& ep, cudaStream_t s) {
   F32Params p{};
   p.M = (int)g.M; p.N = (int)g.N; p.K = (int)g.K;
   p.a_row = g.a_row; p.a_col = g.a_col; p.a_batch = g.a_batch;
@@ -387,14 +389,15 @@ int gemm_f32(const GemmGeom& g, const void* A, const void* B, void* C, const Epi
   const bool avec = g.a_col == 1 && g.K % 4 == 0 && g.a_row % 4 == 0 && g.a_batch % 4 == 0 && (uintptr_t)A % 16 == 0;
   // (pieces past K are zero on the A side, so a B row padded to a multiple of four floats may hold anything there)
   const bool bvec = g.b_row == 1 && g.b_col % 4 == 0 && (g.K % 4 == 0 || g.b_batch == 0) && g.b_batch % 4 == 0 && (uintptr_t)B % 16 == 0;
-  // up to 16384 results the warps of one launch fit the chip at once and the operands are re-read from L2 only
-  if (avec && bvec && g.K % 4 == 0 && g.batch > 0 && g.batch * g.M * g.N <= 16384) {
-    p.splits = (int)g.batch;
+  // up to 16384 results (of the whole recorded batch, see pick_splits) the warps of one launch fit the chip at once and the
+  // operands are re-read from L2 only
+  if (avec && bvec && g.K % 4 == 0 && g.batch > 0 && batch_full * rows_full * g.N <= 16384) {
+    p.batches = (int)g.batch;
     const int64_t warps = g.batch * ((g.M + kFewRows - 1) / kFewRows) * ((g.N + kFewCols - 1) / kFewCols);
     b200::launch(f32_few_results_kernel, (unsigned)((warps + 3) / 4), 128, 0, s, p);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
   }
-  return run(p, avec ? LOAD_GEMM_VEC : LOAD_GEMM_SCALAR, bvec, g.batch, s);
+  return run(p, avec ? LOAD_GEMM_VEC : LOAD_GEMM_SCALAR, bvec, g.batch, batch_full, rows_full, s);
 }
 
 }  // namespace b200

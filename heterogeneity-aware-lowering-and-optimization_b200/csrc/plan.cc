@@ -1069,7 +1069,8 @@ odla_status Builder::emit_fused(const Item& it) {
         auto wb = prepared(f.w, "conv_f32_kmajor", [&] { return f32_rows_kmajor(const_as_f32(f.w), kd, K, pitch); });
         const void* wk = upload(wb->data(), wb->size());
         if (!wk) return err_status_;
-        add_launch("conv_simt", f.out, flops, bytes, [=](cudaStream_t s) { return conv_f32(g, x, wk, pitch, y, ep, s); });
+        const int64_t images_full = rows_of_batch(root, g.N);
+        add_launch("conv_simt", f.out, flops, bytes, [=](cudaStream_t s) { return conv_f32(g, images_full, x, wk, pitch, y, ep, s); });
         return ODLA_SUCCESS;
       }
     }
@@ -1250,7 +1251,11 @@ odla_status Builder::emit_fused(const Item& it) {
     bp = dev_ptr(f.w);
   }
   if (!bp) return err_status_;
-  add_launch("gemm_simt", f.out, flops, bytes, with_move([=](cudaStream_t s) { return f32_tiled ? gemm_f32(g, x, bp, y, ep, s) : gemm_simt(g, in_dt, x, bp, y, ep, s); }));
+  // the whole recorded batch lies along the leading axis: the batch of a batched product, the rows of a plain one
+  const int64_t all_rows = rows_of_batch(root, batch * M), batch_full = ra > 2 && M > 0 ? all_rows / M : batch, rows_full = ra > 2 ? M : all_rows;
+  add_launch("gemm_simt", f.out, flops, bytes, with_move([=](cudaStream_t s) {
+    return f32_tiled ? gemm_f32(g, batch_full, rows_full, x, bp, y, ep, s) : gemm_simt(g, in_dt, x, bp, y, ep, s);
+  }));
   if (perm_via_move) p_->launches.back().n_kernels = 2;
   return ODLA_SUCCESS;
 }

@@ -52,3 +52,29 @@ def test_gemm_f32_matches_float64(odla, gpu_lib, dims):
     g.close()
     af, bf = a.astype(np.float64), b.astype(np.float64)
     close(got, 0.5 * ((af.swapaxes(-1, -2) if ta else af) @ (bf.swapaxes(-1, -2) if tb else bf)) + 2.0 * c, K)
+
+
+def test_f32_results_do_not_depend_on_how_the_batch_is_cut(odla, gpu_lib):
+    """A long convolution, a batched product and two classifiers whose shares of the reduction (and, for the last, whose
+    kernel) would differ between six images and the one to five of a sub-batch: equal bits however the batch is cut."""
+    B = 6
+    rng = np.random.default_rng(8)
+    n = lambda *s: (rng.standard_normal(s) / np.sqrt(np.prod(s[:-1]))).astype(np.float32)
+    x = rng.standard_normal((B, 7, 7, 512)).astype(np.float32)
+    wc, w1, w2 = n(3, 3, 512, 512), n(512, 3000), n(512, 40)
+    outs = []
+    for s in (1, 2, 3, 6):
+        g = odla.Graph(gpu_lib, "cut", n_gpus=1, sub_batches=s)
+        y = g.Conv(g.Argument("x", x.shape), odla.CHANNELS_LAST, 1, g.Constant("wc", wc), odla.SIO, (1, 1), (1, 1), (1, 1), (1, 1), None, x.shape, "conv")
+        g.Output(y)
+        t = g.Reshape(y, (B, 49, 512), "rows")
+        g.Output(g.Gemm(t, False, t, True, 1.0, 0.0, None, (B, 49, 49), "gram"))
+        v = g.Reshape(g.ReduceMean(y, (1, 2), True, (B, 1, 1, 512), "gap"), (B, 512), "flat")
+        g.Output(g.Gemm(v, False, g.Constant("w1", w1), False, 1.0, 0.0, None, (B, 3000), "wide"))
+        g.Output(g.Gemm(v, False, g.Constant("w2", w2), False, 1.0, 0.0, None, (B, 40), "narrow"))
+        outs.append(g.run({"x": x}))
+        assert g.describe().count("gpu ") == s
+        g.close()
+    for o in outs[1:]:
+        for name in outs[0]:
+            assert np.array_equal(o[name], outs[0][name]), name
