@@ -381,6 +381,7 @@ int conv_f32(const ConvGeom& g, int64_t images_full, const void* x, const void* 
 }
 bool gemm_f32_supported(const GemmGeom& g) { return g.M < (1ll << 31) && g.N < (1ll << 31) && g.K < (1ll << 30) && g.K > 0; }
 int gemm_f32(const GemmGeom& g, int64_t batch_full, int64_t rows_full, const void* A, const void* B, void* C, const Epilogue& ep, cudaStream_t s) {
+  if (g.batch <= 0 || g.M <= 0 || g.N <= 0) return 0;
   F32Params p{};
   p.M = (int)g.M; p.N = (int)g.N; p.K = (int)g.K;
   p.a_row = g.a_row; p.a_col = g.a_col; p.a_batch = g.a_batch;
@@ -391,7 +392,7 @@ int gemm_f32(const GemmGeom& g, int64_t batch_full, int64_t rows_full, const voi
   const bool bvec = g.b_row == 1 && g.b_col % 4 == 0 && (g.K % 4 == 0 || g.b_batch == 0) && g.b_batch % 4 == 0 && (uintptr_t)B % 16 == 0;
   // up to 16384 results (of the whole recorded batch, see pick_splits) the warps of one launch fit the chip at once and the
   // operands are re-read from L2 only
-  if (avec && bvec && g.K % 4 == 0 && g.batch > 0 && batch_full * rows_full * g.N <= 16384) {
+  if (avec && bvec && g.K % 4 == 0 && batch_full * rows_full * g.N <= 16384) {
     p.batches = (int)g.batch;
     const int64_t warps = g.batch * ((g.M + kFewRows - 1) / kFewRows) * ((g.N + kFewCols - 1) / kFewCols);
     b200::launch(f32_few_results_kernel, (unsigned)((warps + 3) / 4), 128, 0, s, p);

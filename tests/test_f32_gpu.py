@@ -78,3 +78,12 @@ def test_f32_results_do_not_depend_on_how_the_batch_is_cut(odla, gpu_lib):
     for o in outs[1:]:
         for name in outs[0]:
             assert np.array_equal(o[name], outs[0][name]), name
+
+
+@pytest.mark.parametrize("dims", [(0, 16, 8), (4, 16, 0), (0, 15, 8)])
+def test_f32_product_without_results(odla, gpu_lib, dims):
+    M, K, N = dims
+    g = odla.Graph(gpu_lib, "none", n_gpus=1)
+    g.Output(g.Gemm(g.Argument("a", (M, K)), False, g.Constant("w", np.ones((K, N), np.float32)), False, 1.0, 0.0, None, (M, N), "y"))
+    assert g.run({"a": np.ones((M, K), np.float32)})["y"].shape == (M, N)
+    g.close()
