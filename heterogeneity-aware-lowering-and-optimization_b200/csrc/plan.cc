@@ -1064,7 +1064,11 @@ odla_status Builder::emit_fused(const Item& it) {
     if (in_dt == DT_F32 && nhwc) {
       // fp32 storage: the tiled CUDA-core kernel, filters HWIO -> [K][R*S*C] with rows of whole 16-byte pieces
       g.xs_c = 1; g.xs_w = g.C; g.xs_h = (int64_t)g.W * g.C; g.xs_n = (int64_t)g.H * g.W * g.C;
-      if (conv_f32_supported(g)) {
+      // ... which multiplies the zeros of the padding by the filter: an infinity or NaN there would spread to border pixels
+      // that its tap does not reach, so such filters keep the kernel that leaves the padding out
+      const bool padded_window = g.pad_t > 0 || g.pad_l > 0 || (g.P - 1) * g.stride_h - g.pad_t + g.R > g.H || (g.Q - 1) * g.stride_w - g.pad_l + g.S > g.W;
+      auto all_finite = [&] { const auto wf = const_as_f32(f.w); return std::all_of(wf.begin(), wf.end(), [](float v) { return std::isfinite(v); }); };
+      if (conv_f32_supported(g) && (!padded_window || all_finite())) {
         const int64_t kd = (int64_t)g.R * g.S * g.C, pitch = (kd + 3) / 4 * 4;
         auto wb = prepared(f.w, "conv_f32_kmajor", [&] { return f32_rows_kmajor(const_as_f32(f.w), kd, K, pitch); });
         const void* wk = upload(wb->data(), wb->size());

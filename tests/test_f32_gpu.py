@@ -87,3 +87,26 @@ def test_f32_product_without_results(odla, gpu_lib, dims):
     g.Output(g.Gemm(g.Argument("a", (M, K)), False, g.Constant("w", np.ones((K, N), np.float32)), False, 1.0, 0.0, None, (M, N), "y"))
     assert g.run({"a": np.ones((M, K), np.float32)})["y"].shape == (M, N)
     g.close()
+
+
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+@pytest.mark.parametrize("pads", [((1, 1), (1, 1)), ((0, 0), (1, 1))])
+def test_conv_f32_padding_meets_no_filter_value(odla, gpu_lib, bad, pads):
+    """A filter with one infinite (or NaN) tap: pixels whose window has padding under that tap stay finite."""
+    (pt, pl), (pb, pr) = pads
+    H, C, K = 6, 8, 16
+    P = H + pt + pb - 2
+    x = np.random.default_rng(2).uniform(1, 2, (1, H, H, C)).astype(np.float32)
+    w = np.full((3, 3, C, K), 0.125, np.float32)
+    at = 0 if pt else 2
+    w[at, at] = bad
+    g = odla.Graph(gpu_lib, "c", n_gpus=1)
+    g.Output(g.Conv(g.Argument("x", x.shape), odla.CHANNELS_LAST, 1, g.Constant("w", w), odla.SIO, (1, 1), (1, 1), (pt, pl), (pb, pr), None, (1, P, P, K), "y"))
+    got = g.run({"x": x})["y"][0, :, :, 0]
+    g.close()
+    reached = np.zeros((P, P), bool)
+    reached[slice(1, None) if pt else slice(None, -1), slice(1, None) if pl else slice(None, -1)] = True
+    assert np.array_equal(np.isfinite(got), ~reached)
+    s = np.pad(x.sum(-1)[0].astype(np.float64) * 0.125, ((pt, pb), (pl, pr)))
+    want = sum(s[i:i + P, j:j + P] for i in range(3) for j in range(3))
+    np.testing.assert_allclose(got[~reached], want[~reached], rtol=1e-5)
