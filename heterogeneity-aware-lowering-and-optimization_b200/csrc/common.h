@@ -91,6 +91,7 @@ struct Launch {
   const void* out_ptr = nullptr;
   int out_dt = 0;
   int64_t out_count = 0, out_channels = 1;
+  int64_t out_cols = 0, out_pitch = 0;   // != 0: the value is out_cols columns of a matrix with out_pitch columns
   unsigned* range_stats = nullptr;   // device: [2 + 2 * out_channels] order-preserving keys of min / max, whole tensor then per channel
 };
 

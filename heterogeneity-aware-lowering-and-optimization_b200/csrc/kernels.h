@@ -235,7 +235,9 @@ int gather(int esz, const void* x, const void* idx, int idx_dt, void* y, int64_t
 // Running minimum / maximum of a dense float tensor (fp32 / fp16 / bf16) whose last axis has `channels` entries:
 // stats[0], stats[1] = whole tensor, stats[2 + c], stats[2 + channels + c] = channel c, all as order-preserving
 // unsigned keys (range_key_init / range_key_decode) updated with atomicMin / atomicMax, so calls accumulate.
-int range_minmax(int dt, const void* x, int64_t count, int64_t channels, unsigned* stats, cudaStream_t stream);
+// The rows of `channels` values lie one after the other, or, with row_cols > 0, row_cols / channels of them side by side in
+// each row of row_pitch values (a column group of a wider matrix).
+int range_minmax(int dt, const void* x, int64_t count, int64_t channels, unsigned* stats, cudaStream_t stream, int64_t row_cols = 0, int64_t row_pitch = 0);
 int range_stats_reset(unsigned* stats, int64_t channels, cudaStream_t stream);
 inline float range_key_decode(unsigned k) { unsigned b = (k & 0x80000000u) ? (k & 0x7fffffffu) : ~k; float f; memcpy(&f, &b, 4); return f; }
 

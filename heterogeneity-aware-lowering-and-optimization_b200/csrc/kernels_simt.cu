@@ -1360,7 +1360,7 @@ __global__ void range_reset_kernel(unsigned* stats, int64_t channels) {
 }
 // A block takes a contiguous run of rows; thread t keeps channels t, t + 256, ... (up to 16 of them) in registers and
 // publishes them with one atomic pair per channel at the end.
-__global__ void range_minmax_kernel(int dt, const void* __restrict__ x, int64_t rows, int channels, unsigned* __restrict__ stats) {
+__global__ void range_minmax_kernel(int dt, const void* __restrict__ x, int64_t rows, int channels, int64_t side_by_side, int64_t row_pitch, unsigned* __restrict__ stats) {
   dependency_wait();
   const int64_t per_block = (rows + gridDim.x - 1) / gridDim.x, r0 = blockIdx.x * per_block, r1 = min(rows, r0 + per_block);
   for (int c0 = 0; c0 < channels; c0 += 16 * blockDim.x) {
@@ -1368,10 +1368,11 @@ __global__ void range_minmax_kernel(int dt, const void* __restrict__ x, int64_t 
 #pragma unroll
     for (int k = 0; k < 16; ++k) { mn[k] = 3.402823466e+38f; mx[k] = -3.402823466e+38f; }
     for (int64_t r = r0; r < r1; ++r) {
+      const int64_t at = r / side_by_side * row_pitch + r % side_by_side * channels;
 #pragma unroll
       for (int k = 0; k < 16; ++k) {
         const int c = c0 + threadIdx.x + k * blockDim.x;
-        if (c < channels) { const float v = load_as_float(x, dt, r * channels + c); mn[k] = fminf(mn[k], v); mx[k] = fmaxf(mx[k], v); }
+        if (c < channels) { const float v = load_as_float(x, dt, at + c); mn[k] = fminf(mn[k], v); mx[k] = fmaxf(mx[k], v); }
       }
     }
     if (r1 > r0) {
@@ -1390,12 +1391,14 @@ int range_stats_reset(unsigned* stats, int64_t channels, cudaStream_t s) {
   launch(range_reset_kernel, grid_for(2 + 2 * channels, 256), 256, 0, s, stats, channels);
   return check_launch();
 }
-int range_minmax(int dt, const void* x, int64_t count, int64_t channels, unsigned* stats, cudaStream_t s) {
+int range_minmax(int dt, const void* x, int64_t count, int64_t channels, unsigned* stats, cudaStream_t s, int64_t row_cols, int64_t row_pitch) {
   if (count <= 0 || channels <= 0 || count % channels != 0 || channels > (1 << 30)) return 0;
+  if (row_cols <= 0) row_cols = row_pitch = channels;
+  if (row_cols % channels != 0) return 0;
   if (dt != DT_F32 && dt != DT_F16 && dt != DT_BF16) return 0;
   const int64_t rows = count / channels;
   int grid = (int)std::min<int64_t>(rows, (int64_t)sm_count() * 8);
-  launch(range_minmax_kernel, grid > 0 ? grid : 1, 256, 0, s, dt, x, rows, (int)channels, stats);
+  launch(range_minmax_kernel, grid > 0 ? grid : 1, 256, 0, s, dt, x, rows, (int)channels, row_cols / channels, row_pitch, stats);
   return check_launch();
 }
 // out[b][n][k] = in[b][k][n]: the last two axes swapped, through 32 x 32 shared-memory tiles so that both the reads

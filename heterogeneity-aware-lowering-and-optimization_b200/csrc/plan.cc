@@ -768,13 +768,20 @@ odla_status Builder::emit_group(const Item& it) {
   UmmaLaunch* ul = umma_conv_prepare(uc, dev_ptr(it.fused->x), wd, dev_ptr(it.out), ep, p_->status, sms);
   if (!ul) return fail(ODLA_FAILURE, "'" + root->name + "': tensor-map encoding failed");
   p_->umma.push_back(ul);
-  // one entry of the launch list per value; the kernel belongs to the first
-  add_launch("gemm_umma", it.out, 2.0 * M * N * Kd * G, tensor_bytes(it.fused->x) + G * tensor_bytes(it.out) + (double)(G * N * Kd) * storage_size(in_dt),
-             [ul](cudaStream_t s) { return umma_conv_run(ul, s); });
-  p_->launches.back().out_ptr = nullptr;   // (not a dense tensor of the value's own size: no range record)
-  for (size_t i = 1; i < it.group.size(); ++i) {
-    add_launch("gemm_umma", fused_[it.group[i]]->out, 0, 0, [](cudaStream_t) { return 0; });
-    p_->launches.back().n_kernels = 0;
+  // One entry of the launch list per value, each with its columns of the result for the range records; the kernel belongs to
+  // the first.
+  for (int64_t i = 0; i < G; ++i) {
+    V out = fused_[it.group[(size_t)i]]->out;
+    if (i == 0)
+      add_launch("gemm_umma", out, 2.0 * M * N * Kd * G, tensor_bytes(it.fused->x) + G * tensor_bytes(it.out) + (double)(G * N * Kd) * storage_size(in_dt),
+                 [ul](cudaStream_t s) { return umma_conv_run(ul, s); });
+    else add_launch("gemm_umma", out, 0, 0, [](cudaStream_t) { return 0; });
+    Launch& l = p_->launches.back();
+    const odla_value_shape sh = shape(out);
+    l.n_kernels = i == 0 ? 1 : 0;
+    l.out_ptr = (const char*)dev_ptr(it.out) + i * N * storage_size(ep.out_dt);
+    l.out_dt = ep.out_dt; l.out_count = count(out); l.out_channels = sh.dims[sh.size - 1];
+    l.out_cols = N; l.out_pitch = G * N;
   }
   return ODLA_SUCCESS;
 }
@@ -1929,7 +1936,7 @@ int run_launches(Replica& r, _odla_context* ctx, bool use_graph, long long* n_la
       *n_launched += l.n_kernels;
       if (!l.out_ptr || (l.out_dt != DT_F32 && l.out_dt != DT_F16 && l.out_dt != DT_BF16)) continue;
       if (!stats_for(l.range_stats, l.out_channels)) return -2;
-      if (range_minmax(l.out_dt, l.out_ptr, l.out_count, l.out_channels, l.range_stats, r.stream)) return -2;
+      if (range_minmax(l.out_dt, l.out_ptr, l.out_count, l.out_channels, l.range_stats, r.stream, l.out_cols, l.out_pitch)) return -2;
     }
     return 0;
   }

@@ -412,7 +412,8 @@ int odla_b200_DescribePlan(odla_computation computation, char* buf, int capacity
  * writes the table in halo_pgq's layout -- per value one record with ch_idx = -channels, scale = max(|min|, |max|) / 127
  * and offset 0 (the symmetric int8 scheme of this library), followed by one record per channel -- ready for
  * ODLA_QUANT_TABLE.  Values that a fused kernel never writes to memory (a convolution's result before its bias and
- * ReLU) have no record; every tensor a convolution or Gemm READS has one.  Returns the number of records; call with
+ * ReLU, the scores and probabilities inside a fused attention) have no record; every tensor that a convolution, or a Gemm
+ * with constant weights, READS has one, and so have the queries, keys and values an attention reads.  Returns the number of records; call with
  * records == NULL to size the array.  The value ids point into the computation and live as long as it does. */
 odla_status odla_b200_SetRangeProfiling(odla_context context, int enabled);
 int odla_b200_GetQuantTable(odla_context context, odla_value_quant_info* records, int capacity);
