@@ -1895,6 +1895,7 @@ int run_launches(Replica& r, _odla_context* ctx, bool use_graph, long long* n_la
     cudaEvent_t a, b;
     cudaEventCreate(&a); cudaEventCreate(&b);
     for (auto& l : p.launches) {
+      if (!l.n_kernels) continue;   // (written by the launch of an earlier entry, which has the time)
       cudaEventRecord(a, r.stream);
       int rc = inject_fault("launch") ? -2 : l.fn(r.stream);
       cudaEventRecord(b, r.stream);
@@ -2227,7 +2228,7 @@ int odla_b200_DescribePlan(odla_computation c, char* buf, int capacity) {
   for (auto& r : c->replicas) {
     snprintf(line, sizeof(line), "gpu %d rows [%lld,%lld) arena %lld bytes\n", r.device, (long long)r.shard_start, (long long)(r.shard_start + r.shard_batch), (long long)r.plan->arena_bytes);
     s += line;
-    for (auto& l : r.plan->launches) { snprintf(line, sizeof(line), "  %-12s %s\n", l.op.c_str(), l.name.c_str()); s += line; }
+    for (auto& l : r.plan->launches) { snprintf(line, sizeof(line), "  %-12s %s%s\n", l.op.c_str(), l.name.c_str(), l.n_kernels ? "" : " (by the launch above)"); s += line; }
   }
   if (buf && capacity > 0) { snprintf(buf, (size_t)capacity, "%s", s.c_str()); }
   return (int)s.size() + 1;

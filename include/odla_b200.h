@@ -391,7 +391,7 @@ typedef struct {
   char op[32];          /* kernel family, e.g. "conv_umma", "maxpool" */
   char name[64];        /* id of the ODLA value the launch produces */
   double total_ms;      /* summed event time over the profiled executions */
-  long long launches;   /* how many times it ran while profiling was on */
+  long long launches;   /* how many times it ran while profiling was on (0: the launch of an earlier entry writes the value too) */
   double flops;         /* algorithmic 2*MAC per launch (0 for memory-bound kernels) */
   double bytes;         /* algorithmic bytes read + written per launch */
 } odla_b200_profile_entry;
@@ -401,7 +401,8 @@ int odla_b200_GetProfile(odla_context context, odla_b200_profile_entry* entries,
 /* Number of kernel launches the most recent odla_ExecuteComputation issued, all GPUs. */
 long long odla_b200_LastExecuteLaunches(odla_context context);
 
-/* Text description of the launch list (one line per kernel) into buf; returns bytes needed. */
+/* Text description of the launch list into buf, one line per value that is written to memory (a value that the launch of an
+ * earlier line writes too is marked); returns bytes needed. */
 int odla_b200_DescribePlan(odla_computation computation, char* buf, int capacity);
 
 /* Range profiling on the GPU -- what the reference does with a wrapper platform that evaluates every op on the host and

@@ -48,3 +48,27 @@ def test_records_of_q_k_v_are_those_of_the_unfused_graph(odla, gpu_lib, monkeypa
         for ch, (mn, mx) in want.items():
             np.testing.assert_allclose(fused[n + "t"][ch], (mn, mx), rtol=2.0 ** -10, atol=2.0 ** -10)   # one rounding to fp16
             np.testing.assert_allclose(plain[n + "t"][ch], (mn, mx), rtol=2.0 ** -10, atol=2.0 ** -10)
+
+
+def test_launch_list_tells_launches_from_values(odla, gpu_lib):
+    """The keys and values of grouped projections have entries of their own, marked as written by the launch above, and the
+    profile counts no launch for them."""
+    B, S, NH, D, E = 2, 32, 2, 64, 64
+    rng = np.random.default_rng(0)
+    g = odla.Graph(gpu_lib, "list", fp16=True, n_gpus=1)
+    x = g.Argument("x", (B * S, E))
+    heads = []
+    for n in "qkv":
+        y = g.Gemm(x, False, g.Constant("w" + n, rng.standard_normal((E, NH * D)).astype(np.float32) * 0.1), False, 1.0, 0.0, None, (B * S, NH * D), n)
+        heads.append(g.Transpose(g.Reshape(y, (B, S, NH, D), n + "4"), (0, 2, 1, 3), (B, NH, S, D), n + "t"))
+    sc = g.Mul(g.Gemm(heads[0], False, heads[1], True, 1.0, 0.0, None, (B, NH, S, S), "scores"), g.Constant("scale", np.array([0.125], np.float32)), "scaled")
+    ctx = g.Gemm(g.Softmax(sc, -1, "probs"), False, heads[2], False, 1.0, 0.0, None, (B, NH, S, D), "ctx")
+    g.Output(g.Transpose(ctx, (0, 2, 1, 3), (B, S, NH, D), "merged"))
+    xin, out = rng.standard_normal((B * S, E)).astype(np.float32), np.empty((B, S, NH, D), np.float32)
+    g.bind_input("x", xin.ctypes.data)
+    g.bind_output("merged", out.ctypes.data)
+    lines = {l.split()[1]: l for l in g.describe().splitlines() if l.startswith("  ")}
+    runs = {p["name"]: p["launches"] for p in g.profile(runs=2)}
+    g.close()
+    for n, of_its_own in (("qt", True), ("kt", False), ("vt", False), ("merged", True)):
+        assert ("(by the launch above)" in lines[n]) == (not of_its_own) and runs[n] == (2 if of_its_own else 0)
