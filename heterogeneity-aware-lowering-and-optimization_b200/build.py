@@ -14,6 +14,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libodla_b200.so")
+REPORTS = os.path.join(CSRC, "build")   # what ptxas says of every kernel (registers, spills), one file per source
 SOURCES = ["api.cc", "plan.cc", "quant_table.cc", "executable.cc", "kabi.cu", "noalloc.cu", "kernels_simt.cu", "kernels_f32.cu", "kernels_detect.cu", "kernels_umma.cu"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -40,8 +41,12 @@ def build(force=False, verbose=False):
         if force or _stale(o, [s] + headers):
             jobs.append([NVCC] + FLAGS + ["-c", s, "-o", o])
 
+    os.makedirs(REPORTS, exist_ok=True)
+
     def run(cmd):
         r = subprocess.run(cmd, capture_output=True, text=True)
+        with open(os.path.join(REPORTS, os.path.basename(cmd[-3]) + ".ptxas"), "w") as f:
+            f.write(r.stderr)
         return cmd, r
 
     with concurrent.futures.ThreadPoolExecutor(max_workers=max(1, len(jobs))) as ex:

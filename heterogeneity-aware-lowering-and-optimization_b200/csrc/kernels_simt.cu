@@ -493,11 +493,16 @@ __global__ void softmax_rows_vec_kernel(const uint4* __restrict__ x, uint4* __re
 // rows are under way: blocks of four warps, seven to an SM (72 registers a thread), leave no gap that blocks of eight do.
 // 8192 rows of 768 two-byte values: 15.8 -> 13.9 us, with their int8 copy 18.2 -> 16.8 (a bracketed launch alone is 2.6).
 // Ten blocks spill.
-// EARLY: gamma and beta are requested with the row instead of after its sums.  That takes 48 more registers, i.e. rows under
-// way, and so pays where all rows are under way anyway (693 rows: 9.2 -> 7.6 us) and loses where they queue (8192: 15.8).
-constexpr int kLayernormThreads = 128;
+// A lane holds 8 * NP values of its row, so the blocks an SM can take fall with NP.  Six at NP = 4 (8192 rows of 1024:
+// 14.0 us; seven spill beside the int8 copy).  NP = 8 needs 128 registers and keeps two blocks of eight warps; seven blocks of four would hold the row in
+// local memory (8192 rows of 2048: 25.2 -> 30.6 us, with their int8 copy 39 -> 46; 2000 rows 10.5 -> 20).
+// EARLY: gamma and beta are requested with the row instead of after its sums.  That takes 16 * NP more registers, i.e. rows under
+// way, and so pays where all rows are under way anyway (693 rows of 768: 9.2 -> 7.6 us) and loses where they queue (8192: 15.8).
+// At NP = 8 the two do not fit a thread's registers beside the row: no EARLY form.
+constexpr int layernorm_threads(int np) { return np <= 4 ? 128 : 256; }
+constexpr int layernorm_blocks(int np, bool early) { return np <= 3 ? (early ? 4 : 7) : np == 4 ? (early ? 3 : 6) : 2; }
 template <typename T, int NP, int LPR, bool QUANT, bool EARLY>
-__global__ void __launch_bounds__(kLayernormThreads, EARLY ? 4 : 7) layernorm_rows_vec_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, const float* __restrict__ gamma,
+__global__ void __launch_bounds__(layernorm_threads(NP), layernorm_blocks(NP, EARLY)) layernorm_rows_vec_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, const float* __restrict__ gamma,
                                           const float* __restrict__ beta, int64_t rows, int pieces, float eps, uint2* __restrict__ qout, const float* __restrict__ qscale) {
   dependency_wait();
   const QuantDiv qd(QUANT ? qscale[0] : 1.f);
@@ -542,12 +547,18 @@ __global__ void __launch_bounds__(kLayernormThreads, EARLY ? 4 : 7) layernorm_ro
       if (have[i]) {
         const int d0 = (l + LPR * i) * 8;
         float gm[8], bt[8];
-        if (!EARLY) {
+        if (!EARLY && NP <= 4) {
           if (gamma) { gm4[i][0] = __ldg((const float4*)(gamma + d0)); gm4[i][1] = __ldg((const float4*)(gamma + d0 + 4)); }
           if (beta) { bt4[i][0] = __ldg((const float4*)(beta + d0)); bt4[i][1] = __ldg((const float4*)(beta + d0 + 4)); }
         }
-        if (gamma) { const float4 g0 = gm4[i][0], g1 = gm4[i][1]; gm[0] = g0.x; gm[1] = g0.y; gm[2] = g0.z; gm[3] = g0.w; gm[4] = g1.x; gm[5] = g1.y; gm[6] = g1.z; gm[7] = g1.w; }
-        if (beta) { const float4 b0 = bt4[i][0], b1 = bt4[i][1]; bt[0] = b0.x; bt[1] = b0.y; bt[2] = b0.z; bt[3] = b0.w; bt[4] = b1.x; bt[5] = b1.y; bt[6] = b1.z; bt[7] = b1.w; }
+        if (gamma) {
+          const float4 g0 = NP <= 4 ? gm4[i][0] : __ldg((const float4*)(gamma + d0)), g1 = NP <= 4 ? gm4[i][1] : __ldg((const float4*)(gamma + d0 + 4));
+          gm[0] = g0.x; gm[1] = g0.y; gm[2] = g0.z; gm[3] = g0.w; gm[4] = g1.x; gm[5] = g1.y; gm[6] = g1.z; gm[7] = g1.w;
+        }
+        if (beta) {
+          const float4 b0 = NP <= 4 ? bt4[i][0] : __ldg((const float4*)(beta + d0)), b1 = NP <= 4 ? bt4[i][1] : __ldg((const float4*)(beta + d0 + 4));
+          bt[0] = b0.x; bt[1] = b0.y; bt[2] = b0.z; bt[3] = b0.w; bt[4] = b1.x; bt[5] = b1.y; bt[6] = b1.z; bt[7] = b1.w;
+        }
         uint32_t w[4];
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
@@ -578,12 +589,13 @@ bool launch_rows_vec(bool is_softmax, const void* x, void* y, const float* gamma
   const int pieces = (int)(dim / 8);
   const int lpr = pieces <= 8 ? 8 : (pieces <= 16 ? 16 : 32), np = (pieces + lpr - 1) / lpr;
   const int grid = grid_for(rows * lpr, 256);
-  const int norm_grid = grid_for(rows * lpr, kLayernormThreads);
-  const bool early = rows * lpr <= (int64_t)sm_count() * 16 * 32;   // 16 warps of the EARLY form fit an SM
+  const int norm_threads = layernorm_threads(np);
+  const int norm_grid = grid_for(rows * lpr, norm_threads);
+  const bool early = np <= 4 && rows * lpr <= (int64_t)sm_count() * layernorm_blocks(np, true) * layernorm_threads(np);   // all rows under way
 #define B2_NORM(NP, LPR, Q, EARLY)                                                                                                            \
   do {                                                                                                                                        \
-    if (EARLY) launch(layernorm_rows_vec_kernel<T, NP, LPR, Q, true>, norm_grid, kLayernormThreads, 0, s, (const uint4*)x, (uint4*)y, gamma, beta, rows, pieces, eps, (uint2*)q, qscale); \
-    else launch(layernorm_rows_vec_kernel<T, NP, LPR, Q, false>, norm_grid, kLayernormThreads, 0, s, (const uint4*)x, (uint4*)y, gamma, beta, rows, pieces, eps, (uint2*)q, qscale); \
+    if ((EARLY) && NP <= 4) launch(layernorm_rows_vec_kernel<T, NP <= 4 ? NP : 4, LPR, Q, true>, norm_grid, norm_threads, 0, s, (const uint4*)x, (uint4*)y, gamma, beta, rows, pieces, eps, (uint2*)q, qscale); \
+    else launch(layernorm_rows_vec_kernel<T, NP, LPR, Q, false>, norm_grid, norm_threads, 0, s, (const uint4*)x, (uint4*)y, gamma, beta, rows, pieces, eps, (uint2*)q, qscale); \
   } while (0)
 #define B2_ROWS(NP, LPR)                                                                                                                      \
   do {                                                                                                                                        \
