@@ -76,6 +76,7 @@ __device__ __forceinline__ bool overlaps_yolo(const float (&s)[4], const float (
 constexpr int kGathered = 1024;   // candidates of one problem kept in shared memory: boxes 16 KB, scores and indices 8 KB
 constexpr int kNmsThreads = 512;
 constexpr int kNmsSmem = kGathered * 24;
+constexpr int kNmsMaxBoxes = 1500000;   // their mask takes 183 KB of shared memory
 
 // grid = problems (batch x class); sel[p][k] = k-th selected box of problem p, cnt[p] = how many.
 template <int MODE>
@@ -317,8 +318,10 @@ __global__ void yolo_emit_kernel(const int* __restrict__ sel, const int* __restr
 int nms(int B, int C, int N, int max_sel, float iou_thr, float score_thr, int box_dt, const void* boxes, int score_dt, const void* scores, int out_rows,
         int out64, void* out, int* sel, int* cnt, cudaStream_t s) {
   if (B * C <= 0 || out_rows <= 0) return 0;
-  if (B * C > 1024 || N > 1500000) return -1;
+  if (B * C > 1024 || N > kNmsMaxBoxes) return -1;
   if (N > 0 && max_sel > 0) {
+    if (((N + 31) / 32) * 4 > 40 * 1024 &&   // the mask and the kernel's own arrays may pass the 48 KB every launch gets
+        cudaFuncSetAttribute(greedy_nms_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (kNmsMaxBoxes + 31) / 32 * 4) != cudaSuccess) { check_launch(); return -2; }
     launch(greedy_nms_kernel<0>, B * C, kNmsThreads, std::max(kNmsSmem, ((N + 31) / 32) * 4), s, boxes, box_dt, scores, score_dt, C, N, max_sel, iou_thr, score_thr, sel, cnt);
     if (int rc = check_launch()) return rc;
   } else if (cudaMemsetAsync(cnt, 0, sizeof(int) * B * C, s) != cudaSuccess) return -2;

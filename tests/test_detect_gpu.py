@@ -109,3 +109,23 @@ def test_yolo_postprocess_matches_the_oracle(odla, gpu_lib, ref, layout, mode):
     tol = 1e-3 if mode == "fp32" else 0.5          # pixels; fp16 storage rounds the result
     assert np.abs(got["det0"][..., :4] - want["det0"][..., :4]).max() <= tol
     assert np.abs(got["det0"][..., 4] - want["det0"][..., 4]).max() <= (1e-5 if mode == "fp32" else 2e-3)
+
+
+@pytest.mark.parametrize("N,candidates", [(400000, 30), (400000, 3000), (1500000, 30)])
+def test_nms_over_very_many_boxes(odla, gpu_lib, N, candidates):
+    """Numbers of boxes whose mask of one bit each passes 48 KB, with candidates that are gathered and with more than are."""
+    rng = np.random.default_rng(N)
+    boxes = random_boxes(rng, 1, N, size=20000.0)
+    scores = np.zeros((1, 2, N), np.float32)
+    for c in range(2):
+        at = rng.choice(N, candidates, replace=False)
+        scores[0, c, at] = rng.uniform(0.5, 1.0, candidates).astype(np.float32)
+    g = odla.Graph(gpu_lib, "nms")
+    g.Output(g.NMS(g.Argument("boxes", boxes.shape), g.Argument("scores", scores.shape), 12, 0.5, 0.35, 24, "sel"))
+    got = g.run({"boxes": boxes, "scores": scores})["sel"]
+    g.close()
+    # the rule over the candidates alone, with their own numbers put back
+    cand = np.unique(np.nonzero(scores[0] > 0.35)[1])
+    want = numpy_nms(boxes[:, cand], scores[:, :, cand], 12, np.float32(0.5), np.float32(0.35), 24)
+    want[:, 2] = np.where(want[:, 2] >= 0, cand[want[:, 2]], -1)
+    assert np.array_equal(got.astype(np.int64), want)
