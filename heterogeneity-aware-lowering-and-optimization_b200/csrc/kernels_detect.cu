@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(kNmsThreads)
 greedy_nms_kernel(const void* __restrict__ boxes, int box_dt, const void* __restrict__ scores, int score_dt, int C, int N, int max_sel,
                   float iou_thr, float score_thr, int* __restrict__ sel, int* __restrict__ cnt) {
   dependency_wait();
-  extern __shared__ uint32_t alive[];          // the gathered candidates; MODE 0 without them: one bit per candidate
+  extern __shared__ __align__(16) uint32_t alive[];   // the gathered candidates, boxes first; MODE 0 without them: one bit per candidate
   __shared__ Cand warp_c[32];
   __shared__ Cand chosen;
   __shared__ int n_gathered;
