@@ -357,17 +357,21 @@ int run(F32Params p, int la, bool bvec, int64_t batch, int64_t batch_full, int64
   p.n_tiles = (p.N + kTile - 1) / kTile;
   const int64_t tiles = batch * p.m_tiles * p.n_tiles;
   if (tiles <= 0) return 0;
-  if (tiles > 0x7fffffffLL) return -1;
   p.splits = pick_splits(batch_full * ((rows_full + kTile - 1) / kTile) * p.n_tiles, p.num_kb);
   if (la == LOAD_CONV_VEC) return launch_tiles<LOAD_CONV_VEC, true>(p, tiles, s);
   if (la == LOAD_CONV_SCALAR) return launch_tiles<LOAD_CONV_SCALAR, true>(p, tiles, s);
   if (la == LOAD_GEMM_VEC) return bvec ? launch_tiles<LOAD_GEMM_VEC, true>(p, tiles, s) : launch_tiles<LOAD_GEMM_VEC, false>(p, tiles, s);
   return bvec ? launch_tiles<LOAD_GEMM_SCALAR, true>(p, tiles, s) : launch_tiles<LOAD_GEMM_SCALAR, false>(p, tiles, s);
 }
+// What the kernels' 32-bit indices can address: rows and columns of the last tile included, and one block per tile.
+bool indexable(int64_t batch, int64_t M, int64_t N, int64_t K) {
+  const int64_t most = (1ll << 31) - kTile;
+  return M < most && N < most && K < (1ll << 30) && batch < (1ll << 31) && (double)batch * ((M + kTile - 1) / kTile) * ((N + kTile - 1) / kTile) < 2147483648.0;
+}
 }  // namespace
 
 bool conv_f32_supported(const ConvGeom& g) {
-  return g.groups == 1 && g.xs_c == 1 && (int64_t)g.N * g.P * g.Q < (1ll << 31) && (int64_t)g.R * g.S * g.C < (1ll << 30) && g.P > 0 && g.Q > 0;
+  return g.groups == 1 && g.xs_c == 1 && g.P > 0 && g.Q > 0 && indexable(1, (int64_t)g.N * g.P * g.Q, g.K, (int64_t)g.R * g.S * g.C);
 }
 int conv_f32(const ConvGeom& g, int64_t images_full, const void* x, const void* w, int64_t w_pitch, void* y, const Epilogue& ep, cudaStream_t s) {
   F32Params p{};
@@ -379,7 +383,7 @@ int conv_f32(const ConvGeom& g, int64_t images_full, const void* x, const void* 
   const bool vec = g.C % 4 == 0 && (uintptr_t)x % 16 == 0;
   return run(p, vec ? LOAD_CONV_VEC : LOAD_CONV_SCALAR, true, 1, 1, images_full * g.P * g.Q, s);
 }
-bool gemm_f32_supported(const GemmGeom& g) { return g.M < (1ll << 31) && g.N < (1ll << 31) && g.K < (1ll << 30) && g.K > 0; }
+bool gemm_f32_supported(const GemmGeom& g) { return g.K > 0 && indexable(g.batch, g.M, g.N, g.K); }
 int gemm_f32(const GemmGeom& g, int64_t batch_full, int64_t rows_full, const void* A, const void* B, void* C, const Epilogue& ep, cudaStream_t s) {
   if (g.batch <= 0 || g.M <= 0 || g.N <= 0) return 0;
   F32Params p{};
