@@ -2065,7 +2065,7 @@ constexpr int kLongReduction = 12;   // k-blocks from which a tile's time is its
 void choose_split(const UmmaConv& c, int sms, UmmaParams& p) {
   p.splits = 1;
   p.bm = BM;
-  if (c.store_mode != 0 || getenv("ODLA_B200_NO_SPLIT") || getenv("ODLA_B200_PAIR_MIN_KB")) return;
+  if (c.store_mode != 0 || getenv("ODLA_B200_NO_SPLIT")) return;
   auto tiles = [](int64_t n, int64_t t) { return (n + t - 1) / t; };
   const int64_t rows_full = std::max<int64_t>(c.rows_full, p.M_total);
   double best = 176.0 * p.num_kb;

@@ -53,3 +53,35 @@ def test_long_reductions(odla, gpu_lib, size, residual, dtype):
     # one rounding of the sum before the residual and one after it, of values below eight
     step = 2.0 ** (-10 if dtype == "f16" else -7)
     np.testing.assert_allclose(got, ref, rtol=step, atol=2 * step)
+
+
+def raw_conv(odla, lib, dtype, N, H, W, C, K, R, out_kind, seed=3, **epilogue):
+    """odla_b200_conv_umma over integers (int8) or values of the type; (result, the operands as float64 / int64)."""
+    import ctypes
+    rng = np.random.default_rng(seed)
+    if dtype == "s8":
+        x, w = (torch.from_numpy(rng.integers(-127, 128, s, dtype=np.int8)).cuda() for s in ((N, H, W, C), (K, R * R * C)))
+    else:
+        t = {"f16": torch.float16, "bf16": torch.bfloat16}[dtype]
+        x, w = (torch.from_numpy(rng.standard_normal(s).astype(np.float32) * k).to(t).cuda() for s, k in (((N, H, W, C), 1.0), ((K, R * R * C), (R * R * C) ** -0.5)))
+    y = torch.zeros((N, H, W, K), dtype={1: torch.float32, 2: torch.int8, 3: torch.int32}[out_kind], device="cuda")
+    tensors = {n: torch.from_numpy(v).cuda() for n, v in epilogue.items() if isinstance(v, np.ndarray)}
+    ptr = lambda n: tensors[n].data_ptr() if n in tensors else None
+    d = odla.ConvDesc(n=N, h=H, w=W, c=C, k=K, r=R, s=R, stride_h=1, stride_w=1, pad_top=R // 2, pad_left=R // 2, p=H, q=W, dtype=["f16", "bf16", "s8"].index(dtype), out_kind=out_kind,
+                      res_kind=2 if "res" in tensors else 0, act=epilogue.get("act", 0), alpha=0, res_scale=epilogue.get("res_scale", 1), out_scale=epilogue.get("out_scale", 1),
+                      out_multiply=epilogue.get("out_multiply", 0))
+    torch.cuda.synchronize()
+    assert lib.b200_conv_umma(ctypes.byref(d), x.data_ptr(), w.data_ptr(), ptr("mul"), ptr("add"), ptr("res"), y.data_ptr(), None) == 0
+    acc = torch.nn.functional.conv2d(x.double().permute(0, 3, 1, 2), w.double().view(K, R, R, C).permute(0, 3, 1, 2), padding=R // 2).permute(0, 2, 3, 1)
+    return y.cpu().numpy(), acc.cpu().numpy()
+
+
+def test_the_switch_for_pairs_leaves_shared_reductions_on(odla, gpu_lib, monkeypatch):
+    """ODLA_B200_PAIR_MIN_KB at its own default changes nothing, here for a layer whose reduction eight CTAs share."""
+    size = (1, 7, 7, 512, 512, 3)
+    default, _ = raw_conv(odla, gpu_lib, "f16", *size, out_kind=1)
+    monkeypatch.setenv("ODLA_B200_PAIR_MIN_KB", "12")
+    switched, _ = raw_conv(odla, gpu_lib, "f16", *size, out_kind=1)
+    monkeypatch.setenv("ODLA_B200_NO_SPLIT", "1")
+    unshared, _ = raw_conv(odla, gpu_lib, "f16", *size, out_kind=1)
+    assert np.array_equal(default, switched) and not np.array_equal(default, unshared)
