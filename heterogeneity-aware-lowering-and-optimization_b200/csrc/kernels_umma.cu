@@ -2238,8 +2238,11 @@ UmmaLaunch* umma_conv_prepare(const UmmaConv& c, const void* x, const void* w, v
     p.box_arrivals = 4 * (groups_per_box < 1 ? 1 : groups_per_box);
     // Contiguous runs let the groups work on different boxes at once, which pays when boxes need no residual and
     // the CTA has many tiles to stream through; otherwise finishing box after box gets the first store out sooner.
-    p.epi_interleave = ep.res != nullptr || (p.total_tiles << p.pair) < 16 * sms || p.ring_boxes < p.stage_boxes || p.BN == 192;
+    p.epi_interleave = ep.res != nullptr || (p.total_tiles << p.pair) < 16 * sms;
     if (getenv("ODLA_B200_EPI_INTERLEAVE")) p.epi_interleave = atoi(getenv("ODLA_B200_EPI_INTERLEAVE"));
+    // Runs need a box of its own for every group of the tile, and whole groups to a box: with fewer boxes a group would find the
+    // phase before last of its box complete, with 192 columns a box would count its arrivals short.
+    if (p.ring_boxes < p.stage_boxes || p.BN == 192) p.epi_interleave = 1;
     if (p.epi_interleave) p.box_arrivals = 16;
   }
   p.stages = (budget - p.ring_boxes * 16384) / stage_bytes;

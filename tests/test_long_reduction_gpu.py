@@ -85,3 +85,12 @@ def test_the_switch_for_pairs_leaves_shared_reductions_on(odla, gpu_lib, monkeyp
     monkeypatch.setenv("ODLA_B200_NO_SPLIT", "1")
     unshared, _ = raw_conv(odla, gpu_lib, "f16", *size, out_kind=1)
     assert np.array_equal(default, switched) and not np.array_equal(default, unshared)
+
+
+@pytest.mark.parametrize("chunks", ["0", "1"])
+@pytest.mark.parametrize("size", [(16, 26, 26, 256, 512, 3), (1, 65, 100, 768, 320, 1), (1, 64, 128, 768, 256, 1)])
+def test_epilogue_chunk_assignment_on_long_reductions(odla, gpu_lib, monkeypatch, size, chunks):
+    """ODLA_B200_EPI_INTERLEAVE either way, where two boxes go round for a tile of three or four and where a tile has 192 columns."""
+    monkeypatch.setenv("ODLA_B200_EPI_INTERLEAVE", chunks)
+    got, ref = run_conv(odla, gpu_lib, *size, False, "f16")
+    np.testing.assert_allclose(got, ref, rtol=2.0 ** -10, atol=2.0 ** -9)   # one rounding of the result, values below eight
