@@ -130,16 +130,21 @@ __device__ __forceinline__ void load_b(const F32Params& p, uint32_t dst, const f
   }
 }
 
-// Four neighbouring results of one row: the common forms on vectors, everything else through the scalar epilogue.
+// Four neighbouring results of one row: the common forms on vectors, everything else through the scalar epilogue.  Every step is
+// rounded by itself, as there.
 __device__ __forceinline__ void finish4(const F32Params& p, float4 v, int64_t row, int col, bool plain) {
   const Epilogue& ep = p.ep;
   float t[4] = {v.x, v.y, v.z, v.w};
   if (plain) {
-    if (ep.alpha != 1.f) { t[0] *= ep.alpha; t[1] *= ep.alpha; t[2] *= ep.alpha; t[3] *= ep.alpha; }
-    if (ep.add1) { const float4 a = __ldg((const float4*)(ep.add1 + col)); t[0] = __fadd_rn(t[0], a.x); t[1] = __fadd_rn(t[1], a.y); t[2] = __fadd_rn(t[2], a.z); t[3] = __fadd_rn(t[3], a.w); }
-    if (ep.add2) { const float4 a = __ldg((const float4*)(ep.add2 + col)); t[0] += a.x; t[1] += a.y; t[2] += a.z; t[3] += a.w; }
+    auto add = [&](const float4& a) { t[0] = __fadd_rn(t[0], a.x); t[1] = __fadd_rn(t[1], a.y); t[2] = __fadd_rn(t[2], a.z); t[3] = __fadd_rn(t[3], a.w); };
+    if (ep.alpha != 1.f) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) t[j] = __fmul_rn(t[j], ep.alpha);
+    }
+    if (ep.add1) add(__ldg((const float4*)(ep.add1 + col)));
+    if (ep.add2) add(__ldg((const float4*)(ep.add2 + col)));
     if (ep.act_first) apply_act_all<4>(ep.act, t, ep.act_a, ep.act_b);
-    if (ep.res) { const float4 a = *(const float4*)((const float*)ep.res + row * p.N + col); t[0] += a.x; t[1] += a.y; t[2] += a.z; t[3] += a.w; }
+    if (ep.res) add(*(const float4*)((const float*)ep.res + row * p.N + col));
     if (!ep.act_first) apply_act_all<4>(ep.act, t, ep.act_a, ep.act_b);
     *(float4*)((float*)p.y + row * p.N + col) = make_float4(t[0], t[1], t[2], t[3]);
   } else {

@@ -110,3 +110,22 @@ def test_conv_f32_padding_meets_no_filter_value(odla, gpu_lib, bad, pads):
     s = np.pad(x.sum(-1)[0].astype(np.float64) * 0.125, ((pt, pb), (pl, pr)))
     want = sum(s[i:i + P, j:j + P] for i in range(3) for j in range(3))
     np.testing.assert_allclose(got[~reached], want[~reached], rtol=1e-5)
+
+
+@pytest.mark.parametrize("N", [4096, 4095, 12])   # four results at a time, one at a time, a warp per 4 x 2 results
+def test_f32_epilogue_rounds_every_step(odla, gpu_lib, N):
+    """alpha, per-channel addend, LeakyReLU and residual on products with a single term: numpy's fp32 steps, bit for bit."""
+    M, K = 8, 4
+    rng = np.random.default_rng(N)
+    a, w = np.zeros((M, K), np.float32), np.zeros((K, N), np.float32)
+    a[:, 0], w[0] = rng.standard_normal(M), rng.standard_normal(N)
+    b, r = rng.standard_normal((1, N)).astype(np.float32), rng.standard_normal((M, N)).astype(np.float32)
+    alpha, slope = np.float32(0.3), np.float32(0.1)
+    g = odla.Graph(gpu_lib, "r", n_gpus=1)
+    aa, ra = g.Argument("a", a.shape), g.Argument("r", r.shape)
+    y = g.Add(g.Gemm(aa, False, g.Constant("w", w), False, float(alpha), 0.0, None, (M, N), "gemm"), g.Constant("b", b), "bias")
+    g.Output(g.Add(g.LeakyRelu(y, float(slope), "act"), ra, "y"))
+    got = g.run({"a": a, "r": r})["y"]
+    g.close()
+    t = alpha * (a[:, :1] * w[:1]) + b
+    assert np.array_equal(got, np.where(t < 0, slope * t, t) + r)
