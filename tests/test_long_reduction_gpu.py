@@ -94,3 +94,57 @@ def test_epilogue_chunk_assignment_on_long_reductions(odla, gpu_lib, monkeypatch
     monkeypatch.setenv("ODLA_B200_EPI_INTERLEAVE", chunks)
     got, ref = run_conv(odla, gpu_lib, *size, False, "f16")
     np.testing.assert_allclose(got, ref, rtol=2.0 ** -10, atol=2.0 ** -9)   # one rounding of the result, values below eight
+
+
+@pytest.mark.parametrize("K", [255, 10, 64])
+@pytest.mark.parametrize("residual", [False, True])
+def test_shared_reductions_store_any_number_of_columns(odla, gpu_lib, K, residual):
+    """Results of two-byte storage that leave as fp32: rows padded to 16 bytes inside (255 and 10 columns without a residual),
+    finished value by value, or, with a residual, stored densely."""
+    got, ref = run_conv(odla, gpu_lib, 1, 7, 9, 2048, K, 1, residual, "bf16")
+    np.testing.assert_allclose(got, ref, rtol=2.0 ** -7, atol=2.0 ** -6)
+
+
+@pytest.mark.parametrize("dtype", ["f16", "bf16", "s8"])
+@pytest.mark.parametrize("K", [255, 10, 512])
+def test_shared_reductions_raw_accumulators(odla, gpu_lib, dtype, K):
+    """fp32 and int32 results of a reduction over 4608 products: exact integers, fp32 sums in any order."""
+    got, acc = raw_conv(odla, gpu_lib, dtype, 1, 7, 7, 512, K, 3, out_kind=3 if dtype == "s8" else 1)
+    if dtype == "s8":
+        assert np.array_equal(got, acc.astype(np.int64))
+    else:   # partial sums of up to 4608 exact products of magnitude 4608^-1/2
+        np.testing.assert_allclose(got, acc, rtol=0, atol=4608 ** 0.5 * 2.0 ** -24 * 16)
+
+
+@pytest.mark.parametrize("multiply", [0, 1])
+@pytest.mark.parametrize("K", [512, 72, 130])
+def test_shared_reductions_requantise_bit_exact(odla, gpu_lib, K, multiply):
+    rng = np.random.default_rng(K)
+    e = dict(mul=rng.uniform(1e-5, 1e-4, K).astype(np.float32), add=rng.standard_normal(K).astype(np.float32), res=rng.integers(-128, 128, (1, 7, 7, K), dtype=np.int8),
+             act=1, res_scale=float(np.float32(0.037)), out_scale=float(np.float32(0.021)), out_multiply=multiply)
+    got, acc = raw_conv(odla, gpu_lib, "s8", 1, 7, 7, 512, K, 3, out_kind=2, **e)
+    v = acc.astype(np.float32) * e["mul"] + e["add"] + e["res"].astype(np.float32) * np.float32(0.037)     # numpy rounds every step to fp32, as the kernel does
+    v = np.maximum(v, np.float32(0))
+    scaled = v * (np.float32(1.0) / np.float32(0.021)) if multiply else v / np.float32(0.021)
+    assert np.array_equal(got, np.clip(np.rint(scaled), -128, 127).astype(np.int8))
+
+
+@pytest.mark.parametrize("N,transposed", [(64, False), (64, True), (96, False), (96, True)])
+def test_shared_reductions_of_batched_products(odla, gpu_lib, monkeypatch, N, transposed):
+    """Two run-time operands, 2 x [128, 2048] x [2048, N]: the right one read as it lies (64 columns), transposed first, or K-major."""
+    B, M, K = 2, 128, 2048
+    rng = np.random.default_rng(N)
+    a, b = [torch.from_numpy(rng.standard_normal(s).astype(np.float32)).half() for s in ((B, M, K), (B, N, K) if transposed else (B, K, N))]
+    b = (b.float() / K ** 0.5).half()
+    outs = []
+    for unshared in (False, True):
+        if unshared:
+            monkeypatch.setenv("ODLA_B200_NO_SPLIT", "1")
+        g = odla.Graph(gpu_lib, "g", fp16=True, n_gpus=1)
+        g.Output(g.Gemm(g.Argument("a", a.shape, odla.FLOAT16), False, g.Argument("b", b.shape, odla.FLOAT16), transposed, 1.0, 0.0, None, (B, M, N), "y"))
+        outs.append(g.run({"a": a.numpy(), "b": b.numpy()})["y"])
+        assert "gemm_umma" in g.describe()
+        g.close()
+    want = np.einsum("bmk,bnk->bmn" if transposed else "bmk,bkn->bmn", a.double().numpy(), b.double().numpy())
+    for o in outs:
+        np.testing.assert_allclose(o.astype(np.float64), want, rtol=2.0 ** -11, atol=4e-5)   # one rounding to fp16 of values up to five
