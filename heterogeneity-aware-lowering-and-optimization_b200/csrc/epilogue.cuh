@@ -13,15 +13,15 @@
 namespace b200 {
 
 // ---- launches ----
-// Every kernel of this library is launched as a programmatic dependent of the one in front of it (its blocks may be placed
-// while that one drains) and therefore begins with dependency_wait(): wait until the kernels it depends on have completed and
-// their writes are visible, then let the next kernel's blocks come.
+// Every kernel of this library begins with dependency_wait(): wait until the kernels it depends on have completed and their
+// writes are visible, then let the next kernel's blocks come.  Nearly all are launched as programmatic dependents of the kernel in
+// front, i.e. their blocks may be placed while that one drains.
 __device__ __forceinline__ void dependency_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 template <typename... P, typename... A>
-inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+inline void launch_as(bool dependent, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
   static const bool pdl = !getenv("ODLA_B200_NO_PDL");
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
@@ -32,10 +32,20 @@ inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cud
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
-  cfg.numAttrs = pdl ? 1 : 0;
+  cfg.numAttrs = dependent && pdl ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);   // (the caller asks cudaGetLastError)
 }
-
+template <typename... P, typename... A>
+inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) { launch_as(true, kernel, grid, block, smem, s, args...); }
+// For kernels that read their operands several times through L1.  A block placed beside a tensor-core CTA finds an SM with all but
+// 28 KB given to shared memory, and the SM keeps that split until it has been idle, which is as long as the kernel runs.
+// Behind a tensor-core convolution, as dependents and alone: grouped 3x3 of 64 x 28 x 28 x 128 (three of each) 1454 and 1060 us, soft-max
+// along H 250 and 218; batched products of 252 heads x 219 x 128 behind their projections 11.4 and 7.0 ms.  Up to half a megabyte of
+// operands the early start is worth more (2 x 28 x 28 x 128: 109 and 112 us; 4 images: 141 and 135).
+template <typename... P, typename... A>
+inline void launch_cached(int64_t operand_bytes, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+  launch_as(operand_bytes <= (512 << 10), kernel, grid, block, smem, s, args...);
+}
 
 __device__ __forceinline__ float load_as_float(const void* p, int dt, int64_t i) {
   switch (dt) {

@@ -835,11 +835,12 @@ int conv_simt(const ConvGeom& g, int in_dt, const void* x, const void* w, void* 
   int64_t total = (int64_t)g.N * g.P * g.Q * g.K;
   if (total <= 0) return 0;
   int grid = grid_for(total, 256);
+  const int64_t bytes = (int64_t)g.N * g.H * g.W * g.C * (in_dt == DT_F32 ? 4 : in_dt == DT_S8 ? 1 : 2);
   switch (in_dt) {
-    case DT_F32: launch(conv_direct_kernel<float, float>, grid, 256, 0, s, g, (const float*)x, (const float*)w, y, ep); break;
-    case DT_F16: launch(conv_direct_kernel<__half, float>, grid, 256, 0, s, g, (const __half*)x, (const __half*)w, y, ep); break;
-    case DT_BF16: launch(conv_direct_kernel<__nv_bfloat16, float>, grid, 256, 0, s, g, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, y, ep); break;
-    case DT_S8: launch(conv_direct_kernel<int8_t, int>, grid, 256, 0, s, g, (const int8_t*)x, (const int8_t*)w, y, ep); break;
+    case DT_F32: launch_cached(bytes, conv_direct_kernel<float, float>, grid, 256, 0, s, g, (const float*)x, (const float*)w, y, ep); break;
+    case DT_F16: launch_cached(bytes, conv_direct_kernel<__half, float>, grid, 256, 0, s, g, (const __half*)x, (const __half*)w, y, ep); break;
+    case DT_BF16: launch_cached(bytes, conv_direct_kernel<__nv_bfloat16, float>, grid, 256, 0, s, g, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, y, ep); break;
+    case DT_S8: launch_cached(bytes, conv_direct_kernel<int8_t, int>, grid, 256, 0, s, g, (const int8_t*)x, (const int8_t*)w, y, ep); break;
     default: return -1;
   }
   return check_launch();
@@ -848,11 +849,12 @@ int gemm_simt(const GemmGeom& g, int in_dt, const void* A, const void* B, void* 
   int64_t total = g.batch * g.M * g.N;
   if (total <= 0) return 0;
   int grid = grid_for(total, 256);
+  const int64_t bytes = g.batch * (g.M + g.N) * g.K * (in_dt == DT_F32 ? 4 : in_dt == DT_S8 ? 1 : 2);
   switch (in_dt) {
-    case DT_F32: launch(gemm_direct_kernel<float, float>, grid, 256, 0, s, g, (const float*)A, (const float*)B, C, ep); break;
-    case DT_F16: launch(gemm_direct_kernel<__half, float>, grid, 256, 0, s, g, (const __half*)A, (const __half*)B, C, ep); break;
-    case DT_BF16: launch(gemm_direct_kernel<__nv_bfloat16, float>, grid, 256, 0, s, g, (const __nv_bfloat16*)A, (const __nv_bfloat16*)B, C, ep); break;
-    case DT_S8: launch(gemm_direct_kernel<int8_t, int>, grid, 256, 0, s, g, (const int8_t*)A, (const int8_t*)B, C, ep); break;
+    case DT_F32: launch_cached(bytes, gemm_direct_kernel<float, float>, grid, 256, 0, s, g, (const float*)A, (const float*)B, C, ep); break;
+    case DT_F16: launch_cached(bytes, gemm_direct_kernel<__half, float>, grid, 256, 0, s, g, (const __half*)A, (const __half*)B, C, ep); break;
+    case DT_BF16: launch_cached(bytes, gemm_direct_kernel<__nv_bfloat16, float>, grid, 256, 0, s, g, (const __nv_bfloat16*)A, (const __nv_bfloat16*)B, C, ep); break;
+    case DT_S8: launch_cached(bytes, gemm_direct_kernel<int8_t, int>, grid, 256, 0, s, g, (const int8_t*)A, (const int8_t*)B, C, ep); break;
     default: return -1;
   }
   return check_launch();
@@ -1015,8 +1017,8 @@ int softmax(int dt, const void* x, void* y, int64_t outer, int64_t dim, int64_t 
   if (inner == 1 && dt == DT_F32 && launch_rows_f32(true, x, y, nullptr, nullptr, outer, dim, 0.f, log_form, s)) return check_launch();
   if (inner == 1 && dt == DT_F16 && launch_rows_vec<__half>(true, x, y, nullptr, nullptr, outer, dim, 0.f, log_form, s)) return check_launch();
   if (inner == 1 && dt == DT_BF16 && launch_rows_vec<__nv_bfloat16>(true, x, y, nullptr, nullptr, outer, dim, 0.f, log_form, s)) return check_launch();
-  if (inner == 1) launch(softmax_rows_kernel, grid_for(outer * 32, 256), 256, 0, s, dt, x, y, outer, dim, log_form);
-  else launch(softmax_strided_kernel, grid_for(outer * inner, 128), 128, 0, s, dt, x, y, outer, dim, inner, log_form);
+  if (inner == 1) launch_cached(outer * dim * (dt == DT_F32 ? 4 : 2), softmax_rows_kernel, grid_for(outer * 32, 256), 256, 0, s, dt, x, y, outer, dim, log_form);
+  else launch_cached(outer * dim * inner * (dt == DT_F32 ? 4 : 2), softmax_strided_kernel, grid_for(outer * inner, 128), 128, 0, s, dt, x, y, outer, dim, inner, log_form);
   return check_launch();
 }
 // Mean along one axis with 16-byte loads across the kept inner axis: a thread owns VEC neighbouring outputs and adds
@@ -1129,7 +1131,7 @@ int layernorm(int dt, const void* x, void* y, const float* gamma, const float* b
   if (dt == DT_F16 && launch_rows_vec<__half>(false, x, y, gamma, beta, rows, dim, eps, 0, s)) return check_launch();
   if (dt == DT_BF16 && launch_rows_vec<__nv_bfloat16>(false, x, y, gamma, beta, rows, dim, eps, 0, s)) return check_launch();
   if (dt == DT_F32 && launch_rows_f32(false, x, y, gamma, beta, rows, dim, eps, 0, s)) return check_launch();
-  launch(layernorm_kernel, grid_for(rows * 32, 256), 256, 0, s, dt, x, y, gamma, beta, rows, dim, eps);
+  launch_cached(rows * dim * (dt == DT_F32 ? 4 : 2), layernorm_kernel, grid_for(rows * 32, 256), 256, 0, s, dt, x, y, gamma, beta, rows, dim, eps);
   return check_launch();
 }
 int quantize(int dt_in, const void* x, void* q, const float* scale, const int* zp, int64_t outer, int64_t adim, int64_t inner,
