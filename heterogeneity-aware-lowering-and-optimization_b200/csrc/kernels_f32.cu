@@ -130,26 +130,22 @@ __device__ __forceinline__ void load_b(const F32Params& p, uint32_t dst, const f
   }
 }
 
-// Four neighbouring results of one row: the common forms on vectors, everything else through the scalar epilogue.  Every step is
-// rounded by itself, as there.
-__device__ __forceinline__ void finish4(const F32Params& p, float4 v, int64_t row, int col, bool plain) {
+// Four neighbouring results of one row, fp32 in and out without multiplier or full-matrix addend.  Every step is rounded by itself,
+// as in epilogue_value.
+__device__ __forceinline__ void finish4(const F32Params& p, float4 v, int64_t row, int col) {
   const Epilogue& ep = p.ep;
   float t[4] = {v.x, v.y, v.z, v.w};
-  if (plain) {
-    auto add = [&](const float4& a) { t[0] = __fadd_rn(t[0], a.x); t[1] = __fadd_rn(t[1], a.y); t[2] = __fadd_rn(t[2], a.z); t[3] = __fadd_rn(t[3], a.w); };
-    if (ep.alpha != 1.f) {
+  auto add = [&](const float4& a) { t[0] = __fadd_rn(t[0], a.x); t[1] = __fadd_rn(t[1], a.y); t[2] = __fadd_rn(t[2], a.z); t[3] = __fadd_rn(t[3], a.w); };
+  if (ep.alpha != 1.f) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) t[j] = __fmul_rn(t[j], ep.alpha);
-    }
-    if (ep.add1) add(__ldg((const float4*)(ep.add1 + col)));
-    if (ep.add2) add(__ldg((const float4*)(ep.add2 + col)));
-    if (ep.act_first) apply_act_all<4>(ep.act, t, ep.act_a, ep.act_b);
-    if (ep.res) add(*(const float4*)((const float*)ep.res + row * p.N + col));
-    if (!ep.act_first) apply_act_all<4>(ep.act, t, ep.act_a, ep.act_b);
-    *(float4*)((float*)p.y + row * p.N + col) = make_float4(t[0], t[1], t[2], t[3]);
-  } else {
-    for (int j = 0; j < 4 && col + j < p.N; ++j) store_from_float(p.y, ep.out_dt, row * p.N + col + j, epilogue_value(ep, t[j], row, col + j, p.N));
+    for (int j = 0; j < 4; ++j) t[j] = __fmul_rn(t[j], ep.alpha);
   }
+  if (ep.add1) add(__ldg((const float4*)(ep.add1 + col)));
+  if (ep.add2) add(__ldg((const float4*)(ep.add2 + col)));
+  if (ep.act_first) apply_act_all<4>(ep.act, t, ep.act_a, ep.act_b);
+  if (ep.res) add(*(const float4*)((const float*)ep.res + row * p.N + col));
+  if (!ep.act_first) apply_act_all<4>(ep.act, t, ep.act_a, ep.act_b);
+  *(float4*)((float*)p.y + row * p.N + col) = make_float4(t[0], t[1], t[2], t[3]);
 }
 
 template <int LA, bool BVEC>
@@ -226,27 +222,85 @@ __global__ void __launch_bounds__(kThreads, 4) f32_tile_kernel(const F32Params p
       out[(ty + 8 * i) * kPitch + tx + 8 * j] = f.x + f.y;
     }
   const Epilogue& ep = p.ep;
-  const bool plain = !ep.mul && !ep.add_full && (!ep.res || ep.res_dt == DT_F32) && ep.out_dt == DT_F32 && (p.N & 3) == 0;
-  const int r_lo = kTile * rank / p.splits, r_hi = kTile * (rank + 1) / p.splits;
+  const bool f32_io = !ep.mul && !ep.add_full && (!ep.res || ep.res_dt == DT_F32) && ep.out_dt == DT_F32;
+  const int r_lo = kTile * rank / p.splits, r_hi = min(kTile * (rank + 1) / p.splits, p.M - m0);
   if (p.splits > 1) {
     asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
   } else __syncthreads();
-  for (int e = t; e < (r_hi - r_lo) * (kTile / 4); e += kThreads) {
-    const int r = r_lo + e / (kTile / 4), c = (e % (kTile / 4)) * 4;
-    if (m0 + r >= p.M || n0 + c >= p.N) continue;
-    const uint32_t at = sbase + (uint32_t)((r * kPitch + c) * 4);
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (p.splits == 1) v = *(const float4*)(out + r * kPitch + c);
-    else
-      for (int k = 0; k < p.splits; ++k) {
-        uint32_t peer;
-        float4 u;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(at), "r"(k));
-        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(u.x), "=f"(u.y), "=f"(u.z), "=f"(u.w) : "r"(peer) : "memory");
-        v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+  if (f32_io && (p.N & 3) == 0) {
+    for (int e = t; e < (r_hi - r_lo) * (kTile / 4); e += kThreads) {
+      const int r = r_lo + e / (kTile / 4), c = (e % (kTile / 4)) * 4;
+      if (n0 + c >= p.N) continue;
+      const uint32_t at = sbase + (uint32_t)((r * kPitch + c) * 4);
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (p.splits == 1) v = *(const float4*)(out + r * kPitch + c);
+      else
+        for (int k = 0; k < p.splits; ++k) {
+          uint32_t peer;
+          float4 u;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(at), "r"(k));
+          asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(u.x), "=f"(u.y), "=f"(u.z), "=f"(u.w) : "r"(peer) : "memory");
+          v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+        }
+      finish4(p, v, (int64_t)batch * p.M + m0 + r, n0 + c);
+    }
+  } else {
+    // One result at a time: a thread keeps its column, whose addends it reads once, and the threads that the columns leave over
+    // take further rows; eight results are read before the first is finished, because the stores keep the compiler from
+    // gathering the reads.
+    constexpr int kAhead = 8;
+    const int cols = min(kTile, p.N - n0);
+    int width = 1;
+    while (width < cols) width *= 2;
+    const int c = t & (width - 1), col = n0 + c, step = kThreads / width;
+    if (c < cols) {
+      const float a1 = ep.add1 ? __ldg(ep.add1 + col) : 0.f, a2 = ep.add2 ? __ldg(ep.add2 + col) : 0.f;
+      for (int r0 = r_lo + t / width; r0 < r_hi; r0 += kAhead * step) {
+        float v[kAhead], res[kAhead];
+        const int64_t row0 = (int64_t)batch * p.M + m0 + r0;
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) {
+          const bool here = r0 + i * step < r_hi;
+          v[i] = here && p.splits == 1 ? out[(r0 + i * step) * kPitch + c] : 0.f;
+          res[i] = here && f32_io && ep.res ? ((const float*)ep.res)[(row0 + i * step) * p.N + col] : 0.f;
+        }
+        if (p.splits > 1)
+          for (int k = 0; k < p.splits; ++k) {   // every result adds its parts in rank order
+            uint32_t peer;
+            float u[kAhead];
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(sbase + (uint32_t)((r0 * kPitch + c) * 4)), "r"(k));
+#pragma unroll
+            for (int i = 0; i < kAhead; ++i) {
+              u[i] = 0.f;
+              if (r0 + i * step < r_hi) asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(u[i]) : "r"(peer + (uint32_t)(i * step * kPitch * 4)) : "memory");
+            }
+#pragma unroll
+            for (int i = 0; i < kAhead; ++i) v[i] += u[i];
+          }
+        if (f32_io) {
+#pragma unroll
+          for (int i = 0; i < kAhead; ++i) {
+            if (ep.alpha != 1.f) v[i] = __fmul_rn(v[i], ep.alpha);
+            if (ep.add1) v[i] = __fadd_rn(v[i], a1);
+            if (ep.add2) v[i] = __fadd_rn(v[i], a2);
+          }
+          if (ep.act_first) apply_act_all<kAhead>(ep.act, v, ep.act_a, ep.act_b);
+          if (ep.res) {
+#pragma unroll
+            for (int i = 0; i < kAhead; ++i) v[i] = __fadd_rn(v[i], res[i]);
+          }
+          if (!ep.act_first) apply_act_all<kAhead>(ep.act, v, ep.act_a, ep.act_b);
+        }
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) {
+          const int64_t row = row0 + i * step;
+          if (r0 + i * step >= r_hi) break;
+          if (f32_io) ((float*)p.y)[row * p.N + col] = v[i];
+          else store_from_float(p.y, ep.out_dt, row * p.N + col, epilogue_value(ep, v[i], row, col, p.N));
+        }
       }
-    finish4(p, v, (int64_t)batch * p.M + m0 + r, n0 + c, plain);
+    }
   }
   if (p.splits > 1) {   // nobody leaves while a peer may still read its partial tile
     asm volatile("barrier.cluster.arrive.release;" ::: "memory");
