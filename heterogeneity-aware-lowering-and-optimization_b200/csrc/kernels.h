@@ -84,10 +84,12 @@ int gemm_simt(const GemmGeom& g, int in_dt, const void* A, const void* B, void* 
 // (r, s, c) order and w_pitch a multiple of 4 (the padding holds zeros).  images_full: images of the whole recorded batch, of
 // which g.N are here.  It alone decides the order of the sums, so that an image's result does not depend on how a batch is cut.
 bool conv_f32_supported(const ConvGeom& g);
+bool conv_f32_pays(const ConvGeom& g, int64_t images_full);   // ... and is faster than conv_simt
 int conv_f32(const ConvGeom& g, int64_t images_full, const void* x, const void* w, int64_t w_pitch, void* y, const Epilogue& ep, cudaStream_t stream);
 // fp32 batched GEMM, any strides (a B with unit b_row and 16-byte rows loads widest).  batch_full and rows_full: g.batch and g.M
 // of the whole recorded batch, as above.
 bool gemm_f32_supported(const GemmGeom& g);
+bool gemm_f32_pays(const GemmGeom& g, int64_t batch_full, int64_t rows_full, bool b_kmajor);   // ... and is faster than gemm_simt; b_kmajor: B's rows will be contiguous along K
 int gemm_f32(const GemmGeom& g, int64_t batch_full, int64_t rows_full, const void* A, const void* B, void* C, const Epilogue& ep, cudaStream_t stream);
 
 // ---- tensor-core path (kernels_umma.cu) ----

@@ -370,7 +370,8 @@ int device_sms() {
 // writing the tile, a cluster 2 us more for its barriers and remote reads (measured on ResNet-50's layers at batch 8).
 // `tiles` are those of the whole recorded batch: the number of shares is the order of the sums, and a launch that computes a
 // part of the batch (another GPU's or sub-batch's rows) has to take the same one.
-int pick_splits(int64_t tiles, int num_kb) {
+struct Splits { int n; double us; };
+Splits pick_splits(int64_t tiles, int num_kb) {
   const int sms = device_sms();
   int best = 1;
   double best_cost = 0;
@@ -379,8 +380,25 @@ int pick_splits(int64_t tiles, int num_kb) {
     const double cost = (double)((per_sm + 1) / 2 * 2) * ((num_kb + n - 1) / n) * 1.04 + (double)((per_sm + 3) / 4) * 4.0 + (n > 1 ? 2.0 : 0.0);
     if (n == 1 || cost < best_cost) { best = n; best_cost = cost; }
   }
-  return best;
+  return {best, best_cost};
 }
+// Whether a short reduction over few or narrow results is better off on the one-thread-per-output kernel, which has nothing to
+// set up.  In us, fitted to 630 shapes (1 to 256 columns, 4 to 2048 values, 16 to 131072 rows; convolutions of 1 to 64 channels
+// with 1x1 to 7x7 windows of 8 x 8 to 16 x 56 x 56 pixels), each launch bracketed: the tiles as pick_splits counts them and 5, 4-byte loads 1.35
+// times; one thread per output 85 ns a value and 250 ns a tap until the chip is full, then a throughput per result and value.
+// The fit is within a quarter on either side for most, so the tiles keep whatever is close.  131072 x 2 results of 10 values: 33 us on tiles, 9 on
+// threads; 3x3 of 16 x 56 x 56 x 5 -> 1: 30 and 10; 16384 x 64 results of 16 values: 14 and 18.  Sums of up to 256 values in one chain only:
+// beyond, the tiles are both faster and more exact.
+bool direct_pays(int64_t M, int64_t N, int64_t K, int taps, bool wide_loads) {
+  if (K > 256) return false;
+  const double tiles = 5.0 + pick_splits((M + kTile - 1) / kTile * ((N + kTile - 1) / kTile), (int)((K + kBK - 1) / kBK)).us * (wide_loads ? 1.0 : 1.35);
+  const double results = (double)M * N, chain = 1.0 + 0.085 * K + (taps > 1 ? 0.25 * taps : 0.0);
+  const double rate = taps ? results * (12e-6 + (taps > 1 ? 1.7e-6 * taps : 0.0) + 3.4e-7 * K) : results * (8e-6 + 3.4e-7 * K) + 1.5e-6 * M * K;
+  return 6.0 + std::max(chain, rate) < 0.9 * tiles;
+}
+// Up to this many results (of the whole recorded batch, see pick_splits) the warps of one launch fit the chip at once and the
+// operands are re-read from L2 only.
+constexpr int64_t kFewResults = 16384;
 template <int LA, bool BVEC>
 int launch_tiles(const F32Params& p, int64_t blocks, cudaStream_t s) {
   static bool set[16] = {false};
@@ -416,7 +434,7 @@ int run(F32Params p, int la, bool bvec, int64_t batch, int64_t batch_full, int64
   p.n_tiles = (p.N + kTile - 1) / kTile;
   const int64_t tiles = batch * p.m_tiles * p.n_tiles;
   if (tiles <= 0) return 0;
-  p.splits = pick_splits(batch_full * ((rows_full + kTile - 1) / kTile) * p.n_tiles, p.num_kb);
+  p.splits = pick_splits(batch_full * ((rows_full + kTile - 1) / kTile) * p.n_tiles, p.num_kb).n;
   if (la == LOAD_CONV_VEC) return launch_tiles<LOAD_CONV_VEC, true>(p, tiles, s);
   if (la == LOAD_CONV_SCALAR) return launch_tiles<LOAD_CONV_SCALAR, true>(p, tiles, s);
   if (la == LOAD_GEMM_VEC) return bvec ? launch_tiles<LOAD_GEMM_VEC, true>(p, tiles, s) : launch_tiles<LOAD_GEMM_VEC, false>(p, tiles, s);
@@ -432,6 +450,7 @@ bool indexable(int64_t batch, int64_t M, int64_t N, int64_t K) {
 bool conv_f32_supported(const ConvGeom& g) {
   return g.groups == 1 && g.xs_c == 1 && g.P > 0 && g.Q > 0 && indexable(1, (int64_t)g.N * g.P * g.Q, g.K, (int64_t)g.R * g.S * g.C);
 }
+bool conv_f32_pays(const ConvGeom& g, int64_t images_full) { return !direct_pays(images_full * g.P * g.Q, g.K, (int64_t)g.R * g.S * g.C, g.R * g.S, g.C % 4 == 0); }
 int conv_f32(const ConvGeom& g, int64_t images_full, const void* x, const void* w, int64_t w_pitch, void* y, const Epilogue& ep, cudaStream_t s) {
   F32Params p{};
   p.M = g.N * g.P * g.Q; p.N = g.K; p.K = g.R * g.S * g.C;
@@ -443,6 +462,11 @@ int conv_f32(const ConvGeom& g, int64_t images_full, const void* x, const void* 
   return run(p, vec ? LOAD_CONV_VEC : LOAD_CONV_SCALAR, true, 1, 1, images_full * g.P * g.Q, s);
 }
 bool gemm_f32_supported(const GemmGeom& g) { return g.K > 0 && indexable(g.batch, g.M, g.N, g.K); }
+bool gemm_f32_pays(const GemmGeom& g, int64_t batch_full, int64_t rows_full, bool b_kmajor) {
+  const bool wide = g.a_col == 1 && b_kmajor && g.K % 4 == 0;
+  if (batch_full > 1 || (wide && rows_full * g.N <= kFewResults)) return true;
+  return !direct_pays(rows_full, g.N, g.K, 0, wide);
+}
 int gemm_f32(const GemmGeom& g, int64_t batch_full, int64_t rows_full, const void* A, const void* B, void* C, const Epilogue& ep, cudaStream_t s) {
   if (g.batch <= 0 || g.M <= 0 || g.N <= 0) return 0;
   F32Params p{};
@@ -453,9 +477,7 @@ int gemm_f32(const GemmGeom& g, int64_t batch_full, int64_t rows_full, const voi
   const bool avec = g.a_col == 1 && g.K % 4 == 0 && g.a_row % 4 == 0 && g.a_batch % 4 == 0 && (uintptr_t)A % 16 == 0;
   // (pieces past K are zero on the A side, so a B row padded to a multiple of four floats may hold anything there)
   const bool bvec = g.b_row == 1 && g.b_col % 4 == 0 && (g.K % 4 == 0 || g.b_batch == 0) && g.b_batch % 4 == 0 && (uintptr_t)B % 16 == 0;
-  // up to 16384 results (of the whole recorded batch, see pick_splits) the warps of one launch fit the chip at once and the
-  // operands are re-read from L2 only
-  if (avec && bvec && g.K % 4 == 0 && batch_full * rows_full * g.N <= 16384) {
+  if (avec && bvec && g.K % 4 == 0 && batch_full * rows_full * g.N <= kFewResults) {
     p.batches = (int)g.batch;
     const int64_t warps = g.batch * ((g.M + kFewRows - 1) / kFewRows) * ((g.N + kFewCols - 1) / kFewCols);
     b200::launch(f32_few_results_kernel, (unsigned)((warps + 3) / 4), 128, 0, s, p);

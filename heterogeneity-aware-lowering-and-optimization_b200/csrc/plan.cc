@@ -1075,12 +1075,12 @@ odla_status Builder::emit_fused(const Item& it) {
       // that its tap does not reach, so such filters keep the kernel that leaves the padding out
       const bool padded_window = g.pad_t > 0 || g.pad_l > 0 || (g.P - 1) * g.stride_h - g.pad_t + g.R > g.H || (g.Q - 1) * g.stride_w - g.pad_l + g.S > g.W;
       auto all_finite = [&] { const auto wf = const_as_f32(f.w); return std::all_of(wf.begin(), wf.end(), [](float v) { return std::isfinite(v); }); };
-      if (conv_f32_supported(g) && (!padded_window || all_finite())) {
+      const int64_t images_full = rows_of_batch(root, g.N);
+      if (conv_f32_supported(g) && conv_f32_pays(g, images_full) && (!padded_window || all_finite())) {
         const int64_t kd = (int64_t)g.R * g.S * g.C, pitch = (kd + 3) / 4 * 4;
         auto wb = prepared(f.w, "conv_f32_kmajor", [&] { return f32_rows_kmajor(const_as_f32(f.w), kd, K, pitch); });
         const void* wk = upload(wb->data(), wb->size());
         if (!wk) return err_status_;
-        const int64_t images_full = rows_of_batch(root, g.N);
         add_launch("conv_simt", f.out, flops, bytes, [=](cudaStream_t s) { return conv_f32(g, images_full, x, wk, pitch, y, ep, s); });
         return ODLA_SUCCESS;
       }
@@ -1249,9 +1249,11 @@ odla_status Builder::emit_fused(const Item& it) {
   g.a_row = ta ? 1 : ac; g.a_col = ta ? ac : 1; g.a_batch = ar * ac;
   g.b_row = tb ? 1 : bc; g.b_col = tb ? bc : 1; g.b_batch = bbatch == 1 ? 0 : br * bc;
   const void* bp;
-  const bool f32_tiled = in_dt == DT_F32 && gemm_f32_supported(g);
-  if (f.w->kind == OP_CONST && f32_tiled && bbatch == 1 && !tb) {
-    // [K][N] weights as [N][K] rows of whole 16-byte pieces
+  // the whole recorded batch lies along the leading axis: the batch of a batched product, the rows of a plain one
+  const int64_t all_rows = rows_of_batch(root, batch * M), batch_full = ra > 2 && M > 0 ? all_rows / M : batch, rows_full = ra > 2 ? M : all_rows;
+  const bool kmajor_weights = f.w->kind == OP_CONST && bbatch == 1 && !tb;   // [K][N] weights are repacked as [N][K] rows
+  const bool f32_tiled = in_dt == DT_F32 && gemm_f32_supported(g) && gemm_f32_pays(g, batch_full, rows_full, tb || kmajor_weights);
+  if (f32_tiled && kmajor_weights) {   // ... of whole 16-byte pieces
     const int64_t pitch = (Kd + 3) / 4 * 4;
     auto wb = prepared(f.w, "gemm_f32_kmajor", [&] { return f32_rows_kmajor(const_as_f32(f.w), Kd, N, pitch); });
     bp = upload(wb->data(), wb->size());
@@ -1262,8 +1264,6 @@ odla_status Builder::emit_fused(const Item& it) {
     bp = dev_ptr(f.w);
   }
   if (!bp) return err_status_;
-  // the whole recorded batch lies along the leading axis: the batch of a batched product, the rows of a plain one
-  const int64_t all_rows = rows_of_batch(root, batch * M), batch_full = ra > 2 && M > 0 ? all_rows / M : batch, rows_full = ra > 2 ? M : all_rows;
   add_launch("gemm_simt", f.out, flops, bytes, with_move([=](cudaStream_t s) {
     return f32_tiled ? gemm_f32(g, batch_full, rows_full, x, bp, y, ep, s) : gemm_simt(g, in_dt, x, bp, y, ep, s);
   }));

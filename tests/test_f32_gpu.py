@@ -129,3 +129,26 @@ def test_f32_epilogue_rounds_every_step(odla, gpu_lib, N):
     g.close()
     t = alpha * (a[:, :1] * w[:1]) + b
     assert np.array_equal(got, np.where(t < 0, slope * t, t) + r)
+
+
+@pytest.mark.parametrize("images", [1, 4, 16])
+@pytest.mark.parametrize("shape", [(9, 5, 4, 3), (9, 8, 255, 1), (14, 1, 64, 3), (20, 3, 1, 5), (28, 16, 16, 1)])   # H, C, K, window: either side of the choice
+def test_short_reductions_on_whichever_kernel(odla, gpu_lib, shape, images):
+    """fp32 layers at the line between the tiles and the one-thread-per-output kernel, cut in two as well."""
+    H, C, K, R = shape
+    rng = np.random.default_rng(H * C + K)
+    x = rng.standard_normal((images, H, H, C)).astype(np.float32)
+    w = (rng.standard_normal((R, R, C, K)) / np.sqrt(R * R * C)).astype(np.float32)
+    outs = []
+    for s in (1, 2):
+        g = odla.Graph(gpu_lib, "c", n_gpus=1, sub_batches=s)
+        p = R // 2
+        y = g.Conv(g.Argument("x", x.shape), odla.CHANNELS_LAST, 1, g.Constant("w", w), odla.SIO, (1, 1), (1, 1), (p, p), (p, p), None, (images, H, H, K), "y")
+        g.Output(y)
+        rows = g.Reshape(g.ReduceMean(y, (1, 2), True, (images, 1, 1, K), "m"), (images, K), "rows")
+        g.Output(g.Gemm(rows, False, g.Constant("v", w[0, 0].T.copy()), False, 1.0, 0.0, None, (images, C), "z"))
+        outs.append(g.run({"x": x}))
+        g.close()
+    t = torch.nn.functional.conv2d(torch.from_numpy(x).double().permute(0, 3, 1, 2), torch.from_numpy(w).double().permute(3, 2, 0, 1), padding=p).permute(0, 2, 3, 1).numpy()
+    close(outs[0]["y"], t, R * R * C)
+    assert all(np.array_equal(outs[0][n], outs[1][n]) for n in outs[0])
