@@ -235,11 +235,12 @@ def bind_to_gpu_numa_node(index):
 
 
 # ResNet-50 dram__bytes_read.sum + dram__bytes_write.sum of the tensor-core kernel, summed over its launches of one
-# execute and divided by their number: one ncu capture at a smaller batch (the full batch breaks the capture-size rule),
+# execute and divided by their number: one ncu capture of the single-producer form of the kernel (the later forms move the same
+# tensors, with smaller tiles for a few long reductions) at a smaller batch (the full batch breaks the capture-size rule),
 # scaled in proportion to the batch (activation traffic grows with it; the 25 / 51 MB of weights do not, which makes the
 # scaled figure a slight over-estimate).  See profiles/.
-NCU_TRAFFIC = {"f16": {"bytes_per_launch": 9.8226e7, "launches": 54, "at_batch": 128, "source": "ncu capture of all 54 launches at B=128 (4.066 GB read + 1.238 GB written), scaled by batch / 128"},
-               "s8": {"bytes_per_launch": 4.1931e7, "launches": 54, "at_batch": 128, "source": "ncu capture of all 54 launches at B=128 (1.975 GB read + 0.290 GB written), scaled by batch / 128"}}
+NCU_TRAFFIC = {"f16": {"bytes_per_launch": 9.8226e7, "launches": 54, "at_batch": 128, "source": "ncu capture of all 54 launches of the single-producer kernel at B=128 (4.066 GB read + 1.238 GB written), scaled by batch / 128"},
+               "s8": {"bytes_per_launch": 4.1931e7, "launches": 54, "at_batch": 128, "source": "ncu capture of all 54 launches of the single-producer kernel at B=128 (1.975 GB read + 0.290 GB written), scaled by batch / 128"}}
 
 
 def tensor_roofline(prof, ms_per_step, peaks, peak_kind, clocks, int8, batch):

@@ -53,8 +53,9 @@ extern "C" int odla_b200_conv_umma(const odla_b200_conv_desc* d, const void* x, 
     cudaMemcpy(ts, (char*)status + 32, sizeof(ts), cudaMemcpyDeviceToHost);
     fprintf(stderr, "ts(ns rel. to kernel entry): sync=%lld tfull0=%lld epi0_end=%lld teardown=%lld | cycles %lld\n", (long long)(ts[0] - ts[7]),
             (long long)(ts[4] - ts[7]), (long long)(ts[5] - ts[7]), (long long)(ts[6] - ts[7]), (long long)(ts[16 + 6] - ts[16 + 7]));
-    static const char* site[8] = {"", "producer<-empty", "mma<-tempty", "mma<-full", "epi<-tfull", "loader<-box_free", "epi<-box_full", "storer<-box_done"};
-    for (int code = 1; code < 8; ++code) {
+    static const char* site[9] = {"", "A producer<-empty", "mma<-tempty", "mma<-full", "epi<-tfull", "", "epi<-box_full", "storer<-box_done", "B producer<-empty"};
+    for (int code = 1; code < 9; ++code) {
+      if (!*site[code]) continue;
       const unsigned long long* c4 = ts + 28 + code * 4;  // ts[] starts at status + 32 bytes = 4 words
       fprintf(stderr, "  wait %-18s %10llu %10llu %10llu %10llu\n", site[code], c4[0], c4[1], c4[2], c4[3]);
     }

@@ -1303,7 +1303,7 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const uint32_t staging_u32 = smem_u32(staging);
     if constexpr (STAGED) {
       // Per output tile the staging ring supplies stage_boxes boxes of 128 rows x 128 bytes; the
-      // loader warp has already put the residual there, this warp overwrites its part of the box
+      // storer warp has already had the residual put there, this warp overwrites its part of the box
       // with the result and the storer warp sends the box out.
       const int cols_per_box = 128 / p.out_esz, chunks_per_box = cols_per_box / CW;
       // Which 16-column chunks of a tile the four warps of a group (one per lane quarter) take: either a
@@ -2100,7 +2100,8 @@ void choose_split(const UmmaConv& c, int sms, UmmaParams& p) {
 // are two rounds as long as 148 would be.  192 columns make them 128 shorter ones.  In clocks, from the walk's own
 // timing: a k-block of 256, 192, 128 columns takes 560, 430, 390 on pairs and 600, 470, 415 on single CTAs, a tile 1200 to
 // start, the last tile's epilogue 20 a column and a pair's setting up 400.  3x3 512 -> 1024 at 13 x 13 x 16: 43 -> 35 us, a
-// 3072 -> 768 projection of 8192 rows with a residual: 49 -> 45 us.  (192 columns are one and a half boxes of one-byte results: not there.)
+// 3072 -> 768 projection of 8192 rows with a residual: 49 -> 45 us.  (192 columns are one and a half boxes of one-byte results: not there.)  The clocks are those of
+// k-blocks of 128 bytes, measured on the layers named here; shorter k-blocks are given the same, which only scales both sides.
 void choose_tile(const UmmaConv& c, const Epilogue& ep, int sms, UmmaParams& p) {
   p.pair = 0;
   p.bn_load = p.BN;

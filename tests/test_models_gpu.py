@@ -161,8 +161,8 @@ def test_bert_encoder_matches_oracle(odla, gpu_lib, ref, models, mode, cfg):
     err = float(np.abs(got["encoder_out"] - want["encoder_out"]).max())
     assert err <= (2e-4 if mode == "fp32" else 3e-2), err
     if mode == "fp16":
-        # Q/K/V/out/FFN on the tensor-core Gemm; heads of 128 positions x 64 channels take the fused attention launch
-        # (scores product, 1/sqrt(d) Mul, soft-max and context product in one), other shapes the separate kernels
+        # Q/K/V/out/FFN on the tensor-core Gemm; heads of 64 channels take the fused attention launch (scores product,
+        # 1/sqrt(d) Mul, soft-max and context product in one), other widths the separate kernels
         fused_attention = cfg["seq"] == 128 and cfg["hidden"] // cfg["heads"] == 64
         assert desc.count("gemm_umma") == 6 * cfg["layers"] and "layernorm" in desc and "gather" in desc
         assert desc.count("attention") == (cfg["layers"] if fused_attention else 0)
