@@ -92,6 +92,24 @@ bool gemm_f32_supported(const GemmGeom& g);
 bool gemm_f32_pays(const GemmGeom& g, int64_t batch_full, int64_t rows_full, bool b_kmajor);   // ... and is faster than gemm_simt; b_kmajor: B's rows will be contiguous along K
 int gemm_f32(const GemmGeom& g, int64_t batch_full, int64_t rows_full, const void* A, const void* B, void* C, const Epilogue& ep, cudaStream_t stream);
 
+// ---- fp32 on the tensor cores (kernels_f32_umma.cu) ----
+// A dense NHWC convolution with one group, or a product with constant weights (H = W = R = S = 1, N = rows).  `planes` holds the
+// weights as three bf16 values each, [block][3][K][64]: block b covers channels (b % c) * 64 and on of tap b / c for c = ceil(C / 64),
+// zeros past C.  The weights are finite and at most 2^20 (results below 2^-70 are then computed from the operands as they are).
+struct F32Umma {
+  int N, H, W, C, K, R, S, P, Q, stride_h, stride_w, pad_t, pad_l;
+  int64_t rows_full;   // output rows of the whole recorded batch: alone they decide the order of the sums
+  // Byte strides of the W and H dimensions of x (0 = dense): a W stride smaller than a pixel describes overlapping windows.
+  long long x_w_stride = 0, x_h_stride = 0;
+};
+bool f32_umma_supported(const F32Umma& c);
+bool f32_umma_pays(const F32Umma& c);       // ... and is faster than the CUDA-core kernels
+int64_t f32_umma_blocks(const F32Umma& c);
+struct F32UmmaLaunch;
+F32UmmaLaunch* f32_umma_prepare(const F32Umma& c, const void* x, const void* planes, void* y, const Epilogue& ep, int* status_word, int device_sms);
+int f32_umma_run(F32UmmaLaunch* l, cudaStream_t stream);
+void f32_umma_destroy(F32UmmaLaunch* l);
+
 // ---- tensor-core path (kernels_umma.cu) ----
 // NHWC implicit-GEMM convolution: x [N,H,W,C], w repacked to [K][R*S*C] (K-major), y [N,P,Q,K].
 // A 1x1/stride-1 convolution with H=W=1 is a plain GEMM, which is how Gemm uses it.

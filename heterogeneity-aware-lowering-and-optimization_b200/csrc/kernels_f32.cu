@@ -1,5 +1,5 @@
-// fp32 convolution (NHWC, one group) and batched GEMM on the CUDA cores, for graphs that run in the library's default
-// storage type.  The tensor cores have no fp32 operand type, so the bound is the FMA pipe: 128 fp32 FMA per clock and
+// fp32 convolution (NHWC, one group) and batched GEMM on the CUDA cores, for what kernels_f32_umma.cu does not take: products of two
+// run-time tensors, few results, short reductions, channels that are no multiple of four.  The bound is the FMA pipe: 128 fp32 FMA per clock and
 // SM, 74 TFLOP/s at 1965 MHz.
 //
 //   C[b][M, N] = A[b][M, K] * B[b][N, K]^T      convolution: M = N*P*Q pixels, K = R*S*C gathered on the fly

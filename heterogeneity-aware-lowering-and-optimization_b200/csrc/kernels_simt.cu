@@ -1534,6 +1534,7 @@ int stem_pad(int esz, const void* x, void* y, int N, int H, int W, int C, int pi
   else if (esz == 1 && cp == 8) launch(stem_pad_kernel<uint8_t, 8>, grid, 256, 0, s, (const uint8_t*)x, (uint8_t*)y, rows, W, C, lp, Wp);
   else if (esz == 1 && cp == 16) launch(stem_pad_kernel<uint8_t, 16>, grid, 256, 0, s, (const uint8_t*)x, (uint8_t*)y, rows, W, C, lp, Wp);
   else if (esz == 2 && cp == 4) launch(stem_pad_kernel<uint16_t, 4>, grid, 256, 0, s, (const uint16_t*)x, (uint16_t*)y, rows, W, C, lp, Wp);
+  else if (esz == 4 && cp == 4) launch(stem_pad_kernel<uint32_t, 4>, grid, 256, 0, s, (const uint32_t*)x, (uint32_t*)y, rows, W, C, lp, Wp);
   else if (esz == 2 && cp == 8) launch(stem_pad_kernel<uint16_t, 8>, grid, 256, 0, s, (const uint16_t*)x, (uint16_t*)y, rows, W, C, lp, Wp);
   else return -1;
   return check_launch();

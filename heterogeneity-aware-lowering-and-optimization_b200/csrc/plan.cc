@@ -39,6 +39,7 @@ Plan::~Plan() {
   for (auto& l : launches) l.fn = nullptr;
   for (auto* u : umma) umma_conv_destroy(u);
   for (auto* a : attn) attn_destroy(a);
+  for (auto* f : f32_umma) f32_umma_destroy(f);
   for (void* p : extra_allocs) cudaFree(p);
   if (arena) cudaFree(arena);
 }
@@ -133,6 +134,30 @@ std::vector<float> transpose_rows(const std::vector<float>& w, int64_t k, int64_
   return o;
 }
 std::vector<uint8_t> f32_rows_kmajor(const std::vector<float>& w, int64_t k, int64_t n, int64_t pitch) { return f32_to_storage(transpose_rows(w, k, n, pitch), DT_F32); }
+// fp32 weights [taps * channels][n] (or [n][taps * channels] when `transposed`) as the three bf16 values whose sum each is,
+// [block][3][n][64] for blocks of 64 channels of one tap (see F32Umma).
+std::vector<uint8_t> f32_planes(const std::vector<float>& w, int64_t taps, int64_t channels, int64_t n, bool transposed) {
+  const int64_t chunks = (channels + 63) / 64, kd = taps * channels;
+  std::vector<uint8_t> bytes((size_t)(taps * chunks * 3 * n * 64 * 2), 0);
+  uint16_t* out = (uint16_t*)bytes.data();
+  auto round = [](float v) { uint32_t b; memcpy(&b, &v, 4); return (uint16_t)((b + 0x7fffu + ((b >> 16) & 1u)) >> 16); };
+  auto value = [](uint16_t h) { const uint32_t b = (uint32_t)h << 16; float v; memcpy(&v, &b, 4); return v; };
+  for (int64_t b = 0; b < taps * chunks; ++b) {
+    const int64_t k0 = b / chunks * channels + b % chunks * 64, here = std::min<int64_t>(64, channels - b % chunks * 64);
+    uint16_t* plane = out + b * 3 * n * 64;
+    for (int64_t j0 = 0; j0 < n; j0 += 32)   // (square blocks: neither side is walked a line at a time)
+      for (int64_t c = 0; c < here; ++c)
+        for (int64_t j = j0; j < std::min(n, j0 + 32); ++j) {
+          float v = transposed ? w[(size_t)(j * kd + k0 + c)] : w[(size_t)((k0 + c) * n + j)];
+          for (int64_t i = 0; i < 3; ++i) {
+            const uint16_t h = round(v);
+            plane[(i * n + j) * 64 + c] = h;
+            v -= value(h);
+          }
+        }
+  }
+  return bytes;
+}
 // A Gemm's weights as K-major rows [n][k] of storage type dt; `w` is [k][n], or already [n][k] when `transposed`.
 std::vector<uint8_t> rows_kmajor(const std::vector<float>& w, int64_t k, int64_t n, bool transposed, int dt) {
   return f32_to_storage(transposed ? w : transpose_rows(w, k, n, k), dt);
@@ -270,6 +295,8 @@ class Builder {
   odla_status emit_group(const Item& it);
   odla_status emit_fused(const Item& it);
   odla_status emit_plain(const Item& it);
+  F32UmmaLaunch* prepare_f32_umma(const F32Umma& fu, const Fused& f, const std::string& form, const std::function<std::vector<uint8_t>(const std::vector<float>&)>& make,
+                                  const void* x, void* y, const Epilogue& ep, int sms);
   void add_launch(const char* op, V out, double flops, double bytes, std::function<int(cudaStream_t)> fn) {
     Launch l; l.op = op; l.name = out->name; l.flops = flops; l.bytes = bytes; l.fn = std::move(fn);
     l.out_v = out;
@@ -1076,6 +1103,48 @@ odla_status Builder::emit_fused(const Item& it) {
       const bool padded_window = g.pad_t > 0 || g.pad_l > 0 || (g.P - 1) * g.stride_h - g.pad_t + g.R > g.H || (g.Q - 1) * g.stride_w - g.pad_l + g.S > g.W;
       auto all_finite = [&] { const auto wf = const_as_f32(f.w); return std::all_of(wf.begin(), wf.end(), [](float v) { return std::isfinite(v); }); };
       const int64_t images_full = rows_of_batch(root, g.N);
+      const F32Umma fu{g.N, g.H, g.W, g.C, g.K, g.R, g.S, g.P, g.Q, g.stride_h, g.stride_w, g.pad_t, g.pad_l, images_full * g.P * g.Q};
+      const int64_t taps = (int64_t)g.R * g.S;
+      if (allow_umma && groups == 1 && f32_umma_pays(fu)) {
+        F32UmmaLaunch* fl = prepare_f32_umma(fu, f, "f32_planes", [&](const std::vector<float>& w) { return f32_planes(w, taps, g.C, K, false); }, x, y, ep, sms);
+        if (err_status_ != ODLA_SUCCESS) return err_status_;
+        if (fl) {
+          add_launch("conv_f32_umma", f.out, flops, bytes, [fl](cudaStream_t s) { return f32_umma_run(fl, s); });
+          return ODLA_SUCCESS;
+        }
+      }
+      if (allow_umma && groups == 1 && g.C <= 4 && g.S <= 32) {
+        // A few-channel image has pixels that TMA cannot address: a pass pads them to four channels and every row with zeros, and the S pixels
+        // that a row of taps reads are one window of 4 * S values, neighbouring windows overlapping -- an (R x 1) convolution with the padding
+        // along W in memory.  7x7 of 8 x 224 x 224 x 3 -> 64: 111 -> 50 us with its launches bracketed.
+        const int Wp = std::max(g.pad_l + g.W, (g.Q - 1) * g.stride_w + g.S);
+        F32Umma fw{g.N, g.H, g.Q, 4 * g.S, g.K, g.R, 1, g.P, g.Q, g.stride_h, 1, g.pad_t, 0, images_full * g.P * g.Q};
+        fw.x_w_stride = 16ll * g.stride_w;
+        fw.x_h_stride = 16ll * Wp;
+        void* image = nullptr;
+        if (f32_umma_pays(fw) && f32_umma_supported(fw) && !inject_fault("alloc")) {
+          if (cudaMalloc(&image, (size_t)fw.x_h_stride * g.H * g.N) != cudaSuccess) { cudaGetLastError(); image = nullptr; }
+        }
+        if (image) {
+          p_->extra_allocs.push_back(image);
+          F32UmmaLaunch* fl = prepare_f32_umma(fw, f, "f32_planes wide", [&](const std::vector<float>& w) {
+            std::vector<float> wide((size_t)g.R * 4 * g.S * K, 0.f);
+            for (int64_t t = 0; t < taps; ++t)
+              for (int64_t c = 0; c < g.C; ++c) std::copy_n(&w[(size_t)((t * g.C + c) * K)], K, &wide[(size_t)((t * 4 + c) * K)]);
+            return f32_planes(wide, g.R, 4 * g.S, K, false);
+          }, image, y, ep, sms);
+          if (err_status_ != ODLA_SUCCESS) return err_status_;
+          if (fl) {
+            const ConvGeom gg = g;
+            add_launch("conv_f32_umma", f.out, flops, bytes + 2.0 * (double)fw.x_h_stride * g.H * g.N, [=](cudaStream_t s) {
+              const int rc = stem_pad(4, x, image, gg.N, gg.H, gg.W, gg.C, 16, gg.pad_l, Wp, s);
+              return rc ? rc : f32_umma_run(fl, s);
+            });
+            p_->launches.back().n_kernels = 2;
+            return ODLA_SUCCESS;
+          }
+        }
+      }
       if (conv_f32_supported(g) && conv_f32_pays(g, images_full) && (!padded_window || all_finite())) {
         const int64_t kd = (int64_t)g.R * g.S * g.C, pitch = (kd + 3) / 4 * 4;
         auto wb = prepared(f.w, "conv_f32_kmajor", [&] { return f32_rows_kmajor(const_as_f32(f.w), kd, K, pitch); });
@@ -1251,6 +1320,17 @@ odla_status Builder::emit_fused(const Item& it) {
   const void* bp;
   // the whole recorded batch lies along the leading axis: the batch of a batched product, the rows of a plain one
   const int64_t all_rows = rows_of_batch(root, batch * M), batch_full = ra > 2 && M > 0 ? all_rows / M : batch, rows_full = ra > 2 ? M : all_rows;
+  if (in_dt == DT_F32 && allow_umma && !ta && f.w->kind == OP_CONST && bbatch == 1 && M > 0 && batch * M < (1ll << 31) && Kd < (1ll << 31) && N < (1ll << 31)) {
+    const F32Umma fu{1, 1, (int)(batch * M), (int)Kd, (int)N, 1, 1, 1, (int)(batch * M), 1, 1, 0, 0, batch_full * rows_full};
+    F32UmmaLaunch* fl = !f32_umma_pays(fu) ? nullptr
+                        : prepare_f32_umma(fu, f, tb ? "f32_planes t" : "f32_planes", [&](const std::vector<float>& w) { return f32_planes(w, 1, Kd, N, tb); }, x, y, ep, sms);
+    if (fl) {
+      add_launch("gemm_f32_umma", f.out, flops, bytes, with_move([fl](cudaStream_t s) { return f32_umma_run(fl, s); }));
+      if (perm_via_move) p_->launches.back().n_kernels = 2;
+      return ODLA_SUCCESS;
+    }
+    if (err_status_ != ODLA_SUCCESS) return err_status_;
+  }
   const bool kmajor_weights = f.w->kind == OP_CONST && bbatch == 1 && !tb;   // [K][N] weights are repacked as [N][K] rows
   const bool f32_tiled = in_dt == DT_F32 && gemm_f32_supported(g) && gemm_f32_pays(g, batch_full, rows_full, tb || kmajor_weights);
   if (f32_tiled && kmajor_weights) {   // ... of whole 16-byte pieces
@@ -1269,6 +1349,20 @@ odla_status Builder::emit_fused(const Item& it) {
   }));
   if (perm_via_move) p_->launches.back().n_kernels = 2;
   return ODLA_SUCCESS;
+}
+
+// An fp32 layer as three bf16 values an operand on the tensor cores; null when it stays on the CUDA cores (or, with err_ set, fails).
+F32UmmaLaunch* Builder::prepare_f32_umma(const F32Umma& fu, const Fused& f, const std::string& form, const std::function<std::vector<uint8_t>(const std::vector<float>&)>& make,
+                                         const void* x, void* y, const Epilogue& ep, int sms) {
+  if (!f32_umma_supported(fu) || (uintptr_t)x % 16 || (uintptr_t)y % 16) return nullptr;
+  const auto w = const_as_f32(f.w);
+  if (!std::all_of(w.begin(), w.end(), [](float v) { return std::fabs(v) <= 1048576.f; })) return nullptr;   // (a NaN fails as well)
+  auto planes = prepared(f.w, form, [&] { return make(w); });
+  const void* wd = upload(planes->data(), planes->size());
+  F32UmmaLaunch* l = wd ? f32_umma_prepare(fu, x, wd, y, ep, p_->status, sms) : nullptr;
+  if (l) p_->f32_umma.push_back(l);
+  else if (!fu.x_w_stride) fail(ODLA_FAILURE, "'" + f.root->name + "': fp32 tensor-core launch could not be prepared");
+  return l;
 }
 
 odla_status Builder::emit_plain(const Item& it) {

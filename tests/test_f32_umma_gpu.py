@@ -1,0 +1,106 @@
+"""fp32 layers as three bf16 values an operand on the tensor cores (kernels_f32_umma.cu) against a float64 evaluation, and against
+the CUDA-core kernels where an operand is not an ordinary number."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def conv(odla, lib, x, w, b, r=None, stride=1, pad=1, act=0.0, sub_batches=None, launch="conv_f32_umma"):
+    """act: slope of a LeakyReLU (0: ReLU), None: no activation."""
+    N, H, W, C = x.shape
+    R, _, _, K = w.shape
+    P, Q = (H + 2 * pad - R) // stride + 1, (W + 2 * pad - R) // stride + 1
+    g = odla.Graph(lib, "c", n_gpus=1, sub_batches=sub_batches)
+    y = g.Conv(g.Argument("x", x.shape), odla.CHANNELS_LAST, 1, g.Constant("w", w), odla.SIO, (stride, stride), (1, 1), (pad, pad), (pad, pad), None, (N, P, Q, K), "conv")
+    y = g.Add(y, g.Constant("b", b.reshape(1, 1, 1, K)), "bias")
+    if r is not None:
+        y = g.Add(y, g.Argument("r", r.shape), "sum")
+    if act is not None:
+        y = g.LeakyRelu(y, act, "act") if act else g.Relu(y, "act")
+    g.Output(y)
+    ins = {"x": x} if r is None else {"x": x, "r": r}
+    out = next(iter(g.run(ins).values()))
+    assert launch in g.describe()
+    g.close()
+    return out
+
+
+def float64(x, w, b, r, stride, pad, act):
+    t = torch.nn.functional.conv2d(torch.from_numpy(x).double().permute(0, 3, 1, 2), torch.from_numpy(w).double().permute(3, 2, 0, 1), stride=stride, padding=pad)
+    y = t.permute(0, 2, 3, 1).numpy() + b + (0 if r is None else r)
+    return y if act is None else np.where(y < 0, y * np.float64(np.float32(act)), y)
+
+
+# N, H, C, K, window, stride, pad: one stage and several, half stages (channels past the last 32), 64- and 128-column tiles with ragged
+# rows and columns, columns that are no multiple of four, a reduction shared by a cluster, three- and four-channel images as windows
+SHAPES = [(4, 56, 64, 64, 1, 1, 0), (4, 30, 96, 128, 3, 1, 1), (9, 33, 36, 72, 3, 2, 1), (3, 29, 100, 255, 1, 1, 0), (2, 14, 512, 130, 3, 1, 1), (1, 7, 2048, 512, 1, 1, 0),
+          (2, 7, 512, 512, 3, 1, 1), (8, 28, 128, 512, 1, 1, 0), (2, 112, 3, 64, 7, 2, 3), (1, 200, 4, 32, 3, 1, 1), (2, 60, 68, 64, 5, 1, 2)]
+
+
+@pytest.mark.parametrize("act", [0.0, 0.1, None])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_conv_matches_float64(odla, gpu_lib, shape, act):
+    N, H, C, K, R, stride, pad = shape
+    P = (H + 2 * pad - R) // stride + 1
+    rng = np.random.default_rng(sum(shape))
+    x = rng.standard_normal((N, H, H, C)).astype(np.float32)
+    w = (rng.standard_normal((R, R, C, K)) / np.sqrt(R * R * C)).astype(np.float32)
+    b = rng.standard_normal(K).astype(np.float32)
+    r = rng.standard_normal((N, P, P, K)).astype(np.float32) if act != 0.1 else None
+    got = conv(odla, gpu_lib, x, w, b, r, stride, pad, act)
+    want = float64(x, w, b, r, stride, pad, act)
+    # sums of 64 products each (a few roundings of 2^-24) and the chain over them, next to the largest of the results
+    n = R * R * C
+    err = np.abs(got - want).max() / np.sqrt(np.mean(want ** 2))
+    assert err < 4e-7 * np.sqrt(max(n / 64, 4)) + 1e-6, err
+
+
+@pytest.mark.parametrize("sub_batches", [2, 3])
+def test_results_do_not_depend_on_the_cut(odla, gpu_lib, sub_batches):
+    rng = np.random.default_rng(1)
+    x, w = rng.standard_normal((6, 14, 14, 256)).astype(np.float32), (rng.standard_normal((3, 3, 256, 200)) / 48).astype(np.float32)
+    b = rng.standard_normal(200).astype(np.float32)
+    assert np.array_equal(conv(odla, gpu_lib, x, w, b), conv(odla, gpu_lib, x, w, b, sub_batches=sub_batches))
+
+
+@pytest.mark.parametrize("shape", [(2, 28, 64, 128, 3), (1, 14, 256, 320, 3)])   # boxes of results; a shared reduction
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan, 3.4e38, 1e-30, 1e-38])
+def test_values_the_split_does_not_hold(odla, gpu_lib, shape, bad, monkeypatch):
+    """Infinities, NaN, the largest fp32 values and operands whose last bits no bf16 can carry: what the CUDA-core kernel gives."""
+    N, H, C, K, R = shape
+    rng = np.random.default_rng(5)
+    x = rng.standard_normal((N, H, H, C)).astype(np.float32)
+    w = (rng.standard_normal((R, R, C, K)) / np.sqrt(R * R * C)).astype(np.float32)
+    b = np.zeros(K, np.float32)
+    if abs(bad) < 1:
+        x *= np.float32(bad)
+    else:
+        x[0, 3, 4, 5] = x[0, H - 1, 0, C - 1] = bad
+    got = conv(odla, gpu_lib, x, w, b, act=None)
+    monkeypatch.setenv("ODLA_B200_NO_F32_UMMA", "1")
+    want = conv(odla, gpu_lib, x, w, b, act=None, launch="conv_simt")
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isposinf(got), np.isposinf(want)) and np.array_equal(np.isneginf(got), np.isneginf(want))
+    ok = np.isfinite(want)
+    # both are chains of roundings of 2^-24 (subnormal results: of 2^-149) relative to the largest terms
+    assert np.abs(got[ok].astype(np.float64) - want[ok]).max() <= 2e-5 * np.abs(want[ok]).max() + 1e-43
+
+
+@pytest.mark.parametrize("tb", [False, True])
+@pytest.mark.parametrize("dims", [(2, 130, 768, 768), (1, 700, 100, 999)])   # batch, M, K, N
+def test_products_match_float64(odla, gpu_lib, dims, tb):
+    batch, M, K, N = dims
+    rng = np.random.default_rng(M)
+    lead = (batch,) if batch > 1 else ()
+    a = rng.standard_normal(lead + (M, K)).astype(np.float32)
+    w = (rng.standard_normal((N, K) if tb else (K, N)) / np.sqrt(K)).astype(np.float32)
+    c = rng.standard_normal(N).astype(np.float32)
+    g = odla.Graph(gpu_lib, "g", n_gpus=1)
+    g.Output(g.Gelu(g.Gemm(g.Argument("a", a.shape), False, g.Constant("w", w), tb, 0.5, 2.0, g.Constant("c", c), lead + (M, N), "y"), False, "act"))
+    got = next(iter(g.run({"a": a}).values()))
+    assert "gemm_f32_umma" in g.describe()
+    g.close()
+    t = torch.from_numpy(0.5 * (a.astype(np.float64) @ (w.T if tb else w).astype(np.float64)) + 2.0 * c)
+    want = torch.nn.functional.gelu(t).numpy()
+    assert np.abs(got - want).max() / np.sqrt(np.mean(want ** 2)) < 4e-7 * np.sqrt(max(K / 64, 4)) + 1e-6
