@@ -29,6 +29,7 @@
 //                has filled with the residual), the others through shared memory in whole rows of 16-byte pieces
 // With few tiles over a long reduction the CTAs of a cluster share it, as in kernels_umma.cu; partial tiles meet through distributed
 // shared memory in rank order.
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 
@@ -61,6 +62,8 @@ struct F32UmmaParams {
   Epilogue ep;
 };
 struct SharedState { uint64_t full[kMaxStages], empty[kMaxStages], split[4], slot_empty[4], sum_empty[2], low_empty, res_full; uint32_t tmem; int abort; };
+static_assert(offsetof(SharedState, split) == 16 * kMaxStages && offsetof(SharedState, sum_empty) == 16 * kMaxStages + 64 && offsetof(SharedState, res_full) == 16 * kMaxStages + 88,
+              "the barriers are initialised as one array");
 
 template <int BN> struct Tile {
   static constexpr uint32_t kABytes = kRows * kDepth * 4, kPlane = BN * kDepth * 2, kStage = kABytes + 3 * kPlane, kOut = kRows * BN * 4;
@@ -312,13 +315,10 @@ f32_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   const int rank = (int)blockIdx.x % p.splits, first = (int)blockIdx.x / p.splits, step = (int)gridDim.x / p.splits;
   const int kb_lo = (int)((int64_t)p.num_kb * rank / p.splits), kb_hi = (int)((int64_t)p.num_kb * (rank + 1) / p.splits);
   const int tiles = first < p.total_tiles ? (p.total_tiles - first + step - 1) / step : 0, its = tiles * (kb_hi - kb_lo);
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < p.stages; ++s) { mbar_init(&sh.full[s], 1); mbar_init(&sh.empty[s], 1); }
-    for (int s = 0; s < T::kSlots; ++s) { mbar_init(&sh.split[s], kSplitWarps); mbar_init(&sh.slot_empty[s], 1); }
-    for (int d = 0; d < 2; ++d) mbar_init(&sh.sum_empty[d], kSumWarps);
-    mbar_init(&sh.low_empty, kSumWarps);
-    mbar_init(&sh.res_full, 1);
-    sh.abort = 0;
+  if (warp == 0) {   // a lane per barrier
+    constexpr int kSplit = 2 * kMaxStages, kSum = kSplit + 8;
+    if (lane < kSum + 4) mbar_init(&sh.full[lane], lane >= kSplit && lane < kSplit + 4 ? kSplitWarps : lane >= kSum && lane < kSum + 3 ? kSumWarps : 1);
+    if (lane == 0) { sh.abort = 0; prefetch_map(&tmA); prefetch_map(&tmB); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -334,8 +334,6 @@ f32_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   if (warp == 0) {
     // ---------------------------------------------------------------------- loads ----
     if (elect_one()) {
-      prefetch_map(&tmA);
-      prefetch_map(&tmB);
       // A and W are walked separately: the weights of the first stages are constants and do not wait for the kernel in front
       int a_tile = first, a_kb = kb_lo, chunk = 0, c0 = 0, fr = 0, fs = 0, m0 = 0, w0 = 0, h0 = 0, img = 0, b_tile = first, b_kb = kb_lo;
       auto load_a = [&](int s) {

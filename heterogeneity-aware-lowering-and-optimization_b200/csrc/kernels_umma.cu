@@ -30,6 +30,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -756,6 +757,7 @@ __device__ __forceinline__ void issue_one(uint32_t d, uint64_t da, uint64_t db, 
   else if constexpr (INT) umma_i8(d, da, db, idesc, accum);
   else umma_f16(d, da, db, idesc, accum);
 }
+// (a pair's commit arrives on the barrier at this offset in both CTAs once the MMAs issued so far have completed)
 template <bool PAIR> __device__ __forceinline__ void commit_at(uint32_t bar) {
   if constexpr (PAIR)
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
@@ -822,16 +824,29 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < p.stages; ++s) { mbar_init(&full_bar[s], 2); mbar_init(&empty_bar[s], 1); }   // (a full stage: both producers have armed it and every byte has landed)
-    // in pair mode the epilogue warps of both CTAs release an accumulator on the first CTA's barrier
-    for (int a = 0; a < 2; ++a) { mbar_init(&tfull_bar[a], 1); mbar_init(&tempty_bar[a], (uint32_t)(kEpilogueWarps << kPair)); }
-    for (int b = 0; b < kMaxRing; ++b) { mbar_init(&box_full[b], 1); mbar_init(&box_done[b], (uint32_t)p.box_arrivals); }
-    *abort_flag = 0;
+  // A lane per barrier: 52 initialisations in a row would be on every launch's way.
+  if (warp == 0) {
+    constexpr int kTempty = 34, kBoxes = 36, kAll = kBoxes + 2 * kMaxRing;
+    for (int i = lane; i < kAll; i += 32) {
+      // full (both producers have armed the stage and every byte has landed), empty, accumulator full, accumulator empty (in pair mode the
+      // epilogue warps of both CTAs release it on the first CTA's barrier), box armed, box done
+      const uint32_t count = i < 16 ? 2u : i < kTempty ? 1u : i < kBoxes ? (uint32_t)(kEpilogueWarps << kPair) : i < kBoxes + kMaxRing ? 1u : (uint32_t)p.box_arrivals;
+      mbar_init(&full_bar[i], count);
+    }
+    if (lane == 0) *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  if constexpr (PAIR) cluster_sync_all();  // the peer's barriers exist before anything of this CTA can reach them
+  if (warp == kStorerWarp && lane == 0) {
+    prefetch_map(&tmA);
+    prefetch_map(&tmB);
+    if (STAGED) prefetch_map(&tmY);
+    if (p.res_tma) prefetch_map(&tmR);
+  }
+  if constexpr (PAIR) {   // the peer's barriers exist before anything of this CTA can reach them
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  }
   if (warp == 1) {
     if constexpr (PAIR) {  // the same warp of both CTAs allocates the same columns in both tensor memories
       asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)p.tmem_cols) : "memory");
@@ -841,6 +856,7 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
   }
+  if constexpr (PAIR) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -859,7 +875,6 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // ------------------------------------------------------------ producer of A ----
     // One lane; its instruction rate bounds the rate of stages.  The pixel a tile starts at is carried from tile to tile.
     if (elect_one()) {
-      prefetch_map(&tmA);
       grid_dependency_wait();
       asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the next kernel may start its own prologue now
       const uint32_t bytes_kb = PAIR ? 2u * a_box : a_box;              // the first CTA's barrier counts the bytes of both
@@ -929,7 +944,6 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   } else if (warp == kFilterWarp) {
     // ------------------------------------------------------------ producer of B ----
     if (elect_one()) {
-      prefetch_map(&tmB);
       if (!p.b_constant) grid_dependency_wait();
       const uint32_t bytes_kb = PAIR ? 2u * b_box : b_box;
       const uint32_t sb0 = smem_u32(smem) + (uint32_t)p.bps * a_box, full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
@@ -1024,8 +1038,6 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   } else if (warp == kStorerWarp) {
     // -------------------------- staging ring: store finished boxes, arm them again (residual loads) ----
     if (STAGED && elect_one()) {
-      prefetch_map(&tmY);
-      if (p.res_tma) prefetch_map(&tmR);
       grid_dependency_wait();   // earlier kernels may still read what the stores overwrite, and write the residual
       const int cols_per_box = 128 / p.out_esz;
       const uint32_t staging_u32 = smem_u32(staging);
@@ -1279,6 +1291,7 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 constexpr int kSplitThreads = 352, kSplitEpiWarps = 8;   // producer of A, MMA issuer, eight warps that empty tensor memory, producer of B
 constexpr int kSplitRows = 4;                             // rows one thread finishes, at most (128 rows x 16 pieces / 2 CTAs / 256 threads)
 struct SplitShared { uint64_t full[8], empty[8], done; uint32_t tmem; int abort; };
+static_assert(offsetof(SplitShared, empty) == 64 && offsetof(SplitShared, done) == 128, "the barriers are initialised as one array");
 
 // What four neighbouring columns need from the epilogue's per-channel vectors; one thread keeps the same columns for all its rows.
 struct FourColumns { float mul[4], add1[4], add2[4]; };
@@ -1366,10 +1379,9 @@ umma_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int swz = p.BN >= 32 ? 7 : 3;   // a row of the partial tile has BN / 4 pieces, at least 4
   const int rank = (int)blockIdx.x % p.splits, tile = (int)blockIdx.x / p.splits;
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < p.stages; ++s) { mbar_init(&sh.full[s], 2); mbar_init(&sh.empty[s], 1); }
-    mbar_init(&sh.done, 1);
-    sh.abort = 0;
+  if (warp == 0) {   // a lane per barrier
+    if (lane < 17) mbar_init(&sh.full[lane], lane < 8 ? 2u : 1u);
+    if (lane == 0) { sh.abort = 0; prefetch_map(&tmA); prefetch_map(&tmB); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -1394,7 +1406,6 @@ umma_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     // ------------------------------------------------------------ producers of A and B ----
     if (elect_one()) {
       const bool do_a = warp == 0;
-      prefetch_map(do_a ? &tmA : &tmB);
       if (do_a || !p.b_constant) grid_dependency_wait();
       if (do_a) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
       int w0 = 0, h0 = 0, img = 0;

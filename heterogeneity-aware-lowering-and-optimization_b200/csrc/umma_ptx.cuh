@@ -170,11 +170,6 @@ __device__ __forceinline__ void umma_i8_pair(uint32_t tmem_d, uint64_t da, uint6
       "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// arrives on the barrier at this offset in both CTAs of the pair once the MMAs issued so far have completed
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"((uint16_t)3)
-               : "memory");
-}
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
