@@ -92,6 +92,7 @@ struct UmmaParams {
   int bm;              // rows of its tiles: 128 or 64
   int split_data_bytes;  // ... shared memory before its barriers: the operand stages, reused by the partial tile
   int y_ld;            // row pitch of y in elements (split kernel)
+  int split_plain;     // ... whose results take finish_plain
   int b_constant;      // B is written by no kernel: its loads need not wait for the kernel in front
   int test_skip_stage;  // test hook: the producer of CTA 0 leaves the last stage of its first tile unarmed, so the MMA lane's wait runs out
   void* y;
@@ -1369,6 +1370,44 @@ __device__ __forceinline__ void finish_four(const UmmaParams& p, float (&v)[4], 
   }
 }
 
+// The form nearly every layer of a two-byte network has: fp32 sums, one per-channel addend, a residual of the result's type, ReLU or LeakyReLU
+// (p.split_plain, decided when planning).  The same steps as finish_four, without its twenty decisions on the way of every result.
+template <bool BF16>
+__device__ __forceinline__ void finish_plain(const UmmaParams& p, float (&v)[4], int64_t row, int col, const float4& add, const uint4& res) {
+  const Epilogue& ep = p.ep;
+  const float a[4] = {add.x, add.y, add.z, add.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) v[j] = __fadd_rn(v[j], a[j]);
+  if (ep.act == ACT_LEAKY && ep.act_first) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = apply_act(ACT_LEAKY, v[j], ep.act_a, 0.f);
+  }
+  if (ep.res) {
+    const uint32_t w[2] = {res.x, res.y};
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      const float2 h = BF16 ? __bfloat1622float2(*(const __nv_bfloat162*)&w[t]) : __half22float2(*(const __half2*)&w[t]);
+      v[2 * t] = __fadd_rn(v[2 * t], h.x);
+      v[2 * t + 1] = __fadd_rn(v[2 * t + 1], h.y);
+    }
+  }
+  if (ep.act == ACT_RELU) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = apply_act(ACT_RELU, v[j], 0.f, 0.f);
+  } else if (ep.act == ACT_LEAKY && !ep.act_first) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = apply_act(ACT_LEAKY, v[j], ep.act_a, 0.f);
+  }
+  uint2 u;
+  uint32_t* w = (uint32_t*)&u;
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    if (BF16) { const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * t], v[2 * t + 1]); w[t] = *(const uint32_t*)&h; }
+    else { const __half2 h = __floats2half2_rn(v[2 * t], v[2 * t + 1]); w[t] = *(const uint32_t*)&h; }
+  }
+  *(uint2*)((uint16_t*)p.y + row * p.y_ld + col) = u;
+}
+
 __global__ void __launch_bounds__(kSplitThreads, 2)
 umma_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const UmmaParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -1401,6 +1440,7 @@ umma_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   const int rows = min(p.bm, p.M_total - m0), r_lo = rows * rank / p.splits, r_hi = rows * (rank + 1) / p.splits;
   const bool vec = (p.K_out & 3) == 0, finisher = warp >= 2 && warp < 2 + kSplitEpiWarps && col < p.K_out;
   FourColumns fc;
+  float4 plain_add = make_float4(0.f, 0.f, 0.f, 0.f);
   uint4 res[kSplitRows];
   if (warp == 0 || warp == 2 + kSplitEpiWarps) {
     // ------------------------------------------------------------ producers of A and B ----
@@ -1476,7 +1516,8 @@ umma_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       if (ok) umma_commit(&sh.done);
     }
   } else {
-    if (finisher && vec) load_four_columns(p.ep, col, fc);
+    if (finisher && p.split_plain) plain_add = __ldg((const float4*)((p.ep.add1 ? p.ep.add1 : p.ep.add2) + col));
+    else if (finisher && vec) load_four_columns(p.ep, col, fc);
     grid_dependency_wait();   // residuals are read, and tensors earlier kernels may still read overwritten, from here on
     if (finisher && vec && p.ep.res) {
 #pragma unroll
@@ -1541,7 +1582,8 @@ umma_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         for (int k = 1; k < 8; ++k)
           if (k < p.splits) { v[0] += __uint_as_float(u[k].x); v[1] += __uint_as_float(u[k].y); v[2] += __uint_as_float(u[k].z); v[3] += __uint_as_float(u[k].w); }
       }
-      if (vec && !p.ep.add_full) finish_four(p, v, row, col, fc, res[i]);
+      if (p.split_plain) { if (p.ep.out_dt == DT_BF16) finish_plain<true>(p, v, row, col, plain_add, res[i]); else finish_plain<false>(p, v, row, col, plain_add, res[i]); }
+      else if (vec && !p.ep.add_full) finish_four(p, v, row, col, fc, res[i]);
       else
         for (int j = 0; j < 4 && col + j < p.K_out; ++j) store_from_float(p.y, p.ep.out_dt, row * p.y_ld + col + j, epilogue_value(p.ep, v[j], row, col + j, p.K_out));
     }
@@ -2084,6 +2126,9 @@ UmmaLaunch* umma_conv_prepare(const UmmaConv& c, const void* x, const void* w, v
   if (p.splits > 1) {
     p.stages = std::max(1, std::min({200 * 1024 / stage_bytes, 8, (share_kb + p.bps - 1) / p.bps}));
     p.split_data_bytes = (std::max(p.stages * stage_bytes, p.bm * p.BN * 4) + 1023) / 1024 * 1024;
+    p.split_plain = !p.acc_int && c.K % 4 == 0 && !ep.mul && ep.alpha == 1.f && ((ep.add1 != nullptr) != (ep.add2 != nullptr)) && !ep.add_full &&
+                    (ep.act == ACT_NONE || (ep.act == ACT_RELU && !ep.act_first) || ep.act == ACT_LEAKY) && (ep.out_dt == DT_F16 || ep.out_dt == DT_BF16) &&
+                    (!ep.res || ep.res_dt == ep.out_dt);
     L->grid = p.total_tiles * p.splits;
     L->smem = (size_t)p.split_data_bytes + 1024 /*alignment slack*/ + 256 /*barriers*/;
   }
