@@ -52,7 +52,8 @@ constexpr float kLeast = 8.47032947e-22f;             // 2^-70
 struct F32UmmaParams {
   int M, N, C, H, W, R, S, P, Q, stride_h, stride_w, pad_t, pad_l;
   int im2col, chunks, tail_halves, num_kb, splits, m_tiles, total_tiles, stages;
-  int boxed;                 // results leave (and residuals arrive) through boxes of 128 rows x 32 columns by TMA
+  int plain;                 // fp32 results in rows of whole 16-byte pieces, at most one addend, no activation or a last ReLU
+  int boxed;                 // ... which leave (and residuals arrive) through boxes of 128 rows x 32 columns by TMA
   int64_t a_row, a_img, a_h, a_w;   // floats from row to row of a product's A, from image to image, line to line and pixel to pixel of a convolution's
   uint32_t spin_limit;
   const float* A;
@@ -242,6 +243,36 @@ __device__ __forceinline__ void finish_rows(const F32UmmaParams& p, bool f32_io,
   }
   if (again) finish_doubtful<BN, W>(p, out, m0, n0, c, r_lo + t / kPerRow, r_hi);   // (over what was just stored)
 }
+// The plain form (p.plain) of a shared reduction, with nothing left to decide for a result.
+template <int BN>
+__device__ __forceinline__ void finish_plain_rows(const F32UmmaParams& p, uint32_t out, int m0, int n0, int r_lo, int r_hi, int t) {
+  constexpr int kPerRow = BN / 4, kStep = 32 * kSumWarps / kPerRow;
+  const Epilogue& ep = p.ep;
+  const int c = t % kPerRow * 4, col = n0 + c;
+  if (col >= p.N) return;
+  const float* addv = ep.add1 ? ep.add1 : ep.add2;
+  const float4 add = addv ? __ldg((const float4*)(addv + col)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float* res = (const float*)ep.res;
+  float* y = (float*)p.y;
+  bool again = false;
+#pragma unroll 2
+  for (int r = r_lo + t / kPerRow; r < r_hi; r += kStep) {
+    const int64_t at = ((int64_t)m0 + r) * p.N + col;
+    const float4 f = res ? *(const float4*)(res + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float x[4];
+    read_result<BN, 4>(p, out, r, c, x);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) again = again || doubtful(x[j]);
+    if (addv) { x[0] = __fadd_rn(x[0], add.x); x[1] = __fadd_rn(x[1], add.y); x[2] = __fadd_rn(x[2], add.z); x[3] = __fadd_rn(x[3], add.w); }
+    if (res) { x[0] = __fadd_rn(x[0], f.x); x[1] = __fadd_rn(x[1], f.y); x[2] = __fadd_rn(x[2], f.z); x[3] = __fadd_rn(x[3], f.w); }
+    if (ep.act == ACT_RELU) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) x[j] = apply_act(ACT_RELU, x[j], 0.f, 0.f);
+    }
+    *(float4*)(y + at) = make_float4(x[0], x[1], x[2], x[3]);
+  }
+  if (again) finish_doubtful<BN, 4>(p, out, m0, n0, c, r_lo + t / kPerRow, r_hi);   // (over what was just stored)
+}
 // COLS columns of one row, straight from their sums into the row's places in the boxes of 32 columns that start at `at` (128-byte swizzle:
 // 16-byte piece j of a row at j ^ (row & 7)); the residual lies there already.  Columns past N hold anything: the store clips them.
 template <int COLS>
@@ -296,6 +327,7 @@ __device__ __forceinline__ void finish_in_boxes(const F32UmmaParams& p, float (&
 template <int BN>
 __device__ __forceinline__ void finish_tile(const F32UmmaParams& p, uint32_t out, int m0, int n0, int r_lo, int r_hi, int t) {
   const Epilogue& ep = p.ep;
+  if (p.plain) return finish_plain_rows<BN>(p, out, m0, n0, r_lo, r_hi, t);
   const bool f32_io = !ep.mul && !ep.add_full && (!ep.res || ep.res_dt == DT_F32) && ep.out_dt == DT_F32;
   if (f32_io && (p.N & 3) == 0) finish_rows<BN, 4>(p, true, out, m0, n0, r_lo, r_hi, t);
   else finish_rows<BN, 1>(p, f32_io, out, m0, n0, r_lo, r_hi, t);
@@ -713,9 +745,9 @@ F32UmmaLaunch* f32_umma_prepare(const F32Umma& c, const void* x, const void* pla
     r = g_encode_tiled(&L->tmB, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, (void*)planes, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   }
-  // fp32 results and residuals in rows of whole 16-byte pieces go through boxes
-  p.boxed = p.splits == 1 && c.K % 4 == 0 && !ep.mul && !ep.add_full && ep.out_dt == DT_F32 && ep.alpha == 1.f && !(ep.add1 && ep.add2) &&
+  p.plain = c.K % 4 == 0 && !ep.mul && !ep.add_full && ep.out_dt == DT_F32 && ep.alpha == 1.f && !(ep.add1 && ep.add2) &&
             (ep.act == ACT_NONE || (ep.act == ACT_RELU && !ep.act_first)) && (!ep.res || (ep.res_dt == DT_F32 && (uintptr_t)ep.res % 16 == 0));
+  p.boxed = p.plain && p.splits == 1;
   L->tmY = L->tmR = L->tmA;
   if (r == CUDA_SUCCESS && p.boxed) {
     cuuint64_t dims[2] = {(cuuint64_t)c.K, (cuuint64_t)p.M};
