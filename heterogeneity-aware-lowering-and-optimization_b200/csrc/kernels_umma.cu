@@ -2068,13 +2068,20 @@ UmmaLaunch* umma_conv_prepare(const UmmaConv& c, const void* x, const void* w, v
     const int per_group = std::max(p.BN / 64, 1), per_box = 128 / p.out_esz / 16;
     const int groups_per_box = per_box / per_group < 4 ? per_box / per_group : 4;
     p.box_arrivals = 4 * (groups_per_box < 1 ? 1 : groups_per_box);
-    // Contiguous runs let the groups work on different boxes at once, which pays when boxes need no residual and
-    // the CTA has many tiles to stream through; otherwise finishing box after box gets the first store out sooner.
-    p.epi_interleave = ep.res != nullptr || (p.total_tiles << p.pair) < 16 * sms;
+    // Contiguous runs let the groups work on different boxes at once; finishing box after box gets the first store out sooner,
+    // which only still pays for the long arithmetic of MODE 3 (LeakyReLU, GELU) with a residual or few tiles: a feed-forward layer of
+    // 8192 x 768 -> 3072 in int8 takes 31.6 us box after box and 32.6 in runs, its Q, K and V product 20.6 and 18.3; ResNet-50 of 45
+    // images 819 and 805, of 256 in int8 3330 and 3290.
+    p.epi_interleave = p.epi_mode == 3 && (ep.res != nullptr || (p.total_tiles << p.pair) < 16 * sms);
     if (getenv("ODLA_B200_EPI_INTERLEAVE")) p.epi_interleave = atoi(getenv("ODLA_B200_EPI_INTERLEAVE"));
-    // Runs need a box of its own for every group of the tile, and whole groups to a box: with fewer boxes a group would find the
-    // phase before last of its box complete, with 192 columns a box would count its arrivals short.
-    if (p.ring_boxes < p.stage_boxes || p.BN == 192) p.epi_interleave = 1;
+    // In runs a group waits only for its own boxes, by the parity of the box's phase, so the use of the same box one
+    // turn of the ring earlier has to have been full by then.  That use lies in the tile before, at or below the group's
+    // own box there (ring of at least a tile's boxes; every tile with all its boxes; groups whole to a box, which 192 columns are
+    // not) -- and boxes without a residual fill in order.  Residuals land in any order: there it has to be the group's own box
+    // (ring of exactly a tile) or lie two tiles back, which every group has left before the accumulator could be reused.
+    const bool whole_tiles = p.K_out > (p.n_tiles - 1) * p.BN + (p.stage_boxes - 1) * (128 / p.out_esz);
+    const bool in_order = !ep.res || p.ring_boxes == p.stage_boxes || p.ring_boxes >= 2 * p.stage_boxes;
+    if (p.ring_boxes < p.stage_boxes || p.BN == 192 || !whole_tiles || !in_order) p.epi_interleave = 1;
     if (p.epi_interleave) p.box_arrivals = 16;
   }
   p.stages = (budget - p.ring_boxes * 16384) / stage_bytes;
