@@ -6,7 +6,7 @@
 // mantissa, the same exponent range): a = a1 + a2 + a3, each the leading bits of what the ones before leave.  The product a * w is then
 // a1 w1 + (a1 w2 + a2 w1) + (a1 w3 + a2 w2 + a3 w1) up to 2^-26 of its size, six bf16 products that are exact in fp32.  Six of them at
 // 4096 a clock and SM are 683 fp32 products against the FMA pipe's 128, of which the tiles of kernels_f32.cu reach a third.
-// ResNet-50 of 8 images 2747 -> 1046 us, YOLOv3 of one 416 x 416 picture 3115 -> 1506, BERT of 2 x 128 2464 -> 1747; one 3x3 layer of
+// ResNet-50 of 8 images 2747 -> 957 us, YOLOv3 of one 416 x 416 picture 3115 -> 1506, BERT of 2 x 128 2464 -> 1747; one 3x3 layer of
 // 8 x 28 x 28 x 128 -> 128 56 -> 19 us, of 2 x 52 x 52 x 128 -> 256 93 -> 28.  What bounds it: half a stage of 64 columns takes some 800 clocks
 // where its products take 400 (the splitting warps' chain of load, split, store and signal), one of 128 columns 1100 where they take
 // 770; short reductions their first loads and the finishing of the tile.
