@@ -596,14 +596,14 @@ __device__ __forceinline__ void box_fast(const UmmaParams& p, uint32_t taddr, in
 // The Darknet layer form as straight-line code (MODE 3): fp32 accumulators, one per-channel addend, LeakyReLU with a
 // slope in [0, 1], then (optionally) the residual tile, two-byte outputs.  For such a slope x < 0 ? fl(a*x) : x equals
 // max(x, fl(a*x)): the product rounds monotonically and keeps the sign.
-// GELU (erf form) without branches, used only where the result is rounded to a two-byte type or to int8 right after (the
+// GELU (erf form) without branches, used only where the result is rounded to a two-byte type right after (the
 // library erff takes two different paths by magnitude, which a warp's 32 rows then both execute):
 //   x Phi(x) = x / 2 + |x| (1/2 - Phi(-|x|)),   Phi(-a) = 2^P(a),
 // with P of degree 8, the minimax fit (a linear programme over the error of 2^P) of log2 Phi(-a) on [0, 5.7]: 7.6e-9 in Phi.  P stays
 // below -26 beyond and goes to minus infinity, so infinities and NaN come out as from the formula.  Largest error against 64 bits
 // 3.4e-7, the roundings of fp32 included (4.7e-7 for erf as a polynomial in 1 / (1 + 0.33 |z|), which takes a reciprocal more).
 // A feed-forward layer's epilogue is bound by instruction issue: this is 13 packed and 4 scalar instructions for two values; BERT-base
-// of 64 x 128 1568 -> 1517 us in int8 and 1707 -> 1664 in fp16 against the reciprocal's form, 1530 and 1687 with scalar instructions.
+// of 64 x 128 1707 -> 1664 us in fp16 against the reciprocal's form, 1687 with scalar instructions.
 __device__ __forceinline__ void ffma2(float& a0, float& a1, float b0, float b1, float c0, float c1) {   // a = a * b + c
   asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %3};\n\tmov.b64 z, {%4, %5};\n\tfma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
       : "+f"(a0), "+f"(a1)
@@ -622,6 +622,33 @@ __device__ __forceinline__ void gelu_erf_two_byte_pair(float& t0, float& t1) {
   fmul2_rn(t0, t1, 0.5f, 0.5f);
   ffma2(p0, p1, a0, a1, t0, t1);
   t0 = p0; t1 = p1;
+}
+// The form for results that are requantised: erf by Abramowitz & Stegun 7.1.26 (the whole expression within 5e-7).  A value next to a
+// rounding boundary moves by a whole step with any other last bits, and twelve layers carry such steps to 2 % of the output; the
+// shorter form above would save 3 % of an int8 BERT-base at that price.
+__device__ __forceinline__ void gelu_erf_requantised_pair(float& t0, float& t1) {
+  float z0 = t0, z1 = t1;
+  fmul2_rn(z0, z1, 0.70710678118654752440f, 0.70710678118654752440f);
+  const float a0 = fabsf(z0), a1 = fabsf(z1);
+  float d0 = a0, d1 = a1;
+  ffma2(d0, d1, 0.3275911f, 0.3275911f, 1.0f, 1.0f);
+  const float k0 = __fdividef(1.0f, d0), k1 = __fdividef(1.0f, d1);
+  float p0 = k0, p1 = k1;
+  ffma2(p0, p1, 1.061405429f, 1.061405429f, -1.453152027f, -1.453152027f);
+  ffma2(p0, p1, k0, k1, 1.421413741f, 1.421413741f);
+  ffma2(p0, p1, k0, k1, -0.284496736f, -0.284496736f);
+  ffma2(p0, p1, k0, k1, 0.254829592f, 0.254829592f);
+  fmul2_rn(p0, p1, -k0, -k1);                       // -(polynomial * k)
+  float e0 = a0, e1 = a1;
+  fmul2_rn(e0, e1, a0, a1);
+  fmul2_rn(e0, e1, -1.4426950408889634f, -1.4426950408889634f);
+  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(e0));
+  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(e1));
+  ffma2(p0, p1, e0, e1, 1.0f, 1.0f);                // 1 - polynomial * k * exp(-z^2)
+  p0 = copysignf(p0, z0); p1 = copysignf(p1, z1);
+  fadd2_rn(p0, p1, 1.0f, 1.0f);
+  fmul2_rn(t0, t1, 0.5f, 0.5f);
+  fmul2_rn(t0, t1, p0, p1);
 }
 // ACTF 0: LeakyReLU, 1: GELU (erf form)
 template <int OUT, int ACTF, bool RES>
@@ -705,7 +732,7 @@ __device__ __forceinline__ void chunk_gelu_s8(const uint32_t (&r)[16], const flo
 #pragma unroll
   for (int j = 0; j < 16; j += 2) {   // scalar sums after a packed product (see fadd2_rn)
     v[j] = __fadd_rn(v[j], cv[j]); v[j + 1] = __fadd_rn(v[j + 1], cv[j + 1]);
-    gelu_erf_two_byte_pair(v[j], v[j + 1]);
+    gelu_erf_requantised_pair(v[j], v[j + 1]);
   }
   uint4 u;
   uint32_t* w = (uint32_t*)&u;
