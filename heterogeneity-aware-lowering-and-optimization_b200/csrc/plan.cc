@@ -134,14 +134,26 @@ std::vector<float> transpose_rows(const std::vector<float>& w, int64_t k, int64_
   return o;
 }
 std::vector<uint8_t> f32_rows_kmajor(const std::vector<float>& w, int64_t k, int64_t n, int64_t pitch) { return f32_to_storage(transpose_rows(w, k, n, pitch), DT_F32); }
+// The bf16 value nearest to a finite fp32 value, and the value a bf16 stands for.
+uint16_t nearest_bf16(float v) { uint32_t b; memcpy(&b, &v, 4); return (uint16_t)((b + 0x7fffu + ((b >> 16) & 1u)) >> 16); }
+float bf16_value(uint16_t h) { const uint32_t b = (uint32_t)h << 16; float v; memcpy(&v, &b, 4); return v; }
+// Whether f32_planes can hold these weights: at most 2^20 in magnitude (a NaN fails as well), and each the exact sum of its three
+// parts.  Below 2^-110 the last ones fall under bf16's smallest subnormal, 2^-133: a weight of 1e-36 would be off by 2e-5, one of 1e-40 by 8 %.
+bool f32_planes_hold(const std::vector<float>& w) {
+  return std::all_of(w.begin(), w.end(), [](float v) {
+    const float a = std::fabs(v);
+    if (!(a <= 1048576.f)) return false;
+    if (a >= 0x1p-110f) return true;   // (24 bits down to 2^-133)
+    for (int i = 0; i < 3; ++i) v -= bf16_value(nearest_bf16(v));
+    return v == 0.f;
+  });
+}
 // fp32 weights [taps * channels][n] (or [n][taps * channels] when `transposed`) as the three bf16 values whose sum each is,
 // [block][3][n][64] for blocks of 64 channels of one tap (see F32Umma).
 std::vector<uint8_t> f32_planes(const std::vector<float>& w, int64_t taps, int64_t channels, int64_t n, bool transposed) {
   const int64_t chunks = (channels + 63) / 64, kd = taps * channels;
   std::vector<uint8_t> bytes((size_t)(taps * chunks * 3 * n * 64 * 2), 0);
   uint16_t* out = (uint16_t*)bytes.data();
-  auto round = [](float v) { uint32_t b; memcpy(&b, &v, 4); return (uint16_t)((b + 0x7fffu + ((b >> 16) & 1u)) >> 16); };
-  auto value = [](uint16_t h) { const uint32_t b = (uint32_t)h << 16; float v; memcpy(&v, &b, 4); return v; };
   for (int64_t b = 0; b < taps * chunks; ++b) {
     const int64_t k0 = b / chunks * channels + b % chunks * 64, here = std::min<int64_t>(64, channels - b % chunks * 64);
     uint16_t* plane = out + b * 3 * n * 64;
@@ -150,9 +162,9 @@ std::vector<uint8_t> f32_planes(const std::vector<float>& w, int64_t taps, int64
         for (int64_t j = j0; j < std::min(n, j0 + 32); ++j) {
           float v = transposed ? w[(size_t)(j * kd + k0 + c)] : w[(size_t)((k0 + c) * n + j)];
           for (int64_t i = 0; i < 3; ++i) {
-            const uint16_t h = round(v);
+            const uint16_t h = nearest_bf16(v);
             plane[(i * n + j) * 64 + c] = h;
-            v -= value(h);
+            v -= bf16_value(h);
           }
         }
   }
@@ -1356,7 +1368,7 @@ F32UmmaLaunch* Builder::prepare_f32_umma(const F32Umma& fu, const Fused& f, cons
                                          const void* x, void* y, const Epilogue& ep, int sms) {
   if (!f32_umma_supported(fu) || (uintptr_t)x % 16 || (uintptr_t)y % 16) return nullptr;
   const auto w = const_as_f32(f.w);
-  if (!std::all_of(w.begin(), w.end(), [](float v) { return std::fabs(v) <= 1048576.f; })) return nullptr;   // (a NaN fails as well)
+  if (!f32_planes_hold(w)) return nullptr;
   auto planes = prepared(f.w, form, [&] { return make(w); });
   const void* wd = upload(planes->data(), planes->size());
   F32UmmaLaunch* l = wd ? f32_umma_prepare(fu, x, wd, y, ep, p_->status, sms) : nullptr;

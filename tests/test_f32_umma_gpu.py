@@ -87,6 +87,26 @@ def test_values_the_split_does_not_hold(odla, gpu_lib, shape, bad, monkeypatch):
     assert np.abs(got[ok].astype(np.float64) - want[ok]).max() <= 2e-5 * np.abs(want[ok]).max() + 1e-43
 
 
+@pytest.mark.parametrize("scale, value, launch", [(2.0 ** -126, 0, "conv_simt"), (1e-40, 0, "conv_simt"), (1, 1e-36, "conv_simt"), (1, 1.5 * 2.0 ** 20, "conv_simt"),
+                                                  (1, -2.0 ** 20, "conv_f32_umma"), (1, 1.2345678 * 2.0 ** -110, "conv_f32_umma"), (1, 2.0 ** -133, "conv_f32_umma"), (1, 2.0 ** -134, "conv_simt")])
+def test_weights_the_split_does_not_hold(odla, gpu_lib, scale, value, launch):
+    """Filters with values that are no sum of three bf16 values, or too large, stay with the CUDA-core kernel; either way the results
+    are the products of the filter as given, also where large activations meet filters that are all tiny."""
+    N, H, C, K, R = 2, 28, 64, 128, 3
+    rng = np.random.default_rng(6)
+    x = rng.standard_normal((N, H, H, C)).astype(np.float32)
+    w = (rng.standard_normal((R, R, C, K)) / 24 * scale).astype(np.float32)
+    if scale < 1:
+        x *= np.float32(1e30)
+    if value:
+        w[1, 1, 7, 5] = value
+    got = conv(odla, gpu_lib, x, w, np.zeros(K, np.float32), act=None, launch=launch)
+    want = float64(x, w, 0, None, 1, 1, None)
+    # a column against its own size (one holds the large weight); sums as in test_conv_matches_float64, on the CUDA cores a chain of all products
+    err = np.abs(got - want).max(axis=(0, 1, 2)) / np.sqrt(np.mean(want ** 2, axis=(0, 1, 2)))
+    assert err.max() < 4e-7 * (3 if launch == "conv_f32_umma" else 24) + 1e-6, err.max()
+
+
 @pytest.mark.parametrize("tb", [False, True])
 @pytest.mark.parametrize("dims", [(2, 130, 768, 768), (1, 700, 100, 999)])   # batch, M, K, N
 def test_products_match_float64(odla, gpu_lib, dims, tb):
