@@ -137,6 +137,22 @@ __device__ __noinline__ float replay(const F32UmmaParams& p, int row, int col) {
   return sum;
 }
 __device__ __forceinline__ bool doubtful(float v) { return !(fabsf(v) < __int_as_float(0x7f800000)) || (v != 0.f && fabsf(v) < kLeast); }
+// Whether any of N is, in short independent chains: twice the bits less one is least for the smallest value that is not zero, and
+// zero times a value is not zero where it is not finite.
+template <int N> __device__ __forceinline__ bool any_doubtful(const float (&v)[N]) {
+  constexpr int kChains = N < 4 ? N : 4;
+  uint32_t least[kChains];
+  float zero[kChains];
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const uint32_t u = 2u * __float_as_uint(v[j]) - 1u;
+    least[j % kChains] = j < kChains ? u : min(least[j % kChains], u);
+    zero[j % kChains] = __fmaf_rn(v[j], 0.f, j < kChains ? 0.f : zero[j % kChains]);
+  }
+#pragma unroll
+  for (int c = 1; c < kChains; ++c) { least[0] = min(least[0], least[c]); zero[0] = __fadd_rn(zero[0], zero[c]); }
+  return least[0] < 2u * __float_as_uint(kLeast) - 1u || !(zero[0] == 0.f);
+}
 
 // A tile's result lies in shared memory at `out`, row r's 16-byte piece c at c ^ (r & 7); with a shared reduction every CTA of the
 // cluster has its part there.
@@ -273,22 +289,27 @@ __device__ __forceinline__ void finish_plain_rows(const F32UmmaParams& p, uint32
   }
   if (again) finish_doubtful<BN, 4>(p, out, m0, n0, c, r_lo + t / kPerRow, r_hi);   // (over what was just stored)
 }
+// COLS sums of one row, the doubtful ones among them computed again -- these alone: a result may not depend on which others lie
+// beside it, as the width of the tiles follows this launch's share of the batch.
+template <int COLS>
+__device__ __noinline__ void sum_doubtful(const F32UmmaParams& p, float* acc, int row, int col0) {
+  if (row >= p.M) return;
+  for (int j = 0; j < COLS && col0 + j < p.N; ++j)
+    if (doubtful(acc[j])) acc[j] = replay(p, row, col0 + j);
+}
 // COLS columns of one row, straight from their sums into the row's places in the boxes of 32 columns that start at `at` (128-byte swizzle:
 // 16-byte piece j of a row at j ^ (row & 7)); the residual lies there already.  Columns past N hold anything: the store clips them.
 template <int COLS>
-__device__ __noinline__ void finish_doubtful_row(const F32UmmaParams& p, uint32_t at, int row, int m0, int col0) {
-  if (m0 + row >= p.M) return;
-  for (int j = 0; j < COLS && col0 + j < p.N; ++j) {
-    const float v = epilogue_value(p.ep, replay(p, m0 + row, col0 + j), (int64_t)m0 + row, col0 + j, p.N);
-    asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + (uint32_t)(j / 32) * kBox + (uint32_t)((((j % 32) >> 2) ^ (row & 7)) << 4) + (uint32_t)(j & 3) * 4u), "f"(v) : "memory");
-  }
-}
-template <int COLS>
 __device__ __forceinline__ void finish_in_boxes(const F32UmmaParams& p, float (&acc)[COLS], uint32_t at, int row, int m0, int col0) {
   const Epilogue& ep = p.ep;
-  bool bad = false;
+  if (any_doubtful<COLS>(acc)) {   // (through a copy: the sums themselves stay in registers)
+    float copy[COLS];
 #pragma unroll
-  for (int j = 0; j < COLS; ++j) bad = bad || doubtful(acc[j]);
+    for (int j = 0; j < COLS; ++j) copy[j] = acc[j];
+    sum_doubtful<COLS>(p, copy, m0 + row, col0);
+#pragma unroll
+    for (int j = 0; j < COLS; ++j) acc[j] = copy[j];
+  }
   const float* addv = ep.add1 ? ep.add1 : ep.add2;
 #pragma unroll
   for (int q0 = 0; q0 < COLS / 4; q0 += 4) {
@@ -322,7 +343,6 @@ __device__ __forceinline__ void finish_in_boxes(const F32UmmaParams& p, float (&
       asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(place(q)), "f"(x[0]), "f"(x[1]), "f"(x[2]), "f"(x[3]) : "memory");
     }
   }
-  if (bad) finish_doubtful_row<COLS>(p, at, row, m0, col0);
 }
 template <int BN>
 __device__ __forceinline__ void finish_tile(const F32UmmaParams& p, uint32_t out, int m0, int n0, int r_lo, int r_hi, int t) {

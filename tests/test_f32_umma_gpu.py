@@ -65,6 +65,25 @@ def test_results_do_not_depend_on_the_cut(odla, gpu_lib, sub_batches):
     assert np.array_equal(conv(odla, gpu_lib, x, w, b), conv(odla, gpu_lib, x, w, b, sub_batches=sub_batches))
 
 
+@pytest.mark.parametrize("exponent", [-70, -100, 128])
+@pytest.mark.parametrize("shape", [(28, 128, 512, 1), (28, 64, 260, 3)])   # tiles of 128 columns for four images and of 64 for two
+def test_results_computed_again_do_not_depend_on_the_cut(odla, gpu_lib, shape, exponent):
+    """Results on both sides of where they are computed again (too small for the split, sums that overflow on the way): whether a
+    neighbour in the tile is on the other side makes no difference to any bit."""
+    H, C, K, R = shape
+    rng = np.random.default_rng(2)
+    x = rng.standard_normal((4, H, H, C)).astype(np.float32) * np.float32(2.0 ** (exponent / 2))
+    w = (rng.standard_normal((R, R, C, K)) / np.sqrt(R * R * C) * 2.0 ** min(exponent / 2, 19)).astype(np.float32)
+    x *= np.float32(2.0 ** (exponent / 2 - 20 if exponent > 0 else 5))   # (a few of a hundred are on the other side)
+    b = np.zeros(K, np.float32)
+    outs = [conv(odla, gpu_lib, x, w, b, pad=R // 2, act=None, sub_batches=s) for s in (1, 2, 4)]
+    with np.errstate(over="ignore"):
+        size = np.abs(float64(x, w, 0, None, 1, R // 2, None))
+    assert 0.01 < np.mean(size < 2.0 ** exponent) < 0.99
+    for o in outs[1:]:
+        assert np.array_equal(o.view(np.uint32), outs[0].view(np.uint32))
+
+
 @pytest.mark.parametrize("shape", [(2, 28, 64, 128, 3), (1, 14, 256, 320, 3)])   # boxes of results; a shared reduction
 @pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan, 3.4e38, 1e-30, 1e-38])
 def test_values_the_split_does_not_hold(odla, gpu_lib, shape, bad, monkeypatch):
