@@ -21,9 +21,11 @@ def conv(odla, lib, x, w, b, r=None, stride=1, pad=1, act=0.0, sub_batches=None,
         y = g.LeakyRelu(y, act, "act") if act else g.Relu(y, "act")
     g.Output(y)
     ins = {"x": x} if r is None else {"x": x, "r": r}
-    out = next(iter(g.run(ins).values()))
-    assert launch in g.describe()
-    g.close()
+    try:
+        out = next(iter(g.run(ins).values()))
+        assert launch in g.describe()
+    finally:
+        g.close()
     return out
 
 
@@ -143,3 +145,26 @@ def test_products_match_float64(odla, gpu_lib, dims, tb):
     t = torch.from_numpy(0.5 * (a.astype(np.float64) @ (w.T if tb else w).astype(np.float64)) + 2.0 * c)
     want = torch.nn.functional.gelu(t).numpy()
     assert np.abs(got - want).max() / np.sqrt(np.mean(want ** 2)) < 4e-7 * np.sqrt(max(K / 64, 4)) + 1e-6
+
+
+@pytest.mark.parametrize("residual", [False, True])
+@pytest.mark.parametrize("shape", [(8, 56, 64, 256, 1), (1, 7, 2048, 512, 1), (1, 14, 256, 320, 3), (3, 29, 100, 255, 1)])   # boxes, shared reductions, rows
+def test_wait_that_runs_out(odla, gpu_lib, monkeypatch, shape, residual):
+    """A stage that is never loaded: every role's bounded wait gives up after a short limit, the execute returns ODLA_TIMEOUT and the same
+    layer planned without the hook is right."""
+    N, H, C, K, R = shape
+    rng = np.random.default_rng(3)
+    x, w = rng.standard_normal((N, H, H, C)).astype(np.float32), (rng.standard_normal((R, R, C, K)) / np.sqrt(R * R * C)).astype(np.float32)
+    b, r = rng.standard_normal(K).astype(np.float32), rng.standard_normal((N, H, H, K)).astype(np.float32) if residual else None
+    monkeypatch.setenv("ODLA_B200_TEST_SPIN_LIMIT", "256")
+    monkeypatch.setenv("ODLA_B200_TEST_SKIP_STAGE", "1")
+    gpu_lib.SetLogLevel(0)
+    try:
+        with pytest.raises(RuntimeError, match="odla_status %d" % odla.TIMEOUT):
+            conv(odla, gpu_lib, x, w, b, r, pad=R // 2)
+    finally:
+        gpu_lib.SetLogLevel(3)
+    monkeypatch.delenv("ODLA_B200_TEST_SKIP_STAGE")
+    monkeypatch.delenv("ODLA_B200_TEST_SPIN_LIMIT")
+    got, want = conv(odla, gpu_lib, x, w, b, r, pad=R // 2), float64(x, w, b, r, 1, R // 2, 0.0)
+    assert np.abs(got - want).max() / np.sqrt(np.mean(want ** 2)) < 4e-7 * 6 + 1e-6
