@@ -431,10 +431,7 @@ f32_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         load_b(s);
         if (++s == p.stages) { s = 0; ph ^= 1; }
       }
-      if (!ok)   // copies in flight get a bounded chance to land before shared memory goes away
-        for (int i = 0; i < p.stages; ++i)
-          for (uint32_t n = 0; n < 4096; ++n)
-            if (mbar_try_wait(&sh.full[i], 0) || mbar_try_wait(&sh.full[i], 1)) break;
+      if (!ok) await_stages(sh.full, p.stages, s, ph);
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------- products ----

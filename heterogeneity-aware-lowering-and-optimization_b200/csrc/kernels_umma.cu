@@ -952,12 +952,7 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             }
           }
         }
-        if (!ok) {
-          // give copies already in flight a bounded chance to land before shared memory goes away
-          for (int i = 0; i < p.stages; ++i)
-            for (uint32_t n = 0; n < 4096; ++n)
-              if (mbar_try_wait(&full_bar[i], 0) || mbar_try_wait(&full_bar[i], 1)) break;
-        }
+        if (!ok) await_stages(full_bar, p.stages, (int)(bar - full0) >> 3, ph);
       };
       if (p.im2col) produce(BoolConst<true>{}); else produce(BoolConst<false>{});
     }
@@ -996,11 +991,7 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           if (bar == full_end) { bar = full0; ph ^= 1; sb_stage = sb0; }
         }
       }
-      if (!ok) {
-        for (int i = 0; i < p.stages; ++i)
-          for (uint32_t n = 0; n < 4096; ++n)
-            if (mbar_try_wait(&full_bar[i], 0) || mbar_try_wait(&full_bar[i], 1)) break;
-      }
+      if (!ok) await_stages(full_bar, p.stages, (int)(bar - full0) >> 3, ph);
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer ----
@@ -1063,6 +1054,7 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const uint32_t staging_u32 = smem_u32(staging);
       // Arming runs ring_boxes ahead of storing: a box is armed for its next use as soon as its store has read it.
       int a_tile = tile_first, a_bx = 0, a_slot = 0;
+      uint32_t a_ph = 1;   // (as if waiting for boxes to be empty)
       TileWalk a_at(p, tile_first);
       auto arm = [&]() {
         if (a_tile >= p.total_tiles) return;
@@ -1072,7 +1064,7 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         } else {
           mbar_arrive(box_full + a_slot);
         }
-        if (++a_slot == p.ring_boxes) a_slot = 0;
+        if (++a_slot == p.ring_boxes) { a_slot = 0; a_ph ^= 1; }
         if (++a_bx == p.stage_boxes || a_at.ni * p.BN + a_bx * cols_per_box >= p.K_out) { a_bx = 0; a_tile += tile_step; a_at.next(p, tile_step); }
       };
       for (int b = 0; b < p.ring_boxes; ++b) arm();
@@ -1119,12 +1111,7 @@ umma_conv_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           if (++slot == p.ring_boxes) { slot = 0; ph ^= 1; }
         }
       }
-      if (!ok && p.res_tma) {
-        // residual loads already in flight get a bounded chance to land before shared memory goes away
-        for (int i = 0; i < p.ring_boxes; ++i)
-          for (uint32_t k = 0; k < 4096; ++k)
-            if (mbar_try_wait(&box_full[i], 0) || mbar_try_wait(&box_full[i], 1)) break;
-      }
+      if (!ok && p.res_tma) await_stages(box_full, p.ring_boxes, a_slot, a_ph);
       asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // stores complete before shared memory is released
     }
   } else {
@@ -1503,10 +1490,7 @@ umma_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         at_stage += (uint32_t)stage_bytes;
         if (++s == p.stages) { s = 0; ph ^= 1; at_stage = first; }
       }
-      if (!ok)   // copies in flight get a bounded chance to land before shared memory goes away
-        for (int i = 0; i < p.stages; ++i)
-          for (uint32_t n = 0; n < 4096; ++n)
-            if (mbar_try_wait(&sh.full[i], 0) || mbar_try_wait(&sh.full[i], 1)) break;
+      if (!ok) await_stages(sh.full, p.stages, s, ph);
     }
   } else if (warp == 1) {
     if (elect_one()) {
@@ -1713,10 +1697,7 @@ attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
         asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the box is V again: the next loads are issued by this thread
       }
       asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-      // copies that were armed but never consumed (an aborted run) get a bounded chance to land
-      if (*abort_flag)
-        for (uint32_t k = 0; k < 4096; ++k)
-          if (mbar_try_wait(b_full, 0) || mbar_try_wait(b_full, 1)) break;
+      if (*abort_flag && n > 0) await_landing(b_full, (n - 1) & 1);   // (armed but never consumed)
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------- the two products ----

@@ -71,6 +71,18 @@ __device__ __forceinline__ bool mbar_wait_impl(uint64_t* bar, uint32_t parity, v
   if (status) { *(volatile int*)status = code; ((volatile int*)status)[1] = (int)blockIdx.x; __threadfence_system(); }
   return false;
 }
+// For loads in flight when a wait has run out: shared memory stays until they have landed, or about a millisecond.  A barrier answers for the
+// phase of the given parity, which therefore has to be that of the load (either parity's answer would be yes for one of the two).
+__device__ __noinline__ void await_landing(uint64_t* bar, uint32_t parity) {
+#pragma unroll 1
+  for (int i = 0; i < 256 && !mbar_try_wait_suspend(bar, parity, 4000u); ++i) {}
+}
+// ... of a ring of stages whose next one to load is `next`, with `ph` as the parity of the wait for it to be empty: those before it were loaded
+// in this turn of the ring, the others in the one before (in the first turn not at all: their barriers answer at once).
+__device__ __noinline__ void await_stages(uint64_t* full, int stages, int next, uint32_t ph) {
+#pragma unroll 1
+  for (int i = 0; i < stages; ++i) await_landing(&full[i], i < next ? ph ^ 1u : ph);
+}
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(dst)),
                "l"((uint64_t)map), "r"(smem_u32(bar)), "r"(x), "r"(y)
