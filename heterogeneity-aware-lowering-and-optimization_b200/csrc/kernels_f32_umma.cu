@@ -18,7 +18,7 @@
 // 4608 values have 5e-8 to 9e-8, the CUDA-core kernels 7e-8 to 2e-7.
 // Values for which the split does not hold -- an infinity or NaN among the operands, results so small that the operands' last parts
 // may lie below the smallest bf16 -- show up in the sum (not finite, or not zero and below 2^-70) and such results are computed
-// again as an fp32 FMA chain (replay) from the original operands.
+// again as an fp32 FMA chain (replay) from the operands: A as it lies, W as the sum of its three parts, which it is exactly.
 //
 // One CTA per SM walks tiles of 128 rows x BN columns, 64 values of the reduction a stage:
 //   warp 0       TMA: fp32 rows of A as they lie, the three planes of W (split once on the host)
@@ -108,6 +108,16 @@ __device__ __forceinline__ uint32_t split_off(float& x, float& y) {
   y = __fsub_rn(y, __uint_as_float(b & 0xffff0000u));
   return __byte_perm(a, b, 0x7632);
 }
+// The third parts.  They are all that is left of a value of 2^-110 or more.  Of a smaller one bits below bf16's smallest, 2^-133, would be cut
+// off, and nothing be left of many: it is rounded away from zero instead, so that a result of such values does not become a zero that
+// hides among the true ones.  (`one` is 1, which the compiler does not know: a multiply-add has a pipe that stands idle here, an addition
+// would queue with the other integer instructions.  ResNet-50 of 8 images 964 us without either, 976 and 979 with.)
+__device__ __forceinline__ uint32_t split_last(float x, float y, uint32_t one) {
+  uint32_t a, b;
+  asm("mad.lo.u32 %0, %1, %2, 65535;" : "=r"(a) : "r"(__float_as_uint(x)), "r"(one));
+  asm("mad.lo.u32 %0, %1, %2, 65535;" : "=r"(b) : "r"(__float_as_uint(y)), "r"(one));
+  return __byte_perm(a, b, 0x7632);
+}
 // How many halves of a stage hold values: the last stage of a tap may have one.
 __device__ __forceinline__ int halves_of(const F32UmmaParams& p, int chunk) { return chunk + 1 == p.chunks ? p.tail_halves : 2; }
 __device__ __forceinline__ int next_chunk(const F32UmmaParams& p, int chunk) { return chunk + 1 == p.chunks ? 0 : chunk + 1; }
@@ -138,6 +148,12 @@ __device__ __noinline__ float replay(const F32UmmaParams& p, int row, int col) {
   return sum;
 }
 __device__ __forceinline__ bool doubtful(float v) { return !(fabsf(v) < __int_as_float(0x7f800000)) || (v != 0.f && fabsf(v) < kLeast); }
+// Beside a tiny result a zero is doubtful as well: the coarse last parts of subnormals may have cancelled.
+__device__ __forceinline__ bool any_tiny(const float* v, int n) {
+  bool tiny = false;
+  for (int j = 0; j < n; ++j) tiny = tiny || (v[j] != 0.f && fabsf(v[j]) < kLeast);
+  return tiny;
+}
 // Whether any of N is, in short independent chains: twice the bits less one is least for the smallest value that is not zero, and
 // zero times a value is not zero where it is not finite.
 template <int N> __device__ __forceinline__ bool any_doubtful(const float (&v)[N]) {
@@ -181,13 +197,15 @@ template <int BN, int W> __device__ __forceinline__ void read_result(const F32Um
 // The doubtful ones among a thread's results, one at a time.
 template <int BN, int W>
 __device__ __noinline__ void finish_doubtful(const F32UmmaParams& p, uint32_t out, int m0, int n0, int c, int r0, int r_hi) {
-  for (int r = r0; r < r_hi; r += 32 * kSumWarps * W / BN)
+  for (int r = r0; r < r_hi; r += 32 * kSumWarps * W / BN) {
+    float x[W];
+    read_result<BN, W>(p, out, r, c, x);
+    const bool tiny = any_tiny(x, W);
     for (int j = 0; j < W && n0 + c + j < p.N; ++j) {
-      float x[1];
-      read_result<BN, 1>(p, out, r, c + j, x);
       const int64_t row = (int64_t)m0 + r;
-      if (doubtful(x[0])) store_from_float(p.y, p.ep.out_dt, row * p.N + n0 + c + j, epilogue_value(p.ep, replay(p, (int)row, n0 + c + j), row, n0 + c + j, p.N));
+      if (doubtful(x[j]) || (tiny && x[j] == 0.f)) store_from_float(p.y, p.ep.out_dt, row * p.N + n0 + c + j, epilogue_value(p.ep, replay(p, (int)row, n0 + c + j), row, n0 + c + j, p.N));
     }
+  }
 }
 // Rows [r_lo, r_hi) of the tile that starts at (m0, n0): the epilogue (every step rounded by itself) and the store.  A thread keeps W
 // columns, whose addends it reads once, and has several rows' residuals and results on the way at a time.
@@ -295,8 +313,11 @@ __device__ __forceinline__ void finish_plain_rows(const F32UmmaParams& p, uint32
 template <int COLS>
 __device__ __noinline__ void sum_doubtful(const F32UmmaParams& p, float* acc, int row, int col0) {
   if (row >= p.M) return;
-  for (int j = 0; j < COLS && col0 + j < p.N; ++j)
-    if (doubtful(acc[j])) acc[j] = replay(p, row, col0 + j);
+  for (int g = 0; g < COLS; g += 32) {   // (32 columns are together in tiles of either width)
+    const bool tiny = any_tiny(acc + g, 32);
+    for (int j = g; j < g + 32 && col0 + j < p.N; ++j)
+      if (doubtful(acc[j]) || (tiny && acc[j] == 0.f)) acc[j] = replay(p, row, col0 + j);
+  }
 }
 // COLS columns of one row, straight from their sums into the row's places in the boxes of 32 columns that start at `at` (128-byte swizzle:
 // 16-byte piece j of a row at j ^ (row & 7)); the residual lies there already.  Columns past N hold anything: the store clips them.
@@ -496,7 +517,7 @@ f32_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   } else if (warp < kFirstSummer) {
     // ------------------------------------------------------------------- splits A ----
     const int quarter = warp & 3, row = quarter * 32 + lane;
-    const uint32_t rx = (uint32_t)(row & 7), lane_addr = (uint32_t)(quarter * 32) << 16;
+    const uint32_t one = (uint32_t)min(p.stages, 1), rx = (uint32_t)(row & 7), lane_addr = (uint32_t)(quarter * 32) << 16;
     int s = 0, slot = 0;
     uint32_t ph = 0, slot_ph = 1;   // (the first round of slots is free)
     bool ok = true;   // (a lane's own: whatever becomes of the waits, the warp stays together for its collective stores)
@@ -513,7 +534,7 @@ f32_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           float4 v = lds4(at + ((q ^ rx) << 4));
           w1[2 * q] = split_off(v.x, v.y); w1[2 * q + 1] = split_off(v.z, v.w);
           w2[2 * q] = split_off(v.x, v.y); w2[2 * q + 1] = split_off(v.z, v.w);
-          w3[2 * q] = split_off(v.x, v.y); w3[2 * q + 1] = split_off(v.z, v.w);
+          w3[2 * q] = split_last(v.x, v.y, one); w3[2 * q + 1] = split_last(v.z, v.w, one);
         }
         if (ok) ok = mbar_wait(&sh.slot_empty[slot], slot_ph, abort_flag, p.status, 37, p.spin_limit);
         tc_fence_after();

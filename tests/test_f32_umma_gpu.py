@@ -87,7 +87,7 @@ def test_results_computed_again_do_not_depend_on_the_cut(odla, gpu_lib, shape, e
 
 
 @pytest.mark.parametrize("shape", [(2, 28, 64, 128, 3), (1, 14, 256, 320, 3)])   # boxes of results; a shared reduction
-@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan, 3.4e38, 1e-30, 1e-38])
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan, 3.4e38, 1e-30, 1e-38, 1e-41])
 def test_values_the_split_does_not_hold(odla, gpu_lib, shape, bad, monkeypatch):
     """Infinities, NaN, the largest fp32 values and operands whose last bits no bf16 can carry: what the CUDA-core kernel gives."""
     N, H, C, K, R = shape
