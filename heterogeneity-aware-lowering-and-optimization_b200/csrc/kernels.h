@@ -95,11 +95,11 @@ int gemm_f32(const GemmGeom& g, int64_t batch_full, int64_t rows_full, const voi
 // ---- fp32 on the tensor cores (kernels_f32_umma.cu) ----
 // A dense NHWC convolution with one group, or a product with constant weights (H = W = R = S = 1, N = rows).  `planes` holds the
 // weights as three bf16 values each, [block][3][K][64]: block b covers channels (b % c) * 64 and on of tap b / c for c = ceil(C / 64),
-// zeros past C.  The weights are at most 2^20 and each is the exact sum of its three values (results below 2^-70 are then computed
-// from the operands as they are).
+// zeros past C.  The weights are at most 2^20 and each is the exact sum of its three values.
 struct F32Umma {
   int N, H, W, C, K, R, S, P, Q, stride_h, stride_w, pad_t, pad_l;
   int64_t rows_full;   // output rows of the whole recorded batch: alone they decide the order of the sums
+  float largest_weight = 1048576.f;   // in magnitude: decides below which size results are computed again from the operands as they are
   // Byte strides of the W and H dimensions of x (0 = dense): a W stride smaller than a pixel describes overlapping windows.
   long long x_w_stride = 0, x_h_stride = 0;
 };

@@ -16,9 +16,12 @@
 // added up in registers with ordinary fp32 additions while the other fills; the five small products, a 2^-8th of the result, share
 // one accumulator for the whole tile, where the drift is a 2^-8th as well.  Against float64 (rms error over rms result) layers of 64 to
 // 4608 values have 5e-8 to 9e-8, the CUDA-core kernels 7e-8 to 2e-7.
-// Values for which the split does not hold -- an infinity or NaN among the operands, results so small that the operands' last parts
-// may lie below the smallest bf16 -- show up in the sum (not finite, or not zero and below 2^-70) and such results are computed
-// again as an fp32 FMA chain (replay) from the operands: A as it lies, W as the sum of its three parts, which it is exactly.
+// Values for which the split does not hold -- an infinity among the operands, a sum that overflows on the way, results so small that bits
+// of A below the smallest bf16 count -- show up in the sum (not finite, or not zero and below p.least) and such results are computed
+// again: from the infinities' signs where there are any, else as an fp32 FMA chain (replay) from the operands, A as it lies, W as the sum
+// of its three parts, which it is exactly.  A NaN in the row needs nothing: its sums are NaN.  An FMA chain takes a hundred times as long as
+// the tensor cores, so that it has to be rare: hence p.least as low as the layer's weights allow.  ResNet-50 of 8 images, waited for after
+// each call: 985 us, with an image of NaN 991, of infinities 1083, of 1e-40 1272, all of them of 1e-40 2603.
 //
 // One CTA per SM walks tiles of 128 rows x BN columns, 64 values of the reduction a stage:
 //   warp 0       TMA: fp32 rows of A as they lie, the three planes of W (split once on the host)
@@ -47,7 +50,6 @@ constexpr int kSplitWarps = 4, kSumWarps = 8, kFirstSplitter = 2, kFirstSummer =
 constexpr int kThreads = 32 * (kFirstSummer + kSumWarps);
 constexpr int kMaxStages = 8;
 constexpr uint32_t kBox = 16384;                       // 128 rows x 32 columns
-constexpr float kLeast = 8.47032947e-22f;             // 2^-70
 
 struct F32UmmaParams {
   int M, N, C, H, W, R, S, P, Q, stride_h, stride_w, pad_t, pad_l;
@@ -56,6 +58,7 @@ struct F32UmmaParams {
   int boxed;                 // ... which leave (and residuals arrive) through boxes of 128 rows x 32 columns by TMA
   int64_t a_row, a_img, a_h, a_w;   // floats from row to row of a product's A, from image to image, line to line and pixel to pixel of a convolution's
   uint32_t spin_limit;
+  float least;               // results below this, zero apart, are computed again
   int test_skip_stage;       // test hook, as in kernels_umma.cu: the last stage of CTA 0's first tile is neither armed nor loaded
   const float* A;
   const uint16_t* planes;    // [num_kb][3][N][32]
@@ -127,36 +130,96 @@ __device__ __forceinline__ void summers_sync() {
   asm volatile("bar.sync 1, %0;" ::"n"(32 * kSumWarps) : "memory");
 }
 
-// One result from the operands as they are: values in memory order, FMAs, padding left out.
-__device__ __noinline__ float replay(const F32UmmaParams& p, int row, int col) {
-  float sum = 0.f;
+// Where the values of block kb of a row lie, and how many there are; null in the padding.
+__device__ __forceinline__ const float* values_at(const F32UmmaParams& p, int row, int kb, int& count) {
+  const int tap = kb / p.chunks, c0 = (kb - tap * p.chunks) * kDepth;
+  count = min(kDepth, p.C - c0);
+  if (!p.im2col) return p.A + (int64_t)row * p.a_row + c0;
   const int pq = p.P * p.Q, img = row / pq, op = (row - img * pq) / p.Q, oq = row - img * pq - op * p.Q;
+  const int h = op * p.stride_h - p.pad_t + tap / p.S, w = oq * p.stride_w - p.pad_l + tap % p.S;
+  if ((unsigned)h >= (unsigned)p.H || (unsigned)w >= (unsigned)p.W) return nullptr;
+  return p.A + img * p.a_img + h * p.a_h + w * p.a_w + c0;
+}
+// What a row's values are: all finite, infinities among them (in blocks [first, last]), or a NaN, which makes every result NaN.
+enum { ROW_FINITE, ROW_INFINITE, ROW_NAN };
+struct RowKind { int kind, first, last; };
+__device__ __noinline__ RowKind look_at_row(const F32UmmaParams& p, int row) {
+  RowKind k{ROW_FINITE, 0, 0};
   for (int kb = 0; kb < p.num_kb; ++kb) {
-    const int tap = kb / p.chunks, c0 = (kb - tap * p.chunks) * kDepth;
-    const float* a = p.A + (int64_t)row * p.a_row;
-    if (p.im2col) {
-      const int h = op * p.stride_h - p.pad_t + tap / p.S, w = oq * p.stride_w - p.pad_l + tap % p.S;
-      if ((unsigned)h >= (unsigned)p.H || (unsigned)w >= (unsigned)p.W) continue;
-      a = p.A + img * p.a_img + h * p.a_h + w * p.a_w;
+    int count;
+    const float* a = values_at(p, row, kb, count);
+    if (!a) continue;
+    uint32_t top = 0;
+#pragma unroll 4
+    for (int c = 0; c < count; c += 4) {
+      const uint4 v = *(const uint4*)(a + c);
+      top = max(max(max(top, v.x & 0x7fffffffu), v.y & 0x7fffffffu), max(v.z & 0x7fffffffu, v.w & 0x7fffffffu));
     }
-    const uint16_t* w1 = p.planes + ((int64_t)kb * 3 * p.N + col) * kDepth;
-    for (int c = 0; c < kDepth && c0 + c < p.C; ++c) {
-      auto part = [&](int i) { return __uint_as_float((uint32_t)w1[(int64_t)i * p.N * kDepth + c] << 16); };
-      sum = fmaf(a[c0 + c], part(0) + (part(1) + part(2)), sum);   // (both sums are exact)
+    if (top > 0x7f800000u) { k.kind = ROW_NAN; return k; }
+    if (top == 0x7f800000u) {
+      if (k.kind == ROW_FINITE) { k.kind = ROW_INFINITE; k.first = kb; }
+      k.last = kb;
     }
   }
-  return sum;
+  return k;
 }
-__device__ __forceinline__ bool doubtful(float v) { return !(fabsf(v) < __int_as_float(0x7f800000)) || (v != 0.f && fabsf(v) < kLeast); }
+// The result of a row with infinities: they alone decide it.  Random signs meet within a few of them, where the walk ends.
+__device__ __noinline__ float infinite_sum(const F32UmmaParams& p, int row, int col, int first, int last) {
+  uint32_t sign = 2;   // none so far
+  for (int kb = first; kb <= last; ++kb) {
+    int count;
+    const float* a = values_at(p, row, kb, count);
+    if (!a) continue;
+    const uint16_t* w1 = p.planes + ((int64_t)kb * 3 * p.N + col) * kDepth;   // (zero where the weight is, and of its sign)
+    for (int c = 0; c < count; ++c) {
+      const uint32_t v = __float_as_uint(a[c]);
+      if ((v & 0x7fffffffu) != 0x7f800000u) continue;
+      const uint32_t w = w1[c], here = (v >> 31) ^ (w >> 15);
+      if ((w & 0x7fffu) == 0 || (sign != 2 && sign != here)) return __int_as_float(0x7fffffff);
+      sign = here;
+    }
+  }
+  return __uint_as_float(sign << 31 | 0x7f800000u);
+}
+// Two results of a row from the operands as they are: values in memory order, FMAs, padding left out.  Bound by its loads' latency; four
+// chains at a time with loads ahead take half as long, but the registers of the call then cost the kernel 2 % on its ordinary way.
+__device__ __noinline__ float2 replay(const F32UmmaParams& p, int row, int col0, int col1) {
+  float sum[2] = {};
+  const int64_t at[2] = {(int64_t)col0 * kDepth, (int64_t)col1 * kDepth};
+  for (int kb = 0; kb < p.num_kb; ++kb) {
+    int count;
+    const float* a = values_at(p, row, kb, count);
+    if (!a) continue;
+    const uint16_t* w = p.planes + (int64_t)kb * 3 * p.N * kDepth;   // [3][p.N][64]
+#pragma unroll 1
+    for (int c = 0; c < count; c += 4) {
+      const float4 v = *(const float4*)(a + c);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        uint2 u[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) u[i] = __ldg((const uint2*)(w + (int64_t)i * p.N * kDepth + at[j] + c));
+        auto part = [&](int i, int k) { const uint32_t h = k < 2 ? u[i].x : u[i].y; return __uint_as_float(k & 1 ? h & 0xffff0000u : h << 16); };
+        auto weight = [&](int k) { return part(0, k) + (part(1, k) + part(2, k)); };   // (both sums are exact)
+        sum[j] = fmaf(v.x, weight(0), sum[j]);
+        sum[j] = fmaf(v.y, weight(1), sum[j]);
+        sum[j] = fmaf(v.z, weight(2), sum[j]);
+        sum[j] = fmaf(v.w, weight(3), sum[j]);
+      }
+    }
+  }
+  return make_float2(sum[0], sum[1]);
+}
+__device__ __forceinline__ bool doubtful(const F32UmmaParams& p, float v) { return !(fabsf(v) < __int_as_float(0x7f800000)) || (v != 0.f && fabsf(v) < p.least); }
 // Beside a tiny result a zero is doubtful as well: the coarse last parts of subnormals may have cancelled.
-__device__ __forceinline__ bool any_tiny(const float* v, int n) {
+__device__ __forceinline__ bool any_tiny(const F32UmmaParams& p, const float* v, int n) {
   bool tiny = false;
-  for (int j = 0; j < n; ++j) tiny = tiny || (v[j] != 0.f && fabsf(v[j]) < kLeast);
+  for (int j = 0; j < n; ++j) tiny = tiny || (v[j] != 0.f && fabsf(v[j]) < p.least);
   return tiny;
 }
 // Whether any of N is, in short independent chains: twice the bits less one is least for the smallest value that is not zero, and
 // zero times a value is not zero where it is not finite.
-template <int N> __device__ __forceinline__ bool any_doubtful(const float (&v)[N]) {
+template <int N> __device__ __forceinline__ bool any_doubtful(const F32UmmaParams& p, const float (&v)[N]) {
   constexpr int kChains = N < 4 ? N : 4;
   uint32_t least[kChains];
   float zero[kChains];
@@ -168,7 +231,7 @@ template <int N> __device__ __forceinline__ bool any_doubtful(const float (&v)[N
   }
 #pragma unroll
   for (int c = 1; c < kChains; ++c) { least[0] = min(least[0], least[c]); zero[0] = __fadd_rn(zero[0], zero[c]); }
-  return least[0] < 2u * __float_as_uint(kLeast) - 1u || !(zero[0] == 0.f);
+  return least[0] < 2u * __float_as_uint(p.least) - 1u || !(zero[0] == 0.f);
 }
 
 // A tile's result lies in shared memory at `out`, row r's 16-byte piece c at c ^ (r & 7); with a shared reduction every CTA of the
@@ -194,17 +257,40 @@ template <int BN, int W> __device__ __forceinline__ void read_result(const F32Um
     for (int j = 0; j < W; ++j) x[j] = __fadd_rn(x[j], u[j]);
   }
 }
-// The doubtful ones among a thread's results, one at a time.
+// `n` sums of one row, of columns from `col` on, the doubtful ones among them computed again -- these alone: a result may not depend on
+// which others lie beside it, as the width of the tiles follows this launch's share of the batch (32 columns are together in either).
+__device__ __noinline__ void sum_doubtful(const F32UmmaParams& p, float* sums, int n, int row, int col) {
+  if (row >= p.M) return;
+  RowKind k{-1, 0, 0};
+  bool tiny = false;
+  int held = -1;   // two are computed at a time
+  for (int j = 0; j < n && col + j < p.N; ++j) {
+    if (j % 32 == 0) tiny = any_tiny(p, sums + j, min(n - j, 32));
+    if (!doubtful(p, sums[j]) && !(tiny && sums[j] == 0.f)) continue;
+    if (k.kind < 0) k = look_at_row(p, row);
+    if (k.kind == ROW_NAN) return;   // (they are NaN)
+    if (k.kind == ROW_INFINITE) sums[j] = infinite_sum(p, row, col + j, k.first, k.last);
+    else if (held < 0) held = j;
+    else {
+      const float2 s = replay(p, row, col + held, col + j);
+      sums[held] = s.x;
+      sums[j] = s.y;
+      held = -1;
+    }
+  }
+  if (held >= 0) sums[held] = replay(p, row, col + held, col + held).x;
+}
+// The doubtful ones among a thread's results, stored again where that changes anything.
 template <int BN, int W>
 __device__ __noinline__ void finish_doubtful(const F32UmmaParams& p, uint32_t out, int m0, int n0, int c, int r0, int r_hi) {
   for (int r = r0; r < r_hi; r += 32 * kSumWarps * W / BN) {
-    float x[W];
+    float x[W], again[W];
     read_result<BN, W>(p, out, r, c, x);
-    const bool tiny = any_tiny(x, W);
-    for (int j = 0; j < W && n0 + c + j < p.N; ++j) {
-      const int64_t row = (int64_t)m0 + r;
-      if (doubtful(x[j]) || (tiny && x[j] == 0.f)) store_from_float(p.y, p.ep.out_dt, row * p.N + n0 + c + j, epilogue_value(p.ep, replay(p, (int)row, n0 + c + j), row, n0 + c + j, p.N));
-    }
+    for (int j = 0; j < W; ++j) again[j] = x[j];
+    sum_doubtful(p, again, W, m0 + r, n0 + c);
+    const int64_t row = (int64_t)m0 + r;
+    for (int j = 0; j < W; ++j)
+      if (__float_as_uint(again[j]) != __float_as_uint(x[j])) store_from_float(p.y, p.ep.out_dt, row * p.N + n0 + c + j, epilogue_value(p.ep, again[j], row, n0 + c + j, p.N));
   }
 }
 // Rows [r_lo, r_hi) of the tile that starts at (m0, n0): the epilogue (every step rounded by itself) and the store.  A thread keeps W
@@ -242,7 +328,7 @@ __device__ __forceinline__ void finish_rows(const F32UmmaParams& p, bool f32_io,
       bool bad = false;
 #pragma unroll
       for (int j = 0; j < W; ++j) {
-        bad = bad || doubtful(x[i][j]);
+        bad = bad || doubtful(p, x[i][j]);
         if (ep.alpha != 1.f) x[i][j] = __fmul_rn(x[i][j], ep.alpha);
         if (ep.add1) x[i][j] = __fadd_rn(x[i][j], a1[j]);
         if (ep.add2) x[i][j] = __fadd_rn(x[i][j], a2[j]);
@@ -297,7 +383,7 @@ __device__ __forceinline__ void finish_plain_rows(const F32UmmaParams& p, uint32
     float x[4];
     read_result<BN, 4>(p, out, r, c, x);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) again = again || doubtful(x[j]);
+    for (int j = 0; j < 4; ++j) again = again || doubtful(p, x[j]);
     if (addv) { x[0] = __fadd_rn(x[0], add.x); x[1] = __fadd_rn(x[1], add.y); x[2] = __fadd_rn(x[2], add.z); x[3] = __fadd_rn(x[3], add.w); }
     if (res) { x[0] = __fadd_rn(x[0], f.x); x[1] = __fadd_rn(x[1], f.y); x[2] = __fadd_rn(x[2], f.z); x[3] = __fadd_rn(x[3], f.w); }
     if (ep.act == ACT_RELU) {
@@ -308,27 +394,16 @@ __device__ __forceinline__ void finish_plain_rows(const F32UmmaParams& p, uint32
   }
   if (again) finish_doubtful<BN, 4>(p, out, m0, n0, c, r_lo + t / kPerRow, r_hi);   // (over what was just stored)
 }
-// COLS sums of one row, the doubtful ones among them computed again -- these alone: a result may not depend on which others lie
-// beside it, as the width of the tiles follows this launch's share of the batch.
-template <int COLS>
-__device__ __noinline__ void sum_doubtful(const F32UmmaParams& p, float* acc, int row, int col0) {
-  if (row >= p.M) return;
-  for (int g = 0; g < COLS; g += 32) {   // (32 columns are together in tiles of either width)
-    const bool tiny = any_tiny(acc + g, 32);
-    for (int j = g; j < g + 32 && col0 + j < p.N; ++j)
-      if (doubtful(acc[j]) || (tiny && acc[j] == 0.f)) acc[j] = replay(p, row, col0 + j);
-  }
-}
 // COLS columns of one row, straight from their sums into the row's places in the boxes of 32 columns that start at `at` (128-byte swizzle:
 // 16-byte piece j of a row at j ^ (row & 7)); the residual lies there already.  Columns past N hold anything: the store clips them.
 template <int COLS>
 __device__ __forceinline__ void finish_in_boxes(const F32UmmaParams& p, float (&acc)[COLS], uint32_t at, int row, int m0, int col0) {
   const Epilogue& ep = p.ep;
-  if (any_doubtful<COLS>(acc)) {   // (through a copy: the sums themselves stay in registers)
+  if (__any_sync(0xffffffffu, any_doubtful<COLS>(p, acc))) {   // (one branch for the warp, and through a copy: the sums themselves stay in registers)
     float copy[COLS];
 #pragma unroll
     for (int j = 0; j < COLS; ++j) copy[j] = acc[j];
-    sum_doubtful<COLS>(p, copy, m0 + row, col0);
+    sum_doubtful(p, copy, COLS, m0 + row, col0);
 #pragma unroll
     for (int j = 0; j < COLS; ++j) acc[j] = copy[j];
   }
@@ -719,7 +794,8 @@ bool f32_umma_supported(const F32Umma& c) {
   if (c.pad_t > 127 || c.pad_l > 127) return false;   // the corners of an im2col map have eight bits
   const int64_t lim = 127, dw = (int64_t)(c.Q - 1) * c.stride_w - c.pad_l - (c.W - 1), dh = (int64_t)(c.P - 1) * c.stride_h - c.pad_t - (c.H - 1);
   if (dw < -128 || dw > lim || dh < -128 || dh > lim) return false;
-  return (int64_t)c.N * c.P * c.Q < (1ll << 31) - kRows && c.K < (1 << 30) && f32_umma_blocks(c) < (1 << 24) && c.rows_full < (1ll << 40);
+  // (blocks: while a row is computed again, other roles' waits go on; half a million values take about a third of their limit)
+  return (int64_t)c.N * c.P * c.Q < (1ll << 31) - kRows && c.K < (1 << 30) && f32_umma_blocks(c) < (1 << 13) && c.rows_full < (1ll << 40);
 }
 int64_t f32_umma_blocks(const F32Umma& c) { return (int64_t)c.R * c.S * ((c.C + kDepth - 1) / kDepth); }
 
@@ -755,6 +831,9 @@ F32UmmaLaunch* f32_umma_prepare(const F32Umma& c, const void* x, const void* pla
   p.stages = L->bn == 128 ? 2 : 3;
   L->grid = p.splits > 1 ? p.total_tiles * p.splits : std::min(p.total_tiles, sms);
   L->smem = L->bn == 128 ? smem_bytes<128>() : smem_bytes<64>();
+  // What a value of A is off by is below 2^-133 (split_last), what a product may lose below the smallest fp32 2^-149 six times; against 2^-26
+  // of a result.  (Measured with nothing computed again, 2048 x 576 x 256: errors are those of ordinary sizes down to results of 2^-104.)
+  p.least = std::max(0x1p-100f, (float)((double)c.R * c.S * c.C * 0x1p-107) * std::max(c.largest_weight, 0x1p-13f));
   p.spin_limit = kSpinLimit;
   p.test_skip_stage = getenv("ODLA_B200_TEST_SKIP_STAGE") != nullptr;   // (the hooks of umma_conv_prepare)
   if (const char* e = getenv("ODLA_B200_TEST_SPIN_LIMIT")) { const long v = atol(e); if (v >= 64 && v <= (1l << 18)) p.spin_limit = (uint32_t)v; }

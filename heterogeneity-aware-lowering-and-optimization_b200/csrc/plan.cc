@@ -1369,9 +1369,12 @@ F32UmmaLaunch* Builder::prepare_f32_umma(const F32Umma& fu, const Fused& f, cons
   if (!f32_umma_supported(fu) || (uintptr_t)x % 16 || (uintptr_t)y % 16) return nullptr;
   const auto w = const_as_f32(f.w);
   if (!f32_planes_hold(w)) return nullptr;
+  F32Umma c = fu;
+  c.largest_weight = 0.f;
+  for (float v : w) c.largest_weight = std::max(c.largest_weight, std::fabs(v));
   auto planes = prepared(f.w, form, [&] { return make(w); });
   const void* wd = upload(planes->data(), planes->size());
-  F32UmmaLaunch* l = wd ? f32_umma_prepare(fu, x, wd, y, ep, p_->status, sms) : nullptr;
+  F32UmmaLaunch* l = wd ? f32_umma_prepare(c, x, wd, y, ep, p_->status, sms) : nullptr;
   if (l) p_->f32_umma.push_back(l);
   else if (!fu.x_w_stride) fail(ODLA_FAILURE, "'" + f.root->name + "': fp32 tensor-core launch could not be prepared");
   return l;

@@ -29,6 +29,12 @@ def conv(odla, lib, x, w, b, r=None, stride=1, pad=1, act=0.0, sub_batches=None,
     return out
 
 
+def plain_size(x, w, pad):
+    """Sums of the terms' magnitudes: what an error is to be measured against where terms cancel."""
+    t = torch.nn.functional.conv2d(torch.from_numpy(np.abs(x)).double().permute(0, 3, 1, 2), torch.from_numpy(np.abs(w)).double().permute(3, 2, 0, 1), padding=pad)
+    return t.permute(0, 2, 3, 1).numpy()
+
+
 def float64(x, w, b, r, stride, pad, act):
     t = torch.nn.functional.conv2d(torch.from_numpy(x).double().permute(0, 3, 1, 2), torch.from_numpy(w).double().permute(3, 2, 0, 1), stride=stride, padding=pad)
     y = t.permute(0, 2, 3, 1).numpy() + b + (0 if r is None else r)
@@ -106,6 +112,74 @@ def test_values_the_split_does_not_hold(odla, gpu_lib, shape, bad, monkeypatch):
     ok = np.isfinite(want)
     # both are chains of roundings of 2^-24 (subnormal results: of 2^-149) relative to the largest terms
     assert np.abs(got[ok].astype(np.float64) - want[ok]).max() <= 2e-5 * np.abs(want[ok]).max() + 1e-43
+
+
+# N, H, C, K, window: boxes of results, two tiles a CTA and more, a shared reduction, columns that are no multiple of four (and shared)
+@pytest.mark.parametrize("act, residual", [(None, False), (0.0, True), (0.1, True), ("gelu", False)])
+@pytest.mark.parametrize("shape", [(6, 28, 64, 128, 3), (6, 56, 64, 320, 1), (6, 7, 256, 320, 3), (6, 14, 64, 255, 1), (6, 7, 512, 130, 1)])
+def test_images_that_are_no_ordinary_numbers(odla, gpu_lib, monkeypatch, shape, act, residual):
+    """A batch of an ordinary image, one of NaN, one of infinities, one with a single infinity and one with a single NaN, one of subnormals;
+    a filter that is all zeros and one that has all but vanished.  Infinities and NaN as from the CUDA-core kernel, every other result
+    next to the sum of its own terms' magnitudes."""
+    N, H, C, K, R = shape
+    rng = np.random.default_rng(sum(shape))
+    x = rng.standard_normal((N, H, H, C)).astype(np.float32)
+    w = (rng.standard_normal((R, R, C, K)) / np.sqrt(R * R * C)).astype(np.float32)
+    w[..., 3] = 0
+    w[..., 9] *= np.float32(1e-25)
+    x[1] = np.nan
+    x[2] = np.where(x[2] < 0, -np.inf, np.inf)
+    x[3, 2, 3, 5] = -np.inf
+    x[4, H - 1, 0, C - 1] = np.nan
+    x[5] *= np.float32(1e-40)
+    r = np.abs(rng.standard_normal((N, H, H, K))).astype(np.float32) if residual else None
+
+    def layer(launch):
+        if act != "gelu":
+            return conv(odla, gpu_lib, x, w, np.zeros(K, np.float32), r, pad=R // 2, act=act, launch=launch)
+        g = odla.Graph(gpu_lib, "c", n_gpus=1)
+        y = g.Conv(g.Argument("x", x.shape), odla.CHANNELS_LAST, 1, g.Constant("w", w), odla.SIO, (1, 1), (1, 1), (R // 2, R // 2), (R // 2, R // 2), None, (N, H, H, K), "conv")
+        g.Output(g.Gelu(y, False, "act"))
+        try:
+            out = g.run({"x": x})["act"]
+            assert launch in g.describe()
+        finally:
+            g.close()
+        return out
+
+    got = layer("conv_f32_umma")
+    monkeypatch.setenv("ODLA_B200_NO_F32_UMMA", "1")
+    want = layer("conv_simt")
+    for same in (np.isnan, np.isposinf, np.isneginf):
+        assert np.array_equal(same(got), same(want))
+    ok = np.isfinite(want)
+    xf = np.where(np.isfinite(x), x, 0)
+    # two fp32 chains: roundings of 2^-24 of the terms (of the residual too, of 2^-149 among subnormals), erf's 5e-7
+    size = plain_size(xf, w, R // 2) + (0 if r is None else np.abs(r))
+    assert (np.abs(got[ok].astype(np.float64) - want[ok]) <= 2e-6 * size[ok] + 1e-43).all()
+
+
+def test_rows_computed_again_in_a_deep_product(odla, gpu_lib):
+    """Several tiles a CTA over a long reduction, most rows of which are computed again while the other roles wait."""
+    M, K, N = 40000, 2304, 64
+    rng = np.random.default_rng(4)
+    a = rng.standard_normal((M, K), dtype=np.float32)
+    w = (rng.standard_normal((K, N)) / 48).astype(np.float32)
+    a[:10000] *= np.float32(1e-40)
+    a[10000:20000] = np.nan
+    a[20000:30000, 7] = np.inf
+    g = odla.Graph(gpu_lib, "g", n_gpus=1)
+    g.Output(g.Gemm(g.Argument("a", a.shape), False, g.Constant("w", w), False, 1.0, 0.0, None, (M, N), "y"))
+    got = g.run({"a": a})["y"]
+    assert "gemm_f32_umma" in g.describe()
+    g.close()
+    assert np.isnan(got[10000:20000]).all()
+    assert np.array_equal(got[20000:30000], np.broadcast_to(np.where(w[7] < 0, -np.inf, np.inf).astype(np.float32), (10000, N)))
+    want = (torch.from_numpy(a).cuda().double() @ torch.from_numpy(w).cuda().double()).cpu().numpy()
+    size = (torch.from_numpy(np.abs(a)).cuda().double() @ torch.from_numpy(np.abs(w)).cuda().double()).cpu().numpy()
+    # a chain of 2304 roundings: of 2^-24 of the terms, of 2^-149 among subnormals
+    for rows in (slice(0, 10000), slice(30000, M)):
+        assert (np.abs(got[rows] - want[rows]) <= 1e-6 * size[rows] + K * 2.0 ** -149).all()
 
 
 @pytest.mark.parametrize("scale, value, launch", [(2.0 ** -126, 0, "conv_simt"), (1e-40, 0, "conv_simt"), (1, 1e-36, "conv_simt"), (1, 1.5 * 2.0 ** 20, "conv_simt"),
