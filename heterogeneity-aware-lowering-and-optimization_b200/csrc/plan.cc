@@ -271,6 +271,12 @@ class Builder {
     p_->const_bytes += (int64_t)bytes;
     return d;
   }
+  // Gives back what upload or a cudaMalloc registered last, when the launch it was for is not made after all.
+  void release_last(void* d) {
+    if (p_->extra_allocs.empty() || p_->extra_allocs.back() != d) return;
+    p_->extra_allocs.pop_back();
+    cudaFree(d);
+  }
   void* const_dev(V v, int dt) {  // constant converted to storage type dt, uploaded once
     auto key = std::make_pair(v, dt);
     auto it = const_cache_.find(key);
@@ -1363,7 +1369,8 @@ odla_status Builder::emit_fused(const Item& it) {
   return ODLA_SUCCESS;
 }
 
-// An fp32 layer as three bf16 values an operand on the tensor cores; null when it stays on the CUDA cores (or, with err_ set, fails).
+// An fp32 layer as three bf16 values an operand on the tensor cores; null when it stays on the CUDA cores, for want of memory as well (or,
+// with err_ set, fails).
 F32UmmaLaunch* Builder::prepare_f32_umma(const F32Umma& fu, const Fused& f, const std::string& form, const std::function<std::vector<uint8_t>(const std::vector<float>&)>& make,
                                          const void* x, void* y, const Epilogue& ep, int sms) {
   if (!f32_umma_supported(fu) || (uintptr_t)x % 16 || (uintptr_t)y % 16) return nullptr;
@@ -1373,10 +1380,14 @@ F32UmmaLaunch* Builder::prepare_f32_umma(const F32Umma& fu, const Fused& f, cons
   c.largest_weight = 0.f;
   for (float v : w) c.largest_weight = std::max(c.largest_weight, std::fabs(v));
   auto planes = prepared(f.w, form, [&] { return make(w); });
-  const void* wd = upload(planes->data(), planes->size());
-  F32UmmaLaunch* l = wd ? f32_umma_prepare(c, x, wd, y, ep, p_->status, sms) : nullptr;
-  if (l) p_->f32_umma.push_back(l);
-  else if (!fu.x_w_stride) fail(ODLA_FAILURE, "'" + f.root->name + "': fp32 tensor-core launch could not be prepared");
+  void* wd = nullptr;   // (half as much again as the weights: where that does not fit, the CUDA cores' form may)
+  if (inject_fault("alloc") || cudaMalloc(&wd, planes->size()) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+  p_->extra_allocs.push_back(wd);
+  if (cudaMemcpy(wd, planes->data(), planes->size(), cudaMemcpyHostToDevice) != cudaSuccess) { fail(ODLA_FAILURE, "constant upload failed"); return nullptr; }
+  F32UmmaLaunch* l = f32_umma_prepare(c, x, wd, y, ep, p_->status, sms);
+  if (!l) { release_last(wd); return nullptr; }
+  p_->const_bytes += (int64_t)planes->size();
+  p_->f32_umma.push_back(l);
   return l;
 }
 

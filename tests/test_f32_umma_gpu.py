@@ -242,3 +242,33 @@ def test_wait_that_runs_out(odla, gpu_lib, monkeypatch, shape, residual):
     monkeypatch.delenv("ODLA_B200_TEST_SPIN_LIMIT")
     got, want = conv(odla, gpu_lib, x, w, b, r, pad=R // 2), float64(x, w, b, r, 1, R // 2, 0.0)
     assert np.abs(got - want).max() / np.sqrt(np.mean(want ** 2)) < 4e-7 * 6 + 1e-6
+
+
+def test_weights_without_memory_for_their_parts(odla, gpu_lib, monkeypatch):
+    """Each allocation of a plan fails in turn (on the host, nothing touches the device): the one for the bf16 parts of the weights, half as
+    much again as the weights, leaves the layer to the CUDA cores; the others are refused as before."""
+    rng = np.random.default_rng(7)
+    x, w = rng.standard_normal((2, 28, 28, 64)).astype(np.float32), (rng.standard_normal((3, 3, 64, 128)) / 24).astype(np.float32)
+    b, launches = rng.standard_normal(128).astype(np.float32), []
+    gpu_lib.SetLogLevel(0)
+    try:
+        for n in range(1, 9):
+            monkeypatch.setenv("ODLA_B200_INJECT", "alloc@%d" % n)
+            for launch in ("conv_f32_umma", "conv_simt", "refused"):
+                monkeypatch.delenv("ODLA_B200_INJECT")
+                conv(odla, gpu_lib, x, w, b)   # (forgets the count)
+                monkeypatch.setenv("ODLA_B200_INJECT", "alloc@%d" % n)
+                try:
+                    got = conv(odla, gpu_lib, x, w, b, launch=launch)
+                except AssertionError:
+                    continue
+                except RuntimeError:
+                    launches.append("refused")
+                    break
+                launches.append(launch)
+                want = float64(x, w, b, None, 1, 1, 0.0)
+                assert np.abs(got - want).max() / np.sqrt(np.mean(want ** 2)) < 4e-7 * 24 + 1e-6
+                break
+    finally:
+        gpu_lib.SetLogLevel(3)
+    assert launches.count("conv_simt") == 1 and "refused" in launches and launches[-1] == "conv_f32_umma", launches
