@@ -1140,7 +1140,7 @@ odla_status Builder::emit_fused(const Item& it) {
         fw.x_w_stride = 16ll * g.stride_w;
         fw.x_h_stride = 16ll * Wp;
         void* image = nullptr;
-        if (f32_umma_pays(fw) && f32_umma_supported(fw) && !inject_fault("alloc")) {
+        if (f32_umma_pays(fw) && f32_umma_supported(fw) && f32_planes_hold(const_as_f32(f.w)) && !inject_fault("alloc")) {
           if (cudaMalloc(&image, (size_t)fw.x_h_stride * g.H * g.N) != cudaSuccess) { cudaGetLastError(); image = nullptr; }
         }
         if (image) {
@@ -1161,6 +1161,7 @@ odla_status Builder::emit_fused(const Item& it) {
             p_->launches.back().n_kernels = 2;
             return ODLA_SUCCESS;
           }
+          release_last(image);
         }
       }
       if (conv_f32_supported(g) && conv_f32_pays(g, images_full) && (!padded_window || all_finite())) {

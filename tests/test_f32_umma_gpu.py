@@ -1,5 +1,7 @@
 """fp32 layers as three bf16 values an operand on the tensor cores (kernels_f32_umma.cu) against a float64 evaluation, and against
 the CUDA-core kernels where an operand is not an ordinary number."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -272,3 +274,39 @@ def test_weights_without_memory_for_their_parts(odla, gpu_lib, monkeypatch):
     finally:
         gpu_lib.SetLogLevel(3)
     assert launches.count("conv_simt") == 1 and "refused" in launches and launches[-1] == "conv_f32_umma", launches
+
+
+def test_refused_filters_leave_no_scratch_behind(odla, gpu_lib, monkeypatch):
+    """Filters of an RGB image that stay with the CUDA cores, because the split does not hold them or because their parts find no memory: the
+    plan holds no padded copy of the images (128 of 224 x 224: 420 MB)."""
+    N, H, K = 128, 224, 64
+    w = np.full((7, 7, 3, K), 1e-40, np.float32)
+
+    def memory():
+        g = odla.Graph(gpu_lib, "c", n_gpus=1)
+        g.Output(g.Conv(g.Argument("x", (N, H, H, 3)), odla.CHANNELS_LAST, 1, g.Constant("w", w), odla.SIO, (2, 2), (1, 1), (3, 3), (3, 3), None, (N, 112, 112, K), "y"))
+        before = torch.cuda.mem_get_info()[0]
+        g.context()
+        exe = C.c_void_p()
+        done = gpu_lib.CompileComputation(g.comp, None, C.byref(exe)) == odla.SUCCESS
+        taken = before - torch.cuda.mem_get_info()[0] if done and "conv_simt" in g.describe() else None
+        g.close()
+        return taken
+
+    memory()   # (what the first plan of a process takes besides)
+    refused = memory()
+    w[:] = 1
+    assert memory() is None   # on the tensor cores
+    gpu_lib.SetLogLevel(0)
+    failed = []
+    for n in range(1, 9):
+        monkeypatch.setenv("ODLA_B200_INJECT", "alloc@%d" % n)
+        failed.append(memory())
+        monkeypatch.delenv("ODLA_B200_INJECT")
+        memory()   # (forgets the count)
+    gpu_lib.SetLogLevel(3)
+    failed = [taken for taken in failed if taken is not None]
+    assert len(failed) == 2   # the padded images, the parts of the filter
+    monkeypatch.setenv("ODLA_B200_NO_F32_UMMA", "1")
+    want = memory()
+    assert all(abs(taken - want) < 100e6 for taken in failed + [refused]), (failed, refused, want)
