@@ -259,13 +259,14 @@ template <int BN, int W> __device__ __forceinline__ void read_result(const F32Um
 }
 // `n` sums of one row, of columns from `col` on, the doubtful ones among them computed again -- these alone: a result may not depend on
 // which others lie beside it, as the width of the tiles follows this launch's share of the batch (32 columns are together in either).
-__device__ __noinline__ void sum_doubtful(const F32UmmaParams& p, float* sums, int n, int row, int col) {
+// `beside_tiny`: there is a tiny one among those 32.
+__device__ __noinline__ void sum_doubtful(const F32UmmaParams& p, float* sums, int n, int row, int col, bool beside_tiny) {
   if (row >= p.M) return;
   RowKind k{-1, 0, 0};
-  bool tiny = false;
+  bool tiny = beside_tiny;
   int held = -1;   // two are computed at a time
   for (int j = 0; j < n && col + j < p.N; ++j) {
-    if (j % 32 == 0) tiny = any_tiny(p, sums + j, min(n - j, 32));
+    if (!beside_tiny && j % 32 == 0) tiny = any_tiny(p, sums + j, min(n - j, 32));
     if (!doubtful(p, sums[j]) && !(tiny && sums[j] == 0.f)) continue;
     if (k.kind < 0) k = look_at_row(p, row);
     if (k.kind == ROW_NAN) return;   // (they are NaN)
@@ -282,25 +283,33 @@ __device__ __noinline__ void sum_doubtful(const F32UmmaParams& p, float* sums, i
 }
 // The doubtful ones among a thread's results, stored again where that changes anything.
 template <int BN, int W>
-__device__ __noinline__ void finish_doubtful(const F32UmmaParams& p, uint32_t out, int m0, int n0, int c, int r0, int r_hi) {
+__device__ __noinline__ void finish_doubtful(const F32UmmaParams& p, uint32_t out, int m0, int n0, int r_lo, int r_hi, int t) {
+  const int c = t % (BN / W) * W, r0 = r_lo + t / (BN / W);
+  if (n0 + c >= p.N) return;
   for (int r = r0; r < r_hi; r += 32 * kSumWarps * W / BN) {
     float x[W], again[W];
     read_result<BN, W>(p, out, r, c, x);
-    for (int j = 0; j < W; ++j) again[j] = x[j];
-    sum_doubtful(p, again, W, m0 + r, n0 + c);
+    bool zero = false, tiny = false;
+    for (int j = 0; j < W; ++j) { again[j] = x[j]; zero = zero || x[j] == 0.f; }
+    for (int k = c & ~31; zero && !tiny && k < (c | 31); k += 4) {
+      float beside[4];
+      read_result<BN, 4>(p, out, r, k, beside);
+      tiny = any_tiny(p, beside, 4);
+    }
+    sum_doubtful(p, again, W, m0 + r, n0 + c, tiny);
     const int64_t row = (int64_t)m0 + r;
     for (int j = 0; j < W; ++j)
       if (__float_as_uint(again[j]) != __float_as_uint(x[j])) store_from_float(p.y, p.ep.out_dt, row * p.N + n0 + c + j, epilogue_value(p.ep, again[j], row, n0 + c + j, p.N));
   }
 }
 // Rows [r_lo, r_hi) of the tile that starts at (m0, n0): the epilogue (every step rounded by itself) and the store.  A thread keeps W
-// columns, whose addends it reads once, and has several rows' residuals and results on the way at a time.
+// columns, whose addends it reads once, and has several rows' residuals and results on the way at a time.  Returns whether any is doubtful.
 template <int BN, int W>
-__device__ __forceinline__ void finish_rows(const F32UmmaParams& p, bool f32_io, uint32_t out, int m0, int n0, int r_lo, int r_hi, int t) {
+__device__ __forceinline__ bool finish_rows(const F32UmmaParams& p, bool f32_io, uint32_t out, int m0, int n0, int r_lo, int r_hi, int t) {
   constexpr int kPerRow = BN / W, kStep = 32 * kSumWarps / kPerRow, kAhead = W == 4 ? 4 : 8;
   const Epilogue& ep = p.ep;
   const int c = t % kPerRow * W, col = n0 + c;
-  if (col >= p.N) return;
+  if (col >= p.N) return false;
   float a1[W], a2[W];
 #pragma unroll
   for (int j = 0; j < W; ++j) {
@@ -362,15 +371,15 @@ __device__ __forceinline__ void finish_rows(const F32UmmaParams& p, bool f32_io,
       }
     }
   }
-  if (again) finish_doubtful<BN, W>(p, out, m0, n0, c, r_lo + t / kPerRow, r_hi);   // (over what was just stored)
+  return again;
 }
 // The plain form (p.plain) of a shared reduction, with nothing left to decide for a result.
 template <int BN>
-__device__ __forceinline__ void finish_plain_rows(const F32UmmaParams& p, uint32_t out, int m0, int n0, int r_lo, int r_hi, int t) {
+__device__ __forceinline__ bool finish_plain_rows(const F32UmmaParams& p, uint32_t out, int m0, int n0, int r_lo, int r_hi, int t) {
   constexpr int kPerRow = BN / 4, kStep = 32 * kSumWarps / kPerRow;
   const Epilogue& ep = p.ep;
   const int c = t % kPerRow * 4, col = n0 + c;
-  if (col >= p.N) return;
+  if (col >= p.N) return false;
   const float* addv = ep.add1 ? ep.add1 : ep.add2;
   const float4 add = addv ? __ldg((const float4*)(addv + col)) : make_float4(0.f, 0.f, 0.f, 0.f);
   const float* res = (const float*)ep.res;
@@ -392,7 +401,7 @@ __device__ __forceinline__ void finish_plain_rows(const F32UmmaParams& p, uint32
     }
     *(float4*)(y + at) = make_float4(x[0], x[1], x[2], x[3]);
   }
-  if (again) finish_doubtful<BN, 4>(p, out, m0, n0, c, r_lo + t / kPerRow, r_hi);   // (over what was just stored)
+  return again;
 }
 // COLS columns of one row, straight from their sums into the row's places in the boxes of 32 columns that start at `at` (128-byte swizzle:
 // 16-byte piece j of a row at j ^ (row & 7)); the residual lies there already.  Columns past N hold anything: the store clips them.
@@ -403,7 +412,7 @@ __device__ __forceinline__ void finish_in_boxes(const F32UmmaParams& p, float (&
     float copy[COLS];
 #pragma unroll
     for (int j = 0; j < COLS; ++j) copy[j] = acc[j];
-    sum_doubtful(p, copy, COLS, m0 + row, col0);
+    sum_doubtful(p, copy, COLS, m0 + row, col0, false);
 #pragma unroll
     for (int j = 0; j < COLS; ++j) acc[j] = copy[j];
   }
@@ -444,10 +453,14 @@ __device__ __forceinline__ void finish_in_boxes(const F32UmmaParams& p, float (&
 template <int BN>
 __device__ __forceinline__ void finish_tile(const F32UmmaParams& p, uint32_t out, int m0, int n0, int r_lo, int r_hi, int t) {
   const Epilogue& ep = p.ep;
-  if (p.plain) return finish_plain_rows<BN>(p, out, m0, n0, r_lo, r_hi, t);
-  const bool f32_io = !ep.mul && !ep.add_full && (!ep.res || ep.res_dt == DT_F32) && ep.out_dt == DT_F32;
-  if (f32_io && (p.N & 3) == 0) finish_rows<BN, 4>(p, true, out, m0, n0, r_lo, r_hi, t);
-  else finish_rows<BN, 1>(p, f32_io, out, m0, n0, r_lo, r_hi, t);
+  const bool f32_io = !ep.mul && !ep.add_full && (!ep.res || ep.res_dt == DT_F32) && ep.out_dt == DT_F32, four = p.plain || (f32_io && (p.N & 3) == 0);
+  const bool again = p.plain ? finish_plain_rows<BN>(p, out, m0, n0, r_lo, r_hi, t)
+                     : four  ? finish_rows<BN, 4>(p, true, out, m0, n0, r_lo, r_hi, t)
+                             : finish_rows<BN, 1>(p, f32_io, out, m0, n0, r_lo, r_hi, t);
+  if (__any_sync(0xffffffffu, again)) {   // (over what was just stored; 32 columns of a row are one warp's, so that zeros beside a tiny result come along)
+    if (four) finish_doubtful<BN, 4>(p, out, m0, n0, r_lo, r_hi, t);
+    else finish_doubtful<BN, 1>(p, out, m0, n0, r_lo, r_hi, t);
+  }
 }
 
 template <int BN>

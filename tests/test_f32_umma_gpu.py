@@ -185,6 +185,27 @@ def test_rows_computed_again_in_a_deep_product(odla, gpu_lib):
         assert (np.abs(got[rows] - want[rows]) <= 1e-6 * size[rows] + K * 2.0 ** -149).all()
 
 
+@pytest.mark.parametrize("gelu", [False, True])
+@pytest.mark.parametrize("dims", [(6000, 256, 640), (1000, 768, 255), (130, 2048, 512), (130, 2048, 510)])   # boxes, rows, a shared reduction of either kind
+def test_zeros_beside_tiny_results(odla, gpu_lib, dims, gelu):
+    """One subnormal a row, so that every result is one product: where the parts' products all vanish, the product may not."""
+    M, K, N = dims
+    rng = np.random.default_rng(N)
+    at = rng.integers(0, K, M)
+    a = np.zeros((M, K), np.float32)
+    a[np.arange(M), at] = rng.uniform(1, 2, M) * rng.choice([-1, 1], M) * 2.0 ** rng.integers(-136, -128, M)
+    w = (rng.uniform(1, 2, (K, N)) * rng.choice([-1, 1], (K, N)) * 2.0 ** rng.integers(-20, 20, (K, N))).astype(np.float32)
+    g = odla.Graph(gpu_lib, "g", n_gpus=1)
+    y = g.Gemm(g.Argument("a", a.shape), False, g.Constant("w", w), False, 1.0, 0.0, None, (M, N), "y")
+    g.Output(g.Gelu(y, False, "act") if gelu else y)
+    got = next(iter(g.run({"a": a}).values()))
+    assert "gemm_f32_umma" in g.describe()
+    g.close()
+    want = a[np.arange(M), at].astype(np.float64)[:, None] * w[at].astype(np.float64)
+    want = np.where(gelu, 0.5, 1.0) * want
+    assert (np.abs(got - want) <= 2.0 ** -24 * np.abs(want) + 2.0 ** -149).all()   # (a rounding; GELU halves them exactly, but for the last bit)
+
+
 @pytest.mark.parametrize("scale, value, launch", [(2.0 ** -126, 0, "conv_simt"), (1e-40, 0, "conv_simt"), (1, 1e-36, "conv_simt"), (1, 1.5 * 2.0 ** 20, "conv_simt"),
                                                   (1, -2.0 ** 20, "conv_f32_umma"), (1, 1.2345678 * 2.0 ** -110, "conv_f32_umma"), (1, 2.0 ** -133, "conv_f32_umma"), (1, 2.0 ** -134, "conv_simt")])
 def test_weights_the_split_does_not_hold(odla, gpu_lib, scale, value, launch):
