@@ -4,7 +4,8 @@
 //
 // The tensor cores have no fp32 operand type, but an fp32 value is exactly the sum of three bf16 values (8 + 8 + 8 bits of
 // mantissa, the same exponent range): a = a1 + a2 + a3, each the leading bits of what the ones before leave.  The product a * w is then
-// a1 w1 + (a1 w2 + a2 w1) + (a1 w3 + a2 w2 + a3 w1) up to 2^-26 of its size, six bf16 products that are exact in fp32.  Six of them at
+// a1 w1 + (a1 w2 + a2 w1) + (a1 w3 + a2 w2 + a3 w1), six bf16 products that are exact in fp32; what the other three add up to is at most
+// 1.5 * 2^-24 of a * w, 2^-26.5 rms (a rounding to fp32: 2^-24, 2^-25.3).  Six of them at
 // 4096 a clock and SM are 683 fp32 products against the FMA pipe's 128, of which the tiles of kernels_f32.cu reach a third.
 // ResNet-50 of 8 images 2747 -> 957 us, YOLOv3 of one 416 x 416 picture 3115 -> 1506, BERT of 2 x 128 2464 -> 1747; one 3x3 layer of
 // 8 x 28 x 28 x 128 -> 128 56 -> 19 us, of 2 x 52 x 52 x 128 -> 256 93 -> 28.  What bounds it: half a stage of 64 columns takes some 800 clocks
@@ -14,8 +15,9 @@
 // Precision.  The tensor cores add into their accumulators without rounding to nearest, so that a long reduction kept there
 // drifts.  The leading products a1 w1 of 64 values therefore go to an accumulator of their own, two of which take turns, and are
 // added up in registers with ordinary fp32 additions while the other fills; the five small products, a 2^-8th of the result, share
-// one accumulator for the whole tile, where the drift is a 2^-8th as well.  Against float64 (rms error over rms result) layers of 64 to
-// 4608 values have 5e-8 to 9e-8, the CUDA-core kernels 7e-8 to 2e-7.
+// one accumulator for the whole tile, where the drift is a 2^-8th as well.  Against float64 (rms error over rms result, products of 64 to
+// 4608 values) N(0, 1) operands have 7e-8 to 1.4e-7, on the CUDA cores 1.1e-7 to 3.1e-7; after a ReLU 5e-8 to 1.3e-7 and 8e-8 to 2.3e-7.  Only where
+// both operands have one sign throughout is the drift the larger part: 8.5e-8 to 1.1e-7 and 5.8e-8 to 9.0e-8.
 // Values for which the split does not hold -- an infinity among the operands, a sum that overflows on the way, results so small that bits
 // of A below the smallest bf16 count -- show up in the sum (not finite, or not zero and below p.least) and such results are computed
 // again: from the infinities' signs where there are any, else as an fp32 FMA chain (replay) from the operands, A as it lies, W as the sum
@@ -103,13 +105,27 @@ __device__ __forceinline__ float4 lds4(uint32_t addr) {
   asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
   return v;
 }
-// The upper halves of two values (x at the lower address), which are bf16 values; the rest of both replaces them.  (Cutting off instead of
-// rounding leaves 8 + 8 + 8 bits as well; what it biases, the parts of A, only meets rounded parts of W in the products left out.)
+// The upper halves of two values (x at the lower address), which are bf16 values; the rest of both replaces them.  (After a first part that
+// was rounded, cutting off leaves 8 + 8 + 8 bits as rounding does.)
 __device__ __forceinline__ uint32_t split_off(float& x, float& y) {
   const uint32_t a = __float_as_uint(x), b = __float_as_uint(y);
   x = __fsub_rn(x, __uint_as_float(a & 0xffff0000u));
   y = __fsub_rn(y, __uint_as_float(b & 0xffff0000u));
   return __byte_perm(a, b, 0x7632);
+}
+// The first parts, rounded to nearest: the rests are half as large as with bits cut off, and of either sign, so that the small products' sums
+// stay small where all operands have one sign (4608 of them: rms error 1.7e-7 -> 1.1e-7; ResNet-50 of 8 images 988 -> 1005 us).  Subnormals
+// have none: a value of 2^-133 or less, rounded up here and away from zero below, could end as zero.  Above 3.396e38 they are infinite, and such
+// results computed again.
+__device__ __forceinline__ uint32_t split_first(float& x, float& y) {
+  float a, b;
+  uint32_t w;
+  asm("mul.ftz.f32 %0, %1, 0f3F800000;" : "=f"(a) : "f"(x));
+  asm("mul.ftz.f32 %0, %1, 0f3F800000;" : "=f"(b) : "f"(y));
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w) : "f"(b), "f"(a));
+  x = __fsub_rn(x, __uint_as_float(w << 16));
+  y = __fsub_rn(y, __uint_as_float(w & 0xffff0000u));
+  return w;
 }
 // The third parts.  They are all that is left of a value of 2^-110 or more.  Of a smaller one bits below bf16's smallest, 2^-133, would be cut
 // off, and nothing be left of many: it is rounded away from zero instead, so that a result of such values does not become a zero that
@@ -620,7 +636,7 @@ f32_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 #pragma unroll
         for (uint32_t q = 0; q < 8; ++q) {
           float4 v = lds4(at + ((q ^ rx) << 4));
-          w1[2 * q] = split_off(v.x, v.y); w1[2 * q + 1] = split_off(v.z, v.w);
+          w1[2 * q] = split_first(v.x, v.y); w1[2 * q + 1] = split_first(v.z, v.w);
           w2[2 * q] = split_off(v.x, v.y); w2[2 * q + 1] = split_off(v.z, v.w);
           w3[2 * q] = split_last(v.x, v.y, one); w3[2 * q + 1] = split_last(v.z, v.w, one);
         }

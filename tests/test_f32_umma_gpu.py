@@ -226,6 +226,27 @@ def test_weights_the_split_does_not_hold(odla, gpu_lib, scale, value, launch):
     assert err.max() < 4e-7 * (3 if launch == "conv_f32_umma" else 24) + 1e-6, err.max()
 
 
+@pytest.mark.parametrize("dims", [(8192, 512, 640), (700, 128, 512), (130, 2048, 512), (1000, 768, 255)])   # boxes of 128 and 64 columns, a shared reduction, rows
+def test_single_products(odla, gpu_lib, dims):
+    """One value a row, so that every result is one product, for values whose parts are as large as they get and for subnormals."""
+    M, K, N = dims
+    rng = np.random.default_rng(M)
+    at = rng.integers(0, K, M)
+    value = (1 + rng.uniform(0, 1, M) ** 4) * rng.choice([-1, 1], M) * 2.0 ** rng.integers(-30, 30, M)
+    value[7:71] *= 2.0 ** rng.integers(-136, -128, 64) / 2.0 ** np.floor(np.log2(np.abs(value[7:71])))
+    a = np.zeros((M, K), np.float32)
+    a[np.arange(M), at] = value
+    w = ((1 + rng.uniform(0, 1, (K, N)) ** 4) * rng.choice([-1, 1], (K, N)) * 2.0 ** rng.integers(-20, 20, (K, N))).astype(np.float32)
+    g = odla.Graph(gpu_lib, "g", n_gpus=1)
+    g.Output(g.Gemm(g.Argument("a", a.shape), False, g.Constant("w", w), False, 1.0, 0.0, None, (M, N), "y"))
+    got = g.run({"a": a})["y"]
+    assert "gemm_f32_umma" in g.describe()
+    g.close()
+    want = a[np.arange(M), at].astype(np.float64)[:, None] * w[at].astype(np.float64)
+    # in units of 2^-24 of the product: a rounding, a3 w2 of 2^-16 * 2^-8, a2 w3 of 2^-8 * 2^-17, five sums of at most 2^-7 cut off at their last bit
+    assert (np.abs(got - want) <= 2.6 * 2.0 ** -24 * np.abs(want) + 2.0 ** -149).all(), (np.abs(got - want) / np.abs(want)).max() * 2.0 ** 24
+
+
 @pytest.mark.parametrize("tb", [False, True])
 @pytest.mark.parametrize("dims", [(2, 130, 768, 768), (1, 700, 100, 999)])   # batch, M, K, N
 def test_products_match_float64(odla, gpu_lib, dims, tb):
