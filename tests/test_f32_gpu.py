@@ -6,12 +6,6 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.fixture
-def cuda_cores(monkeypatch):
-    """Plans made by the test stay off the tensor cores (kernels_f32_umma.cu)."""
-    monkeypatch.setenv("ODLA_B200_NO_F32_UMMA", "1")
-
-
 def close(got, want, k):
     # a sum of k products in fp32: a few rounding steps of the result's magnitude
     err = np.abs(got.astype(np.float64) - want).max() / np.sqrt(np.mean(want ** 2))
@@ -22,7 +16,7 @@ def close(got, want, k):
 # leave a k-block nearly empty, few tiles over a long reduction (split over a cluster), one pixel
 @pytest.mark.parametrize("shape", [(2, 17, 19, 3, 64, 7, 2, 3), (1, 9, 11, 36, 65, 3, 1, 1), (1, 7, 7, 512, 72, 3, 1, 1), (3, 13, 13, 64, 255, 1, 1, 0),
                                    (1, 8, 8, 64, 64, 1, 1, 0), (2, 8, 8, 5, 7, 2, 2, 0), (1, 1, 1, 4, 1, 1, 1, 0), (2, 28, 28, 128, 128, 3, 2, 1)])
-def test_conv_f32_matches_float64(odla, gpu_lib, cuda_cores, shape):
+def test_conv_f32_matches_float64(odla, gpu_lib, shape):
     N, H, W, C, K, R, stride, pad = shape
     P, Q = (H + 2 * pad - R) // stride + 1, (W + 2 * pad - R) // stride + 1
     rng = np.random.default_rng(sum(shape))
@@ -34,7 +28,6 @@ def test_conv_f32_matches_float64(odla, gpu_lib, cuda_cores, shape):
     y = g.Conv(xa, odla.CHANNELS_LAST, 1, g.Constant("w", w), odla.SIO, (stride, stride), (1, 1), (pad, pad), (pad, pad), None, (N, P, Q, K), "conv")
     g.Output(g.LeakyRelu(g.Add(g.Add(y, g.Constant("b", b), "bn"), ra, "res"), 0.1, "y"))
     got = g.run({"x": x, "r": r})["y"]
-    assert "conv_simt" in g.describe()
     g.close()
     t = torch.nn.functional.conv2d(torch.from_numpy(x).double().permute(0, 3, 1, 2), torch.from_numpy(w).double().permute(3, 2, 0, 1), stride=stride, padding=pad)
     want = t.permute(0, 2, 3, 1).numpy() + b + r
@@ -44,7 +37,7 @@ def test_conv_f32_matches_float64(odla, gpu_lib, cuda_cores, shape):
 # batch, M, N, K, transposed A, transposed B (None: constant weights)
 @pytest.mark.parametrize("dims", [(1, 64, 10, 784, 0, None), (1, 1, 1000, 2048, 0, None), (1, 65, 63, 33, 0, None), (1, 130, 70, 4, 1, None), (6, 77, 77, 64, 0, 1),
                                   (6, 77, 64, 77, 0, 0), (4, 128, 64, 128, 0, 0), (1, 3, 5, 7, 0, 0)])
-def test_gemm_f32_matches_float64(odla, gpu_lib, cuda_cores, dims):
+def test_gemm_f32_matches_float64(odla, gpu_lib, dims):
     batch, M, N, K, ta, tb = dims
     rng = np.random.default_rng(sum(d or 0 for d in dims))
     lead = (batch,) if batch > 1 else ()
@@ -56,18 +49,14 @@ def test_gemm_f32_matches_float64(odla, gpu_lib, cuda_cores, dims):
     aa = g.Argument("a", a.shape)
     g.Output(g.Gemm(aa, bool(ta), ba, bool(tb), 0.5, 2.0, g.Constant("c", c), lead + (M, N), "y"))
     got = g.run({"a": a, "b": b} if tb is not None else {"a": a})["y"]
-    assert "gemm_simt" in g.describe()
     g.close()
     af, bf = a.astype(np.float64), b.astype(np.float64)
     close(got, 0.5 * ((af.swapaxes(-1, -2) if ta else af) @ (bf.swapaxes(-1, -2) if tb else bf)) + 2.0 * c, K)
 
 
-@pytest.mark.parametrize("tensor_cores", [False, True])
-def test_f32_results_do_not_depend_on_how_the_batch_is_cut(odla, gpu_lib, monkeypatch, tensor_cores):
+def test_f32_results_do_not_depend_on_how_the_batch_is_cut(odla, gpu_lib):
     """A long convolution, a batched product and two classifiers whose shares of the reduction (and, for the last, whose
     kernel) would differ between six images and the one to five of a sub-batch: equal bits however the batch is cut."""
-    if not tensor_cores:
-        monkeypatch.setenv("ODLA_B200_NO_F32_UMMA", "1")
     B = 6
     rng = np.random.default_rng(8)
     n = lambda *s: (rng.standard_normal(s) / np.sqrt(np.prod(s[:-1]))).astype(np.float32)
@@ -84,7 +73,7 @@ def test_f32_results_do_not_depend_on_how_the_batch_is_cut(odla, gpu_lib, monkey
         g.Output(g.Gemm(v, False, g.Constant("w1", w1), False, 1.0, 0.0, None, (B, 3000), "wide"))
         g.Output(g.Gemm(v, False, g.Constant("w2", w2), False, 1.0, 0.0, None, (B, 40), "narrow"))
         outs.append(g.run({"x": x}))
-        assert g.describe().count("gpu ") == s and ("conv_f32_umma" if tensor_cores else "conv_simt") in g.describe()
+        assert g.describe().count("gpu ") == s
         g.close()
     for o in outs[1:]:
         for name in outs[0]:
@@ -163,3 +152,33 @@ def test_short_reductions_on_whichever_kernel(odla, gpu_lib, shape, images):
     t = torch.nn.functional.conv2d(torch.from_numpy(x).double().permute(0, 3, 1, 2), torch.from_numpy(w).double().permute(3, 2, 0, 1), padding=p).permute(0, 2, 3, 1).numpy()
     close(outs[0]["y"], t, R * R * C)
     assert all(np.array_equal(outs[0][n], outs[1][n]) for n in outs[0])
+
+
+@pytest.fixture
+def cuda_cores(odla, monkeypatch):
+    """Plans made by the test stay off the tensor cores (kernels_f32_umma.cu), which is looked up in their launches."""
+    monkeypatch.setenv("ODLA_B200_NO_F32_UMMA", "1")
+    launches, close = [], odla.Graph.close
+
+    def closing(graph):
+        launches.append(graph.describe())
+        close(graph)
+
+    monkeypatch.setattr(odla.Graph, "close", closing)
+    yield
+    assert launches and all("_simt" in text and "f32_umma" not in text for text in launches)
+
+
+@pytest.mark.parametrize("shape", [(2, 17, 19, 3, 64, 7, 2, 3), (1, 9, 11, 36, 65, 3, 1, 1), (1, 7, 7, 512, 72, 3, 1, 1), (3, 13, 13, 64, 255, 1, 1, 0),
+                                   (1, 8, 8, 64, 64, 1, 1, 0), (2, 28, 28, 128, 128, 3, 2, 1)])
+def test_conv_f32_on_the_cuda_cores(odla, gpu_lib, cuda_cores, shape):
+    test_conv_f32_matches_float64(odla, gpu_lib, shape)
+
+
+@pytest.mark.parametrize("dims", [(1, 64, 10, 784, 0, None), (1, 1, 1000, 2048, 0, None), (1, 65, 63, 33, 0, None), (6, 77, 77, 64, 0, 1)])
+def test_gemm_f32_on_the_cuda_cores(odla, gpu_lib, cuda_cores, dims):
+    test_gemm_f32_matches_float64(odla, gpu_lib, dims)
+
+
+def test_f32_results_on_the_cuda_cores_do_not_depend_on_the_cut(odla, gpu_lib, cuda_cores):
+    test_f32_results_do_not_depend_on_how_the_batch_is_cut(odla, gpu_lib)

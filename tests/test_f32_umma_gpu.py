@@ -95,9 +95,31 @@ def test_results_computed_again_do_not_depend_on_the_cut(odla, gpu_lib, shape, e
 
 
 @pytest.mark.parametrize("shape", [(2, 28, 64, 128, 3), (1, 14, 256, 320, 3)])   # boxes of results; a shared reduction
-@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan, 3.4e38, 1e-30, 1e-38, 1e-41])
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan, 3.4e38, 1e-30, 1e-38])
 def test_values_the_split_does_not_hold(odla, gpu_lib, shape, bad, monkeypatch):
     """Infinities, NaN, the largest fp32 values and operands whose last bits no bf16 can carry: what the CUDA-core kernel gives."""
+    N, H, C, K, R = shape
+    rng = np.random.default_rng(5)
+    x = rng.standard_normal((N, H, H, C)).astype(np.float32)
+    w = (rng.standard_normal((R, R, C, K)) / np.sqrt(R * R * C)).astype(np.float32)
+    b = np.zeros(K, np.float32)
+    if abs(bad) < 1:
+        x *= np.float32(bad)
+    else:
+        x[0, 3, 4, 5] = x[0, H - 1, 0, C - 1] = bad
+    got = conv(odla, gpu_lib, x, w, b, act=None)
+    monkeypatch.setenv("ODLA_B200_NO_F32_UMMA", "1")
+    want = conv(odla, gpu_lib, x, w, b, act=None, launch="conv_simt")
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isposinf(got), np.isposinf(want)) and np.array_equal(np.isneginf(got), np.isneginf(want))
+    ok = np.isfinite(want)
+    # both are chains of roundings of 2^-24 (subnormal results: of 2^-149) relative to the largest terms
+    assert np.abs(got[ok].astype(np.float64) - want[ok]).max() <= 2e-5 * np.abs(want[ok]).max() + 1e-43
+
+
+@pytest.mark.parametrize("shape", [(2, 28, 64, 128, 3), (1, 14, 256, 320, 3)])   # boxes of results; a shared reduction
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan, 3.4e38, 1e-30, 1e-38, 1e-41])
+def test_values_the_split_does_not_hold_next_to_their_terms(odla, gpu_lib, shape, bad, monkeypatch):
+    """As above, every result next to the sum of its own terms' magnitudes."""
     N, H, C, K, R = shape
     rng = np.random.default_rng(5)
     x = rng.standard_normal((N, H, H, C)).astype(np.float32)
