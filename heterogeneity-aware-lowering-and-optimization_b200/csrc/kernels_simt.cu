@@ -7,7 +7,6 @@
 #include <cstdio>
 
 #include <algorithm>
-#include <climits>
 
 #include "epilogue.cuh"
 
@@ -1092,6 +1091,7 @@ __global__ void reduce_mean_axis_vec_kernel(int dt_out, const IN* __restrict__ x
 // s - d * q is exact in one FMA and q + r * remainder rounds to fl(s / d), unless something underflows or overflows on the way: outside
 // (1e-30, 1e30), zero apart, the thread starts again with divisions (mean_divided).  2048 channels of 256 two-byte images, where the
 // registers of 21 divisions left two blocks to an SM: 32.4 -> 11.8 us in the network, 45 images 12.1 -> 4.6, one 4.6 -> 2.3.
+// At six blocks to an SM, 80 registers a thread, the two-byte and int8 forms spill 20 to 52 bytes, which is in these times.
 template <typename IN> __device__ __forceinline__ float mean_term(uint32_t raw, int q, float in_scale) {
   if constexpr (sizeof(IN) == 4) return __uint_as_float(raw);
   else if constexpr (sizeof(IN) == 1) return __fmul_rn((float)(int8_t)(raw >> (8 * q)), in_scale);
