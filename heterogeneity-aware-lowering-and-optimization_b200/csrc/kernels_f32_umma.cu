@@ -7,8 +7,8 @@
 // a1 w1 + (a1 w2 + a2 w1) + (a1 w3 + a2 w2 + a3 w1), six bf16 products that are exact in fp32; what the other three add up to is at most
 // 1.5 * 2^-24 of a * w, 2^-26.5 rms (a rounding to fp32: 2^-24, 2^-25.3).  Six of them at
 // 4096 a clock and SM are 683 fp32 products against the FMA pipe's 128, of which the tiles of kernels_f32.cu reach a third.
-// ResNet-50 of 8 images 2747 -> 957 us, YOLOv3 of one 416 x 416 picture 3115 -> 1506, BERT of 2 x 128 2464 -> 1747; one 3x3 layer of
-// 8 x 28 x 28 x 128 -> 128 56 -> 19 us, of 2 x 52 x 52 x 128 -> 256 93 -> 28.  What bounds it: half a stage of 64 columns takes some 800 clocks
+// CUDA cores -> here: ResNet-50 of 8 images 2759 -> 1007 us, YOLOv3 of one 416 x 416 picture 3130 -> 1595, BERT of 2 x 128 2476 -> 1683, each call
+// waited for; a 3x3 layer of 8 x 28 x 28 x 128 -> 128, its launch bracketed, 64 -> 27, of 2 x 52 x 52 x 128 -> 256 101 -> 35.  What bounds it: half a stage of 64 columns takes some 800 clocks
 // where its products take 400 (the splitting warps' chain of load, split, store and signal), one of 128 columns 1100 where they take
 // 770; short reductions their first loads and the finishing of the tile.
 //
@@ -23,7 +23,7 @@
 // again: from the infinities' signs where there are any, else as an fp32 FMA chain (replay) from the operands, A as it lies, W as the sum
 // of its three parts, which it is exactly.  A NaN in the row needs nothing: its sums are NaN.  An FMA chain takes a hundred times as long as
 // the tensor cores, so that it has to be rare: hence p.least as low as the layer's weights allow.  ResNet-50 of 8 images, waited for after
-// each call: 985 us, with an image of NaN 991, of infinities 1083, of 1e-40 1272, all of them of 1e-40 2603.
+// each call: 1007 us, with an image of NaN 1018, of infinities 1111, of 1e-40 1299, all of them of 1e-40 2661.
 //
 // One CTA per SM walks tiles of 128 rows x BN columns, 64 values of the reduction a stage:
 //   warp 0       TMA: fp32 rows of A as they lie, the three planes of W (split once on the host)

@@ -1134,7 +1134,7 @@ odla_status Builder::emit_fused(const Item& it) {
       if (allow_umma && groups == 1 && g.C <= 4 && g.S <= 32) {
         // A few-channel image has pixels that TMA cannot address: a pass pads them to four channels and every row with zeros, and the S pixels
         // that a row of taps reads are one window of 4 * S values, neighbouring windows overlapping -- an (R x 1) convolution with the padding
-        // along W in memory.  7x7 of 8 x 224 x 224 x 3 -> 64: 111 -> 50 us with its launches bracketed.
+        // along W in memory.  7x7 of 8 x 224 x 224 x 3 -> 64: 109 -> 45 us with its launches bracketed.
         const int Wp = std::max(g.pad_l + g.W, (g.Q - 1) * g.stride_w + g.S);
         F32Umma fw{g.N, g.H, g.Q, 4 * g.S, g.K, g.R, 1, g.P, g.Q, g.stride_h, 1, g.pad_t, 0, images_full * g.P * g.Q};
         fw.x_w_stride = 16ll * g.stride_w;
